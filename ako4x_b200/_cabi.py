@@ -2,18 +2,24 @@
 
 The operators have no CPU path: when the shared library is absent every call raises. Arguments
 cross the boundary as raw device pointers, sizes and scalars; the CUDA stream is PyTorch's
-current stream, passed as an opaque handle.
+current stream, passed as an opaque handle. The operators' ``run(...)`` reach the same C ABI through
+a native module (``csrc/bindings.cpp``, loaded by ``native()``): the checks, allocations and
+launches of a call in one C++ function instead of Python statements.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import re
+import sysconfig
 from pathlib import Path
 
 import torch
 
 _PKG = Path(__file__).resolve().parent
 LIB_PATH = _PKG / "lib" / "libako4x_b200.so"
+NATIVE_PATH = _PKG / "lib" / ("_native" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 HEADER_PATH = _PKG.parent / "include" / "ako4x_b200.h"
 
 STATUS = {
@@ -51,6 +57,25 @@ def lib() -> ctypes.CDLL:
         _lib = ctypes.CDLL(str(LIB_PATH))
         _declare(_lib)
     return _lib
+
+
+_native = None
+
+
+def native():
+    """Loads the native binding module once; raises if it has not been built."""
+    global _native
+    if _native is None:
+        lib()   # the module is linked against it
+        if not NATIVE_PATH.exists():
+            raise Ako4xError(
+                f"{NATIVE_PATH} is missing: build it with `python -m ako4x_b200.build` "
+                "(the operators have no fallback path)")
+        loader = importlib.machinery.ExtensionFileLoader("_native", str(NATIVE_PATH))
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_native", loader))
+        loader.exec_module(mod)
+        _native = mod
+    return _native
 
 
 _P = ctypes.c_void_p

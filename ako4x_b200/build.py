@@ -1,4 +1,5 @@
-"""Builds ``lib/libako4x_b200.so`` from ``csrc/*.cu`` with nvcc for sm_100a.
+"""Builds ``lib/libako4x_b200.so`` from ``csrc/*.cu`` with nvcc for sm_100a, and the Python binding
+module ``lib/_native*.so`` from ``csrc/bindings.cpp`` with the host compiler against PyTorch's headers.
 
 Run as ``python -m ako4x_b200.build`` (add ``--force`` to rebuild everything, ``-v`` for the
 ptxas resource report). The library is built in-tree; nothing is installed.
@@ -9,6 +10,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -75,7 +77,31 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         p = subprocess.run(cmd, capture_output=True, text=True)
         if p.returncode != 0:
             raise RuntimeError("link failed:\n" + p.stdout + p.stderr)
+    build_native(force)
     return LIB
+
+
+def build_native(force: bool = False) -> Path:
+    """The binding module; rebuilt when its source, the C-ABI header or PyTorch itself is newer."""
+    import torch
+    from ._cabi import NATIVE_PATH as out
+    src = CSRC / "bindings.cpp"
+    troot = Path(torch.__file__).resolve().parent
+    newest = max(p.stat().st_mtime for p in (src, INCLUDE / "ako4x_b200.h", troot / "version.py"))
+    if not force and out.exists() and out.stat().st_mtime >= newest:
+        return out
+    cuda = Path(_nvcc()).resolve().parents[1]
+    tlib = troot / "lib"
+    cmd = [os.environ.get("CXX") or "g++", "-std=c++17", "-O2", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", str(INCLUDE), "-I", sysconfig.get_paths()["include"], "-I", str(troot / "include"),
+           "-I", str(troot / "include" / "torch" / "csrc" / "api" / "include"), "-I", str(cuda / "include"),
+           str(src), "-o", str(out), "-L", str(LIBDIR), "-lako4x_b200", "-Wl,-rpath,$ORIGIN",
+           "-L", str(tlib), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+    p = subprocess.run(cmd, capture_output=True, text=True)
+    if p.returncode != 0:
+        raise RuntimeError("building the binding module failed:\n" + p.stdout + p.stderr)
+    return out
 
 
 if __name__ == "__main__":
