@@ -512,10 +512,9 @@ PyObject* gdn_prefill(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const bool use_ws = PyObject_IsTrue(a[10]) == 1;
   const Tensor q = dense(q0), k = dense(k0), v = dense(v0), av = dense(a0), bv = dense(b0), A = dense(A0, at::kFloat),
                d = dense(d0, at::kFloat), cu = dense(cu0, at::kLong);
-  // tokens outside every sequence keep a defined value
   Tensor out = empty({T, 8, 128}, at::kBFloat16, q), ns = empty({n, 8, 128, 128}, at::kFloat, q);
-  out.zero_();
   Workspace ws(use_ws ? ako4x_gdn_prefill_workspace_bytes(T, n) : 0, q);
+  if (!ws.p) out.zero_();   // tokens outside every sequence are zero (the chunked form writes them itself)
   void *p0 = ptr(q), *p1 = ptr(k), *p2 = ptr(v), *p3 = has_state ? ptr(sc) : nullptr, *p4 = ptr(A), *p5 = ptr(av), *p6 = ptr(d),
        *p7 = ptr(bv), *p8 = ptr(cu), *st = current_stream();
   check_status(without_gil([&] {

@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(P_THREADS) gdn_prefill_kernel(
 
 extern "C" size_t ako4x_gdn_prefill_workspace_bytes(int64_t total_tokens, int64_t num_seqs) {
   if (total_tokens <= 0 || num_seqs <= 0) return 0;
-  return (size_t)(total_tokens / C_TOK + num_seqs + 1) * P_HQ * C_GSTRIDE * sizeof(float);
+  return (size_t)(total_tokens / C_TOK + num_seqs) * P_HV * C_SLOT_BYTES;
 }
 
 extern "C" int ako4x_gdn_prefill(const void* q, const void* k, const void* v, const float* state, const float* A_log,
@@ -247,42 +247,39 @@ extern "C" int ako4x_gdn_prefill(const void* q, const void* k, const void* v, co
   if (total_tokens > 0 && (!q || !k || !v || !a || !b || !out)) return AKO4X_EINVAL;
   if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out | (uintptr_t)state | (uintptr_t)new_state) & 15)
     return AKO4X_EINVAL;
-  // The chunked form pays per 16 tokens what the token-by-token form pays per 4-5 tokens on its
-  // serial chain, but does more work per token in total: it wins while SMs would otherwise idle.
-  // Measured, chunked against token by token: 1 x 8 192 tokens 1.00 against 1.40 ms, 2 x 4 096 0.79
-  // against 0.90, 4 x 2 048 0.80 against 0.74, 64 x 128 0.64 against 0.51: used for one or two sequences.
-  if (workspace != nullptr && num_seqs <= 2) {
-    // chunked form: the token-only tables first, then 128 CTAs per sequence over 16-token chunks
+  cudaStream_t st = (cudaStream_t)stream;
+  const __nv_bfloat16 *qb = (const __nv_bfloat16*)q, *kb = (const __nv_bfloat16*)k, *vb = (const __nv_bfloat16*)v;
+  const __nv_bfloat16 *ab = (const __nv_bfloat16*)a, *bb = (const __nv_bfloat16*)b;
+  if (workspace != nullptr && total_tokens > 0) {
+    // chunked form: the token-only matrices of every chunk first, then 64 CTAs per sequence
     if (((uintptr_t)workspace & 15) || workspace_bytes < ako4x_gdn_prefill_workspace_bytes(total_tokens, num_seqs))
       return AKO4X_EWORKSPACE;
-    if (total_tokens > 0) {
-      gdn_gram_kernel<<<dim3((unsigned)num_seqs, P_HQ, C_GRAM_Z), 256, 0, (cudaStream_t)stream>>>(
-          (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, cu_seqlens, (float*)workspace);
-      AKO_CHECK_LAUNCH();
-    }
-    if (num_seqs == 1) {
-      gdn_prefill_chunk_kernel<false><<<dim3(P_D / C_ROWS, P_HV, 1), P_THREADS, 0, (cudaStream_t)stream>>>(
-          (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, state, A_log, (const __nv_bfloat16*)a,
-          dt_bias, (const __nv_bfloat16*)b, cu_seqlens, scale, (__nv_bfloat16*)out, new_state, (const float*)workspace);
-    } else {
-      gdn_prefill_chunk_kernel<true><<<dim3(P_D / C_ROWS, P_HV, (unsigned)num_seqs), P_THREADS, 0, (cudaStream_t)stream>>>(
-          (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, state, A_log, (const __nv_bfloat16*)a,
-          dt_bias, (const __nv_bfloat16*)b, cu_seqlens, scale, (__nv_bfloat16*)out, new_state, (const float*)workspace);
-    }
+    const int64_t slots = total_tokens / C_TOK + num_seqs;
+    if (slots > 0x7fffffffLL) return AKO4X_EINVAL;
+    if (!ako::ensure_dynamic_smem<gdn_chunk_kernel>(C_SMEM_ALONE)) return AKO4X_ELAUNCH;
+    gdn_chunk_prep_kernel<<<dim3((unsigned)slots, P_HQ), 128, 0, st>>>(qb, kb, A_log, ab, dt_bias, bb, cu_seqlens,
+                                                                      (int)num_seqs, scale, (unsigned char*)workspace);
     AKO_CHECK_LAUNCH();
+    const int64_t ctas = (int64_t)(P_D / C_ROWS) * P_HV * num_seqs;
+    // A grid that leaves SMs idle asks for so much shared memory that no SM takes two CTAs: launched
+    // while the kernel in front still occupies most SMs, it would otherwise double up on a few (one
+    // sequence of 5 263 tokens: 210 to 280 us from call to call).
+    const int smem = ctas <= ako::sm_count() ? C_SMEM_ALONE : C_SMEM;
+    if (ako::launch_pdl(true, gdn_chunk_kernel, dim3(P_D / C_ROWS, P_HV, (unsigned)num_seqs), dim3(2 * C_WARPS * 32), smem, st, qb,
+                        kb, vb, state, cu_seqlens, total_tokens, scale, (__nv_bfloat16*)out, new_state,
+                        (const unsigned char*)workspace) != cudaSuccess)
+      return AKO4X_ELAUNCH;
     return AKO4X_OK;
   }
-  // Three sequences or more (or no workspace): token by token. One or two sequences: 16 lanes per
-  // row (128 CTAs per sequence, the shorter serial chain per token); more: 8 lanes per row (half the
-  // instructions per row and token; measured better from three sequences on, 4 x 2 048: 675 against 734 us).
+  // No workspace: token by token. One or two sequences: 16 lanes per row (128 CTAs per sequence, the
+  // shorter serial chain per token); more: 8 lanes per row (half the instructions per row and token;
+  // measured better from three sequences on, 4 x 2 048: 675 against 734 us).
   if (num_seqs <= 2) {
-    gdn_prefill_kernel<16><<<dim3(P_D / 8, P_HV, (unsigned)num_seqs), P_THREADS, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, state, A_log, (const __nv_bfloat16*)a,
-        dt_bias, (const __nv_bfloat16*)b, cu_seqlens, scale, (__nv_bfloat16*)out, new_state);
+    gdn_prefill_kernel<16><<<dim3(P_D / 8, P_HV, (unsigned)num_seqs), P_THREADS, 0, st>>>(
+        qb, kb, vb, state, A_log, ab, dt_bias, bb, cu_seqlens, scale, (__nv_bfloat16*)out, new_state);
   } else {
-    gdn_prefill_kernel<8><<<dim3(P_D / 16, P_HV, (unsigned)num_seqs), P_THREADS, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, state, A_log, (const __nv_bfloat16*)a,
-        dt_bias, (const __nv_bfloat16*)b, cu_seqlens, scale, (__nv_bfloat16*)out, new_state);
+    gdn_prefill_kernel<8><<<dim3(P_D / 16, P_HV, (unsigned)num_seqs), P_THREADS, 0, st>>>(
+        qb, kb, vb, state, A_log, ab, dt_bias, bb, cu_seqlens, scale, (__nv_bfloat16*)out, new_state);
   }
   AKO_CHECK_LAUNCH();
   return AKO4X_OK;

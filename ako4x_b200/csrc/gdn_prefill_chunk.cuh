@@ -1,246 +1,576 @@
-// Chunked form of the Gated Delta Net prefill recurrence, in fp32 on the CUDA cores; included by
-// gdn_prefill.cu inside its anonymous namespace.
+// Chunked form of the Gated Delta Net prefill recurrence on the tensor cores (mma.sync, bf16 pieces
+// of fp32 values); included by gdn_prefill.cu inside its anonymous namespace.
 //
-// For a chunk of C = 16 tokens with state S0 at its start, Lc_i = sum_{l<=i} log2 g_l and
-// R_ij = 2^(Lc_i - Lc_j) (the decay between tokens j and i), unrolling
+// For a chunk of C = 32 tokens with state S0 at its start, gam_i = prod_{l<=i} g_l and
+// R_ij = prod_{j<l<=i} g_l (the decay between tokens j and i), unrolling
 //   delta_i = beta_i (v_i - g_i S_{i-1} k_i),   S_i = g_i S_{i-1} + delta_i k_i^T
 // gives, for every state row on its own,
-//   delta_i = beta_i (v_i - 2^Lc_i (S0 k_i) - sum_{j<i} R_ij (k_i.k_j) delta_j)      (a triangular solve)
-//   out_i   = scale (2^Lc_i (S0 q_i) + sum_{j<=i} R_ij (q_i.k_j) delta_j)
-//   S_C     = 2^Lc_C S0 + sum_j R_Cj delta_j k_j^T
-// so the only serial part is the 16-step substitution, one shuffle and two FMAs per step, instead
-// of a full dot product, a reduction and an update per token. The products with S0 are 32 dot
-// products per row with no dependence between them; the 16 x 16 tables k_i.k_j and q_i.k_j depend
-// on the tokens only and are computed once per (chunk, q/k head) by a small kernel in front
-// (every state row of the two v heads that share the q/k head reads them).
+//   delta = T (v - gam (S0 k)),  T = (I + A)^-1 diag(beta),  A_ij = beta_i R_ij (k_i.k_j) for j < i
+//   out_i = gam_i scale (S0 q_i) + sum_{j<=i} P_ij delta_j,  P_ij = scale R_ij (q_i.k_j)
+//   S_C   = gam_C S0 + sum_j (R_Cj delta_j) k_j^T
+// T and P depend on the tokens only: gdn_chunk_prep_kernel makes them for all chunks at once.
+// gdn_chunk_kernel then walks a sequence's chunks with five small matrix products per chunk.
 //
-// A row is held by 16 lanes (8 state values each); lane i of the group is also token i of the
-// chunk: a halving butterfly leaves S0.k_i and S0.q_i in lane i, lane i carries row i of the
-// triangular system, and step j of the substitution broadcasts delta_j from lane j.
+// Precision: q, k and v are bf16 already; S, T, P and delta are fp32 and go to the tensor core as
+// three bf16 pieces each (8 + 8 + 8 mantissa bits: by truncation the three pieces of an fp32 value
+// ADD UP TO IT EXACTLY; T and P are rounded piece by piece, which leaves 2^-26). A product with one
+// bf16 factor takes three mma, a product of two fp32 factors takes the six pairs of pieces down to
+// 2^-24: the sums are those of an fp32 recurrence in another order. R is formed from the sum of its
+// own logarithms, never as a difference of two prefix sums, so strong decay elsewhere in a chunk
+// costs it nothing.
+//
+// Split: the state rows never interact, so a CTA owns 16 rows (v) of one (sequence, head). Two groups
+// of four warps share it. The chain group holds S: its warps split k (32 columns each), which makes
+// S0 k a sum over the warps but keeps every part of S in registers for the whole sequence, as mma
+// accumulators that are at once the A fragments of the next chunk's products. The output group runs
+// one step behind on the pieces of S0 and delta that the chain group hands over, off the serial chain.
+// Per chunk and pair of warps: 96 mma (24 S0 k, 24 S0 q, <= 12 T, <= 12 P, 24 S update) of 8.2 cycles of
+// an SM sub-partition (mma.sync m16n8k16 measured at 2.0 cycles per SM).
+//
+// What bounds it: one CTA per SM, the chain (2 100 cycles per chunk, of which three exchanges through
+// shared memory); two CTAs per SM, the LSU data pipe (ncu: 77 %, 1 130 wavefronts per chunk; tensor pipe
+// 43 %). Measured, whole call against the fp32 CUDA-core form this replaces: 8 ragged sequences of
+// 7 244 tokens 605 -> 121 us, 1 x 8 192 1 000 -> 275, 64 x 128 510 -> 120. One group of four warps that
+// also makes the outputs: 128 us for the 8 (three CTAs per SM) and 1.2 instead of 1.08 us per chunk for
+// one sequence. Loads by TMA instead of cp.async: no difference for 8, 1.22 us per chunk for one.
 #pragma once
 
-constexpr int C_TOK = 16;                 // tokens per chunk
-constexpr int C_GSTRIDE = 2 * C_TOK * C_TOK;   // floats per (slot, q/k head): k.k table then q.k table
-constexpr int C_GRAM_Z = 32;              // chunk lanes per sequence in the table kernel's grid
+constexpr int C_TOK = 32;                                // tokens per chunk
+constexpr int C_ROWS = 16;                               // state rows per CTA (one m16 tile)
+constexpr int C_WARPS = 4;                               // k split
+constexpr int C_FRAG_BYTES = 6 * 3 * 32 * 8;             // six 8 x 16 tiles (i, j) on or below the diagonal, three pieces
+constexpr int C_COEF_FLOATS = 2 * C_TOK;                 // gam_i, then R_Cj
+constexpr int C_SLOT_BYTES = 2 * C_FRAG_BYTES + C_COEF_FLOATS * 4;   // T, P, coefficients of one (chunk, head)
+static_assert(C_SLOT_BYTES % 256 == 0, "slots keep the alignment of the workspace");
 
-// Table slot of chunk c of sequence `seq` that starts at token t0: unique over all sequences
+// Workspace slot of chunk c of sequence `seq` that starts at token t0: unique over all sequences
 // without a scan of cu_seqlens (every sequence start costs at most one extra partial chunk).
 __device__ __forceinline__ int64_t gdn_chunk_slot(int64_t t0, int seq, int c) { return t0 / C_TOK + seq + c; }
 
-// tables[slot][hq][0][i][j] = k_i . k_j, tables[slot][hq][1][i][j] = q_i . k_j (tokens past the end
-// of the sequence count as zero vectors). Grid (sequence, q/k head, C_GRAM_Z), 256 threads = (i, j).
-__global__ void __launch_bounds__(256) gdn_gram_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                                                       const int64_t* __restrict__ cu_seqlens, float* __restrict__ tables) {
-  __shared__ float s_k[C_TOK][P_D + 1], s_q[C_TOK][P_D + 1];
-  const int seq = blockIdx.x, hq = blockIdx.y, tid = threadIdx.x;
-  const int64_t t0 = cu_seqlens[seq], t1 = cu_seqlens[seq + 1];
-  const int chunks = (int)((t1 - t0 + C_TOK - 1) / C_TOK);
-  const int i = tid >> 4, j = tid & 15;
-  for (int c = blockIdx.z; c < chunks; c += gridDim.z) {
-    // 16 tokens x 128 values x {k, q}: thread tid loads 8 k and 8 q values of token tid / 16
-    {
-      const int tok = tid >> 4, part = tid & 15;
-      const int64_t t = t0 + (int64_t)c * C_TOK + tok;
-      uint4 kw = make_uint4(0u, 0u, 0u, 0u), qw = kw;
-      if (t < t1) {
-        kw = __ldg(reinterpret_cast<const uint4*>(k + (t * P_HQ + hq) * P_D + part * 8));
-        qw = __ldg(reinterpret_cast<const uint4*>(q + (t * P_HQ + hq) * P_D + part * 8));
-      }
-      const uint32_t ka[4] = {kw.x, kw.y, kw.z, kw.w}, qa[4] = {qw.x, qw.y, qw.z, qw.w};
+// Tile (w, s) of the fragment arrays: rows i = 8w .. 8w+7, columns j = 16s .. 16s+15, s <= w / 2.
+__host__ __device__ constexpr int gdn_frag_tile(int w, int s) { return (w < 2) ? w : 2 * w - 2 + s; }
+
+// x = the sum of its three bf16 pieces, exactly; the pieces of two values packed as an mma operand pair.
+__device__ __forceinline__ void split3_exact(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
+  const uint32_t u0 = __float_as_uint(x0), u1 = __float_as_uint(x1);
+  h = __byte_perm(u0, u1, 0x7632);
+  const float2 r = __fadd2_rn(make_float2(x0, x1), make_float2(-__uint_as_float(u0 & 0xffff0000u), -__uint_as_float(u1 & 0xffff0000u)));
+  const uint32_t v0 = __float_as_uint(r.x), v1 = __float_as_uint(r.y);
+  m = __byte_perm(v0, v1, 0x7632);
+  const float2 e = __fadd2_rn(r, make_float2(-__uint_as_float(v0 & 0xffff0000u), -__uint_as_float(v1 & 0xffff0000u)));
+  l = __byte_perm(__float_as_uint(e.x), __float_as_uint(e.y), 0x7632);
+}
+__device__ __forceinline__ void split3_rn(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
+  h = ako::pack_bf16x2(x0, x1);
+  x0 -= ako::bf16_lo(h);
+  x1 -= ako::bf16_hi(h);
+  m = ako::pack_bf16x2(x0, x1);
+  l = ako::pack_bf16x2(x0 - ako::bf16_lo(m), x1 - ako::bf16_hi(m));
+}
+
+// ---- T, P and the decay coefficients of one chunk, for the two v heads of one q/k head ------------
+// Grid (slots, q/k heads), 4 warps. k.k and q.k by mma (bf16 operands, exact products); T by forward
+// substitution, one warp per head and one column per lane: 496 FMA and 136 broadcast loads per lane.
+__global__ void __launch_bounds__(128, 7) gdn_chunk_prep_kernel(
+    const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const float* __restrict__ A_log,
+    const __nv_bfloat16* __restrict__ a, const float* __restrict__ dt_bias, const __nv_bfloat16* __restrict__ b,
+    const int64_t* __restrict__ cu_seqlens, int num_seqs, float scale, unsigned char* __restrict__ ws) {
+  // k and q rows; after the products, per warp: A and then T of a head (warps 0, 1), P of a head (2, 3)
+  constexpr int A_PITCH = C_TOK + 4, WARP_FLOATS = C_TOK * A_PITCH;
+  __shared__ __align__(128) unsigned char s_x[4 * WARP_FLOATS * 4];
+  __shared__ float s_g[2][C_TOK][C_TOK + 1];                         // k.k, q.k
+  __shared__ float s_lg[2][C_TOK], s_beta[2][C_TOK];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t slot = blockIdx.x;
+  const int hq = blockIdx.y;
+  ako::pdl_trigger();   // the chunk kernel's prologue may start; it waits before it reads the workspace
+
+  // the sequence of this slot: the last s with cu[s] / 32 + s <= slot, 32 candidates per step
+  int lo = 0, hi = num_seqs;
+  while (true) {
+    const int step = (hi - lo + 31) / 32;
+    const int s = lo + lane * step;
+    const unsigned below = __ballot_sync(0xffffffffu, s < hi && cu_seqlens[s] / C_TOK + s <= slot);
+    const int cnt = __popc(below);
+    if (cnt == 0) return;                   // in front of the first sequence
+    lo += (cnt - 1) * step;
+    hi = min(hi, lo + step);
+    if (step == 1) break;
+  }
+  const int64_t t0 = cu_seqlens[lo], t1 = cu_seqlens[lo + 1];
+  const int64_t tb = t0 + (slot - (t0 / C_TOK + lo)) * C_TOK;
+  if (tb >= t1) return;                     // a slot that no chunk uses
+
+  const uint32_t sx = ako::smem_u32(s_x);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        s_k[tok][part * 8 + 2 * u] = ako::bf16_lo(ka[u]);
-        s_k[tok][part * 8 + 2 * u + 1] = ako::bf16_hi(ka[u]);
-        s_q[tok][part * 8 + 2 * u] = ako::bf16_lo(qa[u]);
-        s_q[tok][part * 8 + 2 * u + 1] = ako::bf16_hi(qa[u]);
+  for (int i = 0; i < 8; ++i) {
+    const int idx = tid + 128 * i;          // 2 x 32 rows x 16 pieces of 16 bytes
+    const int which = idx >> 9, row = (idx >> 4) & 31, piece = idx & 15;
+    const bool valid = tb + row < t1;
+    const __nv_bfloat16* src = (which ? q : k) + ((valid ? tb + row : tb) * P_HQ + hq) * P_D + piece * 8;
+    ako::cp_async16(sx + which * (C_TOK * 256) + row * 256 + ((piece ^ (row & 7)) << 4), src, valid);
+  }
+  ako::cp_async_commit();
+  if (tid < 64) {
+    const int e = tid >> 5, h = 2 * hq + e;
+    const int64_t t = tb + lane;
+    float lg = 0.f, beta = 0.f;             // tokens past the end: no decay, no update
+    if (t < t1) {
+      const float y = __bfloat162float(a[t * P_HV + h]) + dt_bias[h];
+      const float sp = (y > 20.f) ? y : log1pf(expf(y));
+      lg = -expf(A_log[h]) * 1.4426950408889634f * sp;
+      beta = 1.f / (1.f + expf(-__bfloat162float(b[t * P_HV + h])));
+    }
+    s_lg[e][lane] = lg;
+    s_beta[e][lane] = beta;
+  }
+  ako::cp_async_wait<0>();
+  __syncthreads();
+  {
+    // warps 0, 1: k.k, rows 16 (warp & 1) ..; warps 2, 3: q.k
+    const int mt = warp & 1;
+    const uint32_t abase = sx + (warp >> 1) * (C_TOK * 256);
+    float acc[4][4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[n][c] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      uint32_t af[4], bf[8];
+      const int ar = mt * 16 + (lane & 15);
+      ako::ldmatrix_x4(af[0], af[1], af[2], af[3], abase + ar * 256 + (((2 * ks + (lane >> 4)) ^ (ar & 7)) << 4));
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const int br = p * 16 + (lane & 7) + ((lane >> 4) << 3);
+        ako::ldmatrix_x4(bf[4 * p], bf[4 * p + 1], bf[4 * p + 2], bf[4 * p + 3],
+                         sx + br * 256 + (((2 * ks + ((lane >> 3) & 1)) ^ (br & 7)) << 4));
       }
+#pragma unroll
+      for (int n = 0; n < 4; ++n) ako::mma_bf16_16816(acc[n], af, bf[2 * n], bf[2 * n + 1]);
     }
-    __syncthreads();
-    float kk = 0.f, qk = 0.f;
-#pragma unroll 8
-    for (int e = 0; e < P_D; ++e) {
-      const float kj = s_k[j][e];
-      kk = fmaf(s_k[i][e], kj, kk);
-      qk = fmaf(s_q[i][e], kj, qk);
+    float(*g)[C_TOK + 1] = s_g[warp >> 1];
+    const int r = mt * 16 + (lane >> 2), c = 2 * (lane & 3);
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      g[r][8 * n + c] = acc[n][0];
+      g[r][8 * n + c + 1] = acc[n][1];
+      g[r + 8][8 * n + c] = acc[n][2];
+      g[r + 8][8 * n + c + 1] = acc[n][3];
     }
-    float* dst = tables + (gdn_chunk_slot(t0, seq, c) * P_HQ + hq) * C_GSTRIDE;
-    dst[tid] = kk;
-    dst[C_TOK * C_TOK + tid] = qk;
-    __syncthreads();
+  }
+  __syncthreads();
+  // warps 0, 1: T and the coefficients of head e; warps 2, 3: P of head e. Lane = column j.
+  const int e = warp & 1, j = lane;
+  unsigned char* dst = ws + (slot * P_HV + 2 * hq + e) * C_SLOT_BYTES + (warp >> 1) * C_FRAG_BYTES;
+  float* out = reinterpret_cast<float*>(s_x) + warp * WARP_FLOATS;       // [i][j], columns rotated by i
+  if (warp < 2) {
+    float run = 0.f;
+#pragma unroll
+    for (int i = 0; i < C_TOK; ++i) {
+      if (i > j) run += s_lg[e][i];
+      out[i * A_PITCH + j] = (i > j) ? s_beta[e][i] * exp2f(run) * s_g[0][i][j] : 0.f;
+    }
+    float* coef = reinterpret_cast<float*>(ws + (slot * P_HV + 2 * hq + e) * C_SLOT_BYTES + 2 * C_FRAG_BYTES);
+    float lc = s_lg[e][lane];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const float up = __shfl_up_sync(0xffffffffu, lc, off);
+      if (lane >= off) lc += up;
+    }
+    coef[lane] = exp2f(lc);
+    coef[C_TOK + lane] = exp2f(run);
+    __syncwarp();
+    float t[C_TOK];
+#pragma unroll
+    for (int i = 0; i < C_TOK; ++i) {
+      float x[4] = {(i == j) ? 1.f : 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int l = 0; l < i; l += 4) {
+        const float4 w = *reinterpret_cast<const float4*>(out + i * A_PITCH + l);
+        x[0] = fmaf(-w.x, t[l], x[0]);
+        if (l + 1 < i) x[1] = fmaf(-w.y, t[l + 1], x[1]);
+        if (l + 2 < i) x[2] = fmaf(-w.z, t[l + 2], x[2]);
+        if (l + 3 < i) x[3] = fmaf(-w.w, t[l + 3], x[3]);
+      }
+      t[i] = (x[0] + x[1]) + (x[2] + x[3]);
+    }
+    const float bj = s_beta[e][j];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < C_TOK; ++i) out[i * C_TOK + ((j + i) & 31)] = t[i] * bj;
+  } else {
+    float run = 0.f;
+#pragma unroll
+    for (int i = 0; i < C_TOK; ++i) {
+      if (i > j) run += s_lg[e][i];
+      out[i * C_TOK + ((j + i) & 31)] = (i >= j) ? scale * exp2f(run) * s_g[1][i][j] : 0.f;
+    }
+  }
+  __syncwarp();
+  // B fragments of mma.m16n8k16 (n = i, k = j): lane (g, t) holds (i = g; j = 2t, 2t+1 | 2t+8, 2t+9)
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+#pragma unroll
+    for (int s = 0; s <= w / 2; ++s) {
+      const int i = 8 * w + (lane >> 2), c = 16 * s + 2 * (lane & 3);
+      const float* row = out + i * C_TOK;
+      uint32_t f[3][2];
+      split3_rn(row[(c + i) & 31], row[(c + 1 + i) & 31], f[0][0], f[1][0], f[2][0]);
+      split3_rn(row[(c + 8 + i) & 31], row[(c + 9 + i) & 31], f[0][1], f[1][1], f[2][1]);
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+        reinterpret_cast<uint2*>(dst)[(gdn_frag_tile(w, s) * 3 + p) * 32 + lane] = make_uint2(f[p][0], f[p][1]);
+    }
   }
 }
 
-constexpr int C_ROWS = 8;                 // state rows per CTA: 4 warps x 2 groups of 16 lanes
-constexpr int C_TPAD = 20;                // padded row length of the tables in shared memory
+// ---- the recurrence over the chunks of one (sequence, head, 16 state rows) ------------------------
+// Shared memory. Everything a chunk reads from global memory is copied here one chunk ahead (two
+// stages per group): fetching T, P and v into registers instead tied them to the few scoreboards that
+// shared-memory loads wait on as well, 2 700 against 2 240 cycles per chunk in the first version.
+constexpr int C_KQ_WARP = C_TOK * 64;                                 // 32 tokens x the warp's 32 columns of k (or q)
+constexpr int C_CH_SLOT = C_WARPS * C_KQ_WARP;                        // chain stage: k | T | gam, R_C | v
+constexpr int C_CH_COEF = C_CH_SLOT + C_FRAG_BYTES;
+constexpr int C_CH_V = C_CH_COEF + C_COEF_FLOATS * 4;
+constexpr int C_CH_STAGE = C_CH_V + C_TOK * C_ROWS * 2;
+constexpr int C_OUT_SLOT = C_WARPS * C_KQ_WARP;                       // output stage: q | P | gam, R_C
+constexpr int C_OUT_COEF = C_OUT_SLOT + C_FRAG_BYTES;
+constexpr int C_OUT_STAGE = C_OUT_COEF + C_COEF_FLOATS * 4;
+constexpr int C_OFF_OUT = 2 * C_CH_STAGE;
+constexpr int C_OFF_S = C_OFF_OUT + 2 * C_OUT_STAGE;                  // pieces of S0, two chunks: [warp][6][lane] uint4
+constexpr int C_S_BYTES = C_WARPS * 6 * 512;
+constexpr int C_OFF_D = C_OFF_S + 2 * C_S_BYTES;                      // delta pieces, two chunks: [piece][tile][lane] uint2
+constexpr int C_D_BYTES = 3 * 4 * 256;
+constexpr int C_OFF_E = C_OFF_D + 2 * C_D_BYTES;                      // R_Cj delta_j pieces
+constexpr int C_OFF_R = C_OFF_E + C_D_BYTES;                          // right-hand side pieces
+constexpr int C_OFF_X = C_OFF_R + C_D_BYTES;                          // partial S0 k: [tile][3 other warps][lane] float4
+constexpr int C_OFF_Y = C_OFF_X + 4 * 3 * 512;                        // partial S0 q
+constexpr int C_SMEM = C_OFF_Y + 4 * 3 * 512;
+constexpr int C_SMEM_ALONE = 120 * 1024;
+static_assert(2 * (C_SMEM + 1024) <= 228 * 1024, "two CTAs per SM");
 
-// LEAN: a scheduling fence every four tokens of the product loop keeps four tokens' loads in flight
-// instead of sixteen: 124 registers instead of 243, three CTAs per SM instead of one. One sequence
-// (128 CTAs) is faster without it, two sequences with it.
-template <bool LEAN>
-__global__ void __launch_bounds__(P_THREADS) gdn_prefill_chunk_kernel(
+// Named barriers: one per group of four warps, and full / empty pairs for the hand-over of a chunk's
+// S0 and delta pieces from the chain group to the output group.
+constexpr int C_BAR_CHAIN = 1, C_BAR_OUT = 2, C_BAR_FULL = 3, C_BAR_EMPTY = 5;
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
+
+// D = A * B.
+__device__ __forceinline__ void mma_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// d0 + d1 (+)= A * B with A and B given as three pieces each: the six pairs of pieces above 2^-24.
+template <bool FIRST>
+__device__ __forceinline__ void mma_6(float (&d0)[4], float (&d1)[4], const uint32_t (&A)[3][4], const uint2 (&B)[3]) {
+  if (FIRST) {
+    mma_zero(d0, A[0], B[0].x, B[0].y);
+    mma_zero(d1, A[1], B[0].x, B[0].y);
+  } else {
+    ako::mma_bf16_16816(d0, A[0], B[0].x, B[0].y);
+    ako::mma_bf16_16816(d1, A[1], B[0].x, B[0].y);
+  }
+  ako::mma_bf16_16816(d0, A[0], B[1].x, B[1].y);
+  ako::mma_bf16_16816(d1, A[2], B[0].x, B[0].y);
+  ako::mma_bf16_16816(d0, A[1], B[1].x, B[1].y);
+  ako::mma_bf16_16816(d1, A[0], B[2].x, B[2].y);
+}
+// The A fragments (16 rows x 16 tokens, three pieces) of two neighbouring token tiles.
+__device__ __forceinline__ void frag_pieces(uint32_t (&A)[3][4], const uint2* src) {
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    const uint2 x = src[p * 128], y = src[p * 128 + 32];
+    A[p][0] = x.x; A[p][1] = x.y; A[p][2] = y.x; A[p][3] = y.y;
+  }
+}
+// 8 x 8 transpose of bf16 pairs across the warp.
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
+  uint32_t y;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(y) : "r"(x));
+  return y;
+}
+
+// A group's 128 threads copy `bytes` (a multiple of 16, at most 3 x 2 KB) to shared memory.
+template <int BYTES>
+__device__ __forceinline__ void copy_group(uint32_t dst, const unsigned char* src, int tid) {
+#pragma unroll
+  for (int i = 0; i < BYTES / 2048; ++i) ako::cp_async16(dst + (i * 128 + tid) * 16, src + (i * 128 + tid) * 16);
+  if (BYTES % 2048 != 0 && tid < (BYTES % 2048) / 16)
+    ako::cp_async16(dst + BYTES / 2048 * 2048 + tid * 16, src + BYTES / 2048 * 2048 + tid * 16);
+}
+// A warp's 32 columns of a chunk's k (or q) rows: 64-byte rows, 16-byte pieces XOR (row / 2). `src` is the
+// lane's piece of row lane / 4, `left` the sequence's tokens from that row on; rows past the end are zero.
+__device__ __forceinline__ void copy_rows(uint32_t dst, const __nv_bfloat16* src, int left, const __nv_bfloat16* safe) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const bool valid = 8 * i < left;
+    ako::cp_async16(dst + i * 512, valid ? src + i * (8 * P_HQ * P_D) : safe, valid);
+  }
+}
+// B fragments (k = 32 columns, n = 8 tokens) of token tile `tile`: two 16-column steps.
+__device__ __forceinline__ void load_token_tile(uint32_t (&bf)[4], uint32_t base, int tile, int lane) {
+  const int row = 8 * tile + (lane & 7);
+  ako::ldmatrix_x4(bf[0], bf[1], bf[2], bf[3], base + row * 64 + (((lane >> 3) ^ ((row >> 1) & 3)) << 4));
+}
+// acc[n] = (S0 pieces of this warp's 32 columns) x (token tile (w + n) mod 4); the three tiles that other
+// warps finish go to shared memory, tile w itself is accumulator 0.
+__device__ __forceinline__ void partial_products(float (&own)[4], const uint32_t (&As)[2][3][4], uint32_t base, float4* part,
+                                                 int w, int lane) {
+  float acc[4][4];
+  uint32_t bf[4][4];
+#pragma unroll
+  for (int n = 0; n < 4; ++n) load_token_tile(bf[n], base, (w + n) & 3, lane);
+#pragma unroll
+  for (int n = 0; n < 4; ++n) mma_zero(acc[n], As[0][0], bf[n][0], bf[n][1]);
+#pragma unroll
+  for (int n = 0; n < 4; ++n) ako::mma_bf16_16816(acc[n], As[1][0], bf[n][2], bf[n][3]);
+#pragma unroll
+  for (int p = 1; p < 3; ++p)
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int n = 0; n < 4; ++n) ako::mma_bf16_16816(acc[n], As[s][p], bf[n][2 * s], bf[n][2 * s + 1]);
+#pragma unroll
+  for (int n = 1; n < 4; ++n)
+    part[(((w + n) & 3) * 3 + n - 1) * 32 + lane] = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) own[i] = acc[0][i];
+}
+__device__ __forceinline__ void add_partials(float (&own)[4], const float4* part, int w, int lane) {
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    const float4 x = part[(w * 3 + p) * 32 + lane];
+    own[0] += x.x; own[1] += x.y; own[2] += x.z; own[3] += x.w;
+  }
+}
+// A tile of 16 rows x 8 tokens (an mma accumulator) as three exact pieces: half an A fragment.
+__device__ __forceinline__ void store_pieces(uint2* dst, const float (&x)[4]) {
+  uint32_t f[3][2];
+  split3_exact(x[0], x[1], f[0][0], f[1][0], f[2][0]);
+  split3_exact(x[2], x[3], f[0][1], f[1][1], f[2][1]);
+#pragma unroll
+  for (int p = 0; p < 3; ++p) dst[p * 128] = make_uint2(f[p][0], f[p][1]);
+}
+// d0 + d1 (+)= (pieces of token tiles 0 .. w) x (tile w of T or P): one or two 16-token steps.
+template <bool FIRST>
+__device__ __forceinline__ void triangular_tile(float (&d0)[4], float (&d1)[4], const uint2* pieces, const uint2* frag, bool two) {
+  uint32_t A[3][4];
+  uint2 B[3];
+  frag_pieces(A, pieces);
+  B[0] = frag[0]; B[1] = frag[32]; B[2] = frag[64];
+  mma_6<FIRST>(d0, d1, A, B);
+  if (two) {
+    frag_pieces(A, pieces + 64);
+    B[0] = frag[96]; B[1] = frag[128]; B[2] = frag[160];
+    mma_6<false>(d0, d1, A, B);
+  }
+}
+
+__global__ void __launch_bounds__(2 * C_WARPS * 32, 2) gdn_chunk_kernel(
     const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
-    const float* __restrict__ state, const float* __restrict__ A_log, const __nv_bfloat16* __restrict__ a,
-    const float* __restrict__ dt_bias, const __nv_bfloat16* __restrict__ b, const int64_t* __restrict__ cu_seqlens,
-    float scale, __nv_bfloat16* __restrict__ out, float* __restrict__ new_state, const float* __restrict__ tables) {
-  __shared__ __align__(16) float s_kq[2][C_TOK][2][P_D];          // [buffer][token][k | q][128]
-  __shared__ __align__(16) float s_tab[2][2][C_TOK][C_TPAD];      // [buffer][k.k | q.k][i][j]
-  __shared__ float s_lg[2][C_TOK], s_beta[2][C_TOK];              // log2 of the decay, beta
-  __shared__ float s_v[2][C_TOK][C_ROWS];
-  __shared__ __align__(16) __nv_bfloat16 s_out[2][C_TOK][C_ROWS];
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const bool producer = warp == P_CONSUMERS / 32;
-  const int rg = blockIdx.x, h = blockIdx.y, seq = blockIdx.z;
+    const float* __restrict__ state, const int64_t* __restrict__ cu_seqlens, int64_t total_tokens, float scale,
+    __nv_bfloat16* __restrict__ out, float* __restrict__ new_state, const unsigned char* __restrict__ ws) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  constexpr int GROUP = C_WARPS * 32;
+  const int tid = threadIdx.x & (GROUP - 1), lane = tid & 31, w = tid >> 5;
+  const bool chain = threadIdx.x < GROUP;
+  const int slice = blockIdx.x, h = blockIdx.y, seq = blockIdx.z;
   const int hq = h / (P_HV / P_HQ);
+  const int g = lane >> 2, t = lane & 3;
   const int64_t t0 = cu_seqlens[seq], t1 = cu_seqlens[seq + 1];
   const int len = (int)(t1 - t0);
-  const int i = lane & 15;                             // lane of the row's group = token of the chunk
-  const int row_local = warp * 2 + (lane >> 4);
-  const int row = rg * C_ROWS + row_local;
-  // the lane holds state elements 64 p + 4 i + c (p = 0, 1; c = 0..3)
-  float* ns = new_state + (((int64_t)seq * P_HV + h) * P_D + row) * P_D + 4 * i;
-  float S[8];
-  if (len <= 0) {   // the definition leaves the new state of an empty sequence at zero
-    if (!producer) {
-      *reinterpret_cast<float4*>(ns) = make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(ns + 64) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    return;
-  }
-  if (producer) {
+  const int chunks = (len > 0) ? (len + C_TOK - 1) / C_TOK : 0;
+  const uint32_t sm = ako::smem_u32(smem);
+  const bool two = w >= 2;                          // tile w needs two 16-token steps of T and P
+  const int ft = gdn_frag_tile(w, 0) * 96 + lane;   // its first fragment
+  const unsigned char* slot = ws + (gdn_chunk_slot(t0, seq, 0) * P_HV + h) * C_SLOT_BYTES;
+  const int64_t kq_off = ((t0 + g) * P_HQ + hq) * P_D + 32 * w + 8 * t;
+  const uint32_t kq_dst = w * C_KQ_WARP + g * 64 + ((t ^ ((g >> 1) & 3)) << 4);
+
+  if (chain) {
+    // the warp's part of the state: rows g, g + 8, columns 32 w + 8 n + 2 t, + 1
+    const int64_t srow = (((int64_t)seq * P_HV + h) * P_D + slice * C_ROWS + g) * P_D + 32 * w + 2 * t;
+    float S[4][4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) S[e] = 0.f;
-  } else if (state != nullptr) {
-    const float* sp = state + (((int64_t)seq * P_HV + h) * P_D + row) * P_D + 4 * i;
-    const float4 x = __ldcs(reinterpret_cast<const float4*>(sp)), y = __ldcs(reinterpret_cast<const float4*>(sp + 64));
-    S[0] = x.x; S[1] = x.y; S[2] = x.z; S[3] = x.w; S[4] = y.x; S[5] = y.y; S[6] = y.z; S[7] = y.w;
+    for (int n = 0; n < 4; ++n) {
+      float2 x = make_float2(0.f, 0.f), y = x;
+      if (state != nullptr && len > 0) {   // the definition leaves the new state of an empty sequence at zero
+        x = __ldcs(reinterpret_cast<const float2*>(state + srow + 8 * n));
+        y = __ldcs(reinterpret_cast<const float2*>(state + srow + 8 * P_D + 8 * n));
+      }
+      S[n][0] = x.x; S[n][1] = x.y; S[n][2] = y.x; S[n][3] = y.y;
+    }
+    const __nv_bfloat16* kp = k + kq_off;
+    const __nv_bfloat16* vp = v + ((t0 + (tid >> 1)) * P_HV + h) * P_D + slice * C_ROWS + (tid & 1) * 8;
+    auto load_k = [&](int c) {
+      copy_rows(sm + (c & 1) * C_CH_STAGE + kq_dst, kp, len - c * C_TOK - g, k);
+      kp += C_TOK * P_HQ * P_D;
+    };
+    auto load_rest = [&](int c) {   // T, coefficients, v
+      const uint32_t st = sm + (c & 1) * C_CH_STAGE;
+      copy_group<C_FRAG_BYTES>(st + C_CH_SLOT, slot, tid);
+      if (tid < C_COEF_FLOATS / 4) ako::cp_async16(st + C_CH_COEF + tid * 16, slot + 2 * C_FRAG_BYTES + tid * 16);
+      slot += P_HV * C_SLOT_BYTES;
+      if (tid < 2 * C_TOK) {
+        const bool valid = c * C_TOK + (tid >> 1) < len;
+        ako::cp_async16(st + C_CH_V + tid * 16, valid ? vp : v, valid);
+        vp += C_TOK * P_HV * P_D;
+      }
+    };
+    if (chunks > 0) load_k(0);
+    ako::pdl_wait();   // T, P and the coefficients come from the kernel in front
+    if (chunks > 0) load_rest(0);
+    ako::cp_async_commit();
+
+    float4* sX = reinterpret_cast<float4*>(smem + C_OFF_X);
+    uint2* sR = reinterpret_cast<uint2*>(smem + C_OFF_R) + lane;
+    uint2* sE = reinterpret_cast<uint2*>(smem + C_OFF_E) + lane;
+    for (int c = 0; c < chunks; ++c) {
+      const int b = c & 1;
+      if (c + 1 < chunks) load_k(c + 1);
+      ako::cp_async_commit();
+      // A fragments of S (its accumulators as they lie), three exact pieces
+      uint32_t As[2][3][4];
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          split3_exact(S[2 * s + (i >> 1)][2 * (i & 1)], S[2 * s + (i >> 1)][2 * (i & 1) + 1], As[s][0][i], As[s][1][i], As[s][2][i]);
+      ako::cp_async_wait<1>();
+      __syncwarp();
+      const uint32_t kbase = sm + b * C_CH_STAGE + w * C_KQ_WARP;
+      const unsigned char* stage = smem + b * C_CH_STAGE;
+      const float* coef = reinterpret_cast<const float*>(stage + C_CH_COEF);
+
+      // 1. this warp's part of S0 k; the output group gets the pieces of S0
+      float x[4];
+      partial_products(x, As, kbase, sX, w, lane);
+      if (c >= 2) bar_sync(C_BAR_EMPTY + b, 2 * GROUP);
+      {
+        uint4* dst = reinterpret_cast<uint4*>(smem + C_OFF_S + b * C_S_BYTES) + w * 192 + lane;
+#pragma unroll
+        for (int s = 0; s < 2; ++s)
+#pragma unroll
+          for (int p = 0; p < 3; ++p) dst[(s * 3 + p) * 32] = make_uint4(As[s][p][0], As[s][p][1], As[s][p][2], As[s][p][3]);
+      }
+      bar_sync(C_BAR_CHAIN, GROUP);   // the partial sums, and everybody's part of T, coefficients and v
+      if (c + 1 < chunks) load_rest(c + 1);   // no warp reads the other stage any more
+      ako::cp_async_commit();
+
+      // 2. right-hand side of tile w: v - gam (S0 k), as pieces for the group
+      add_partials(x, sX, w, lane);
+      {
+        const float2 gam = *reinterpret_cast<const float2*>(coef + 8 * w + 2 * t);
+        const __nv_bfloat16* vv = reinterpret_cast<const __nv_bfloat16*>(stage + C_CH_V) + (8 * w + 2 * t) * C_ROWS + g;
+        const float r[4] = {__bfloat162float(vv[0]) - gam.x * x[0], __bfloat162float(vv[C_ROWS]) - gam.y * x[1],
+                            __bfloat162float(vv[8]) - gam.x * x[2], __bfloat162float(vv[C_ROWS + 8]) - gam.y * x[3]};
+        store_pieces(sR + w * 32, r);
+      }
+      const float gC = coef[C_TOK - 1];
+      const float2 dec = *reinterpret_cast<const float2*>(coef + C_TOK + 8 * w + 2 * t);
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) S[n][i] *= gC;
+      bar_sync(C_BAR_CHAIN, GROUP);
+
+      // 3. delta of tile w = T (right-hand side)
+      float d0[4], d1[4];
+      triangular_tile<true>(d0, d1, sR, reinterpret_cast<const uint2*>(stage + C_CH_SLOT) + ft, two);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) d0[i] += d1[i];
+      {
+        const float e[4] = {d0[0] * dec.x, d0[1] * dec.y, d0[2] * dec.x, d0[3] * dec.y};
+        store_pieces(sE + w * 32, e);
+      }
+      bar_sync(C_BAR_CHAIN, GROUP);
+      store_pieces(reinterpret_cast<uint2*>(smem + C_OFF_D + b * C_D_BYTES) + lane + w * 32, d0);
+      bar_arrive(C_BAR_FULL + b, 2 * GROUP);
+
+      // 4. the state at the end of the chunk
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        uint32_t A[3][4], bf[8];
+        frag_pieces(A, sE + 64 * s);
+        const int row = 16 * s + (lane & 15);
+#pragma unroll
+        for (int n = 0; n < 4; n += 2)
+          ako::ldmatrix_x4_trans(bf[2 * n], bf[2 * n + 1], bf[2 * n + 2], bf[2 * n + 3],
+                                 kbase + row * 64 + (((n + (lane >> 4)) ^ ((row >> 1) & 3)) << 4));
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+#pragma unroll
+          for (int n = 0; n < 4; ++n) ako::mma_bf16_16816(S[n], A[p], bf[2 * n], bf[2 * n + 1]);
+      }
+      __syncwarp();   // the warp's k of this chunk is read: the next load may overwrite it
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      __stcs(reinterpret_cast<float2*>(new_state + srow + 8 * n), make_float2(S[n][0], S[n][1]));
+      __stcs(reinterpret_cast<float2*>(new_state + srow + 8 * P_D + 8 * n), make_float2(S[n][2], S[n][3]));
+    }
   } else {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) S[e] = 0.f;
-  }
-  const float neg_A = -expf(A_log[h]);
-  const float dtb = dt_bias[h];
-
-  // The producer warp stages chunk c + 1 (and the chunk's two tables, 2 KB) and stores the outputs
-  // of chunk c - 1 while the four compute warps work on chunk c: one barrier per chunk.
-  auto stage = [&](int c, int buf) {
-    gdn_stage_chunk<C_ROWS, true>(lane, c, t0, t1, hq, h, rg, q, k, v, a, b, neg_A, dtb, s_kq[buf], s_lg[buf], s_beta[buf],
-                                  s_v[buf]);
-    const uint4* tp = reinterpret_cast<const uint4*>(tables + (gdn_chunk_slot(t0, seq, c) * P_HQ + hq) * C_GSTRIDE);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int f = lane + 32 * u;                      // float4 number f of the 128 that make both tables
-      const uint4 x = __ldg(tp + f);
-      *reinterpret_cast<uint4*>(&s_tab[buf][f >> 6][(f & 63) >> 2][(f & 3) * 4]) = x;
+    __nv_bfloat16* out_h = out + h * P_D + slice * C_ROWS;
+    const __nv_bfloat16* qp = q + kq_off;
+    auto load = [&](int c) {   // q, P, coefficients
+      const uint32_t st = sm + C_OFF_OUT + (c & 1) * C_OUT_STAGE;
+      copy_rows(st + kq_dst, qp, len - c * C_TOK - g, q);
+      qp += C_TOK * P_HQ * P_D;
+      copy_group<C_FRAG_BYTES + C_COEF_FLOATS * 4>(st + C_OUT_SLOT, slot + C_FRAG_BYTES, tid);
+      slot += P_HV * C_SLOT_BYTES;
+      ako::cp_async_commit();
+    };
+    ako::pdl_wait();
+    if (chunks > 0) load(0);
+    // tokens outside every sequence: zero, by the CTAs of the first and of the last sequence
+    for (int side = 0; side < 2; ++side) {
+      if (seq != (side ? (int)gridDim.z - 1 : 0)) continue;
+      const int64_t z0 = side ? max(t1, (int64_t)0) : 0, z1 = side ? total_tokens : min(t0, total_tokens);
+      for (int64_t i = z0 * 2 + tid; i < z1 * 2; i += GROUP)
+        *reinterpret_cast<uint4*>(out_h + (i >> 1) * (P_HV * P_D) + (i & 1) * 8) = make_uint4(0u, 0u, 0u, 0u);
     }
-  };
-  const int chunks = (len + C_TOK - 1) / C_TOK;
-  if (producer) stage(0, 0);
-  __syncthreads();
-  const bool b3 = (i & 8) != 0, b2 = (i & 4) != 0, b1 = (i & 2) != 0, b0 = (i & 1) != 0;
-  for (int c = 0; c < chunks; ++c) {
-    const int buf = c & 1;
-    if (producer) {
-      if (c > 0) gdn_store_chunk<C_ROWS>(lane, c - 1, t0, len, h, rg, s_out[buf ^ 1], out);
-      if (c + 1 < chunks) stage(c + 1, buf ^ 1);
-      __syncthreads();
-      continue;
-    }
-
-    // 1. this lane's part of S0.k_j and S0.q_j for the 16 tokens: 32 independent short dot products
-    float pa[C_TOK], pc[C_TOK];
+    float4* sY = reinterpret_cast<float4*>(smem + C_OFF_Y);
+    out_h += t0 * (P_HV * P_D);
+    for (int c = 0; c < chunks; ++c) {
+      const int b = c & 1;
+      bar_sync(C_BAR_FULL + b, 2 * GROUP);     // S0 and delta of chunk c; the group is done with chunk c - 1
+      if (c + 1 < chunks) load(c + 1);
+      else ako::cp_async_commit();
+      uint32_t As[2][3][4];
+      {
+        const uint4* src = reinterpret_cast<const uint4*>(smem + C_OFF_S + b * C_S_BYTES) + w * 192 + lane;
 #pragma unroll
-    for (int j = 0; j < C_TOK; ++j) {
-      const float4 k0 = *reinterpret_cast<const float4*>(&s_kq[buf][j][0][4 * i]);
-      const float4 k1 = *reinterpret_cast<const float4*>(&s_kq[buf][j][0][64 + 4 * i]);
-      const float4 q0 = *reinterpret_cast<const float4*>(&s_kq[buf][j][1][4 * i]);
-      const float4 q1 = *reinterpret_cast<const float4*>(&s_kq[buf][j][1][64 + 4 * i]);
-      pa[j] = fmaf(S[0], k0.x, fmaf(S[1], k0.y, fmaf(S[2], k0.z, S[3] * k0.w))) +
-              fmaf(S[4], k1.x, fmaf(S[5], k1.y, fmaf(S[6], k1.z, S[7] * k1.w)));
-      pc[j] = fmaf(S[0], q0.x, fmaf(S[1], q0.y, fmaf(S[2], q0.z, S[3] * q0.w))) +
-              fmaf(S[4], q1.x, fmaf(S[5], q1.y, fmaf(S[6], q1.z, S[7] * q1.w)));
-      if (LEAN && (j & 3) == 3) asm volatile("" ::: "memory");
-    }
-    // 2. halving butterfly over the row's 16 lanes: lane i ends with the complete sums of token i
-    float ai, ci;
-    {
-      float x8[8], x4[4], x2[2];
+        for (int s = 0; s < 2; ++s)
 #pragma unroll
-      for (int t = 0; t < 8; ++t) x8[t] = (b3 ? pa[8 + t] : pa[t]) + __shfl_xor_sync(0xffffffffu, b3 ? pa[t] : pa[8 + t], 8);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) x4[t] = (b2 ? x8[4 + t] : x8[t]) + __shfl_xor_sync(0xffffffffu, b2 ? x8[t] : x8[4 + t], 4);
-#pragma unroll
-      for (int t = 0; t < 2; ++t) x2[t] = (b1 ? x4[2 + t] : x4[t]) + __shfl_xor_sync(0xffffffffu, b1 ? x4[t] : x4[2 + t], 2);
-      ai = (b0 ? x2[1] : x2[0]) + __shfl_xor_sync(0xffffffffu, b0 ? x2[0] : x2[1], 1);
-#pragma unroll
-      for (int t = 0; t < 8; ++t) x8[t] = (b3 ? pc[8 + t] : pc[t]) + __shfl_xor_sync(0xffffffffu, b3 ? pc[t] : pc[8 + t], 8);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) x4[t] = (b2 ? x8[4 + t] : x8[t]) + __shfl_xor_sync(0xffffffffu, b2 ? x8[t] : x8[4 + t], 4);
-#pragma unroll
-      for (int t = 0; t < 2; ++t) x2[t] = (b1 ? x4[2 + t] : x4[t]) + __shfl_xor_sync(0xffffffffu, b1 ? x4[t] : x4[2 + t], 2);
-      ci = (b0 ? x2[1] : x2[0]) + __shfl_xor_sync(0xffffffffu, b0 ? x2[0] : x2[1], 1);
-    }
-    // 3. row i of the triangular system and of the output sum
-    float lc[C_TOK];            // Lc_j for every token of the chunk
-    float Lci = 0.f;
-    {
-      float run = 0.f;
-#pragma unroll
-      for (int j = 0; j < C_TOK; ++j) {
-        run += s_lg[buf][j];
-        lc[j] = run;
-        if (j == i) Lci = run;
+          for (int p = 0; p < 3; ++p) {
+            const uint4 f = src[(s * 3 + p) * 32];
+            As[s][p][0] = f.x; As[s][p][1] = f.y; As[s][p][2] = f.z; As[s][p][3] = f.w;
+          }
+      }
+      ako::cp_async_wait<1>();
+      __syncwarp();
+      const unsigned char* stage = smem + C_OFF_OUT + b * C_OUT_STAGE;
+      float y[4];
+      partial_products(y, As, sm + C_OFF_OUT + b * C_OUT_STAGE + w * C_KQ_WARP, sY, w, lane);
+      bar_sync(C_BAR_OUT, GROUP);
+      add_partials(y, sY, w, lane);
+      const float2 gam = *reinterpret_cast<const float2*>(reinterpret_cast<const float*>(stage + C_OUT_COEF) + 8 * w + 2 * t);
+      float o0[4] = {scale * gam.x * y[0], scale * gam.y * y[1], scale * gam.x * y[2], scale * gam.y * y[3]};
+      float o1[4] = {0.f, 0.f, 0.f, 0.f};
+      triangular_tile<false>(o0, o1, reinterpret_cast<const uint2*>(smem + C_OFF_D + b * C_D_BYTES) + lane,
+                             reinterpret_cast<const uint2*>(stage + C_OUT_SLOT) + ft, two);
+      if (c + 2 < chunks) bar_arrive(C_BAR_EMPTY + b, 2 * GROUP);
+      // transposed across the warp: lane (g, t) gets token g, rows 2t, 2t+1 (and + 8)
+      const uint32_t y0 = movmatrix_trans(ako::pack_bf16x2(o0[0] + o1[0], o0[1] + o1[1]));
+      const uint32_t y1 = movmatrix_trans(ako::pack_bf16x2(o0[2] + o1[2], o0[3] + o1[3]));
+      if (c * C_TOK + 8 * w + g < len) {
+        uint32_t* op = reinterpret_cast<uint32_t*>(out_h + (int64_t)(c * C_TOK + 8 * w + g) * (P_HV * P_D)) + t;
+        op[0] = y0;
+        op[4] = y1;
       }
     }
-    const float beta_i = s_beta[buf][i];
-    float ca[C_TOK], co[C_TOK];  // ca[j] = beta_i R_ij (k_i.k_j) for j < i; co[j] = R_ij (q_i.k_j) for j <= i
-#pragma unroll
-    for (int j4 = 0; j4 < C_TOK; j4 += 4) {
-      const float4 g4 = *reinterpret_cast<const float4*>(&s_tab[buf][0][i][j4]);
-      const float4 m4 = *reinterpret_cast<const float4*>(&s_tab[buf][1][i][j4]);
-      const float gg[4] = {g4.x, g4.y, g4.z, g4.w}, mm[4] = {m4.x, m4.y, m4.z, m4.w};
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int j = j4 + u;
-        const float rij = exp2f(fminf(Lci - lc[j], 0.f));
-        ca[j] = (j < i) ? beta_i * rij * gg[u] : 0.f;
-        co[j] = (j <= i) ? rij * mm[u] : 0.f;
-      }
-    }
-    const float gam_i = exp2f(Lci);
-    float rhs = beta_i * (s_v[buf][i][row_local] - gam_i * ai);
-    float o = gam_i * ci;
-    // 4. forward substitution: delta_j is final in lane j when step j starts
-    float d[C_TOK];
-#pragma unroll
-    for (int j = 0; j < C_TOK; ++j) {
-      const float dj = __shfl_sync(0xffffffffu, rhs, j, 16);
-      d[j] = dj;
-      rhs = fmaf(-ca[j], dj, rhs);
-      o = fmaf(co[j], dj, o);
-    }
-    s_out[buf][i][row_local] = __float2bfloat16_rn(scale * o);
-    // 5. the state at the end of the chunk
-    {
-      const float lend = lc[C_TOK - 1];
-      const float gC = exp2f(lend);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) S[e] *= gC;
-#pragma unroll
-      for (int j = 0; j < C_TOK; ++j) {
-        const float w = exp2f(lend - lc[j]) * d[j];
-        const float4 k0 = *reinterpret_cast<const float4*>(&s_kq[buf][j][0][4 * i]);
-        const float4 k1 = *reinterpret_cast<const float4*>(&s_kq[buf][j][0][64 + 4 * i]);
-        S[0] = fmaf(w, k0.x, S[0]); S[1] = fmaf(w, k0.y, S[1]); S[2] = fmaf(w, k0.z, S[2]); S[3] = fmaf(w, k0.w, S[3]);
-        S[4] = fmaf(w, k1.x, S[4]); S[5] = fmaf(w, k1.y, S[5]); S[6] = fmaf(w, k1.z, S[6]); S[7] = fmaf(w, k1.w, S[7]);
-      }
-    }
-    __syncthreads();                       // chunk c done, chunk c + 1 staged
   }
-  if (producer) {
-    gdn_store_chunk<C_ROWS>(lane, chunks - 1, t0, len, h, rg, s_out[(chunks - 1) & 1], out);
-    return;
-  }
-  __stcs(reinterpret_cast<float4*>(ns), make_float4(S[0], S[1], S[2], S[3]));
-  __stcs(reinterpret_cast<float4*>(ns + 64), make_float4(S[4], S[5], S[6], S[7]));
 }

@@ -95,3 +95,23 @@ def test_long_sequences_sampled():
     ro, rs = oracle.gdn_prefill(*[one[k] for k in KEYS], a["scale"])
     assert (s[1].cpu() - rs[0]).abs().max().item() <= 5e-5 * rs.abs().max().item()
     assert_close_bf16(o[t1 - 64:t1].cpu(), ro[-64:], atol=2e-3, rtol=2e-2)
+
+
+@pytest.mark.parametrize("lens,lead,tail", [([31, 32, 33], 0, 0), ([1, 64, 0, 65, 2], 5, 9), ([96], 33, 1), ([0, 0, 7], 3, 0),
+                                            ([40] * 70, 0, 40)])
+def test_chunk_edges_and_tokens_outside(lens, lead, tail):
+    """Sequences that end at, before and after a 32-token chunk, empty ones, more sequences than the
+    slot search takes per step, and tokens in front of and behind every sequence (their outputs are
+    zero). The chunked and the token-by-token form differ in the order of fp32 sums only: the state
+    of n tokens within 2e-6 * sqrt(n) of its largest value."""
+    a = W.make_gdn_prefill([lead] + lens + [tail], shape_id=31 + len(lens))
+    n = len(lens)
+    a["state"], a["cu_seqlens"] = a["state"][1:n + 1].contiguous(), a["cu_seqlens"][1:n + 2].contiguous()
+    args = [a[k].cuda() for k in KEYS]
+    o1, s1 = gdn_prefill.run(*args, a["scale"], _chunked=False)
+    o2, s2 = gdn_prefill.run(*args, a["scale"])
+    end = lead + sum(lens)
+    assert torch.all(o2[:lead] == 0) and torch.all(o2[end:] == 0)
+    assert (s1 - s2).abs().max().item() <= 2e-6 * max(lens) ** 0.5 * s1.abs().max().item()
+    assert_close_bf16(o2.cpu(), o1.cpu(), atol=2e-3, rtol=2e-2)
+    assert (o1 == o2).float().mean().item() > 0.99
