@@ -5,19 +5,15 @@
 //   delta[v] = beta (v_t[v] - g S[v,:].k_t),  S[v,:] = g S[v,:] + delta[v] k_t,
 //   out_t[v] = scale S[v,:].q_t = scale (g S_old[v,:].q_t + (q_t.k_t) delta[v])
 // (the recurrence reference/gdn-prefill/variants/cuda_graph_v5/kernel.py evaluates in chunked form,
-// :1333-1400 for its entry point). The rows S[v,:] of a state never interact, so this first
-// version runs the recurrence as it is written, token by token, with all the parallelism the rows
-// give: a row is held by 8 or 16 lanes (16 or 8 state values each, in registers for the whole
-// sequence), four compute warps own 16 or 8 rows of one (sequence, head) -- 64 or 128 CTAs per
-// sequence --, q_t / k_t pass through shared memory as fp32 in double-buffered chunks of 16 tokens
-// that a fifth warp stages one chunk ahead (it also stores the finished chunk's outputs). The serial chain per token is one short dot product, three or four
-// shuffle levels and the update; measured about 270 cycles per token and 100 more per token of
-// chunk hand-over, so a single sequence of 8 192 tokens takes 1.5 ms. The chunked form of the
-// recurrence (gdn_prefill_chunk.cuh, fp32 on the CUDA cores) is used for one or two sequences;
-// a tensor-core form is not built. The state crosses HBM once each
-// way; outputs leave in 16- or 32-byte pieces per token and CTA. Processing two tokens per
-// reduction round (both products taken from the same state, the second delta corrected with
-// k1.k2) was built and measured slower (1.97 ms against 1.52 ms): eight values per shuffle level.
+// :1333-1400 for its entry point). Calls with a workspace run it in chunks on the tensor cores
+// (gdn_prefill_chunk.cuh). The kernel in this file needs no workspace: the rows S[v,:] of a state never
+// interact, so it runs the recurrence as it is written, token by token: a row is held by 8 or 16 lanes
+// (16 or 8 state values each, in registers for the whole sequence), four compute warps own 16 or 8
+// rows of one (sequence, head) -- 64 or 128 CTAs per sequence --, q_t / k_t pass through shared memory
+// as fp32 in double-buffered chunks of 16 tokens that a fifth warp stages one chunk ahead (it also
+// stores the finished chunk's outputs). The serial chain per token is one short dot product, three or
+// four shuffle levels and the update: about 270 cycles, 1.4 ms for a sequence of 8 192 tokens. The state
+// crosses HBM once each way; outputs leave in 16- or 32-byte pieces per token and CTA.
 #include "common.cuh"
 
 namespace {
@@ -30,9 +26,9 @@ constexpr int P_THREADS = 160;      // + one producer warp that stages the next 
 // The producer warp's work for one 16-token chunk `c` of the sequence [t0, t1): q and k of head hq
 // as fp32 into kq[token][k | q][128] (token r is one coalesced 512-byte read, lane L converts its 16
 // bytes and writes 32 consecutive bytes: no bank conflict), the v values of the CTA's ROWS rows,
-// and per token the gate pair: gate[token] = g (or log2 g when LOG2) and beta[token]. Tokens past
+// and per token the gate pair: gate[token] = g and beta[token]. Tokens past
 // the end of the sequence are staged as nothing-happens tokens (k = q = v = 0, g = 1, beta = 0).
-template <int ROWS, bool LOG2>
+template <int ROWS>
 __device__ __forceinline__ void gdn_stage_chunk(int lane, int c, int64_t t0, int64_t t1, int hq, int h, int rg,
                                                 const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
                                                 const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ a,
@@ -77,7 +73,7 @@ __device__ __forceinline__ void gdn_stage_chunk(int lane, int c, int64_t t0, int
     }
     const float y = __uint_as_float((uint32_t)graw << 16) + dtb;
     const float sp = (y > 20.f) ? y : log1pf(expf(y));
-    gate[tok] = !valid ? (LOG2 ? 0.f : 1.f) : (LOG2 ? neg_A * 1.4426950408889634f * sp : expf(neg_A * sp));
+    gate[tok] = valid ? expf(neg_A * sp) : 1.f;
   } else {
     beta[tok] = valid ? 1.f / (1.f + expf(-__uint_as_float((uint32_t)graw << 16))) : 0.f;
   }
@@ -155,14 +151,14 @@ __global__ void __launch_bounds__(P_THREADS) gdn_prefill_kernel(
   // outputs of chunk c - 1 and stages chunk c + 1 (global loads, conversion, gate math), so that a
   // chunk costs the compute warps one barrier and nothing else.
   const int chunks = (len + P_CHUNK - 1) / P_CHUNK;
-  if (producer) gdn_stage_chunk<P_ROWS, false>(lane, 0, t0, t1, hq, h, rg, q, k, v, a, b, neg_A, dtb, s_kq[0], s_g[0], s_beta[0], s_v[0]);
+  if (producer) gdn_stage_chunk<P_ROWS>(lane, 0, t0, t1, hq, h, rg, q, k, v, a, b, neg_A, dtb, s_kq[0], s_g[0], s_beta[0], s_v[0]);
   __syncthreads();
   for (int c = 0; c < chunks; ++c) {
     const int buf = c & 1;
     if (producer) {
       if (c > 0) gdn_store_chunk<P_ROWS>(lane, c - 1, t0, len, h, rg, s_out[buf ^ 1], out);
       if (c + 1 < chunks)
-        gdn_stage_chunk<P_ROWS, false>(lane, c + 1, t0, t1, hq, h, rg, q, k, v, a, b, neg_A, dtb, s_kq[buf ^ 1], s_g[buf ^ 1],
+        gdn_stage_chunk<P_ROWS>(lane, c + 1, t0, t1, hq, h, rg, q, k, v, a, b, neg_A, dtb, s_kq[buf ^ 1], s_g[buf ^ 1],
                                        s_beta[buf ^ 1], s_v[buf ^ 1]);
       __syncthreads();
       continue;
@@ -260,6 +256,17 @@ extern "C" int ako4x_gdn_prefill(const void* q, const void* k, const void* v, co
     gdn_chunk_prep_kernel<<<dim3((unsigned)slots, P_HQ), 128, 0, st>>>(qb, kb, A_log, ab, dt_bias, bb, cu_seqlens,
                                                                       (int)num_seqs, scale, (unsigned char*)workspace);
     AKO_CHECK_LAUNCH();
+    // One warp per 16 rows and no exchanges from 20 sequences on, where it fills the GPU: equal at 16
+    // sequences (16 x 200 tokens: 60 against 58 us), ahead from 20 (20 x 200: 60 against 70, 64 x 128: 84
+    // against 128, 64 x 4: 31 against 53) and far behind for few long ones (1 x 8 192: 800 against 275).
+    if (num_seqs >= 20) {
+      if (!ako::ensure_dynamic_smem<gdn_chunk_wide_kernel>(CW_SMEM) ||
+          ako::launch_pdl(true, gdn_chunk_wide_kernel, dim3(P_D / CW_ROWS, P_HV, (unsigned)num_seqs), dim3(128), CW_SMEM, st, qb, kb, vb,
+                          state, cu_seqlens, total_tokens, scale, (__nv_bfloat16*)out, new_state,
+                          (const unsigned char*)workspace) != cudaSuccess)
+        return AKO4X_ELAUNCH;
+      return AKO4X_OK;
+    }
     const int64_t ctas = (int64_t)(P_D / C_ROWS) * P_HV * num_seqs;
     // A grid that leaves SMs idle asks for so much shared memory that no SM takes two CTAs: launched
     // while the kernel in front still occupies most SMs, it would otherwise double up on a few (one

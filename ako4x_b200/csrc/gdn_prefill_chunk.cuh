@@ -574,3 +574,245 @@ __global__ void __launch_bounds__(2 * C_WARPS * 32, 2) gdn_chunk_kernel(
     }
   }
 }
+
+// ---- the same recurrence, one warp per 16 state rows ----------------------------------------------
+// With enough sequences to fill the GPU the exchanges between warps are what costs: here a warp holds
+// all 128 columns of its 16 rows, so that a chunk needs no exchange at all (everything from S0 k to the
+// new S stays in its registers) and the CTA's four warps (64 rows) only share the loads: 264 LSU
+// wavefronts per 16 rows and chunk instead of 1 130, 360 mma in a row instead of 96. Bound by the tensor
+// pipe (2 950 cycles of a sub-partition per chunk and warp) where at least two warps share one.
+constexpr int CW_ROWS = 64;
+constexpr int CW_V_PITCH = CW_ROWS * 2 + 16;                          // ldmatrix of eight rows: no bank conflict
+constexpr int CW_OFF_Q = C_TOK * 256;                                 // stage: k | q | T, P, coefficients | v
+constexpr int CW_OFF_SLOT = 2 * C_TOK * 256;
+constexpr int CW_OFF_V = CW_OFF_SLOT + C_SLOT_BYTES;
+constexpr int CW_STAGE = CW_OFF_V + C_TOK * CW_V_PITCH;
+constexpr int CW_SMEM = 2 * CW_STAGE;
+static_assert(CW_STAGE % 128 == 0 && 3 * (CW_SMEM + 1024) <= 228 * 1024, "three CTAs per SM");
+
+// Pieces of a 16 x 8 accumulator tile: half of the A fragment of a 16-token step.
+__device__ __forceinline__ void tile_pieces(uint32_t (&A)[3][4], int half, const float (&x)[4]) {
+  split3_exact(x[0], x[1], A[0][2 * half], A[1][2 * half], A[2][2 * half]);
+  split3_exact(x[2], x[3], A[0][2 * half + 1], A[1][2 * half + 1], A[2][2 * half + 1]);
+}
+
+__global__ void __launch_bounds__(128, 3) gdn_chunk_wide_kernel(
+    const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
+    const float* __restrict__ state, const int64_t* __restrict__ cu_seqlens, int64_t total_tokens, float scale,
+    __nv_bfloat16* __restrict__ out, float* __restrict__ new_state, const unsigned char* __restrict__ ws) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int half = blockIdx.x, h = blockIdx.y, seq = blockIdx.z;
+  const int hq = h / (P_HV / P_HQ);
+  const int g = lane >> 2, t = lane & 3;
+  const int64_t t0 = cu_seqlens[seq], t1 = cu_seqlens[seq + 1];
+  const int len = (int)(t1 - t0);
+  const int chunks = (len > 0) ? (len + C_TOK - 1) / C_TOK : 0;
+  const uint32_t sm = ako::smem_u32(smem);
+  const unsigned char* slot = ws + (gdn_chunk_slot(t0, seq, 0) * P_HV + h) * C_SLOT_BYTES;
+
+  // thread: 16-byte piece tid % 16 of rows tid / 16 + 8 i of k and q; of v piece tid % 8, rows tid / 8 + 16 i
+  const __nv_bfloat16* kp = k + ((t0 + (tid >> 4)) * P_HQ + hq) * P_D + (tid & 15) * 8;
+  const __nv_bfloat16* qp = q + ((t0 + (tid >> 4)) * P_HQ + hq) * P_D + (tid & 15) * 8;
+  const __nv_bfloat16* vp = v + ((t0 + (tid >> 3)) * P_HV + h) * P_D + half * CW_ROWS + (tid & 7) * 8;
+  auto load_inputs = [&](int c) {
+    const uint32_t st = sm + (c & 1) * CW_STAGE;
+    const int left = len - c * C_TOK;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = (tid >> 4) + 8 * i;
+      const bool valid = row < left;
+      const uint32_t dst = st + row * 256 + (((tid & 15) ^ (row & 7)) << 4);
+      ako::cp_async16(dst, valid ? kp + i * (8 * P_HQ * P_D) : k, valid);
+      ako::cp_async16(dst + CW_OFF_Q, valid ? qp + i * (8 * P_HQ * P_D) : q, valid);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int row = (tid >> 3) + 16 * i;
+      const bool valid = row < left;
+      ako::cp_async16(st + CW_OFF_V + row * CW_V_PITCH + (tid & 7) * 16, valid ? vp + i * (16 * P_HV * P_D) : v, valid);
+    }
+    kp += C_TOK * P_HQ * P_D;
+    qp += C_TOK * P_HQ * P_D;
+    vp += C_TOK * P_HV * P_D;
+  };
+  auto load_slot = [&](int c) {
+    copy_group<C_SLOT_BYTES>(sm + (c & 1) * CW_STAGE + CW_OFF_SLOT, slot, tid);
+    slot += P_HV * C_SLOT_BYTES;
+  };
+  if (chunks > 0) load_inputs(0);
+
+  // the warp's rows of the state: g, g + 8 of its 16, columns 8 n + 2 t, + 1
+  const int64_t srow = (((int64_t)seq * P_HV + h) * P_D + half * CW_ROWS + w * 16 + g) * P_D + 2 * t;
+  float S[16][4];
+#pragma unroll
+  for (int n = 0; n < 16; ++n) {
+    float2 x = make_float2(0.f, 0.f), y = x;
+    if (state != nullptr && len > 0) {   // the definition leaves the new state of an empty sequence at zero
+      x = __ldcs(reinterpret_cast<const float2*>(state + srow + 8 * n));
+      y = __ldcs(reinterpret_cast<const float2*>(state + srow + 8 * P_D + 8 * n));
+    }
+    S[n][0] = x.x; S[n][1] = x.y; S[n][2] = y.x; S[n][3] = y.y;
+  }
+  __nv_bfloat16* out_h = out + h * P_D + half * CW_ROWS;
+  // tokens outside every sequence: zero, by the CTAs of the first and of the last sequence
+  for (int side = 0; side < 2; ++side) {
+    if (seq != (side ? (int)gridDim.z - 1 : 0)) continue;
+    const int64_t z0 = side ? max(t1, (int64_t)0) : 0, z1 = side ? total_tokens : min(t0, total_tokens);
+    for (int64_t i = z0 * 8 + tid; i < z1 * 8; i += 128)
+      *reinterpret_cast<uint4*>(out_h + (i >> 3) * (P_HV * P_D) + (i & 7) * 8) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  out_h += t0 * (P_HV * P_D) + w * 16;
+  ako::pdl_wait();   // T, P and the coefficients come from the kernel in front
+  if (chunks > 0) load_slot(0);
+  ako::cp_async_commit();
+
+  for (int c = 0; c < chunks; ++c) {
+    ako::cp_async_wait<0>();
+    __syncthreads();               // chunk c is here; nobody reads the other stage any more
+    if (c + 1 < chunks) {
+      load_inputs(c + 1);
+      load_slot(c + 1);
+    }
+    ako::cp_async_commit();
+    const uint32_t st = sm + (c & 1) * CW_STAGE;
+    const unsigned char* stage = smem + (c & 1) * CW_STAGE;
+    const uint2* sT = reinterpret_cast<const uint2*>(stage + CW_OFF_SLOT) + lane;
+    const uint2* sP = sT + C_FRAG_BYTES / 8;
+    const float* coef = reinterpret_cast<const float*>(stage + CW_OFF_SLOT + 2 * C_FRAG_BYTES);
+
+    // 1. S0 k and S0 q, four token tiles each
+    float x[4][4], y[4][4];
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      uint32_t As[3][4], bk[8], bq[8];
+      tile_pieces(As, 0, S[2 * ks]);
+      tile_pieces(As, 1, S[2 * ks + 1]);
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const int row = p * 16 + (lane & 7) + ((lane >> 4) << 3);
+        const uint32_t a = st + row * 256 + (((2 * ks + ((lane >> 3) & 1)) ^ (row & 7)) << 4);
+        ako::ldmatrix_x4(bk[4 * p], bk[4 * p + 1], bk[4 * p + 2], bk[4 * p + 3], a);
+        ako::ldmatrix_x4(bq[4 * p], bq[4 * p + 1], bq[4 * p + 2], bq[4 * p + 3], a + CW_OFF_Q);
+      }
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+          if (ks == 0 && p == 0) {
+            mma_zero(x[n], As[0], bk[2 * n], bk[2 * n + 1]);
+            mma_zero(y[n], As[0], bq[2 * n], bq[2 * n + 1]);
+          } else {
+            ako::mma_bf16_16816(x[n], As[p], bk[2 * n], bk[2 * n + 1]);
+            ako::mma_bf16_16816(y[n], As[p], bq[2 * n], bq[2 * n + 1]);
+          }
+        }
+    }
+    // 2. right-hand side v - gam (S0 k), and what S0 adds to the outputs
+#pragma unroll
+    for (int m = 0; m < 4; m += 2) {
+      uint32_t vt[4];                  // tokens 8 m .., rows 0-7 and 8-15; then tokens 8 m + 8 ..
+      ako::ldmatrix_x4_trans(vt[0], vt[1], vt[2], vt[3],
+                             st + CW_OFF_V + (8 * m + (lane & 7) + ((lane >> 4) << 3)) * CW_V_PITCH + w * 32 + ((lane >> 3) & 1) * 16);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float2 gam = *reinterpret_cast<const float2*>(coef + 8 * (m + u) + 2 * t);
+        float(&xr)[4] = x[m + u];
+        float(&yr)[4] = y[m + u];
+        xr[0] = ako::bf16_lo(vt[2 * u]) - gam.x * xr[0];
+        xr[1] = ako::bf16_hi(vt[2 * u]) - gam.y * xr[1];
+        xr[2] = ako::bf16_lo(vt[2 * u + 1]) - gam.x * xr[2];
+        xr[3] = ako::bf16_hi(vt[2 * u + 1]) - gam.y * xr[3];
+        yr[0] *= scale * gam.x; yr[1] *= scale * gam.y; yr[2] *= scale * gam.x; yr[3] *= scale * gam.y;
+      }
+    }
+    // 3. delta = T (right-hand side), tile by tile
+    float d[4][4];
+    {
+      uint32_t A[2][3][4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) tile_pieces(A[n >> 1], n & 1, x[n]);
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        float d1[4];
+#pragma unroll
+        for (int s = 0; s <= n / 2; ++s) {
+          const uint2* f = sT + gdn_frag_tile(n, s) * 96;
+          const uint2 B[3] = {f[0], f[32], f[64]};
+          if (s == 0) mma_6<true>(d[n], d1, A[s], B);
+          else mma_6<false>(d[n], d1, A[s], B);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[n][i] += d1[i];
+      }
+    }
+    // 4. outputs
+    {
+      uint32_t A[2][3][4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) tile_pieces(A[n >> 1], n & 1, d[n]);
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        float o1[4];
+#pragma unroll
+        for (int s = 0; s <= n / 2; ++s) {
+          const uint2* f = sP + gdn_frag_tile(n, s) * 96;
+          const uint2 B[3] = {f[0], f[32], f[64]};
+          if (s == 0) {
+            ako::mma_bf16_16816(y[n], A[0][0], B[0].x, B[0].y);
+            mma_zero(o1, A[0][1], B[0].x, B[0].y);
+            ako::mma_bf16_16816(y[n], A[0][0], B[1].x, B[1].y);
+            ako::mma_bf16_16816(o1, A[0][2], B[0].x, B[0].y);
+            ako::mma_bf16_16816(y[n], A[0][1], B[1].x, B[1].y);
+            ako::mma_bf16_16816(o1, A[0][0], B[2].x, B[2].y);
+          } else {
+            mma_6<false>(y[n], o1, A[s], B);
+          }
+        }
+        // transposed across the warp: lane (g, t) gets token g, rows 2t, 2t+1 (and + 8)
+        const uint32_t y0 = movmatrix_trans(ako::pack_bf16x2(y[n][0] + o1[0], y[n][1] + o1[1]));
+        const uint32_t y1 = movmatrix_trans(ako::pack_bf16x2(y[n][2] + o1[2], y[n][3] + o1[3]));
+        if (c * C_TOK + 8 * n + g < len) {
+          uint32_t* op = reinterpret_cast<uint32_t*>(out_h + (int64_t)(c * C_TOK + 8 * n + g) * (P_HV * P_D)) + t;
+          op[0] = y0;
+          op[4] = y1;
+        }
+      }
+    }
+    // 5. the state at the end of the chunk
+    {
+      uint32_t A[2][3][4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const float2 dec = *reinterpret_cast<const float2*>(coef + C_TOK + 8 * n + 2 * t);
+        const float e[4] = {d[n][0] * dec.x, d[n][1] * dec.y, d[n][2] * dec.x, d[n][3] * dec.y};
+        tile_pieces(A[n >> 1], n & 1, e);
+      }
+      const float gC = coef[C_TOK - 1];
+#pragma unroll
+      for (int n = 0; n < 16; n += 2) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          S[n][i] *= gC;
+          S[n + 1][i] *= gC;
+        }
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          uint32_t bf[4];
+          const int row = 16 * s + (lane & 15);
+          ako::ldmatrix_x4_trans(bf[0], bf[1], bf[2], bf[3], st + row * 256 + (((n + (lane >> 4)) ^ (row & 7)) << 4));
+#pragma unroll
+          for (int p = 0; p < 3; ++p) {
+            ako::mma_bf16_16816(S[n], A[s][p], bf[0], bf[1]);
+            ako::mma_bf16_16816(S[n + 1], A[s][p], bf[2], bf[3]);
+          }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < 16; ++n) {
+    __stcs(reinterpret_cast<float2*>(new_state + srow + 8 * n), make_float2(S[n][0], S[n][1]));
+    __stcs(reinterpret_cast<float2*>(new_state + srow + 8 * P_D + 8 * n), make_float2(S[n][2], S[n][3]));
+  }
+}

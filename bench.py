@@ -405,7 +405,7 @@ def ops_table(peaks, calls=15, only=None):
             T, n = sum(lens), len(lens)
             add("gdn_prefill", f"seqs={n}x{lens[0]}", us, bytes_=T * (2 * 1024 + 2 * 2048 + 32) + n * 8 * 2 * 65536,
                 flops=T * 8 * 128 * 128 * 6, bound="latency",
-                note="token-sequential recurrence, rows in parallel; not the chunked form", e2e=e2e)
+                note="chunked recurrence, fp32 as bf16 pieces on mma.sync", e2e=e2e)
             del a
 
     def _gemm():

@@ -98,7 +98,7 @@ def test_long_sequences_sampled():
 
 
 @pytest.mark.parametrize("lens,lead,tail", [([31, 32, 33], 0, 0), ([1, 64, 0, 65, 2], 5, 9), ([96], 33, 1), ([0, 0, 7], 3, 0),
-                                            ([40] * 70, 0, 40)])
+                                            ([40] * 70, 0, 40), ([31, 32, 33, 1, 0, 64, 65] * 3, 2, 3)])
 def test_chunk_edges_and_tokens_outside(lens, lead, tail):
     """Sequences that end at, before and after a 32-token chunk, empty ones, more sequences than the
     slot search takes per step, and tokens in front of and behind every sequence (their outputs are
