@@ -1,37 +1,37 @@
 // Paged GQA decode: 32 query heads, 8 KV heads, head_dim 128, bf16.
 //
-// HBM-bound: every KV token costs 4096 bytes (8 heads x 128 x bf16 for K and again for V) and
-// only 4 query rows reuse it. One CTA owns (sequence, KV split, half of the KV heads): its 4
-// warps each run flash-decoding for one KV head (the 4 query heads of that group padded to an
-// m16 tile of mma.sync) over a 3-stage ring of 16-token tiles. A token's four K heads are 1 KB
-// contiguous in the cache, so the gather is ONE 1 KB bulk copy (cp.async.bulk, completion counted
-// in bytes on the stage's mbarrier) per token per tensor, issued by 16 lanes of warp 0; 16-byte
-// cp.async copies run out of outstanding-request slots long before HBM is busy. Gather indices are
-// fetched one tile ahead of the copies that need them. Rows sit in shared memory with a 1040-byte
-// pitch, which keeps ldmatrix bank-conflict free without a swizzle. Partials (m, l, acc) go to the
-// workspace in fp32 and a second kernel merges them; with one split the CTA writes o and lse
-// itself. Waits on the mbarriers are bounded: a wait that exceeds its cycle limit records a code in
-// a device status word and the CTA stops consuming.
-#include "lse_merge.cuh"
-#include "tcgen05.cuh"
+// HBM-bound: every KV token costs 4096 bytes (8 heads x 128 x bf16 for K and again for V) and only 4
+// query rows reuse it. With page size 1 a token is a random row of the cache, so the kernel is a gather:
+// a copy-only probe on B200 reaches 6.4 TB/s with 16-byte register loads (64 contiguous bytes of a row
+// per quad of lanes), against 5.4 TB/s with the 1 KB bulk copies that this kernel used before. So
+// nothing is staged: a warp's loads ARE its mma operands, there is no barrier and no shared memory in
+// the loop, and a dozen independent warps per SM keep the loads of 6 to 8 KB each in flight.
+//   * A warp owns one KV head (a CTA: four neighbouring ones of the same tokens, 1 KB of a cache row).
+//     Lane (g, t) loads the 16-byte pieces t + 4 j of K of tokens g and g + 8: the A fragments of
+//     m16n8k16 with tokens as M, over a permuted order of the reduction in which Q's B fragments are
+//     loaded too. S^T = K Q^T is [16 tokens x 8 heads], four of them real.
+//   * V is loaded the same way; movmatrix turns an 8 x 8 block of pairs into the A fragment of
+//     O^T = V^T P^T ([128 x 8 heads], features as M), and P's own pairs into the B fragment.
+//   * K of the next tile is requested when S has been computed, V of it when O has.
+//
+// Work split: flat_share.cuh, tiles of 16 tokens, one share per pair of CTAs (the two halves of the KV
+// heads); a second kernel merges the partials of rows that several shares touch. Measured (whole call,
+// bulk copies through shared memory and a planning kernel before -> now): 64 sequences of up to 8 192 tokens
+// 245 -> 188 us (6.3 TB/s = 0.96 of the measured copy bandwidth), 256 of them 841 -> 680 (0.99), 16 of up to
+// 1 200 25 -> 17, one of 547 12.6 -> 10.2 us.
+#include "flat_share.cuh"
 
 namespace {
 
 constexpr int HQ = 32, HKV = 8, D = 128, GROUP = HQ / HKV;
-constexpr int HPC = 4;        // KV heads per CTA (one per warp); 8 (2 KB rows, one CTA per SM) measured the same
-constexpr int HEAD_GROUPS = HKV / HPC;  // CTAs that share one (sequence, split)
-constexpr int CTAS_PER_SM = (HPC == 4) ? 2 : 1;
-constexpr int TILE = 16;      // tokens per pipeline stage
-constexpr int STAGES = 3;
+constexpr int HPC = 4;                    // KV heads per CTA, one per warp
+constexpr int HALVES = HKV / HPC;         // CTAs per share
+constexpr int TILE = 16;                  // tokens per tile
 constexpr int THREADS = HPC * 32;
-constexpr int ROW_BYTES = HPC * D * 2;            // 1024: the CTA's heads of one token, one tensor
-constexpr int PITCH = ROW_BYTES + 16;             // shared-memory row pitch
-constexpr int TENSOR_TILE_BYTES = TILE * PITCH;   // 16640
-constexpr int STAGE_BYTES = 2 * TENSOR_TILE_BYTES;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES;  // 99840 -> two CTAs per SM
-constexpr int MAX_SPLITS = 64;
+constexpr int CTAS_PER_SM = 3;
+constexpr int ROW_BYTES = HKV * D * 2;    // one token of K (or V)
 
-__device__ int g_gqa_status = 0;  // 0 = ok; set when a bounded wait gave up
+__device__ int g_gqa_status = 0;          // no wait of this kernel can give up: stays 0
 
 struct Params {
   const __nv_bfloat16* q;
@@ -41,380 +41,324 @@ struct Params {
   const int32_t* indices;
   __nv_bfloat16* o;
   float* lse;
-  float* part_acc;  // [batch*32][splits][128]
-  float* part_ml;   // [batch*32][splits][2]
+  float* part_acc;  // [slot][32][128]
+  float* part_ml;   // [slot][32][2]
+  int32_t* prefix;  // [batch + 1] tiles in front of a sequence
   float scale_log2;
   int page_size;
-  int num_splits;       // uniform mode: every sequence is cut into this many chunks
-  // work-list mode (items != nullptr): chunks of `chunk_tokens` tokens; item i = (sequence, chunk
-  // ordinal) or (-1, -1); partials are indexed by item, item_start[b] .. item_start[b+1] are the
-  // items of sequence b.
-  const int2* items;
-  int chunk_tokens;
+  int batch;
+  bool whole_rows;  // a share is one sequence
 };
 
-__global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gqa_decode_kernel(Params p) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) uint64_t s_full[STAGES];
-  __shared__ int s_err;  // code of a wait of this CTA that gave up (0 = none), published on exit
+__device__ __forceinline__ int seq_tokens(const Params& p, int b) {
+  return max(0, p.indptr[b + 1] - p.indptr[b]) * p.page_size;
+}
+__device__ __forceinline__ uint4 ld_row16(const unsigned char* p) {
+  uint4 r;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
+  uint32_t y;
+  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(y) : "r"(x));
+  return y;
+}
 
-  int split, half, b, item = 0;
-  if (p.items) {
-    ako::pdl_wait();  // the work list is written by the planning kernel launched just before
-    item = blockIdx.x / HEAD_GROUPS;
-    half = blockIdx.x % HEAD_GROUPS;
-    const int2 it = p.items[item];
-    b = it.x;
-    split = it.y;
-    if (b < 0) return;  // unused slot of the worst-case grid
-  } else {
-    split = blockIdx.x % p.num_splits;
-    half = (blockIdx.x / p.num_splits) % HEAD_GROUPS;
-    b = blockIdx.x / (p.num_splits * HEAD_GROUPS);
-  }
+__global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gqa_decode_kernel(Params p) {
+  __shared__ int s_scan[6];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int head0 = half * HPC;
-  const int kvh = head0 + warp;
-  const uint32_t smem_base = ako::smem_u32(smem);
-
+  const int half = blockIdx.x % HALVES, share = blockIdx.x / HALVES;
+  const int kvh = half * HPC + warp;
   ako::pdl_trigger();  // the merge kernel may be scheduled early; it waits for this grid to finish
-  const int32_t* idx = p.indices + p.indptr[b];
-  const int len = (int)(p.indptr[b + 1] - p.indptr[b]) * p.page_size;
-  int chunk = p.items ? p.chunk_tokens : (int)ako::round_up(ako::cdiv(len, p.num_splits), TILE);
-  if (chunk < TILE) chunk = TILE;
-  const int tok_begin = min(len, split * chunk);
-  const int tok_end = min(len, tok_begin + chunk);
-  const int ntiles = (tok_end - tok_begin + TILE - 1) / TILE;
+  auto seq_tiles = [&](int b) { return (seq_tokens(p, b) + TILE - 1) / TILE; };
+  ako::Share sh;
+  if (p.whole_rows) {
+    sh = {share, 0, seq_tiles(share)};
+    if (sh.left == 0) {                              // an empty sequence
+      const int64_t h0 = (int64_t)share * HQ + kvh * GROUP;
+      uint4* op = reinterpret_cast<uint4*>(p.o + h0 * D);
+      for (int i = lane; i < GROUP * D / 8; i += 32) op[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (lane < GROUP) p.lse[h0 + lane] = -INFINITY;
+    }
+  } else {
+    sh = ako::find_share(p.batch, share, gridDim.x / HALVES, blockIdx.x == 0, p.prefix, s_scan, seq_tiles);
+  }
 
-  if (ntiles == 0 && (p.num_splits > 1 || p.items)) {
-    // Nothing in this chunk (the sequence is shorter than split * chunk, or empty): an empty
-    // partial, which the merge skips without reading the accumulator.
-    if (g < GROUP && t == 0) {
-      float* ml = p.part_ml + (p.items ? ((int64_t)item * HQ + kvh * GROUP + g)
-                                       : (((int64_t)b * HQ + kvh * GROUP + g) * p.num_splits + split)) * 2;
-      ml[0] = -INFINITY;
-      ml[1] = 0.f;
+  int b = sh.row, ts = sh.skip;
+  while (sh.left > 0) {
+    const int32_t* idx = p.indices + p.indptr[b];
+    const int len = seq_tokens(p, b);
+    const int tiles = (len + TILE - 1) / TILE;
+    const int te = min(tiles, ts + sh.left);
+    if (te <= ts) {                                  // an empty sequence
+      ++b;
+      ts = 0;
+      continue;
+    }
+    sh.left -= te - ts;
+
+    // this lane's two tokens of a tile: byte offset of its pieces in the caches
+    int32_t id[2];
+    auto fetch_ids = [&](int tile) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int tok = min(tile * TILE + 8 * i + g, len - 1);   // past the end: a valid row, masked below
+        id[i] = __ldg(idx + (p.page_size == 1 ? tok : tok / p.page_size));
+      }
+    };
+    int64_t off[2];
+    auto locate = [&](int tile) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        int64_t row = id[i];
+        if (p.page_size != 1) row = row * p.page_size + min(tile * TILE + 8 * i + g, len - 1) % p.page_size;
+        off[i] = row * ROW_BYTES + kvh * (D * 2) + t * 16;
+      }
+    };
+    uint4 kc[2][4], vc[2][4];
+    auto load = [&](uint4 (&x)[2][4], const unsigned char* base) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) x[i][j] = ld_row16(base + off[i] + 64 * j);
+    };
+    fetch_ids(ts);
+    locate(ts);
+    load(kc, p.k);
+    load(vc, p.v);
+    fetch_ids(ts + 1);
+
+    // Q of the four heads as B fragments (n = head g, heads 4-7 are zero), in the order of the K pieces
+    uint4 qb[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      qb[j] = make_uint4(0u, 0u, 0u, 0u);
+      if (g < GROUP)
+        qb[j] = __ldg(reinterpret_cast<const uint4*>(p.q + ((int64_t)b * HQ + kvh * GROUP + g) * D + 32 * j + 8 * t));
+    }
+    float acc[4][2][4];   // [block j][u]: features 32 j + 8 (g / 2) + (g & 1) + 4 u (regs 0, 1) and + 2 (2, 3), heads 2t, 2t+1
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[j][u][i] = 0.f;
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;   // heads 2t, 2t+1; l over this lane's tokens
+
+    for (int tile = ts; tile < te; ++tile) {
+      float s[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t a0[4] = {kc[0][j].x, kc[1][j].x, kc[0][j].y, kc[1][j].y};
+        const uint32_t a1[4] = {kc[0][j].z, kc[1][j].z, kc[0][j].w, kc[1][j].w};
+        ako::mma_bf16_16816(s, a0, qb[j].x, qb[j].y);
+        ako::mma_bf16_16816(s2, a1, qb[j].z, qb[j].w);
+      }
+      const bool more = tile + 1 < te;
+      if (more) {
+        locate(tile + 1);
+        load(kc, p.k);
+      }
+      // softmax over the tokens: rows g and g + 8 of this lane, 8 lanes apart by 4
+      const bool v0 = tile * TILE + g < len, v1 = tile * TILE + 8 + g < len;
+      s[0] = v0 ? (s[0] + s2[0]) * p.scale_log2 : -INFINITY;
+      s[1] = v0 ? (s[1] + s2[1]) * p.scale_log2 : -INFINITY;
+      s[2] = v1 ? (s[2] + s2[2]) * p.scale_log2 : -INFINITY;
+      s[3] = v1 ? (s[3] + s2[3]) * p.scale_log2 : -INFINITY;
+      float n0 = fmaxf(s[0], s[2]), n1 = fmaxf(s[1], s[3]);
+#pragma unroll
+      for (int o = 4; o <= 16; o <<= 1) {
+        n0 = fmaxf(n0, __shfl_xor_sync(0xffffffffu, n0, o));
+        n1 = fmaxf(n1, __shfl_xor_sync(0xffffffffu, n1, o));
+      }
+      if (__any_sync(0xffffffffu, n0 > m0 || n1 > m1)) {   // every tile holds at least one valid token: finite
+        n0 = fmaxf(n0, m0);
+        n1 = fmaxf(n1, m1);
+        const float f0 = ako::fast_exp2(m0 - n0), f1 = ako::fast_exp2(m1 - n1);
+        m0 = n0;
+        m1 = n1;
+        l0 *= f0;
+        l1 *= f1;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            acc[j][u][0] *= f0; acc[j][u][1] *= f1; acc[j][u][2] *= f0; acc[j][u][3] *= f1;
+          }
+      }
+      s[0] = ako::fast_exp2(s[0] - m0);
+      s[1] = ako::fast_exp2(s[1] - m1);
+      s[2] = ako::fast_exp2(s[2] - m0);
+      s[3] = ako::fast_exp2(s[3] - m1);
+      l0 += s[0] + s[2];
+      l1 += s[1] + s[3];
+      const uint32_t b0 = movmatrix_trans(ako::pack_bf16x2(s[0], s[1])), b1 = movmatrix_trans(ako::pack_bf16x2(s[2], s[3]));
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t a0[4] = {movmatrix_trans(vc[0][j].x), movmatrix_trans(vc[0][j].y), movmatrix_trans(vc[1][j].x), movmatrix_trans(vc[1][j].y)};
+        const uint32_t a1[4] = {movmatrix_trans(vc[0][j].z), movmatrix_trans(vc[0][j].w), movmatrix_trans(vc[1][j].z), movmatrix_trans(vc[1][j].w)};
+        ako::mma_bf16_16816(acc[j][0], a0, b0, b1);
+        ako::mma_bf16_16816(acc[j][1], a1, b0, b1);
+      }
+      if (more) {
+        load(vc, p.v);
+        fetch_ids(tile + 2);
+      }
+    }
+
+#pragma unroll
+    for (int o = 4; o <= 16; o <<= 1) {
+      l0 += __shfl_xor_sync(0xffffffffu, l0, o);
+      l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+    }
+    // lanes g = 2 x, 2 x + 1 hold the even and the odd of features 32 j + 8 x .. + 7: swap so that the
+    // even lane has the first four and the odd lane the last four
+    const bool whole = te - ts == tiles;
+    const float i0 = (whole && l0 > 0.f) ? 1.f / l0 : 1.f, i1 = (whole && l1 > 0.f) ? 1.f / l1 : 1.f;
+    const bool odd = g & 1;
+    const int64_t slot = (int64_t)b + share;
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      const int head = kvh * GROUP + 2 * t + hh;
+      const float inv = hh ? i1 : i0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float a = acc[j][0][hh] * inv, c = acc[j][0][2 + hh] * inv, e = acc[j][1][hh] * inv, f = acc[j][1][2 + hh] * inv;
+        const float r0 = __shfl_xor_sync(0xffffffffu, odd ? a : e, 4), r1 = __shfl_xor_sync(0xffffffffu, odd ? c : f, 4);
+        const float4 x = odd ? make_float4(r0, e, r1, f) : make_float4(a, r0, c, r1);
+        if (t < 2) {
+          const int col = 32 * j + 8 * (g >> 1) + 4 * (g & 1);
+          if (whole)
+            *reinterpret_cast<uint2*>(p.o + ((int64_t)b * HQ + head) * D + col) =
+                make_uint2(ako::pack_bf16x2(x.x, x.y), ako::pack_bf16x2(x.z, x.w));
+          else
+            *reinterpret_cast<float4*>(p.part_acc + (slot * HQ + head) * D + col) = x;
+        }
+      }
+      if (t < 2 && g == 0) {
+        const float m = hh ? m1 : m0, l = hh ? l1 : l0;
+        if (whole)
+          p.lse[(int64_t)b * HQ + head] = (l > 0.f) ? m + log2f(l) : -INFINITY;
+        else
+          *reinterpret_cast<float2*>(p.part_ml + (slot * HQ + head) * 2) = make_float2(m, l);
+      }
+    }
+    ++b;
+    ts = 0;
+  }
+}
+
+// Merge: WARPS warps per (sequence, head), every warp 32 threads x 4 columns of every WARPS-th partial;
+// a block holds four heads (WARPS = 1) or one (WARPS = 8: few sequences with many partials each, where
+// one warp would walk up to 222 partials in a row). The partials of sequence b are the slots b + c of
+// the shares c that touch it; a sequence inside one share is already written, an empty one gets its
+// zeros here.
+constexpr int MERGE_MAX = 512;                       // shares of a call never exceed this (three CTAs per SM)
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS == 1 ? 128 : WARPS * 32) gqa_merge_kernel(Params p, int shares) {
+  constexpr int HEADS = (WARPS == 1) ? 4 : 1;
+  __shared__ float s_w[HEADS][MERGE_MAX];
+  __shared__ float4 s_acc[WARPS][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int b = blockIdx.x / (HQ / HEADS), hl = (WARPS == 1) ? w : 0, part = (WARPS == 1) ? 0 : w;
+  const int head = (blockIdx.x % (HQ / HEADS)) * HEADS + hl;
+  ako::pdl_wait();
+  const int t0 = p.prefix[b], t1 = p.prefix[b + 1], total = p.prefix[p.batch];
+  const int64_t oi = (int64_t)b * HQ + head;
+  uint2* op = reinterpret_cast<uint2*>(p.o + oi * D) + lane;
+  if (t1 <= t0) {
+    if (part == 0) {
+      *op = make_uint2(0u, 0u);
+      if (lane == 0) p.lse[oi] = -INFINITY;
     }
     return;
   }
-  // Shared memory starts finite: rows of tokens past the end are never copied, and 0 * stale
-  // must not be NaN in the PV product.
-  for (int i = threadIdx.x; i < SMEM_BYTES / 16; i += THREADS) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) ako::tc::mbar_init(ako::smem_u32(&s_full[s]), 1);
-    ako::tc::mbar_init_fence();
-    s_err = 0;
+  const int per = (total + shares - 1) / shares;
+  const int c0 = t0 / per, n = (t1 - 1) / per - c0 + 1;
+  if (n == 1) return;
+  const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + ((int64_t)(b + c0) * HQ + head);
+  const float4* pa = reinterpret_cast<const float4*>(p.part_acc + ((int64_t)(b + c0) * HQ + head) * D) + lane;
+  // every warp of the head finds the maximum over all partials for itself
+  float2 mine[MERGE_MAX / 32];
+  float M = -INFINITY, L = 0.f;
+#pragma unroll
+  for (int i = 0; i < MERGE_MAX / 32; ++i) {
+    mine[i] = make_float2(-INFINITY, 0.f);
+    if (i * 32 < n && i * 32 + lane < n) mine[i] = ml[(int64_t)(i * 32 + lane) * HQ];
+    M = fmaxf(M, mine[i].x);
   }
-  ako::tc::fence_proxy_async_smem();  // the zero fill is ordered before the bulk copies
-  __syncthreads();
-
-  // ---- producer state (warp 0, lanes 0..15: one token of a tile each) ------------------------
-  const int64_t head_off = (int64_t)head0 * D * 2;
-  // The page id of this lane's token in the next tile to be issued is loaded one iteration early
-  // and only LOADED there: nothing depends on it until issue_tile, so warp 0 never stalls on the
-  // index fetch in front of the barrier the other warps wait at.
-  int32_t page_next = 0;
-  auto fetch_row = [&](int tile) {
-    int tok = tok_begin + tile * TILE + lane;
-    tok = min(tok, max(tok_end - 1, 0));  // a valid address even when this lane has no token
-    if (len > 0) page_next = __ldg(idx + (p.page_size == 1 ? tok : tok / p.page_size));
-  };
-  auto issue_tile = [&](int tile) {  // uses page_next fetched for `tile`
-    const int stage = tile % STAGES;
-    const uint32_t bar = ako::smem_u32(&s_full[stage]);
-    const int tok = tok_begin + tile * TILE + lane;
-    const bool valid = lane < TILE && tok < tok_end;
-    const int64_t row_next = (p.page_size == 1) ? (int64_t)page_next
-                                                : (int64_t)page_next * p.page_size + tok % p.page_size;
-    const unsigned m = __ballot_sync(0xffffffffu, valid);
-    if (lane == 0) ako::tc::mbar_arrive_expect_tx(bar, (uint32_t)__popc(m) * 2 * ROW_BYTES);
-    __syncwarp();
-    if (valid) {
-      const uint32_t dst = smem_base + stage * STAGE_BYTES + lane * PITCH;
-      const int64_t src = row_next * (HKV * D * 2) + head_off;
-      ako::tc::bulk_load_1d(dst, p.k + src, ROW_BYTES, bar);
-      ako::tc::bulk_load_1d(dst + TENSOR_TILE_BYTES, p.v + src, ROW_BYTES, bar);
-    }
-  };
-  if (warp == 0) {
-    for (int s = 0; s < STAGES - 1; ++s) {
-      if (s < ntiles) {
-        fetch_row(s);
-        issue_tile(s);
-      }
-    }
-    fetch_row(STAGES - 1);
-  }
-
-  // Q fragments of this warp's group (rows g<4 real, others zero).
-  uint32_t qa[8][2];
-  {
-    const __nv_bfloat16* qrow = p.q + ((int64_t)b * HQ + kvh * GROUP + (g & 3)) * D;
 #pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      uint32_t v0 = *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 2 * t);
-      uint32_t v1 = *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 8 + 2 * t);
-      qa[ks][0] = (g < GROUP) ? v0 : 0u;
-      qa[ks][1] = (g < GROUP) ? v1 : 0u;
-    }
-  }
-
-  float oacc[16][4];
+  for (int o = 16; o >= 1; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
 #pragma unroll
-  for (int i = 0; i < 16; ++i) oacc[i][0] = oacc[i][1] = oacc[i][2] = oacc[i][3] = 0.f;
-  float m_run = -INFINITY, l_run = 0.f;
-
-  for (int it = 0; it < ntiles; ++it) {
-    const int stage = it % STAGES;
-    const bool landed = ako::tc::mbar_wait(ako::smem_u32(&s_full[stage]), (uint32_t)((it / STAGES) & 1),
-                                           &s_err, 1);
-    // every warp has finished tile it-1: its stage is free for tile it+STAGES-1
-    if (!__syncthreads_and(landed)) break;  // a wait gave up: the whole CTA stops consuming
-    if (warp == 0) {
-      ako::tc::fence_proxy_async_smem();  // generic reads of the freed stage before async writes
-      if (it + STAGES - 1 < ntiles) issue_tile(it + STAGES - 1);
-      fetch_row(it + STAGES);
+  for (int i = 0; i < MERGE_MAX / 32; ++i)
+    if (i * 32 < n) {
+      const float wgt = exp2f(mine[i].x - M);
+      if (part == 0 && i * 32 + lane < n) s_w[hl][i * 32 + lane] = wgt;
+      L = fmaf(mine[i].y, wgt, L);
     }
-    const uint32_t Ks = smem_base + stage * STAGE_BYTES + warp * (D * 2);
-    const uint32_t Vs = Ks + TENSOR_TILE_BYTES;
-
-    // S = Q K^T : 2 n-tiles of 8 tokens
-    float sacc[2][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) sacc[i][0] = sacc[i][1] = sacc[i][2] = sacc[i][3] = 0.f;
-    {
-      const int tok = ((lane >> 4) << 3) + (lane & 7);
-      const int csel = (lane >> 3) & 1;
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        uint32_t b00, b01, b10, b11;
-        ako::ldmatrix_x4(b00, b01, b10, b11, Ks + tok * PITCH + ((2 * ks + csel) << 4));
-        const uint32_t a[4] = {qa[ks][0], 0u, qa[ks][1], 0u};
-        ako::mma_bf16_16816(sacc[0], a, b00, b01);
-        ako::mma_bf16_16816(sacc[1], a, b10, b11);
-      }
-    }
-    // online softmax on row g (tokens: n-tile i, columns 2t, 2t+1)
-    const int tile_tok0 = tok_begin + it * TILE;
-    float mx = -INFINITY;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int tk = tile_tok0 + i * 8 + 2 * t + j;
-        float s = sacc[i][j] * p.scale_log2;
-        s = (tk < tok_end) ? s : -INFINITY;
-        sacc[i][j] = s;
-        mx = fmaxf(mx, s);
-      }
-    }
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    const float m_new = fmaxf(m_run, mx);  // finite: every tile holds at least one valid token
-    const float corr = ako::fast_exp2(m_run - m_new);
-    float psum = 0.f;
-    uint32_t pa[4];
-    {
-      const float p00 = ako::fast_exp2(sacc[0][0] - m_new), p01 = ako::fast_exp2(sacc[0][1] - m_new);
-      const float p10 = ako::fast_exp2(sacc[1][0] - m_new), p11 = ako::fast_exp2(sacc[1][1] - m_new);
-      psum = (p00 + p01) + (p10 + p11);
-      pa[0] = ako::pack_bf16x2(p00, p01);
-      pa[1] = 0u;
-      pa[2] = ako::pack_bf16x2(p10, p11);
-      pa[3] = 0u;
-    }
-    psum += __shfl_xor_sync(0xffffffffu, psum, 1);
-    psum += __shfl_xor_sync(0xffffffffu, psum, 2);
-    l_run = l_run * corr + psum;
-    m_run = m_new;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      oacc[i][0] *= corr;
-      oacc[i][1] *= corr;
-    }
-    // O += P V : 16 n-tiles of 8 dims, k = 16 tokens
-    {
-      const int tok = (((lane >> 3) & 1) << 3) + (lane & 7);
-      const int csel = lane >> 4;
-#pragma unroll
-      for (int nd = 0; nd < 16; nd += 2) {
-        uint32_t v00, v01, v10, v11;
-        ako::ldmatrix_x4_trans(v00, v01, v10, v11, Vs + tok * PITCH + ((nd + csel) << 4));
-        ako::mma_bf16_16816(oacc[nd], pa, v00, v01);
-        ako::mma_bf16_16816(oacc[nd + 1], pa, v10, v11);
-      }
-    }
-  }
-  if (threadIdx.x == 0 && s_err != 0) atomicCAS(&g_gqa_status, 0, s_err);
-
-  if (g < GROUP) {
-    const int64_t rh = (int64_t)b * HQ + kvh * GROUP + g;
-    if (p.num_splits == 1 && !p.items) {
-      const float inv = (l_run > 0.f) ? 1.f / l_run : 0.f;
-      __nv_bfloat16* op = p.o + rh * D;
-#pragma unroll
-      for (int nd = 0; nd < 16; ++nd)
-        *reinterpret_cast<uint32_t*>(op + nd * 8 + 2 * t) =
-            ako::pack_bf16x2(oacc[nd][0] * inv, oacc[nd][1] * inv);
-      if (t == 0) p.lse[rh] = (l_run > 0.f) ? m_run + log2f(l_run) : -INFINITY;
-    } else {
-      const int64_t pidx = p.items ? ((int64_t)item * HQ + kvh * GROUP + g) : (rh * p.num_splits + split);
-      float* pa_out = p.part_acc + pidx * D;
-#pragma unroll
-      for (int nd = 0; nd < 16; ++nd)
-        *reinterpret_cast<float2*>(pa_out + nd * 8 + 2 * t) = make_float2(oacc[nd][0], oacc[nd][1]);
-      if (t == 0) {
-        float* ml = p.part_ml + pidx * 2;
-        ml[0] = m_run;
-        ml[1] = l_run;
-      }
-    }
-  }
-}
-
-// Work list for ragged batches: sequence b is cut into max(1, ceil(len_b / chunk)) chunks of `chunk`
-// tokens, so every CTA has about the same work whatever the mix of lengths. One block.
-__global__ void __launch_bounds__(256) gqa_plan_kernel(const int32_t* __restrict__ indptr, int batch,
-                                                       int page_size, int chunk, int max_items,
-                                                       int32_t* __restrict__ item_start,
-                                                       int2* __restrict__ items) {
-  __shared__ int s_scan[256];
-  __shared__ int s_base;
-  const int tid = threadIdx.x;
-  if (tid == 0) s_base = 0;
-  __syncthreads();
-  for (int b0 = 0; b0 < batch; b0 += 256) {
-    const int b = b0 + tid;
-    int n = 0;
-    if (b < batch) {
-      const int len = (indptr[b + 1] - indptr[b]) * page_size;
-      n = max(1, (len + chunk - 1) / chunk);
-    }
-    s_scan[tid] = n;
-    __syncthreads();
-    for (int off = 1; off < 256; off <<= 1) {  // inclusive Hillis-Steele scan
-      const int add = (tid >= off) ? s_scan[tid - off] : 0;
-      __syncthreads();
-      s_scan[tid] += add;
-      __syncthreads();
-    }
-    const int start = s_base + s_scan[tid] - n;
-    if (b < batch) {
-      // kv_indptr[batch] beyond the num_kv_indices the workspace was sized for: the list is cut at
-      // max_items (those sequences lose their tail), the merge stays inside the partial area, and
-      // the status word records it.
-      item_start[b] = min(start, max_items);
-      for (int c = 0; c < n && start + c < max_items; ++c) items[start + c] = make_int2(b, c);
-    }
-    __syncthreads();
-    if (tid == 255) s_base += s_scan[255];
-    __syncthreads();
-  }
-  if (tid == 0) {
-    item_start[batch] = min(s_base, max_items);
-    if (s_base > max_items) atomicCAS(&g_gqa_status, 0, 20);
-  }
-  for (int i = s_base + tid; i < max_items; i += 256) items[i] = make_int2(-1, -1);
-}
-
-// Merge of the work-list partials: one block per (sequence, head); 32 threads x 4 columns.
-__global__ void __launch_bounds__(D / 4) gqa_merge_items_kernel(
-    const float* __restrict__ part_acc, const float* __restrict__ part_ml,
-    const int32_t* __restrict__ item_start, __nv_bfloat16* __restrict__ o, float* __restrict__ lse) {
-  ako::pdl_wait();
-  const int b = blockIdx.x / HQ, h = blockIdx.x % HQ;
-  const int i0 = item_start[b], i1 = item_start[b + 1];
-  float M = -INFINITY;
-  for (int i = i0; i < i1; ++i) M = fmaxf(M, part_ml[((int64_t)i * HQ + h) * 2]);
-  float L = 0.f;
+  if (WARPS == 1) __syncwarp();
+  else __syncthreads();
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (M > -INFINITY) {
-    for (int i = i0; i < i1; ++i) {
-      const float* ml = part_ml + ((int64_t)i * HQ + h) * 2;
-      if (ml[0] == -INFINITY) continue;
-      const float w = exp2f(ml[0] - M);
-      L = fmaf(ml[1], w, L);
-      const float4 p4 = *reinterpret_cast<const float4*>(part_acc + ((int64_t)i * HQ + h) * D + threadIdx.x * 4);
-      acc.x = fmaf(p4.x, w, acc.x);
-      acc.y = fmaf(p4.y, w, acc.y);
-      acc.z = fmaf(p4.z, w, acc.z);
-      acc.w = fmaf(p4.w, w, acc.w);
+#pragma unroll 8
+  for (int i = part; i < n; i += WARPS) {
+    const float wgt = s_w[hl][i];
+    const float4 x = pa[(int64_t)i * (HQ * D / 4)];
+    acc.x = fmaf(x.x, wgt, acc.x);
+    acc.y = fmaf(x.y, wgt, acc.y);
+    acc.z = fmaf(x.z, wgt, acc.z);
+    acc.w = fmaf(x.w, wgt, acc.w);
+  }
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+  if (WARPS > 1) {
+    s_acc[w][lane] = acc;
+    __syncthreads();
+    if (w != 0) return;
+#pragma unroll
+    for (int i = 1; i < WARPS; ++i) {
+      const float4 x = s_acc[i][lane];
+      acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
     }
   }
   const float inv = (L > 0.f) ? 1.f / L : 0.f;
-  uint2 pk;
-  pk.x = ako::pack_bf16x2(acc.x * inv, acc.y * inv);
-  pk.y = ako::pack_bf16x2(acc.z * inv, acc.w * inv);
-  *reinterpret_cast<uint2*>(o + (int64_t)blockIdx.x * D + threadIdx.x * 4) = pk;
-  if (threadIdx.x == 0) lse[blockIdx.x] = (L > 0.f) ? M + log2f(L) : -INFINITY;
+  *op = make_uint2(ako::pack_bf16x2(acc.x * inv, acc.y * inv), ako::pack_bf16x2(acc.z * inv, acc.w * inv));
+  if (lane == 0) p.lse[oi] = (L > 0.f) ? M + log2f(L) : -INFINITY;
 }
 
-// Work-list mode pays a third launch, so it is used where ragged lengths cost more than that:
-// batches that fill the GPU several times over with long sequences.
-struct Plan {
-  bool on;
-  int chunk;
-  int64_t max_items;
+// Whole sequences as shares, without partials and without the merge: batches that fill the GPU and are
+// short (at most 32 tiles) or many (four times as many sequences as shares fit at once).
+bool whole_rows(int64_t batch, int64_t num_kv_indices, int64_t page_size) {
+  const int64_t most = (int64_t)CTAS_PER_SM * ako::sm_count() / HALVES;
+  return batch >= 4 * most || (batch >= most && num_kv_indices * page_size <= batch * 512);
+}
+// Shares of a call: all CTAs resident at once, and at least one tile (16 tokens, 64 KB of K and V) each.
+int pick_shares(int64_t batch, int64_t num_kv_indices, int64_t page_size) {
+  if (whole_rows(batch, num_kv_indices, page_size)) return (int)batch;
+  const int64_t most = (int64_t)CTAS_PER_SM * ako::sm_count() / HALVES;
+  const int64_t tiles = ako::cdiv(num_kv_indices * page_size, (int64_t)TILE);   // at least; rows round up
+  int64_t s = tiles < most ? tiles : most;
+  if (s > MERGE_MAX) s = MERGE_MAX;
+  return (int)(s < 1 ? 1 : s);
+}
+struct Carve {
+  size_t acc, ml, total;   // offsets; the prefix table is first
 };
-Plan pick_plan(int64_t batch, int64_t num_kv_indices, int64_t page_size) {
-  Plan pl = {false, 0, 0};
-  if (batch <= 0) return pl;
-  const int64_t total = num_kv_indices * page_size;
-  const int64_t avg_len = total / batch;
-  const int64_t slots = 148 * CTAS_PER_SM;
-  if (avg_len < 1024 || total < 64 * 1024 || total / 256 * HEAD_GROUPS < 4 * slots) return pl;
-  // about six waves of equal chunks, at least 256 tokens each
-  int64_t chunk = ako::cdiv(total, 6 * slots / HEAD_GROUPS);
-  if (chunk < 256) chunk = 256;
-  chunk = ako::round_up(chunk, (int64_t)TILE);
-  const int64_t items = ako::cdiv(total, chunk) + batch;
-  if (chunk > 0x3fffffff || items * HEAD_GROUPS > 0x7fffffffLL) return pl;
-  pl.on = true;
-  pl.chunk = (int)chunk;
-  pl.max_items = items;
-  return pl;
-}
-size_t plan_workspace(const Plan& pl, int64_t batch) {
-  // partial accumulators, partial (m, l), item table, item_start
-  return (size_t)pl.max_items * HQ * (D + 2) * sizeof(float) + (size_t)pl.max_items * sizeof(int2) +
-         ((size_t)(batch + 1) * sizeof(int32_t) + 15) / 16 * 16;
-}
-
-int pick_splits(int64_t batch, int64_t num_kv_indices, int64_t page_size) {
-  if (batch <= 0) return 1;
-  const int64_t avg_len = num_kv_indices * page_size / batch;
-  const int64_t slots = 148 * CTAS_PER_SM;                      // resident CTAs
-  const int64_t pairs = HEAD_GROUPS * batch;                    // CTAs per split
-  // Long sequences: chunks of about 300 tokens. Every sequence of a batch gets the same split
-  // count, so with ragged lengths the longest chunks set the makespan; a sweep at B = 64 and 256
-  // (lengths U[128, 8192]) was best between 280 and 450 tokens per chunk and 5 % worse at 900.
-  // Short sequences: 128-token chunks, and at least two waves of CTAs when chunks of 128 allow it.
-  int64_t s = avg_len / (avg_len >= 2048 ? 300 : 128);
-  int64_t t = ako::cdiv(2 * slots, pairs);
-  if (t > avg_len / 128) t = avg_len / 128;
-  if (s < t) s = t;
-  if (s < 1) s = 1;
-  // A small batch that still leaves SMs idle: the call's latency is the chunk length, so go down
-  // to two 16-token tiles per chunk, up to one wave of CTAs.
-  if (pairs * s < slots) {
-    const int64_t fine = avg_len / (2 * TILE) > 1 ? avg_len / (2 * TILE) : 1;
-    const int64_t one_wave = slots / pairs > 1 ? slots / pairs : 1;
-    s = fine < one_wave ? fine : one_wave;
-  }
-  if (s > MAX_SPLITS) s = MAX_SPLITS;
-  return (int)s;
+Carve carve(int64_t batch, int shares) {
+  const size_t slots = (size_t)batch + (size_t)shares;
+  Carve c;
+  c.acc = (((size_t)batch + 1) * sizeof(int32_t) + 255) / 256 * 256;
+  c.ml = c.acc + slots * HQ * D * sizeof(float);
+  c.total = c.ml + slots * HQ * 2 * sizeof(float);
+  return c;
 }
 
 }  // namespace
 
 extern "C" size_t ako4x_gqa_paged_decode_workspace_bytes(int64_t batch, int64_t num_kv_indices,
                                                          int64_t page_size) {
-  const Plan pl = pick_plan(batch, num_kv_indices, page_size);
-  if (pl.on) return plan_workspace(pl, batch);
-  const int s = pick_splits(batch, num_kv_indices, page_size);
-  if (s == 1) return 0;
-  return (size_t)batch * HQ * s * (D + 2) * sizeof(float);
+  if (batch <= 0 || whole_rows(batch, num_kv_indices, page_size)) return 0;
+  return carve(batch, pick_shares(batch, num_kv_indices, page_size)).total;
 }
 
 extern "C" int ako4x_gqa_paged_decode(const void* q, const void* k_cache, const void* v_cache,
@@ -427,11 +371,14 @@ extern "C" int ako4x_gqa_paged_decode(const void* q, const void* k_cache, const 
   if (!q || !k_cache || !v_cache || !kv_indptr || !o || !lse) return AKO4X_EINVAL;
   if (num_kv_indices > 0 && !kv_indices) return AKO4X_EINVAL;
   if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)o) & 15) return AKO4X_EINVAL;
-  const Plan pl = pick_plan(batch, num_kv_indices, page_size);
-  const int splits = pl.on ? 1 : pick_splits(batch, num_kv_indices, page_size);
-  const size_t need = ako4x_gqa_paged_decode_workspace_bytes(batch, num_kv_indices, page_size);
-  if (need > 0 && (!workspace || workspace_bytes < need)) return AKO4X_EWORKSPACE;
-  if (need > 0 && ((uintptr_t)workspace & 15)) return AKO4X_EINVAL;
+  if (batch > 0x7fffffffLL / HQ || page_size > 0x7fffffffLL) return AKO4X_EINVAL;
+  const bool whole = whole_rows(batch, num_kv_indices, page_size);
+  const int shares = pick_shares(batch, num_kv_indices, page_size);
+  const Carve c = carve(batch, shares);
+  if (!whole) {
+    if (!workspace || workspace_bytes < c.total) return AKO4X_EWORKSPACE;
+    if ((uintptr_t)workspace & 15) return AKO4X_EINVAL;
+  }
   cudaStream_t st = (cudaStream_t)stream;
 
   Params p;
@@ -442,79 +389,26 @@ extern "C" int ako4x_gqa_paged_decode(const void* q, const void* k_cache, const 
   p.indices = kv_indices;
   p.o = (__nv_bfloat16*)o;
   p.lse = lse;
-  p.part_acc = (float*)workspace;
-  p.part_ml = p.part_acc ? p.part_acc + (size_t)batch * HQ * splits * D : nullptr;
+  p.prefix = (int32_t*)workspace;
+  p.part_acc = (float*)((unsigned char*)workspace + c.acc);
+  p.part_ml = (float*)((unsigned char*)workspace + c.ml);
   p.scale_log2 = sm_scale * AKO_LOG2E;
   p.page_size = (int)page_size;
-  p.num_splits = splits;
-  p.items = nullptr;
-  p.chunk_tokens = 0;
-
-  if (!ako::ensure_dynamic_smem<gqa_decode_kernel>(SMEM_BYTES)) return AKO4X_ELAUNCH;
-  if (pl.on) {
-    // workspace: [items][32][128] accumulators | [items][32][2] (m, l) | item table | item_start
-    p.part_ml = p.part_acc + (size_t)pl.max_items * HQ * D;
-    int2* items = reinterpret_cast<int2*>(p.part_ml + (size_t)pl.max_items * HQ * 2);
-    int32_t* item_start = reinterpret_cast<int32_t*>(items + pl.max_items);
-    p.items = items;
-    p.chunk_tokens = pl.chunk;
-    gqa_plan_kernel<<<1, 256, 0, st>>>(kv_indptr, (int)batch, (int)page_size, pl.chunk, (int)pl.max_items,
-                                       item_start, items);
-    AKO_CHECK_LAUNCH();
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(pl.max_items * HEAD_GROUPS));
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = SMEM_BYTES;
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, gqa_decode_kernel, p) != cudaSuccess) return AKO4X_ELAUNCH;
-    cudaLaunchConfig_t mcfg = {};
-    mcfg.gridDim = dim3((unsigned)(batch * HQ));
-    mcfg.blockDim = dim3(D / 4);
-    mcfg.stream = st;
-    mcfg.attrs = attr;
-    mcfg.numAttrs = 1;
-    const float* pacc = p.part_acc;
-    const float* pml = p.part_ml;
-    const int32_t* is = item_start;
-    __nv_bfloat16* op = p.o;
-    float* lp = p.lse;
-    if (cudaLaunchKernelEx(&mcfg, gqa_merge_items_kernel, pacc, pml, is, op, lp) != cudaSuccess)
-      return AKO4X_ELAUNCH;
-    return AKO4X_OK;
-  }
-  const int64_t grid = batch * HEAD_GROUPS * splits;
-  if (grid > 0x7fffffffLL) return AKO4X_EINVAL;
-  gqa_decode_kernel<<<(unsigned)grid, THREADS, SMEM_BYTES, st>>>(p);
+  p.batch = (int)batch;
+  p.whole_rows = whole;
+  gqa_decode_kernel<<<(unsigned)(shares * HALVES), THREADS, 0, st>>>(p);
   AKO_CHECK_LAUNCH();
-  if (splits > 1) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(batch * HQ));
-    cfg.blockDim = dim3(D / 4);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const float* pacc = p.part_acc;
-    const float* pml = p.part_ml;
-    __nv_bfloat16* op = p.o;
-    float* lp = p.lse;
-    int ns = splits;
-    if (cudaLaunchKernelEx(&cfg, ako::lse_merge_kernel<D, 4>, pacc, pml, op, lp, ns) != cudaSuccess)
-      return AKO4X_ELAUNCH;
-  }
+  if (whole) return AKO4X_OK;
+  const bool many = shares >= 8 * batch;              // partials per sequence
+  const cudaError_t e = many ? ako::launch_pdl(true, gqa_merge_kernel<8>, dim3((unsigned)(batch * HQ)), dim3(256), 0, st, p, shares)
+                             : ako::launch_pdl(true, gqa_merge_kernel<1>, dim3((unsigned)(batch * (HQ / 4))), dim3(128), 0, st, p, shares);
+  if (e != cudaSuccess)
+    return AKO4X_ELAUNCH;
   return AKO4X_OK;
 }
 
-// Status word of the decode kernel of this file: 0, or the code of a bounded wait that gave up.
-// Synchronises the device; meant for tests and post-mortems.
+// Status word of the decode kernel of this file. Synchronises the device; meant for tests and
+// post-mortems.
 extern "C" int ako4x_gqa_paged_decode_device_status(void) {
   int v = 0;
   if (cudaMemcpyFromSymbol(&v, g_gqa_status, sizeof(int)) != cudaSuccess) return AKO4X_ELAUNCH;

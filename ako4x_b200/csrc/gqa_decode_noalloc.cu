@@ -8,7 +8,7 @@
 // scratch array inside the library image and runs the same kernels on it.
 //
 // Costs and rules, all consequences of the scratch being one static array:
-//   * every GPU that loads the library holds kScratchBytes (16 MiB) of device memory until exit;
+//   * every GPU that loads the library holds kScratchBytes (8 MiB) of device memory until exit;
 //   * a call whose partials would not fit is refused with AKO4X_ETOOLARGE, nothing is launched;
 //   * all calls on a device share the array, so two calls that may overlap on the GPU (different
 //     streams, or different host threads) race; serialise them on one stream;
@@ -23,7 +23,9 @@
 
 namespace {
 
-constexpr size_t kScratchBytes = 16u << 20;
+// Enough for every batch of up to 282 sequences, and for the larger ones whose sequences are short
+// (those need no partials at all).
+constexpr size_t kScratchBytes = 8u << 20;
 
 // In host code this name is only a handle for the runtime, not a device address: it must go
 // through cudaGetSymbolAddress before a kernel can be given the memory.

@@ -49,10 +49,9 @@ int ako4x_rmsnorm_h128(const void* x, const void* weight, void* y, int64_t rows,
  * q bf16 [batch,32,128]; k_cache, v_cache bf16 [pages,page_size,8,128]; kv_indptr int32
  * [batch+1]; kv_indices int32 [kv_indptr[batch]] (page ids); o bf16 [batch,32,128];
  * lse fp32 [batch,32] = log2(sum exp(logit)); empty sequence gives o = 0, lse = -inf.
- * `num_kv_indices` (the length of kv_indices) sizes the split heuristic and the workspace; it is
- * a shape, not device data, and it must bound the device-side list: kv_indptr[batch] <=
- * num_kv_indices. A longer device-side list is cut to what the workspace holds and status code 20
- * is recorded (ako4x_gqa_paged_decode_device_status).
+ * `num_kv_indices` (the length of kv_indices) sizes the work split and the workspace; it is a shape,
+ * not device data, and kv_indptr[batch] <= num_kv_indices must hold. The workspace is 0 bytes for large
+ * batches of short sequences.
  */
 size_t ako4x_gqa_paged_decode_workspace_bytes(int64_t batch, int64_t num_kv_indices,
                                               int64_t page_size);
@@ -62,17 +61,14 @@ int ako4x_gqa_paged_decode(const void* q, const void* k_cache, const void* v_cac
                            int64_t page_size, void* workspace, size_t workspace_bytes,
                            void* stream);
 
-/* The gather pipeline waits on mbarriers with a cycle limit. A wait that gives up makes its CTA
- * stop consuming and stores a non-zero code in a device status word; this call returns that word
- * (0 = no wait has given up since the library was loaded). A non-zero word means that the outputs
- * of the call that set it are invalid; later calls are not affected by it (every launch starts its
- * waits afresh). It synchronises the device: for tests and post-mortems only. */
+/* Status word of the kernel (0: it has no wait that could give up). It synchronises the device: for
+ * tests and post-mortems only. */
 int ako4x_gqa_paged_decode_device_status(void);
 
 /* The same operator for callers that have no scratch memory to pass and cannot allocate any (a
  * plug-in host that supplies only input and output tensors; a serving process whose HBM is fully
  * committed to its KV-cache pool). It has no counterpart in the reference. The split-KV partials
- * live in a 16 MiB array inside the library image (held by every GPU that loads the library);
+ * live in an 8 MiB array inside the library image (held by every GPU that loads the library);
  * ako4x_gqa_paged_decode_noalloc_max_scratch_bytes() returns that limit. A call that would need
  * more (compare ako4x_gqa_paged_decode_workspace_bytes) returns AKO4X_ETOOLARGE and launches
  * nothing. Calls on one device share the array: calls that can overlap on the GPU race, so keep

@@ -119,3 +119,10 @@ def test_same_buffers_new_contents(built_lib):
     a["v_cache"].mul_(-1)
     o2, _ = gqa_decode.run(*[a[k] for k in KEYS])
     assert torch.equal(o2, -o1)
+
+
+@pytest.mark.parametrize("lens", [[15, 16, 17, 0, 33, 1] * 40, [600] * 3 + [0] + [3] * 230, [5, 0, 8192, 2, 0], [7000, 16, 1]])
+def test_shares_and_whole_sequences(built_lib, lens):
+    """Many short sequences (one share each, no partials, no merge), a batch just inside that rule, and
+    few sequences whose partials come from one or from hundreds of shares; empty ones in between."""
+    _check(W.make_gqa_decode(len(lens), shape_id=60 + len(lens) % 7, lens=lens, extra_pages=11))
