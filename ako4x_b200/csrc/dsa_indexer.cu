@@ -6,11 +6,13 @@
 // accumulator. Scores are written as fp32.
 //
 // Select kernel: one CTA per row. Keys are the order-preserving unsigned image of the fp32 scores,
-// read once into shared memory; a three-pass most-significant-digit radix select (11, 11 and 10
-// bits; the heavily repeated leading digit is warp-aggregated) finds the 2048-th largest key, then
-// a stable compaction in token order emits every token above the threshold plus the first tokens
-// equal to it (ties: lower position wins), translated to global cache slots through the block
-// table.
+// read once into shared memory. The 2048-th largest key is found by one histogram over 2048 equal
+// intervals of the row's score range and an exact ranking of the few keys of the interval it falls
+// in; rows where that interval is crowded (many equal scores, outliers that stretch the range, no
+// finite range) and rows of more than 32768 tokens take a three-pass most-significant-digit radix
+// select (11, 11 and 10 bits; the heavily repeated leading digit is warp-aggregated). A stable
+// compaction in token order then emits every token above the threshold plus the first tokens equal
+// to it (ties: lower position wins), translated to global cache slots through the block table.
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include "tma_host.cuh"
@@ -33,6 +35,7 @@ constexpr int SEL_PER = 32;                          // tokens per thread and ch
 constexpr int SEL_CHUNK = SEL_THREADS * SEL_PER;     // 32768 tokens: one shared-memory resident chunk
 constexpr int SEL_BINS = 2048;                       // widest digit: 11 bits
 constexpr int SEL_SMEM = SEL_CHUNK * 4;              // 128 KB of keys
+constexpr int SEL_CAND = 512;                        // most keys of one interval that are ranked directly
 
 __device__ __forceinline__ uint32_t order_key(float s) {
   const uint32_t b = __float_as_uint(s + 0.0f);  // -0 -> +0
@@ -44,23 +47,43 @@ __device__ __forceinline__ uint32_t order_key(float s) {
 // compaction, where a thread reads its own eight consecutive slots.
 __device__ __forceinline__ int sel_slot(int f) { return f ^ ((f >> 3) & 7); }
 
-// Fills the chunk's keys; tokens at or past `sl` get key 0 (below every finite score).
-__device__ __forceinline__ void sel_fill(uint4* skeys, const float* __restrict__ s, int chunk, int sl, int tid) {
+__device__ __forceinline__ float key_score(uint32_t k) {  // inverse of order_key
+  return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k);
+}
+
+// Fills the chunk's keys; tokens at or past `sl` get key 0 (below every finite score). kmin / kmax
+// take in the keys of the tokens this thread fills. Four loads in flight per thread.
+__device__ __forceinline__ void sel_fill(uint4* skeys, const float* __restrict__ s, int chunk, int sl, int tid,
+                                         uint32_t& kmin, uint32_t& kmax) {
   const int nslots = (min(sl - chunk * SEL_CHUNK, SEL_CHUNK) + 3) >> 2;  // slots that hold a token
 #pragma unroll
-  for (int it = 0; it < SEL_PER / 4; ++it) {
-    if (it * SEL_THREADS >= nslots) break;  // short rows: the passes below stop at the same slot
-    const int f = it * SEL_THREADS + tid;
-    const int i = chunk * SEL_CHUNK + 4 * f;  // a row is a whole number of 64-token pages: no overrun
-    uint4 k = make_uint4(0u, 0u, 0u, 0u);
-    if (i < sl) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(s + i));
-      k.x = order_key(v.x);
-      k.y = (i + 1 < sl) ? order_key(v.y) : 0u;
-      k.z = (i + 2 < sl) ? order_key(v.z) : 0u;
-      k.w = (i + 3 < sl) ? order_key(v.w) : 0u;
+  for (int h = 0; h < SEL_PER / 16; ++h) {
+    float4 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = chunk * SEL_CHUNK + 4 * ((4 * h + q) * SEL_THREADS + tid);
+      v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < sl) v[q] = __ldg(reinterpret_cast<const float4*>(s + i));  // a row is whole 64-token pages: no overrun
     }
-    skeys[sel_slot(f)] = k;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if ((4 * h + q) * SEL_THREADS >= nslots) break;  // short rows: the passes below stop at the same slot
+      const int f = (4 * h + q) * SEL_THREADS + tid;
+      const int i = chunk * SEL_CHUNK + 4 * f;
+      uint4 k = make_uint4(0u, 0u, 0u, 0u);
+      if (i < sl) {
+        k.x = order_key(v[q].x);
+        k.y = (i + 1 < sl) ? order_key(v[q].y) : 0u;
+        k.z = (i + 2 < sl) ? order_key(v[q].z) : 0u;
+        k.w = (i + 3 < sl) ? order_key(v[q].w) : 0u;
+        kmax = max(max(kmax, max(k.x, k.y)), max(k.z, k.w));
+        kmin = min(kmin, k.x);
+        if (i + 1 < sl) kmin = min(kmin, k.y);
+        if (i + 2 < sl) kmin = min(kmin, k.z);
+        if (i + 3 < sl) kmin = min(kmin, k.w);
+      }
+      skeys[sel_slot(f)] = k;
+    }
   }
 }
 
@@ -114,13 +137,89 @@ __device__ __forceinline__ void sel_pass(int* hist, const uint4* skeys, uint32_t
   }
 }
 
+// Interval of a key: 2048 equal parts of [lo, lo + 2048 / inv]. Never decreases with the score
+// (each operation is monotonic), which is all that the selection needs of it.
+__device__ __forceinline__ int sel_interval(uint32_t key, float lo, float inv) {
+  return min((int)((key_score(key) - lo) * inv), SEL_BINS - 1);
+}
+
+// The 2048-th largest key of a row in shared memory by intervals. True if found: thr is that key and
+// krem how many keys equal to it are taken. All threads of the block agree.
+__device__ __forceinline__ bool sel_by_intervals(const uint4* skeys, int* hist, int* scan_buf, uint32_t* cand, int* ctl,
+                                                 uint32_t kmin, uint32_t kmax, int nslots, int tid, int lane, int warp,
+                                                 uint32_t& thr, int& krem) {
+  uint32_t* mm = reinterpret_cast<uint32_t*>(hist);  // two words per warp, before the histogram
+  kmin = __reduce_min_sync(0xffffffffu, kmin);
+  kmax = __reduce_max_sync(0xffffffffu, kmax);
+  if (lane == 0) { mm[warp] = kmin; mm[32 + warp] = kmax; }
+  __syncthreads();
+  kmin = __reduce_min_sync(0xffffffffu, mm[lane]);
+  kmax = __reduce_max_sync(0xffffffffu, mm[32 + lane]);
+  __syncthreads();
+  // keys of -inf and +inf: anything at or outside them (infinities, NaN) goes to the radix select
+  if (kmin <= 0x007fffffu || kmax >= 0xff800000u) return false;
+  const float lo = key_score(kmin), inv = (float)SEL_BINS / (key_score(kmax) - lo);
+  hist[tid] = 0;
+  hist[tid + SEL_THREADS] = 0;
+  if (tid < 2) ctl[tid] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < SEL_PER / 4; ++it) {
+    if (it * SEL_THREADS >= nslots) break;
+    const uint4 k = skeys[it * SEL_THREADS + tid];
+    if (k.x) atomicAdd(&hist[sel_interval(k.x, lo, inv)], 1);  // key 0: no token
+    if (k.y) atomicAdd(&hist[sel_interval(k.y, lo, inv)], 1);
+    if (k.z) atomicAdd(&hist[sel_interval(k.z, lo, inv)], 1);
+    if (k.w) atomicAdd(&hist[sel_interval(k.w, lo, inv)], 1);
+  }
+  __syncthreads();
+  const int h0 = hist[2 * tid], h1 = hist[2 * tid + 1];
+  const int incl = block_suffix_sum(h0 + h1, scan_buf, lane, warp);
+  const int gt1 = incl - (h0 + h1), gt0 = gt1 + h1;
+  if (gt1 < TOPK && TOPK <= gt1 + h1) { ctl[1] = 2 * tid + 1; ctl[2] = TOPK - gt1; ctl[3] = h1; }
+  else if (gt0 < TOPK && TOPK <= gt0 + h0) { ctl[1] = 2 * tid; ctl[2] = TOPK - gt0; ctl[3] = h0; }
+  __syncthreads();
+  const int bin = ctl[1], n = ctl[3];
+  krem = ctl[2];
+  if (n > SEL_CAND) return false;
+#pragma unroll
+  for (int it = 0; it < SEL_PER / 4; ++it) {
+    if (it * SEL_THREADS >= nslots) break;
+    const uint4 k = skeys[it * SEL_THREADS + tid];
+    if (k.x && sel_interval(k.x, lo, inv) == bin) cand[atomicAdd(&ctl[0], 1)] = k.x;
+    if (k.y && sel_interval(k.y, lo, inv) == bin) cand[atomicAdd(&ctl[0], 1)] = k.y;
+    if (k.z && sel_interval(k.z, lo, inv) == bin) cand[atomicAdd(&ctl[0], 1)] = k.z;
+    if (k.w && sel_interval(k.w, lo, inv) == bin) cand[atomicAdd(&ctl[0], 1)] = k.w;
+  }
+  __syncthreads();
+  if (tid < n) {  // rank of this key among the interval's; equal keys write the same answer
+    const uint32_t me = cand[tid];
+    int gt = 0, ge = 0;
+    for (int i = 0; i < n; ++i) {
+      const uint32_t c = cand[i];
+      gt += (c > me) ? 1 : 0;
+      ge += (c >= me) ? 1 : 0;
+    }
+    if (gt < krem && krem <= ge) { ctl[4] = (int)me; ctl[5] = krem - gt; }
+  }
+  __syncthreads();
+  thr = (uint32_t)ctl[4];
+  krem = ctl[5];
+  return true;
+}
+
+// What bounded the radix select alone: 25 us a row of 32768 tokens, of it a warp-wide match per key in
+// its first pass, three block-wide scans and, at the end, chains of dependent block-table reads. With
+// intervals and the selected tokens staged in shared memory, index scores + selection + sparse attention
+// went from 53.5 to 38.9 us for one row and from 526 to 496 us for 512 rows of 32768 tokens.
 __global__ void __launch_bounds__(SEL_THREADS, 1) dsa_select_kernel(
     const float* __restrict__ scores, const int32_t* __restrict__ seq_lens,
     const int32_t* __restrict__ block_table, int32_t* __restrict__ out, int max_pages) {
   extern __shared__ __align__(16) unsigned char sel_smem[];
-  __shared__ int hist[SEL_BINS];
+  __shared__ int hist[SEL_BINS];  // at the end: the selected tokens
   __shared__ int scan_buf[SEL_THREADS / 32];
-  __shared__ int scan_buf2[SEL_THREADS / 32];
+  __shared__ uint32_t s_cand[SEL_CAND];
+  __shared__ int s_ctl[6];
   __shared__ uint32_t s_prefix;
   __shared__ int s_krem;
   uint4* skeys = reinterpret_cast<uint4*>(sel_smem);
@@ -142,86 +241,97 @@ __global__ void __launch_bounds__(SEL_THREADS, 1) dsa_select_kernel(
   // Up to 32768 tokens the keys are read from global memory once and stay in shared memory;
   // longer rows are swept chunk by chunk in every pass.
   const int chunks = (sl + SEL_CHUNK - 1) / SEL_CHUNK;
-  sel_fill(skeys, s, 0, sl, tid);
+  uint32_t kmin = 0xffffffffu, kmax = 0u;
+  sel_fill(skeys, s, 0, sl, tid, kmin, kmax);
 
-  // ---- threshold: most-significant-digit radix select, digits of 11, 11 and 10 bits ------------
-  // Padding keys (0) only ever land in the lowest bin, below the 2048-th largest real key.
-  uint32_t prefix = 0u;
+  uint32_t thr = 0u;
   int krem = TOPK;
+  if (chunks > 1 ||
+      !sel_by_intervals(skeys, hist, scan_buf, s_cand, s_ctl, kmin, kmax, (sl + 3) >> 2, tid, lane, warp, thr, krem)) {
+    // ---- threshold: most-significant-digit radix select, digits of 11, 11 and 10 bits ----------
+    // Padding keys (0) only ever land in the lowest bin, below the 2048-th largest real key.
+    uint32_t prefix = 0u;
+    krem = TOPK;
 #pragma unroll 1
-  for (int pass = 0; pass < 3; ++pass) {
-    const int shift = (pass == 0) ? 21 : (pass == 1) ? 10 : 0;
-    hist[tid] = 0;
-    hist[tid + SEL_THREADS] = 0;
-    __syncthreads();  // also: the keys are in place
+    for (int pass = 0; pass < 3; ++pass) {
+      const int shift = (pass == 0) ? 21 : (pass == 1) ? 10 : 0;
+      hist[tid] = 0;
+      hist[tid + SEL_THREADS] = 0;
+      __syncthreads();  // also: the keys are in place
 #pragma unroll 1
-    for (int c = 0; c < chunks; ++c) {
-      if (chunks > 1) {
-        __syncthreads();
-        sel_fill(skeys, s, c, sl, tid);
-        __syncthreads();
+      for (int c = 0; c < chunks; ++c) {
+        if (chunks > 1) {
+          __syncthreads();
+          sel_fill(skeys, s, c, sl, tid, kmin, kmax);
+          __syncthreads();
+        }
+        const int nslots = (min(sl - c * SEL_CHUNK, SEL_CHUNK) + 3) >> 2;
+        if (pass == 0) sel_pass<0>(hist, skeys, prefix, tid, lane, nslots);
+        else if (pass == 1) sel_pass<1>(hist, skeys, prefix, tid, lane, nslots);
+        else sel_pass<2>(hist, skeys, prefix, tid, lane, nslots);
       }
-      const int nslots = (min(sl - c * SEL_CHUNK, SEL_CHUNK) + 3) >> 2;
-      if (pass == 0) sel_pass<0>(hist, skeys, prefix, tid, lane, nslots);
-      else if (pass == 1) sel_pass<1>(hist, skeys, prefix, tid, lane, nslots);
-      else sel_pass<2>(hist, skeys, prefix, tid, lane, nslots);
+      __syncthreads();
+      // thread t owns bins 2t and 2t+1; suffix sums give count(digit >= bin)
+      const int h0 = hist[2 * tid], h1 = hist[2 * tid + 1];
+      const int incl = block_suffix_sum(h0 + h1, scan_buf, lane, warp);
+      const int gt1 = incl - (h0 + h1);  // keys with a larger digit than bin 2t+1
+      const int gt0 = gt1 + h1;
+      if (gt1 < krem && krem <= gt1 + h1) {
+        s_prefix = prefix | ((uint32_t)(2 * tid + 1) << shift);
+        s_krem = krem - gt1;
+      } else if (gt0 < krem && krem <= gt0 + h0) {
+        s_prefix = prefix | ((uint32_t)(2 * tid) << shift);
+        s_krem = krem - gt0;
+      }
+      __syncthreads();
+      prefix = s_prefix;
+      krem = s_krem;  // how many keys of the chosen bin are still to be taken
     }
-    __syncthreads();
-    // thread t owns bins 2t and 2t+1; suffix sums give count(digit >= bin)
-    const int h0 = hist[2 * tid], h1 = hist[2 * tid + 1];
-    const int incl = block_suffix_sum(h0 + h1, scan_buf, lane, warp);
-    const int gt1 = incl - (h0 + h1);  // keys with a larger digit than bin 2t+1
-    const int gt0 = gt1 + h1;
-    if (gt1 < krem && krem <= gt1 + h1) {
-      s_prefix = prefix | ((uint32_t)(2 * tid + 1) << shift);
-      s_krem = krem - gt1;
-    } else if (gt0 < krem && krem <= gt0 + h0) {
-      s_prefix = prefix | ((uint32_t)(2 * tid) << shift);
-      s_krem = krem - gt0;
-    }
-    __syncthreads();
-    prefix = s_prefix;
-    krem = s_krem;  // how many keys of the chosen bin are still to be taken
+    thr = prefix;
   }
-  const uint32_t thr = prefix;
 
   // ---- stable compaction in token order: keys above thr, plus the first `krem` equal to it ----
-  // Thread t owns the 32 consecutive tokens of its eight slots.
+  // Thread t owns the 32 consecutive tokens of its eight slots. The selected tokens go to shared
+  // memory first (the histogram is no longer needed), so that the block-table reads are independent
+  // and the stores coalesced.
   int g_base = 0, e_base = 0;
 #pragma unroll 1
   for (int c = 0; c < chunks; ++c) {
     if (chunks > 1) {
       __syncthreads();
-      sel_fill(skeys, s, c, sl, tid);
+      sel_fill(skeys, s, c, sl, tid, kmin, kmax);
       __syncthreads();
     }
     const int tok0 = c * SEL_CHUNK + tid * SEL_PER;
     const int nvalid = max(0, min(SEL_PER, sl - tok0));
     uint32_t gmask = 0u, emask = 0u;  // bit j: token tok0 + j is above / equal to the threshold
+    if (nvalid > 0) {
 #pragma unroll
-    for (int q = 0; q < SEL_PER / 4; ++q) {
-      const uint4 k = skeys[sel_slot(tid * (SEL_PER / 4) + q)];
-      gmask |= ((k.x > thr) ? 1u : 0u) << (4 * q) | ((k.y > thr) ? 2u : 0u) << (4 * q) |
-               ((k.z > thr) ? 4u : 0u) << (4 * q) | ((k.w > thr) ? 8u : 0u) << (4 * q);
-      emask |= ((k.x == thr) ? 1u : 0u) << (4 * q) | ((k.y == thr) ? 2u : 0u) << (4 * q) |
-               ((k.z == thr) ? 4u : 0u) << (4 * q) | ((k.w == thr) ? 8u : 0u) << (4 * q);
+      for (int q = 0; q < SEL_PER / 4; ++q) {
+        const uint4 k = skeys[sel_slot(tid * (SEL_PER / 4) + q)];
+        gmask |= ((k.x > thr) ? 1u : 0u) << (4 * q) | ((k.y > thr) ? 2u : 0u) << (4 * q) |
+                 ((k.z > thr) ? 4u : 0u) << (4 * q) | ((k.w > thr) ? 8u : 0u) << (4 * q);
+        emask |= ((k.x == thr) ? 1u : 0u) << (4 * q) | ((k.y == thr) ? 2u : 0u) << (4 * q) |
+                 ((k.z == thr) ? 4u : 0u) << (4 * q) | ((k.w == thr) ? 8u : 0u) << (4 * q);
+      }
     }
     const uint32_t vmask = (nvalid >= 32) ? 0xffffffffu : ((1u << nvalid) - 1u);
     gmask &= vmask;
     emask &= vmask;
-    const int ng = __popc(gmask), ne = __popc(emask);
-    const int sg = block_suffix_sum(ng, scan_buf, lane, warp);
-    const int se = block_suffix_sum(ne, scan_buf2, lane, warp);
-    if (tid == 0) { scan_buf[0] = sg; scan_buf2[0] = se; }  // thread 0's suffix sum is the total
+    // one scan for both counts: at most 2047 tokens are above the threshold, at most 32768 of the
+    // chunk equal to it
+    const int cnt = __popc(gmask) << 17 | __popc(emask);
+    const int suf = block_suffix_sum(cnt, scan_buf, lane, warp);
+    if (tid == 0) scan_buf[0] = suf;  // thread 0's suffix sum is the total
     __syncthreads();
-    const int block_g = scan_buf[0], block_e = scan_buf2[0];
-    int G = g_base + block_g - sg;  // above-threshold tokens before this thread's
-    int E = e_base + block_e - se;  // threshold-valued tokens before this thread's
+    const int total = scan_buf[0];
+    const int before = total - suf;       // counts of the tokens before this thread's
+    int G = g_base + (before >> 17);
+    int E = e_base + (before & 0x1ffff);
     uint32_t m = gmask | emask;
     while (m) {
       const int j = __ffs(m) - 1;
       m &= m - 1;
-      const int i = tok0 + j;
       int pos;
       if (gmask >> j & 1u) {
         pos = G + min(E, krem);
@@ -230,11 +340,16 @@ __global__ void __launch_bounds__(SEL_THREADS, 1) dsa_select_kernel(
         pos = (E < krem) ? G + E : TOPK;
         ++E;
       }
-      if (pos < TOPK) o[pos] = bt[i >> 6] * PS + (i & 63);
+      if (pos < TOPK) hist[pos] = tok0 + j;
     }
-    g_base += block_g;
-    e_base += block_e;
+    g_base += total >> 17;
+    e_base += total & 0x1ffff;
     __syncthreads();
+  }
+#pragma unroll
+  for (int k = tid; k < TOPK; k += SEL_THREADS) {
+    const int i = hist[k];
+    o[k] = bt[i >> 6] * PS + (i & 63);
   }
 }
 

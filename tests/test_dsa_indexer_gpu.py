@@ -68,6 +68,40 @@ def test_select_quantised_scores_many_ties(built_lib):
     assert torch.equal(out.cpu(), ref)
 
 
+def _score_rows(kind, n, g):
+    x = torch.randn(n, generator=g)
+    if kind == "outlier":            # everything else shares one interval of the range
+        x[n // 3] = 1e30
+    elif kind == "infinities":
+        x[::50], x[7::501] = float("inf"), float("-inf")
+    elif kind == "widest":           # the range itself overflows fp32
+        x[0], x[1] = 3e38, -3e38
+    elif kind == "denormal":
+        x = (x * 1e-41).float()
+    elif kind == "constant":
+        x = torch.full((n,), -1.25)
+    elif kind == "crowded":          # 513 and more equal scores at the threshold
+        x = torch.where(torch.arange(n) % 4 == 0, torch.full((n,), 0.5), x * 0.1)
+    elif kind == "skewed":
+        x = -torch.rand(n, generator=g) ** 8
+    return x
+
+
+@pytest.mark.parametrize("kind", ["normal", "outlier", "infinities", "widest", "denormal", "constant", "crowded", "skewed"])
+def test_select_by_intervals_and_its_fallback(built_lib, kind):
+    """Rows for the interval histogram and rows that it must hand to the radix select, at lengths around
+    the selection's size, the slot width and the largest resident row."""
+    g = torch.Generator().manual_seed(29)
+    lens = [2049, 2050, 4095, 4097, 8191, 32767, 32768]
+    pages = 512
+    sl = torch.tensor(lens, dtype=torch.int32)
+    bt = torch.stack([torch.randperm(pages, generator=g).to(torch.int32) for _ in lens])
+    scores = torch.stack([torch.nn.functional.pad(_score_rows(kind, n, g), (0, pages * 64 - n)) for n in lens])
+    ref = oracle.dsa_topk_select(scores, sl, bt)
+    out = dsa_indexer.topk_select(scores.cuda(), sl.cuda(), bt.cuda())
+    assert torch.equal(out.cpu(), ref)
+
+
 def test_select_rows_longer_than_one_resident_chunk(built_lib):
     """Rows above 32768 tokens are swept in chunks; ties straddle the chunk boundary."""
     g = torch.Generator().manual_seed(11)
