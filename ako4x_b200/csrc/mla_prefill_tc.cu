@@ -1,29 +1,33 @@
 // Causal paged MLA prefill on the 5th-generation tensor cores (tcgen05 + TMEM) fed by TMA.
 //
 // Two launches. (1) gather: the keys of all sequences are copied from the paged caches into a
-// contiguous [tokens, 576] matrix Kc (ckv | kpe) and, transposed, into Vt [512, columns] (every
-// sequence starts at a multiple of 8 columns so a TMA box may start there). (2) attention: a CTA
-// owns a tile of 8 consecutive query tokens of one sequence (128 rows: token x head) and ONE half of
-// the 512 output columns; the O tile would fill all of TMEM, so the two halves are separate CTAs that
-// both compute S. Per tile of 128 keys:
-//   S  = Q Kc^T        128 x 128, reduction 576 streamed in nine 64-column chunks of Q and Kc through
-//                      a 5-stage TMA ring; 36 tcgen05.mma (bf16, N = 128, K = 16) into one of two
-//                      128-column TMEM buffers;
-//   P  = softmax step  four warps, one thread per row: two sweeps over the S buffer (row maximum,
-//                      then exp2), causal mask, running (m, l); P is written back with tcgen05.st as
-//                      packed bf16 pairs over the first 64 columns of the S buffer it was read from,
-//                      alpha = 2^(m_old-m_new) goes to shared memory;
-//   PV = P Vt^T        128 x 256, 8 MMAs (N = 256) with the A operand (P) taken from TMEM, into a
-//                      256-column TMEM buffer, NOT accumulated; their commit frees the S buffer;
-//   O  = O alpha + PV  eight warps hold the 128 x 256 fp32 O tile in registers (128 per thread) and
-//                      fold every PV tile in -- no rescaling of TMEM contents.
-// S of tile j+1 streams in while the softmax works on tile j; PV of tile j is issued by a thread of
-// its own as soon as P is complete. The kernel is bound by the bytes that cross shared memory (TMA
-// writes + MMA operand reads, 128 B/clk per SM), which is why P stays in TMEM.
-// Warps: 0-7 O accumulation (setmaxnreg 184), 8-11 softmax (104), 12 Q/K producer, 13 S issuer,
-// 14 V producer, 15 PV issuer (40). Rows of a partial last tile and keys past the causal limit are
-// masked; every mbarrier wait is bounded and a timeout sets the status word. Shared memory: ring
-// 160 KB + Vt tile 64 KB + 3 KB (alpha, l, mbarriers) = the whole 227 KB, none of it static.
+// contiguous [tokens, 576] matrix Kc (ckv | kpe). (2) attention: a PAIR of CTAs (a cluster of two,
+// tcgen05 cta_group::2, M = 256) owns 16 consecutive query tokens of one sequence, eight per CTA
+// (128 rows: token x head), and ONE half of the 512 output columns; O and the S buffers together
+// would not fit TMEM otherwise, so the two halves are separate pairs that both compute S. The Q tile
+// (144 KB per CTA) stays in shared memory. Per tile of 128 keys:
+//   S  = Q Kc^T        256 x 128, reduction 576 in nine 64-column chunks of Kc, 64 keys per CTA,
+//                      through a 6-stage TMA ring; 36 MMAs (bf16, K = 16) into one of two 128-column
+//                      TMEM buffers of each CTA;
+//   P  = softmax step  eight warps, two threads per row (64 keys each, held in registers from the
+//                      one TMEM read on), which exchange the row maximum through shared memory;
+//                      P goes back with tcgen05.st as packed bf16 pairs over the first 64 columns of
+//                      the S buffer;
+//   O  = O alpha + P V 256 x 256, 8 MMAs (N = 256): A operand (P) from TMEM, B = the rows of Kc read
+//                      as an MN-major operand (128 columns per CTA), accumulated in TMEM.
+// Where a row's maximum grew, its warps rescale their lanes of O in TMEM once the previous PV is done;
+// a warp none of whose 32 rows grew skips it. (Letting the maximum lag by up to 2^8 instead makes
+// this rare and measured 4 % faster, but then the largest weight of a row is not exactly 1 and its
+// bf16 rounding shows: 1.96e-3 instead of 1.81e-3 from fp64 at 8192 keys. Not done.)
+//
+// Why a pair: one CTA per tile was bound by the bytes that cross shared memory (128 B/clk per SM):
+// 644 KB per 128-key tile, of which 294 KB were TMA writes of Q and K chunks and 288 KB S operands.
+// A pair reads half of every K chunk and half of V per CTA and leaves room for a resident Q tile:
+// 352 KB. Eight ragged prompts (9 101 queries, 39 794 keys): 2 274 -> 1 785 us with the gather, 745
+// TFLOP/s of algorithmic flops, 1 140 counting S of both halves.
+// Warps: 0-7 softmax, rescale and output, 8 Q/K producer, 9 S issuer (even CTA), 10 V producer,
+// 11 PV issuer (even CTA). Rows of a partial last tile and keys past the causal limit are masked;
+// every mbarrier wait is bounded and a timeout sets the status word.
 #include "mla_prefill_tc.h"
 
 #include <cuda_bf16.h>
@@ -36,30 +40,29 @@
 namespace {
 
 constexpr int H = 16, DC = 512, DP = 64, DQK = DC + DP;
-constexpr int QT = 8;                     // query tokens per tile
-constexpr int BM = QT * H;                // 128 rows
+constexpr int QT = 8;                     // query tokens per CTA
+constexpr int PT = 2 * QT;                // query tokens per pair
+constexpr int BM = QT * H;                // 128 rows per CTA
 constexpr int BK = 128;                   // keys per tile
 constexpr int NCH = DQK / 64;             // nine reduction chunks of 64 columns
-constexpr int CH_BYTES = BM * 128;        // one 128-row x 64-column bf16 chunk: 16 KB
-constexpr int ST_BYTES = 2 * CH_BYTES;    // Q chunk + K chunk
-constexpr int NST = 5;
-constexpr int V_BYTES = 2 * 256 * 128;    // two boxes of 256 rows x 64 keys
-constexpr int AUX_BYTES = 3072;           // alpha[4][128], final l[128], mbarriers, TMEM address, work item
+constexpr int Q_CH_BYTES = BM * 128;      // one 128-row x 64-column bf16 chunk: 16 KB
+constexpr int K_CH_BYTES = BK / 2 * 128;  // this CTA's 64 keys of a chunk: 8 KB
+constexpr int Q_BYTES = NCH * Q_CH_BYTES;
+constexpr int NST = 6;
+constexpr int V_BOX_BYTES = BK * 128;     // 128 keys x 64 columns
+constexpr int V_BYTES = 2 * V_BOX_BYTES;  // this CTA's 128 columns
+constexpr int AUX_BYTES = 3072;           // row exchange [2][2][128], mbarriers, TMEM address, work item
 // exactly the 227 KB a CTA may have: no static shared memory in this kernel, so that the dynamic
 // region starts on a 1024-byte boundary (checked at entry) and needs no alignment slack
-constexpr int SMEM = NST * ST_BYTES + V_BYTES + AUX_BYTES;
+constexpr int SMEM = Q_BYTES + NST * K_CH_BYTES + V_BYTES + AUX_BYTES;
 static_assert(SMEM <= 232448, "shared memory per CTA");
-static_assert(2560 + (2 * NST + 11) * 8 + 8 + 16 <= AUX_BYTES, "aux region");
-constexpr int THREADS = 512;
-constexpr int REGS_O = 184, REGS_SOFTMAX = 104, REGS_OTHER = 40;  // 2*184 + 104 + 40 = 4*128
+constexpr int THREADS = 384;
+constexpr int SOFTMAX_WARPS = 8;
 constexpr float NEG = -1.0e30f;           // finite stand-in for -inf
 
 // Wait status of the CURRENT call (cleared by the gather kernel that starts every call, so a code
-// left by an earlier call cannot make this call's waits give up early) and the sticky word that
-// ako_mla_prefill_tc_status() reports. The per-call word stays in global memory on purpose: with
-// the word in shared memory, as in the other kernels, this kernel measured 18 % slower (1 463 ->
-// 1 725 us at the benchmark shape; the roles that run on 40 registers do not take the extra pointer
-// well).
+// left by an earlier call cannot make this call's waits give up early; both CTAs of a pair see it)
+// and the sticky word that ako_mla_prefill_tc_status() reports.
 __device__ int g_pf_status = 0;
 __device__ int g_pf_sticky = 0;
 
@@ -75,52 +78,31 @@ struct PfParams {
 // ---------------------------------------------------------------------------------------------
 // gather: 32 key tokens per CTA
 // ---------------------------------------------------------------------------------------------
-constexpr int G_TOK = 32, G_PITCH = 520;  // bf16 elements per staged row (1040 B: 16-byte aligned)
-
-__host__ __device__ inline int64_t vt_start(int64_t first_token, int b) {
-  return ((first_token + 7) / 8) * 8 + 8 * (int64_t)b;  // non-overlapping and a multiple of 8 columns
-}
+constexpr int G_TOK = 32, G_VEC = DQK * 2 / 16;  // 72 16-byte vectors per token
+static_assert(G_TOK * G_VEC % 256 == 0, "whole passes of the block");
 
 __global__ void __launch_bounds__(256) mla_prefill_gather_kernel(
     const uint4* __restrict__ ckv, const uint4* __restrict__ kpe, const int32_t* __restrict__ kv_indices,
-    const int32_t* __restrict__ kv_indptr, int batch, int page_size, int64_t ntok, uint4* __restrict__ kc,
-    __nv_bfloat16* __restrict__ vt, int64_t vt_cols) {
-  __shared__ __align__(16) __nv_bfloat16 s_v[G_TOK * G_PITCH];
+    int page_size, int64_t ntok, uint4* __restrict__ kc) {
   __shared__ int64_t s_row[G_TOK];
-  __shared__ int64_t s_col[G_TOK];
   const int tid = threadIdx.x;
   const int64_t g0 = (int64_t)blockIdx.x * G_TOK;
   if (blockIdx.x == 0 && tid == 0) g_pf_status = 0;  // this call's wait status starts clean
   if (tid < G_TOK) {
     const int64_t g = g0 + tid;
-    int64_t row = 0, col = -1;
-    if (g < ntok) {
-      const int64_t pg = kv_indices[g / page_size];
-      row = pg * page_size + g % page_size;
-      // sequence of this token: kv_indptr counts pages
-      int b = 0;
-      const int64_t page_slot = g / page_size;
-      while (b + 1 < batch && (int64_t)kv_indptr[b + 1] <= page_slot) ++b;
-      const int64_t first = (int64_t)kv_indptr[b] * page_size;
-      col = vt_start(first, b) + (g - first);
-    }
-    s_row[tid] = row;
-    s_col[tid] = col;
+    s_row[tid] = (g < ntok) ? (int64_t)kv_indices[g / page_size] * page_size + g % page_size : 0;
   }
   __syncthreads();
-  for (int i = tid; i < G_TOK * 72; i += 256) {
-    const int t = i / 72, c = i % 72;
-    if (g0 + t >= ntok) continue;
-    const int64_t row = s_row[t];
-    const uint4 v = (c < 64) ? __ldg(ckv + row * 64 + c) : __ldg(kpe + row * 8 + (c - 64));
-    kc[(g0 + t) * 72 + c] = v;
-    if (c < 64) *reinterpret_cast<uint4*>(s_v + t * G_PITCH + c * 8) = v;
+  uint4 v[G_TOK * G_VEC / 256];
+#pragma unroll
+  for (int k = 0; k < G_TOK * G_VEC / 256; ++k) {
+    const int i = k * 256 + tid, t = i / G_VEC, c = i % G_VEC;
+    if (g0 + t < ntok) v[k] = (c < 64) ? __ldg(ckv + s_row[t] * 64 + c) : __ldg(kpe + s_row[t] * 8 + (c - 64));
   }
-  __syncthreads();
-  for (int i = tid; i < DC * G_TOK; i += 256) {
-    const int d = i / G_TOK, t = i % G_TOK;
-    const int64_t col = s_col[t];
-    if (col >= 0) vt[(int64_t)d * vt_cols + col] = s_v[t * G_PITCH + d];
+#pragma unroll
+  for (int k = 0; k < G_TOK * G_VEC / 256; ++k) {
+    const int i = k * 256 + tid;
+    if (g0 + i / G_VEC < ntok) kc[g0 * G_VEC + i] = v[k];
   }
 }
 
@@ -132,36 +114,34 @@ mla_prefill_tc_kernel(PfParams p, const __grid_constant__ CUtensorMap tm_qn, con
                       const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int crank = (int)ako::tc::t2_cluster_ctarank();
   const int half = blockIdx.y;  // which 256 output columns
-  unsigned char* smem_al = smem_raw;
   if (ako::smem_u32(smem_raw) & 1023u) {  // the swizzled operand tiles need this; nothing is started yet
     if (tid == 0) atomicCAS(&g_pf_sticky, 0, 13);
-    return;
+    return;  // the dynamic region starts at the same address in both CTAs: both return
   }
-  const uint32_t st_base = ako::smem_u32(smem_al);
-  const uint32_t v_base = st_base + NST * ST_BYTES;
-  float* alpha_s = reinterpret_cast<float*>(smem_al + NST * ST_BYTES + V_BYTES);  // [4][128]
-  float* fin_l = alpha_s + 4 * BM;                                                // [128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(fin_l + BM);
-  uint64_t* st_full = bars;
-  uint64_t* st_empty = bars + NST;
-  uint64_t* s_full = bars + 2 * NST;
-  uint64_t* s_empty = bars + 2 * NST + 2;
-  uint64_t& p_full = bars[2 * NST + 4];
-  uint64_t& v_full = bars[2 * NST + 5];
-  uint64_t& v_empty = bars[2 * NST + 6];
-  uint64_t& pv_full = bars[2 * NST + 7];
-  uint64_t& pv_empty = bars[2 * NST + 8];
-  uint64_t& fin = bars[2 * NST + 9];
-  uint32_t& s_tmem = *reinterpret_cast<uint32_t*>(bars + 2 * NST + 10);
-  int* s_work = reinterpret_cast<int*>(bars + 2 * NST + 11);  // sequence, tile inside the sequence (or -1)
+  const uint32_t q_base = ako::smem_u32(smem_raw);
+  const uint32_t k_base = q_base + Q_BYTES;
+  const uint32_t v_base = k_base + NST * K_CH_BYTES;
+  float* xch = reinterpret_cast<float*>(smem_raw + Q_BYTES + NST * K_CH_BYTES + V_BYTES);  // [2][2][128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(xch + 4 * BM);
+  uint64_t* st_full = bars;                // even CTA: bytes of both CTAs
+  uint64_t* st_empty = st_full + NST;      // each CTA
+  uint64_t* s_full = st_empty + NST;       // each CTA
+  uint64_t* pv_done = s_full + 2;          // each CTA: O is up to date, P and V have been read
+  uint64_t* p_full = pv_done + 2;          // even CTA: the softmax warps of both CTAs
+  uint64_t* xch_full = p_full + 2;         // each CTA: the two warps of a lane quarter
+  uint64_t& v_full = xch_full[4];          // even CTA: bytes of both CTAs
+  uint32_t& s_tmem = *reinterpret_cast<uint32_t*>(xch_full + 5);
+  int* s_work = reinterpret_cast<int*>(xch_full + 6);  // sequence, pair tile inside the sequence (or -1)
+  static_assert(4 * BM * 4 + (2 * NST + 6 + 6) * 8 + 8 <= AUX_BYTES, "aux region");
 
   if (tid == 0) {
-    // reversed: within a sequence the later query tiles see more keys, so the long CTAs start
+    // reversed: within a sequence the later query tiles see more keys, so the long pairs start
     // first and the short ones fill the end of the grid
-    int t = (int)(gridDim.x - 1 - blockIdx.x), b = 0;
+    int t = (int)((gridDim.x - 1 - blockIdx.x) >> 1), b = 0;
     for (; b < p.batch; ++b) {
-      const int nt = (p.qo_indptr[b + 1] - p.qo_indptr[b] + QT - 1) / QT;
+      const int nt = (p.qo_indptr[b + 1] - p.qo_indptr[b] + PT - 1) / PT;
       if (t < nt) break;
       t -= nt;
     }
@@ -173,283 +153,283 @@ mla_prefill_tc_kernel(PfParams p, const __grid_constant__ CUtensorMap tm_qn, con
     }
     for (int s = 0; s < 2; ++s) {
       ako::tc::mbar_init(ako::smem_u32(&s_full[s]), 1);
-      ako::tc::mbar_init(ako::smem_u32(&s_empty[s]), 1);
+      ako::tc::mbar_init(ako::smem_u32(&pv_done[s]), 1);
+      ako::tc::mbar_init(ako::smem_u32(&p_full[s]), 2 * SOFTMAX_WARPS);
     }
-    ako::tc::mbar_init(ako::smem_u32(&p_full), 4);
+    for (int q = 0; q < 4; ++q) ako::tc::mbar_init(ako::smem_u32(&xch_full[q]), 2);
     ako::tc::mbar_init(ako::smem_u32(&v_full), 1);
-    ako::tc::mbar_init(ako::smem_u32(&v_empty), 1);
-    ako::tc::mbar_init(ako::smem_u32(&pv_full), 1);
-    ako::tc::mbar_init(ako::smem_u32(&pv_empty), 8);
-    ako::tc::mbar_init(ako::smem_u32(&fin), 4);
     ako::tc::mbar_init_fence();
   }
-  if (warp == 13) ako::tc::tmem_alloc(ako::smem_u32(&s_tmem), 512);
+  if (warp == 9) ako::tc::t2_tmem_alloc(ako::smem_u32(&s_tmem), 512);
   ako::tc::fence_before_thread_sync();
   __syncthreads();
+  ako::tc::t2_cluster_sync();  // both CTAs' barriers are initialised before anybody signals across
   ako::tc::fence_after_thread_sync();
   const uint32_t tmem = s_tmem;
 
   const int b = s_work[0], tile = s_work[1];
-  // geometry of this tile (every thread computes the same values)
+  // geometry of this tile (every thread computes the same values; ntk is the pair's)
   int q0 = 0, nq = 0, kv_len = 0, q_len = 0, ntk = 0;
-  int64_t kbase = 0, vbase = 0;
+  int64_t kbase = 0;
   if (tile >= 0) {
     const int qb = p.qo_indptr[b];
     q_len = p.qo_indptr[b + 1] - qb;
-    q0 = qb + tile * QT;
-    nq = min(QT, q_len - tile * QT);
+    q0 = qb + tile * PT + crank * QT;
+    nq = min(QT, q_len - tile * PT - crank * QT);  // <= 0 for the empty half of an odd last pair
     kbase = (int64_t)p.kv_indptr[b] * p.page_size;
     kv_len = (p.kv_indptr[b + 1] - p.kv_indptr[b]) * p.page_size;
-    vbase = vt_start(kbase, b);
-    // keys visible to the tile's last token: [0, kv_len - q_len + last + 1)
-    const int kv_end = max(0, min(kv_len, kv_len - q_len + tile * QT + nq));
+    // keys visible to the pair's last token: [0, kv_len - q_len + last + 1)
+    const int kv_end = max(0, min(kv_len, kv_len - q_len + min(q_len, (tile + 1) * PT)));
     ntk = (kv_end + BK - 1) / BK;
   }
 
-  if (warp < 8) {
-    // ================================ O accumulation ============================================
-    ako::tc::reg_inc<REGS_O>();
-    const int r = 32 * (warp & 3) + lane;
-    const int ch = warp >> 2;  // which 128 of this CTA's 256 columns
-    const uint32_t taddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 256 + ch * 128;
-    float o[128];
-#pragma unroll
-    for (int i = 0; i < 128; ++i) o[i] = 0.f;
-    bool ok = true;
-    for (int j = 0; j < ntk; ++j) {
-      if (!ako::tc::mbar_wait(ako::smem_u32(&pv_full), (uint32_t)(j & 1), &g_pf_status, 1)) { ok = false; break; }
-      ako::tc::fence_after_thread_sync();
-      const float a = alpha_s[(j & 3) * BM + r];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float v[32];
-        ako::tc::tmem_ld32(taddr + 32 * c, v);
-        ako::tc::tmem_ld_wait_regs(v);
-        if (c == 3) {  // PV buffer and alpha slot are free again
-          ako::tc::fence_before_thread_sync();
-          __syncwarp();
-          if (lane == 0) ako::tc::mbar_arrive(ako::smem_u32(&pv_empty));
-        }
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[32 * c + i] = fmaf(o[32 * c + i], a, v[i]);
-      }
-    }
-    if (ok && tile >= 0 && ako::tc::mbar_wait(ako::smem_u32(&fin), 0u, &g_pf_status, 2)) {
-      const int qtok = r >> 4;
-      if (qtok < nq) {
-        const float l = fin_l[r];
-        const float inv = (l > 0.f) ? 1.0f / l : 0.f;
-        __nv_bfloat16* dst = p.o + ((int64_t)(q0 + qtok) * H + (r & 15)) * DC + half * 256 + ch * 128;
-#pragma unroll
-        for (int i = 0; i < 128; i += 8) {
-          uint4 w;
-          w.x = ako::pack_bf16x2(o[i] * inv, o[i + 1] * inv);
-          w.y = ako::pack_bf16x2(o[i + 2] * inv, o[i + 3] * inv);
-          w.z = ako::pack_bf16x2(o[i + 4] * inv, o[i + 5] * inv);
-          w.w = ako::pack_bf16x2(o[i + 6] * inv, o[i + 7] * inv);
-          *reinterpret_cast<uint4*>(dst + i) = w;
-        }
-      }
-    }
-  } else if (warp < 12) {
-    // ================================ softmax ====================================================
-    ako::tc::reg_dec<REGS_SOFTMAX>();
-    const int r = 32 * (warp & 3) + lane;
+  if (warp < SOFTMAX_WARPS) {
+    // ================================ softmax, rescale, output ===================================
+    const int quarter = warp & 3, ch = warp >> 2;  // ch: keys [64 ch, 64 ch + 64) of a tile; 128 output columns
+    const int r = 32 * quarter + lane;
     const int qtok = r >> 4;
-    const bool row_ok = tile >= 0 && qtok < nq;
-    const int kv_lim = row_ok ? max(0, min(kv_len, kv_len - q_len + tile * QT + qtok + 1)) : 0;
-    const uint32_t tq = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-    float m = NEG, l = 0.f;
+    const bool row_ok = qtok < nq;
+    const int kv_lim = row_ok ? max(0, min(kv_len, kv_len - q_len + tile * PT + crank * QT + qtok + 1)) : 0;
+    const uint32_t tq = tmem + ((uint32_t)(32 * quarter) << 16);
+    const uint32_t to = tq + 256 + 128 * ch;
+    const uint32_t xbar = ako::smem_u32(&xch_full[quarter]);
+    const uint32_t p_full0 = ako::tc::t2_mapa(ako::smem_u32(&p_full[0]), 0);
+    const uint32_t p_full1 = ako::tc::t2_mapa(ako::smem_u32(&p_full[1]), 0);
+    const float scale = p.scale_log2;
+    float m = NEG, l = 0.f;  // running maximum of the row, sum over this thread's keys
     bool ok = true;
+#pragma unroll 1
     for (int j = 0; j < ntk; ++j) {
       const int buf = j & 1;
-      if (!ako::tc::mbar_wait(ako::smem_u32(&s_full[buf]), (uint32_t)((j >> 1) & 1), &g_pf_status, 3)) { ok = false; break; }
+      if (!ako::tc::mbar_wait_warp(ako::smem_u32(&s_full[buf]), (uint32_t)((j >> 1) & 1), &g_pf_status, 3)) { ok = false; break; }
       ako::tc::fence_after_thread_sync();
       const uint32_t ts = tq + buf * BK;
-      const int nvis = kv_lim - j * BK;  // visible keys of this tile for this row (may be <= 0 or > 128)
-      // no masked key for any row of this warp in this tile; warp-uniform, because the aligned TMEM
-      // loads and stores below must be reached by the whole warp together
-      const bool fast = __all_sync(0xffffffffu, nvis >= BK) && p.scale_log2 > 0.f;
+      float v[2][32];
+      ako::tc::tmem_ld32(ts + 64 * ch, v[0]);
+      ako::tc::tmem_ld32(ts + 64 * ch + 32, v[1]);
+      ako::tc::tmem_ld_wait_regs(v[0]);
+      ako::tc::tmem_ld_wait_regs(v[1]);
+      const int nvis = kv_lim - j * BK - 64 * ch;  // visible keys of this thread's 64 (may be <= 0 or > 64)
+      // no masked key for any row of this warp; warp-uniform, because the aligned TMEM stores below
+      // must be reached by the whole warp together
+      const bool fast = __all_sync(0xffffffffu, nvis >= 64) && scale > 0.f;
       float tmax = NEG;
+      if (fast) {  // four independent chains, the (positive) scale applied once
+        float t[4] = {v[0][0], v[0][1], v[0][2], v[0][3]};
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float v[32];
-        ako::tc::tmem_ld32(ts + 32 * c, v);
-        ako::tc::tmem_ld_wait_regs(v);
-        if (fast) {  // four independent chains, the (positive) scale applied once
-          float t0 = v[0], t1 = v[1], t2 = v[2], t3 = v[3];
+        for (int i = 4; i < 64; ++i) t[i & 3] = fmaxf(t[i & 3], v[i >> 5][i & 31]);
+        tmax = fmaxf(tmax, fmaxf(fmaxf(t[0], t[1]), fmaxf(t[2], t[3])) * scale);
+      } else {
 #pragma unroll
-          for (int i = 4; i < 32; i += 4) {
-            t0 = fmaxf(t0, v[i]);
-            t1 = fmaxf(t1, v[i + 1]);
-            t2 = fmaxf(t2, v[i + 2]);
-            t3 = fmaxf(t3, v[i + 3]);
-          }
-          tmax = fmaxf(tmax, fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)) * p.scale_log2);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) tmax = fmaxf(tmax, (32 * c + i < nvis) ? v[i] * p.scale_log2 : NEG);
-        }
+        for (int i = 0; i < 64; ++i) tmax = fmaxf(tmax, (i < nvis) ? v[i >> 5][i & 31] * scale : NEG);
       }
-      const float m_new = fmaxf(m, tmax);
-      const float alpha = ako::fast_exp2(m - m_new);
-      float sum = 0.f;
+      // the row's other 64 keys belong to the same lane of the other warp of the quarter. Its wait
+      // also says that S has been read by both warps, so P may overwrite it.
+      xch[(buf * 2 + ch) * BM + r] = tmax;
+      ako::tc::fence_before_thread_sync();
+      __syncwarp();
+      if (lane == 0) ako::tc::mbar_arrive(xbar);
+      if (!ako::tc::mbar_wait_warp(xbar, (uint32_t)(j & 1), &g_pf_status, 4)) { ok = false; break; }
+      ako::tc::fence_after_thread_sync();
+      tmax = fmaxf(tmax, xch[(buf * 2 + (ch ^ 1)) * BM + r]);
+      const bool moved = tmax > m;
+      const bool rescale = __any_sync(0xffffffffu, moved);  // the same vote in both warps of the quarter
+      const float alpha = moved ? ako::fast_exp2(m - tmax) : 1.0f;
+      m = fmaxf(m, tmax);
+      l *= alpha;
+      if (fast) {
+        const float2 sc2 = make_float2(scale, scale), nm2 = make_float2(-m, -m);
+        float2 sum[2] = {{0.f, 0.f}, {0.f, 0.f}};
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float v[32];
-        ako::tc::tmem_ld32(ts + 32 * c, v);
-        ako::tc::tmem_ld_wait_regs(v);
-        // P overwrites the S buffer it came from, as bf16 pairs: the 32 columns just read become
-        // columns [16c, 16c+16), all of them read already; the PV MMAs take P from there (A operand
-        // in TMEM), so P never crosses shared memory
-        uint32_t w[16];
-        if (fast) {
-          float s0 = 0.f, s1 = 0.f;
+        for (int h = 0; h < 2; ++h) {
+          uint32_t w[16];
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            const float e0 = ako::fast_exp2(v[i] * p.scale_log2 - m_new);
-            const float e1 = ako::fast_exp2(v[i + 1] * p.scale_log2 - m_new);
-            s0 += e0;
-            s1 += e1;
-            w[i >> 1] = ako::pack_bf16x2(e0, e1);
+            const float2 x = __ffma2_rn(make_float2(v[h][i], v[h][i + 1]), sc2, nm2);
+            const float2 e = make_float2(ako::fast_exp2(x.x), ako::fast_exp2(x.y));
+            sum[(i >> 1) & 1] = __fadd2_rn(sum[(i >> 1) & 1], e);
+            w[i >> 1] = ako::pack_bf16x2(e.x, e.y);
           }
-          sum += s0 + s1;
-        } else {
+          ako::tc::tmem_st16(ts + 32 * ch + 16 * h, w);
+        }
+        l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
+      } else {
+        float sum = 0.f;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t w[16];
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            const float e0 = (32 * c + i < nvis) ? ako::fast_exp2(v[i] * p.scale_log2 - m_new) : 0.f;
-            const float e1 = (32 * c + i + 1 < nvis) ? ako::fast_exp2(v[i + 1] * p.scale_log2 - m_new) : 0.f;
+            const float e0 = (32 * h + i < nvis) ? ako::fast_exp2(v[h][i] * scale - m) : 0.f;
+            const float e1 = (32 * h + i + 1 < nvis) ? ako::fast_exp2(v[h][i + 1] * scale - m) : 0.f;
             sum += e0 + e1;
             w[i >> 1] = ako::pack_bf16x2(e0, e1);
           }
+          ako::tc::tmem_st16(ts + 32 * ch + 16 * h, w);
         }
-        ako::tc::tmem_st16(ts + 16 * c, w);
+        l += sum;
+      }
+      if (rescale && j > 0) {
+        // S of this tile came after PV of tile j-2, so the phase before this one (tile j-3) is over
+        if (!ako::tc::mbar_wait_warp(ako::smem_u32(&pv_done[buf ^ 1]), (uint32_t)(((j - 1) >> 1) & 1), &g_pf_status, 2)) { ok = false; break; }
+        ako::tc::fence_after_thread_sync();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          float o[32];
+          uint32_t w[2][16];
+          ako::tc::tmem_ld32(to + 32 * c, o);
+          ako::tc::tmem_ld_wait_regs(o);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) w[i >> 4][i & 15] = __float_as_uint(o[i] * alpha);
+          ako::tc::tmem_st16(to + 32 * c, w[0]);
+          ako::tc::tmem_st16(to + 32 * c + 16, w[1]);
+        }
       }
       ako::tc::tmem_st_wait();
-      l = l * alpha + sum;
-      m = m_new;
-      alpha_s[(j & 3) * BM + r] = alpha;
       ako::tc::fence_before_thread_sync();
-      // Nothing else holds a fast warp back (tiles without masked keys take the short path, a warp
-      // with masked rows does not), so it may finish tile j before a slow warp has finished tile
-      // j-1; its arrival would then complete the phase of tile j-1 in the slow warp's place. Wait
-      // until all four warps have arrived for tile j-1 before arriving for tile j.
-      if (j > 0 && !ako::tc::mbar_wait(ako::smem_u32(&p_full), (uint32_t)((j - 1) & 1), &g_pf_status, 4)) { ok = false; break; }
       __syncwarp();
-      if (lane == 0) ako::tc::mbar_arrive(ako::smem_u32(&p_full));
+      // One barrier per buffer: a warp can be one tile ahead of another, never two (S of tile j+2
+      // needs PV of tile j), so an arrival cannot complete a phase in a slower warp's place.
+      if (lane == 0) ako::tc::t2_arrive_cluster(buf ? p_full1 : p_full0);
     }
     if (ok && tile >= 0) {
-      fin_l[r] = (kv_lim > 0) ? l : 0.f;
-      if (half == 0 && row_ok)
-        p.lse[(int64_t)(q0 + qtok) * H + (r & 15)] = (kv_lim > 0 && l > 0.f) ? m + log2f(l) : -INFINITY;
+      // the slots of the tile before last: every reader has passed the barrier since
+      xch[((ntk & 1) * 2 + ch) * BM + r] = l;
       __syncwarp();
-      if (lane == 0) ako::tc::mbar_arrive(ako::smem_u32(&fin));
-    }
-  } else {
-    ako::tc::reg_dec<REGS_OTHER>();
-    if (warp == 12 && lane == 0 && ntk > 0) {
-      // ================================ Q / K producer =========================================
-      ako::tc::tma_prefetch_desc(&tm_qn);
-      ako::tc::tma_prefetch_desc(&tm_qp);
-      ako::tc::tma_prefetch_desc(&tm_k);
-      int g = 0;
-      for (int j = 0; j < ntk; ++j) {
-        bool ok = true;
-        for (int c = 0; c < NCH; ++c, ++g) {
-          const int stage = g % NST;
-          if (!ako::tc::mbar_wait(ako::smem_u32(&st_empty[stage]), (uint32_t)(((g / NST) & 1) ^ 1), &g_pf_status, 5)) { ok = false; break; }
-          const uint32_t bar = ako::smem_u32(&st_full[stage]);
-          const uint32_t dst = st_base + stage * ST_BYTES;
-          ako::tc::mbar_arrive_expect_tx(bar, ST_BYTES);
-          if (c < DC / 64) ako::tc::tma_load_2d(dst, &tm_qn, c * 64, q0 * H, bar);
-          else ako::tc::tma_load_2d(dst, &tm_qp, 0, q0 * H, bar);
-          ako::tc::tma_load_2d(dst + CH_BYTES, &tm_k, c * 64, (int)(kbase + (int64_t)j * BK), bar);
-        }
-        if (!ok) break;
-      }
-    } else if (warp == 14 && lane == 0 && ntk > 0) {
-      // ================================ V producer ==============================================
-      ako::tc::tma_prefetch_desc(&tm_v);
-      for (int j = 0; j < ntk; ++j) {
-        if (!ako::tc::mbar_wait(ako::smem_u32(&v_empty), (uint32_t)((j & 1) ^ 1), &g_pf_status, 6)) break;
-        const uint32_t bar = ako::smem_u32(&v_full);
-        ako::tc::mbar_arrive_expect_tx(bar, V_BYTES);
-        const int x = (int)(vbase + (int64_t)j * BK);
-        ako::tc::tma_load_2d(v_base, &tm_v, x, half * 256, bar);
-        ako::tc::tma_load_2d(v_base + V_BYTES / 2, &tm_v, x + 64, half * 256, bar);
-      }
-    } else if (warp == 13 && lane == 0 && ntk > 0) {
-      // ================================ S issuer ================================================
-      constexpr uint32_t IDESC_S = ako::tc::idesc_bf16_f32(BM, BK);
-      const uint32_t st_lo0 = ako::tc::smem_desc_lo(st_base);
-      int g = 0;
-      for (int j = 0; j < ntk; ++j) {
-        const int buf = j & 1;
-        // the PV MMAs of tile j-2 have read P out of this buffer
-        if (!ako::tc::mbar_wait(ako::smem_u32(&s_empty[buf]), (uint32_t)(((j >> 1) & 1) ^ 1), &g_pf_status, 7)) break;
-        const uint32_t d = tmem + buf * BK;
-        bool ok = true;
-        for (int c = 0; c < NCH; ++c, ++g) {
-          const int stage = g % NST;
-          if (!ako::tc::mbar_wait(ako::smem_u32(&st_full[stage]), (uint32_t)((g / NST) & 1), &g_pf_status, 8)) { ok = false; break; }
-          ako::tc::fence_after_thread_sync();
-          const uint32_t a_lo = st_lo0 + stage * (ST_BYTES >> 4);
-          const uint32_t b_lo = a_lo + (CH_BYTES >> 4);
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            ako::tc::mma_bf16_lohi(d, a_lo + 2 * ks, b_lo + 2 * ks, IDESC_S, (c > 0 || ks > 0) ? 1u : 0u);
-          ako::tc::mma_commit(ako::smem_u32(&st_empty[stage]));
-        }
-        if (!ok) break;
-        ako::tc::mma_commit(ako::smem_u32(&s_full[buf]));
-      }
-    } else if (warp == 15 && lane == 0 && ntk > 0) {
-      // ================================ PV issuer ===============================================
-      // a thread of its own: PV of tile j goes to the tensor pipe the moment P is written, while
-      // the S issuer is still waiting on the operand stream of a later tile
-      constexpr uint32_t IDESC_PV = ako::tc::idesc_bf16_f32(BM, 256);
-      const uint32_t v_lo0 = ako::tc::smem_desc_lo(v_base);
-      for (int j = 0; j < ntk; ++j) {
-        if (!ako::tc::mbar_wait(ako::smem_u32(&p_full), (uint32_t)(j & 1), &g_pf_status, 9)) break;
-        if (!ako::tc::mbar_wait(ako::smem_u32(&v_full), (uint32_t)(j & 1), &g_pf_status, 10)) break;
-        if (!ako::tc::mbar_wait(ako::smem_u32(&pv_empty), (uint32_t)((j & 1) ^ 1), &g_pf_status, 11)) break;
+      if (lane == 0) ako::tc::mbar_arrive(xbar);
+      if (ako::tc::mbar_wait_warp(xbar, (uint32_t)(ntk & 1), &g_pf_status, 1) &&
+          (ntk == 0 || ako::tc::mbar_wait_warp(ako::smem_u32(&pv_done[(ntk - 1) & 1]), (uint32_t)(((ntk - 1) >> 1) & 1), &g_pf_status, 12))) {
         ako::tc::fence_after_thread_sync();
-        const uint32_t d = tmem + 256;
+        // summed in the order of the keys by both threads of the row
+        l = xch[(ntk & 1) * 2 * BM + r] + xch[((ntk & 1) * 2 + 1) * BM + r];
+        if (kv_lim <= 0) l = 0.f;
+        const float inv = (l > 0.f) ? 1.0f / l : 0.f;
+        if (half == 0 && ch == 0 && row_ok)
+          p.lse[(int64_t)(q0 + qtok) * H + (r & 15)] = (l > 0.f) ? m + log2f(l) : -INFINITY;
+        __nv_bfloat16* dst = p.o + ((int64_t)(q0 + qtok) * H + (r & 15)) * DC + half * 256 + ch * 128;
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          float o[32];
+          if (ntk > 0) {
+            ako::tc::tmem_ld32(to + 32 * c, o);
+            ako::tc::tmem_ld_wait_regs(o);
+          } else {
 #pragma unroll
-        for (int at = 0; at < 2; ++at)
+            for (int i = 0; i < 32; ++i) o[i] = 0.f;
+          }
+          if (row_ok) {
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            ako::tc::mma_bf16_tmem_a(d, tmem + (j & 1) * BK + 8 * (4 * at + ks), v_lo0 + at * ((V_BYTES / 2) >> 4) + 2 * ks,
-                                     IDESC_PV, (at > 0 || ks > 0) ? 1u : 0u);
-        ako::tc::mma_commit(ako::smem_u32(&pv_full));
-        ako::tc::mma_commit(ako::smem_u32(&v_empty));
-        ako::tc::mma_commit(ako::smem_u32(&s_empty[j & 1]));  // P (inside the S buffer) has been read
+            for (int i = 0; i < 32; i += 8) {
+              uint4 w;
+              w.x = ako::pack_bf16x2(o[i] * inv, o[i + 1] * inv);
+              w.y = ako::pack_bf16x2(o[i + 2] * inv, o[i + 3] * inv);
+              w.z = ako::pack_bf16x2(o[i + 4] * inv, o[i + 5] * inv);
+              w.w = ako::pack_bf16x2(o[i + 6] * inv, o[i + 7] * inv);
+              *reinterpret_cast<uint4*>(dst + 32 * c + i) = w;
+            }
+          }
+        }
       }
+    }
+  } else if (warp == 8 && lane == 0 && ntk > 0) {
+    // ================================ Q / K producer (each CTA its rows and keys) ================
+    ako::tc::tma_prefetch_desc(&tm_qn);
+    ako::tc::tma_prefetch_desc(&tm_qp);
+    ako::tc::tma_prefetch_desc(&tm_k);
+    int g = 0;
+    bool ok = true;
+    for (int j = 0; ok && j < ntk; ++j) {
+      for (int c = 0; c < NCH; ++c, ++g) {
+        const int stage = g % NST;
+        if (!ako::tc::mbar_wait(ako::smem_u32(&st_empty[stage]), (uint32_t)(((g / NST) & 1) ^ 1), &g_pf_status, 5)) { ok = false; break; }
+        const uint32_t bar = ako::tc::t2_mapa(ako::smem_u32(&st_full[stage]), 0);
+        // the even CTA announces the bytes of both; the first tile's stages bring the Q chunk along
+        if (crank == 0)
+          ako::tc::mbar_arrive_expect_tx(ako::smem_u32(&st_full[stage]), 2 * (K_CH_BYTES + (j == 0 ? Q_CH_BYTES : 0)));
+        if (j == 0) {
+          if (c < DC / 64) ako::tc::t2_tma_load_2d(q_base + c * Q_CH_BYTES, &tm_qn, c * 64, q0 * H, bar);
+          else ako::tc::t2_tma_load_2d(q_base + c * Q_CH_BYTES, &tm_qp, 0, q0 * H, bar);
+        }
+        ako::tc::t2_tma_load_2d(k_base + stage * K_CH_BYTES, &tm_k, c * 64, (int)(kbase + (int64_t)j * BK + crank * (BK / 2)), bar);
+      }
+    }
+  } else if (warp == 10 && lane == 0 && ntk > 0) {
+    // ================================ V producer (each CTA its 128 columns) ======================
+    ako::tc::tma_prefetch_desc(&tm_v);
+    const uint32_t bar = ako::tc::t2_mapa(ako::smem_u32(&v_full), 0);
+    const int x = half * 256 + crank * 128;
+    for (int j = 0; j < ntk; ++j) {
+      if (j > 0 && !ako::tc::mbar_wait(ako::smem_u32(&pv_done[(j - 1) & 1]), (uint32_t)(((j - 1) >> 1) & 1), &g_pf_status, 6)) break;
+      if (crank == 0) ako::tc::mbar_arrive_expect_tx(ako::smem_u32(&v_full), 2 * V_BYTES);
+      const int y = (int)(kbase + (int64_t)j * BK);
+      ako::tc::t2_tma_load_2d(v_base, &tm_v, x, y, bar);
+      ako::tc::t2_tma_load_2d(v_base + V_BOX_BYTES, &tm_v, x + 64, y, bar);
+    }
+  } else if (warp == 9 && lane == 0 && crank == 0 && ntk > 0) {
+    // ================================ S issuer (for the pair) ====================================
+    constexpr uint32_t IDESC_S = ako::tc::idesc_bf16_f32(2 * BM, BK);
+    const uint32_t q_lo = ako::tc::smem_desc_lo(q_base), k_lo = ako::tc::smem_desc_lo(k_base);
+    int stage = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int j = 0; ok && j < ntk; ++j) {
+      const int buf = j & 1;
+      // the PV MMAs of tile j-2 have read P out of this buffer
+      if (!ako::tc::mbar_wait(ako::smem_u32(&pv_done[buf]), (uint32_t)(((j >> 1) & 1) ^ 1), &g_pf_status, 7)) break;
+      const uint32_t d = tmem + buf * BK;
+      for (int c = 0; c < NCH; ++c) {
+        if (!ako::tc::mbar_wait(ako::smem_u32(&st_full[stage]), ph, &g_pf_status, 8)) { ok = false; break; }
+        ako::tc::fence_after_thread_sync();
+        const uint32_t a_lo = q_lo + c * (Q_CH_BYTES >> 4);
+        const uint32_t b_lo = k_lo + stage * (K_CH_BYTES >> 4);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          ako::tc::t2_mma_bf16(d, a_lo + 2 * ks, b_lo + 2 * ks, IDESC_S, (c > 0 || ks > 0) ? 1u : 0u);
+        ako::tc::t2_commit_both(ako::smem_u32(&st_empty[stage]));
+        if (++stage == NST) { stage = 0; ph ^= 1u; }
+      }
+      if (ok) ako::tc::t2_commit_both(ako::smem_u32(&s_full[buf]));
+    }
+  } else if (warp == 11 && lane == 0 && crank == 0 && ntk > 0) {
+    // ================================ PV issuer (for the pair) ===================================
+    // a thread of its own: PV of tile j goes to the tensor pipe the moment P is written, while
+    // the S issuer is still waiting on the operand stream of a later tile
+    constexpr uint32_t IDESC_PV = ako::tc::idesc_bf16_f32(2 * BM, 256) | ako::tc::kIdescBMnMajor;
+    const uint32_t v_lo = ako::tc::smem_desc_lo_mn(v_base, V_BOX_BYTES);
+    const uint32_t d = tmem + 256;
+    for (int j = 0; j < ntk; ++j) {
+      const int buf = j & 1;
+      if (!ako::tc::mbar_wait(ako::smem_u32(&p_full[buf]), (uint32_t)((j >> 1) & 1), &g_pf_status, 9)) break;
+      if (!ako::tc::mbar_wait(ako::smem_u32(&v_full), (uint32_t)(j & 1), &g_pf_status, 10)) break;
+      ako::tc::fence_after_thread_sync();
+#pragma unroll
+      for (int ks = 0; ks < BK / 16; ++ks)  // 16 keys = two 8-row groups of 1024 bytes
+        ako::tc::t2_mma_bf16_tmem_a(d, tmem + buf * BK + 8 * ks, v_lo + ks * (2048 >> 4), IDESC_PV, (j > 0 || ks > 0) ? 1u : 0u);
+      // P (inside the S buffer) and V have been read, O is up to date. Both CTAs wait for the last of
+      // these, so no signal is on its way to a CTA that leaves.
+      ako::tc::t2_commit_both(ako::smem_u32(&pv_done[buf]));
     }
   }
 
   ako::tc::fence_before_thread_sync();
   __syncthreads();
+  ako::tc::t2_cluster_sync();  // the peer may still be reading this CTA's shared memory or writing its TMEM
   if (tid == 0) {
     const int code = *reinterpret_cast<volatile int*>(&g_pf_status);
     if (code != 0) atomicCAS(&g_pf_sticky, 0, code);
   }
-  if (warp == 13) {
+  if (warp == 9) {
     ako::tc::fence_after_thread_sync();
-    ako::tc::tmem_dealloc(tmem, 512);
+    ako::tc::t2_tmem_dealloc(tmem, 512);
   }
 }
-
-int64_t vt_columns(int64_t ntok, int64_t batch) { return ((ntok + 8 * batch + 8 + 7) / 8) * 8; }
 
 }  // namespace
 
 size_t ako_mla_prefill_tc_workspace_bytes(int64_t batch, int64_t num_kv_indices, int64_t page_size) {
   const int64_t ntok = num_kv_indices * page_size;
   if (ntok <= 0 || batch <= 0) return 0;
-  const size_t kc = ((size_t)ntok * DQK * 2 + 255) / 256 * 256;
-  const size_t vt = (size_t)DC * vt_columns(ntok, batch) * 2;
-  return kc + vt;
+  return ((size_t)ntok * DQK * 2 + 255) / 256 * 256;
 }
 
 int ako_mla_prefill_tc_launch(const void* q_nope, const void* q_pe, const void* ckv_cache, const void* kpe_cache,
@@ -461,21 +441,16 @@ int ako_mla_prefill_tc_launch(const void* q_nope, const void* q_pe, const void* 
   if (ntok <= 0 || ntok > 0x7fffffffLL || total_q * H > 0x7fffffffLL) return AKO4X_EUNSUPPORTED_SHAPE;
   const size_t need = ako_mla_prefill_tc_workspace_bytes(batch, num_kv_indices, page_size);
   if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255)) return AKO4X_EWORKSPACE;
-  const int64_t W = vt_columns(ntok, batch);
   unsigned char* kc = (unsigned char*)workspace;
-  unsigned char* vt = kc + ((size_t)ntok * DQK * 2 + 255) / 256 * 256;
-  // the gaps between sequences in Vt are multiplied by P = 0: they must hold finite values
-  if (cudaMemsetAsync(vt, 0, (size_t)DC * W * 2, st) != cudaSuccess) return AKO4X_ELAUNCH;
   mla_prefill_gather_kernel<<<(unsigned)ako::cdiv(ntok, G_TOK), 256, 0, st>>>(
-      (const uint4*)ckv_cache, (const uint4*)kpe_cache, kv_indices, kv_indptr, (int)batch, (int)page_size, ntok,
-      (uint4*)kc, (__nv_bfloat16*)vt, W);
+      (const uint4*)ckv_cache, (const uint4*)kpe_cache, kv_indices, (int)page_size, ntok, (uint4*)kc);
   AKO_CHECK_LAUNCH();
 
   CUtensorMap tm_qn, tm_qp, tm_k, tm_v;
   if (!ako::tma::bf16_matrix_map(&tm_qn, q_nope, (uint64_t)total_q * H, DC, DC * 2, BM) ||
       !ako::tma::bf16_matrix_map(&tm_qp, q_pe, (uint64_t)total_q * H, DP, DP * 2, BM) ||
-      !ako::tma::bf16_matrix_map(&tm_k, kc, (uint64_t)ntok, DQK, DQK * 2, BK) ||
-      !ako::tma::bf16_matrix_map(&tm_v, vt, DC, (uint64_t)W, (uint64_t)W * 2, 256))
+      !ako::tma::bf16_matrix_map(&tm_k, kc, (uint64_t)ntok, DQK, DQK * 2, BK / 2) ||
+      !ako::tma::bf16_matrix_map(&tm_v, kc, (uint64_t)ntok, DQK, DQK * 2, BK))
     return AKO4X_ELAUNCH;
   if (!ako::ensure_dynamic_smem<mla_prefill_tc_kernel>(SMEM)) return AKO4X_ELAUNCH;
   PfParams p;
@@ -486,9 +461,19 @@ int ako_mla_prefill_tc_launch(const void* q_nope, const void* q_pe, const void* 
   p.scale_log2 = sm_scale * 1.4426950408889634f;
   p.batch = (int)batch;
   p.page_size = (int)page_size;
-  const dim3 grid((unsigned)(ako::cdiv(total_q, QT) + batch), 2);
-  mla_prefill_tc_kernel<<<grid, THREADS, SMEM, st>>>(p, tm_qn, tm_qp, tm_k, tm_v);
-  AKO_CHECK_LAUNCH();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * (ako::cdiv(total_q, PT) + batch)), 2);
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, mla_prefill_tc_kernel, p, tm_qn, tm_qp, tm_k, tm_v) != cudaSuccess) return AKO4X_ELAUNCH;
   return AKO4X_OK;
 }
 

@@ -22,60 +22,6 @@ constexpr int T2_B_BYTES = 128 * 128;                    // this CTA's half of t
 constexpr int T2_STAGE_BYTES = TC_A_BYTES + T2_B_BYTES;  // 32 KB
 constexpr int T2_SMEM = T2_STAGES * T2_STAGE_BYTES + TC_EXTRA_BYTES + 1024;
 
-__device__ __forceinline__ uint32_t t2_cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void t2_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-// shared::cluster address of `addr` (a shared::cta address of this CTA's layout) in CTA `rank`
-__device__ __forceinline__ uint32_t t2_mapa(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-// Arrival on a barrier of the pair's even CTA. Relaxed: what the barrier orders here is TMEM traffic
-// (the tcgen05.ld of this thread's warp against the next MMA into the buffer), which the
-// tcgen05 fences around the arrival and the wait take care of; a release at cluster scope measured
-// 1 500 - 2 400 cycles per arrival, once per warp and K block.
-__device__ __forceinline__ void t2_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void t2_tmem_alloc(uint32_t dst_smem, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(dst_smem), "r"(cols) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ void t2_tmem_dealloc(uint32_t taddr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(cols) : "memory");
-}
-// 2-D tiled load into this CTA's shared memory, bytes counted on the mbarrier at cluster address `bar`
-__device__ __forceinline__ void t2_tma_load_2d(uint32_t dst, const void* tmap, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n" ::
-          "r"(dst),
-      "l"(tmap), "r"(bar), "r"(x), "r"(y)
-      : "memory");
-}
-template <bool ACCUMULATE>
-__device__ __forceinline__ void t2_mma_f8(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
-  asm volatile(
-      "{\n.reg .b64 da, db;\n.reg .pred p;\n"
-      "mov.b64 da, {%1, %4};\n"
-      "mov.b64 db, {%2, %4};\n"
-      "setp.ne.b32 p, %5, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], da, db, %3, p;\n}\n" ::"r"(d_tmem),
-      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(ako::tc::kSmemDescHiSw128), "n"(ACCUMULATE ? 1 : 0)
-      : "memory");
-}
-// arrives (once) on the mbarrier at the same shared-memory offset in both CTAs of the pair
-__device__ __forceinline__ void t2_commit_both(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(bar),
-               "h"((unsigned short)3)
-               : "memory");
-}
-
 // tile = (expert, n-tile, m-tile pair), m-pair fastest; CTA `crank` owns m-tile 2 * mp + crank
 template <int NT_TILES>
 __device__ __forceinline__ TileInfo t2_tile_info(const GemmParams& p, const int* s_cum, int tile, int crank) {
@@ -109,7 +55,7 @@ moe_gemm_tc2_kernel(GemmParams p, const __grid_constant__ CUtensorMap tm_a, cons
   __shared__ int s_cum[MAX_LOCAL + 1];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int crank = (int)t2_cluster_ctarank();
+  const int crank = (int)ako::tc::t2_cluster_ctarank();
   const int pair_id = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const uint32_t smem_base = (ako::smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char* extra = smem_raw + (smem_base - ako::smem_u32(smem_raw)) + T2_STAGES * T2_STAGE_BYTES;
@@ -127,7 +73,7 @@ moe_gemm_tc2_kernel(GemmParams p, const __grid_constant__ CUtensorMap tm_a, cons
     }
     ako::tc::mbar_init_fence();
   }
-  if (warp == 8) t2_tmem_alloc(ako::smem_u32(&s_tmem_base), TC_TMEM_COLS);
+  if (warp == 8) ako::tc::t2_tmem_alloc(ako::smem_u32(&s_tmem_base), TC_TMEM_COLS);
   ako::pdl_wait();
   ako::pdl_trigger();
   if (tid == 0) {
@@ -140,13 +86,13 @@ moe_gemm_tc2_kernel(GemmParams p, const __grid_constant__ CUtensorMap tm_a, cons
   }
   ako::tc::fence_before_thread_sync();
   __syncthreads();
-  t2_cluster_sync();   // both CTAs' barriers are initialised before anybody signals across
+  ako::tc::t2_cluster_sync();   // both CTAs' barriers are initialised before anybody signals across
   ako::tc::fence_after_thread_sync();
   const uint32_t tmem_base = s_tmem_base;
   const int total_tiles = s_cum[p.n_local] * NT_TILES;
   // the even CTA's barriers, as seen from this CTA
-  const uint32_t acc_empty_leader0 = t2_mapa(ako::smem_u32(&s_acc_empty[0]), 0);
-  const uint32_t acc_empty_leader1 = t2_mapa(ako::smem_u32(&s_acc_empty[1]), 0);
+  const uint32_t acc_empty_leader0 = ako::tc::t2_mapa(ako::smem_u32(&s_acc_empty[0]), 0);
+  const uint32_t acc_empty_leader1 = ako::tc::t2_mapa(ako::smem_u32(&s_acc_empty[1]), 0);
 
   if (warp >= 10) {
     ako::tc::reg_dec<TC_REGS_OTHER>();  // donor warps
@@ -166,18 +112,18 @@ moe_gemm_tc2_kernel(GemmParams p, const __grid_constant__ CUtensorMap tm_a, cons
           if (!ako::tc::mbar_wait(ako::smem_u32(&s_empty[stage]), ph ^ 1u, p.error, kErrLoad)) { ok = false; break; }
           const uint32_t sa = smem_base + stage * T2_STAGE_BYTES;
           const uint32_t sb = sa + TC_A_BYTES;
-          const uint32_t bar = t2_mapa(ako::smem_u32(&s_full[stage]), 0);
+          const uint32_t bar = ako::tc::t2_mapa(ako::smem_u32(&s_full[stage]), 0);
           // the even CTA announces the bytes of BOTH CTAs; the odd CTA's copies only count down
           if (crank == 0) ako::tc::mbar_arrive_expect_tx(ako::smem_u32(&s_full[stage]), 2 * T2_STAGE_BYTES);
-          t2_tma_load_2d(sa, &tm_a, kb * 128, ti.row0, bar);
+          ako::tc::t2_tma_load_2d(sa, &tm_a, kb * 128, ti.row0, bar);
           if (WHICH == 1) {
             // rows of the 256-row weight tile: [g1 0-63 | g2 0-63 | g1 64-127 | g2 64-127]; this CTA
             // loads the two 64-row boxes of its half
             const int wr = ti.e * (2 * INTER) + ti.nt * 128 + 64 * crank;
-            t2_tma_load_2d(sb, &tm_b, kb * 128, wr, bar);
-            t2_tma_load_2d(sb + 64 * 128, &tm_b, kb * 128, wr + INTER, bar);
+            ako::tc::t2_tma_load_2d(sb, &tm_b, kb * 128, wr, bar);
+            ako::tc::t2_tma_load_2d(sb + 64 * 128, &tm_b, kb * 128, wr + INTER, bar);
           } else {
-            t2_tma_load_2d(sb, &tm_b, (kb & 15) * 128, ti.e * HID + ti.nt * TC_BN + 128 * crank, bar);
+            ako::tc::t2_tma_load_2d(sb, &tm_b, (kb & 15) * 128, ti.e * HID + ti.nt * TC_BN + 128 * crank, bar);
           }
         }
       }
@@ -201,12 +147,12 @@ moe_gemm_tc2_kernel(GemmParams p, const __grid_constant__ CUtensorMap tm_a, cons
           const uint32_t a_lo = a_lo0 + stage * (T2_STAGE_BYTES >> 4);
           const uint32_t b_lo = b_lo0 + stage * (T2_STAGE_BYTES >> 4);
           const uint32_t d = tmem_base + buf * TC_BN;
-          t2_mma_f8<false>(d, a_lo, b_lo, IDESC);
-          t2_mma_f8<true>(d, a_lo + 2, b_lo + 2, IDESC);
-          t2_mma_f8<true>(d, a_lo + 4, b_lo + 4, IDESC);
-          t2_mma_f8<true>(d, a_lo + 6, b_lo + 6, IDESC);
-          t2_commit_both(ako::smem_u32(&s_empty[stage]));
-          t2_commit_both(ako::smem_u32(&s_acc_full[buf]));
+          ako::tc::t2_mma_f8<false>(d, a_lo, b_lo, IDESC);
+          ako::tc::t2_mma_f8<true>(d, a_lo + 2, b_lo + 2, IDESC);
+          ako::tc::t2_mma_f8<true>(d, a_lo + 4, b_lo + 4, IDESC);
+          ako::tc::t2_mma_f8<true>(d, a_lo + 6, b_lo + 6, IDESC);
+          ako::tc::t2_commit_both(ako::smem_u32(&s_empty[stage]));
+          ako::tc::t2_commit_both(ako::smem_u32(&s_acc_full[buf]));
           if (++stage == T2_STAGES) { stage = 0; ph ^= 1u; }
         }
       }
@@ -270,7 +216,7 @@ moe_gemm_tc2_kernel(GemmParams p, const __grid_constant__ CUtensorMap tm_a, cons
         ako::tc::tmem_ld_wait_regs(v1);
         ako::tc::fence_before_thread_sync();
         __syncwarp();
-        if (lane == 0) t2_arrive_cluster(buf ? acc_empty_leader1 : acc_empty_leader0);
+        if (lane == 0) ako::tc::t2_arrive_cluster(buf ? acc_empty_leader1 : acc_empty_leader0);
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
           acc[64 + j] = fmaf(v0[j], s1, acc[64 + j]);
@@ -359,9 +305,9 @@ moe_gemm_tc2_kernel(GemmParams p, const __grid_constant__ CUtensorMap tm_a, cons
   // ================================ common exit ================================================
   ako::tc::fence_before_thread_sync();
   __syncthreads();
-  t2_cluster_sync();   // the peer may still be reading this CTA's shared memory or writing its TMEM
+  ako::tc::t2_cluster_sync();   // the peer may still be reading this CTA's shared memory or writing its TMEM
   if (warp == 8) {
     ako::tc::fence_after_thread_sync();
-    t2_tmem_dealloc(tmem_base, TC_TMEM_COLS);
+    ako::tc::t2_tmem_dealloc(tmem_base, TC_TMEM_COLS);
   }
 }

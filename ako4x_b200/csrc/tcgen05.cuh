@@ -164,8 +164,9 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n) {
 __device__ __forceinline__ uint32_t smem_desc_lo_mn(uint32_t saddr, uint32_t lbo_bytes) {
   return ((saddr >> 4) & 0x3FFFu) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
 }
-// Instruction descriptor bit that declares the A operand MN-major.
+// Instruction descriptor bits that declare the A or the B operand MN-major.
 constexpr uint32_t kIdescAMnMajor = 1u << 15;
+constexpr uint32_t kIdescBMnMajor = 1u << 16;
 __device__ __forceinline__ void mma_bf16_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
                                               uint32_t accumulate) {
   asm volatile(
@@ -258,6 +259,84 @@ __device__ __forceinline__ void mma_bf16_tmem_a(uint32_t d_tmem, uint32_t a_tmem
       "mov.b64 db, {%2, %4};\n"
       "setp.ne.b32 p, %5, 0;\n"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(kSmemDescHiSw128), "r"(accumulate)
+      : "memory");
+}
+
+// ---- CTA pairs (cta_group::2, a cluster of two) ---------------------------------------------------
+__device__ __forceinline__ uint32_t t2_cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void t2_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// shared::cluster address of `addr` (a shared::cta address of this CTA's layout) in CTA `rank`
+__device__ __forceinline__ uint32_t t2_mapa(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// Arrival on a barrier of the pair's even CTA. Relaxed: what the barrier orders here is TMEM traffic
+// (the tcgen05.ld of this thread's warp against the next MMA into the buffer), which the
+// tcgen05 fences around the arrival and the wait take care of; a release at cluster scope measured
+// 1 500 - 2 400 cycles per arrival, once per warp and K block.
+__device__ __forceinline__ void t2_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void t2_tmem_alloc(uint32_t dst_smem, uint32_t cols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(dst_smem), "r"(cols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ void t2_tmem_dealloc(uint32_t taddr, uint32_t cols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(cols) : "memory");
+}
+// 2-D tiled load into this CTA's shared memory, bytes counted on the mbarrier at cluster address `bar`
+__device__ __forceinline__ void t2_tma_load_2d(uint32_t dst, const void* tmap, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n" ::
+          "r"(dst),
+      "l"(tmap), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+template <bool ACCUMULATE>
+__device__ __forceinline__ void t2_mma_f8(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
+  asm volatile(
+      "{\n.reg .b64 da, db;\n.reg .pred p;\n"
+      "mov.b64 da, {%1, %4};\n"
+      "mov.b64 db, {%2, %4};\n"
+      "setp.ne.b32 p, %5, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], da, db, %3, p;\n}\n" ::"r"(d_tmem),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kSmemDescHiSw128), "n"(ACCUMULATE ? 1 : 0)
+      : "memory");
+}
+// arrives (once) on the mbarrier at the same shared-memory offset in both CTAs of the pair
+__device__ __forceinline__ void t2_commit_both(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(bar),
+               "h"((unsigned short)3)
+               : "memory");
+}
+
+// bf16 operands over the pair: A and B from shared memory, and A from TMEM (each CTA's own lanes).
+__device__ __forceinline__ void t2_mma_bf16(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .b64 da, db;\n.reg .pred p;\n"
+      "mov.b64 da, {%1, %4};\n"
+      "mov.b64 db, {%2, %4};\n"
+      "setp.ne.b32 p, %5, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n}\n" ::"r"(d_tmem),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kSmemDescHiSw128), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void t2_mma_bf16_tmem_a(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc,
+                                                   uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .b64 db;\n.reg .pred p;\n"
+      "mov.b64 db, {%2, %4};\n"
+      "setp.ne.b32 p, %5, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], db, %3, p;\n}\n" ::"r"(d_tmem),
       "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(kSmemDescHiSw128), "r"(accumulate)
       : "memory");
 }

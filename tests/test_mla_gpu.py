@@ -127,6 +127,17 @@ def test_prefill_tensor_core_path(built_lib, q_lens, kv_lens):
                               extra_pages=17))
 
 
+@pytest.mark.parametrize("q_lens,kv_lens,sign", [([64], [1500], 1.0), ([9, 40], [640, 129], 1.0), ([64], [1500], -1.0)])
+def test_prefill_row_maximum_moves(built_lib, q_lens, kv_lens, sign):
+    """Scores that grow along the keys (and, with the sign, fall): the reference maximum of a row
+    moves several times, so the accumulated output is rescaled in the middle of the key loop."""
+    a = W.make_mla_prefill(len(q_lens), shape_id=11, q_lens=q_lens, kv_lens=kv_lens, extra_pages=5)
+    a["q_pe"] = torch.ones_like(a["q_pe"]) * sign
+    ramp = torch.cat([torch.arange(n) / 100.0 for n in kv_lens])    # 64 x ramp x sm_scale: up to 69, or 100 in log2
+    a["kpe_cache"].view(-1, 64)[a["kv_indices"].long()] = ramp[:, None].expand(-1, 64).to(torch.bfloat16)
+    _check(mla_prefill, oracle.mla_paged_prefill, PKEYS, a)
+
+
 @pytest.mark.parametrize("q_len", [20, 100])
 def test_prefill_page_size_4(built_lib, q_len):
     """Pages of four tokens (kv_len = pages x 4), on the small-call kernel and on the tensor-core one."""
