@@ -2,9 +2,10 @@
 // the operand type: the operator family reference/gemm-n2048-k4096 (N = 2048, K = 4096, M from 1
 // to 16 294; the reference's campaign ended with cuBLAS as its best implementation, README.md of
 // that folder). Hand-written for sm_100a:
-//   * persistent CTAs, one per SM, over output tiles of 128 rows x BN columns (BN = 256, 128 or 32
-//     chosen by how many tiles M gives), n fastest so that the CTAs sharing an A tile run side by
-//     side and A crosses HBM once (B, 16 MB, stays in L2);
+//   * persistent CTAs, one per SM, over output tiles of 128 rows x BN columns, or pairs of CTAs
+//     (cta_group::2) over tiles of 256 rows x BN columns (BN = 256, 128 or 32, gemm_plan below), n
+//     fastest so that the CTAs sharing an A tile run side by side and A crosses HBM once (B, 16 MB,
+//     stays in L2). Each CTA of a pair brings its own rows of A and half of B;
 //   * a TMA producer warp fills a ring of K = 64 slices (128-byte-swizzled boxes of A and B);
 //   * one thread issues tcgen05.mma kind::f16 (M128 x BN x K16) into one of TWO TMEM accumulators,
 //     the whole K dimension per tile, so no partial sums leave TMEM;
@@ -16,6 +17,9 @@
 // CTAs per tile and a second kernel sums the fp32 partial products (gemm_plan below).
 // Every wait is bounded; a wait that gives up records its code in the status word below and the
 // CTA unwinds through the common exit that frees TMEM.
+#include <algorithm>
+#include <atomic>
+
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include "tma_host.cuh"
@@ -28,11 +32,13 @@ enum { kErrGLoad = 71, kErrGMma = 72, kErrGAcc = 73, kErrGEpi = 74 };
 
 __device__ int g_gemm_status;
 
-template <int BN>
+// CG: CTAs per tile. A pair (2) computes 256 rows, 128 per CTA, and each CTA brings half of B.
+template <int BN, int CG>
 struct GemmCfg {
-  static constexpr int B_BYTES = BN * G_BK_BYTES;
+  static constexpr int B_ROWS = BN / CG;
+  static constexpr int B_BYTES = B_ROWS * G_BK_BYTES;
   static constexpr int STAGE_BYTES = G_A_BYTES + B_BYTES;
-  static constexpr int STAGES = (BN == 256) ? 4 : (BN == 128) ? 6 : 8;
+  static constexpr int STAGES = (STAGE_BYTES >= 48 * 1024) ? 4 : (STAGE_BYTES >= 32 * 1024) ? 6 : 8;
   static constexpr int TMEM_COLS = (2 * BN < 32) ? 32 : 2 * BN;
   static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024;
 };
@@ -50,12 +56,12 @@ struct GemmArgs {
   int splits;       // CTAs that share one output tile, each over k / splits of the reduction
 };
 
-template <int BN, bool BF16>
+template <int BN, bool BF16, int CG>
 __global__ void __launch_bounds__(G_THREADS, 1)
 gemm_f16_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b) {
-  using Cfg = GemmCfg<BN>;
+  using Cfg = GemmCfg<BN, CG>;
   constexpr int STAGES = Cfg::STAGES;
-  constexpr uint32_t IDESC = idesc_f16(G_BM, BN, BF16);
+  constexpr uint32_t IDESC = idesc_f16(CG * G_BM, BN, BF16);
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t s_full[STAGES];
   __shared__ __align__(8) uint64_t s_empty[STAGES];
@@ -65,6 +71,8 @@ gemm_f16_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tm_a, const _
   __shared__ int s_err;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int crank = (CG == 2) ? (int)ako::tc::t2_cluster_ctarank() : 0;
+  const int worker = blockIdx.x / CG, workers = gridDim.x / CG;
   const uint32_t smem_base = (ako::smem_u32(smem_raw) + 1023u) & ~1023u;
   if (tid == 0) {
     s_err = 0;
@@ -74,79 +82,105 @@ gemm_f16_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tm_a, const _
     }
     for (int b = 0; b < 2; ++b) {
       ako::tc::mbar_init(ako::smem_u32(&s_acc_full[b]), 1);
-      ako::tc::mbar_init(ako::smem_u32(&s_acc_empty[b]), 4);   // one elected arrival per epilogue warp
+      ako::tc::mbar_init(ako::smem_u32(&s_acc_empty[b]), 4 * CG);   // one elected arrival per epilogue warp (even CTA: of both)
     }
     ako::tc::mbar_init_fence();
   }
-  if (warp == 4) ako::tc::tmem_alloc(ako::smem_u32(&s_tmem_base), Cfg::TMEM_COLS);
+  if (warp == 4) {
+    if (CG == 2) ako::tc::t2_tmem_alloc(ako::smem_u32(&s_tmem_base), Cfg::TMEM_COLS);
+    else ako::tc::tmem_alloc(ako::smem_u32(&s_tmem_base), Cfg::TMEM_COLS);
+  }
   ako::tc::fence_before_thread_sync();
   __syncthreads();
+  if (CG == 2) ako::tc::t2_cluster_sync();  // both CTAs' barriers are initialised before anybody signals across
   ako::tc::fence_after_thread_sync();
   const uint32_t tmem_base = s_tmem_base;
 
   // work item = (output tile, K split), the split fastest
-  const int m_tiles = (p.m + G_BM - 1) / G_BM, n_tiles = p.n / BN;
+  const int m_tiles = (p.m + CG * G_BM - 1) / (CG * G_BM), n_tiles = p.n / BN;
   const int total_tiles = m_tiles * n_tiles * p.splits;
   const int nkb = p.k / 64 / p.splits;
-  // bytes one stage receives: A brings a_box_rows rows, B all BN
-  const uint32_t stage_tx = (uint32_t)p.a_box_rows * G_BK_BYTES + (uint32_t)Cfg::B_BYTES;
+  // bytes one stage receives (a pair: in both CTAs): A brings a_box_rows rows, B all of its rows
+  const uint32_t stage_tx = CG * ((uint32_t)p.a_box_rows * G_BK_BYTES + (uint32_t)Cfg::B_BYTES);
 
   if (warp == 4) {
-    // ================================ TMA producer =============================================
-    if (lane == 0) {
+    // ================================ TMA producer (whole warp, one lane issues) ===============
+    if (ako::tc::elect_one()) {
       ako::tc::tma_prefetch_desc(&tm_a);
       ako::tc::tma_prefetch_desc(&tm_b);
-      int g = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-        const int ks = tile % p.splits, ot = tile / p.splits;
-        const int mt = ot / n_tiles, nt = ot % n_tiles;
-        for (int kb0 = 0; kb0 < nkb; ++kb0, ++g) {
-          const int kb = ks * nkb + kb0;
-          const int stage = g % STAGES;
-          const uint32_t ph = (uint32_t)((g / STAGES) & 1);
-          if (!ako::tc::mbar_wait(ako::smem_u32(&s_empty[stage]), ph ^ 1u, &s_err, kErrGLoad)) { ok = false; break; }
-          const uint32_t bar = ako::smem_u32(&s_full[stage]);
-          const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
-          ako::tc::mbar_arrive_expect_tx(bar, stage_tx);
-          ako::tc::tma_load_2d(sa, &tm_a, kb * G_BK_BYTES, mt * G_BM, bar);
-          ako::tc::tma_load_2d(sa + G_A_BYTES, &tm_b, kb * G_BK_BYTES, nt * BN, bar);
+    }
+    int stage = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int tile = worker; ok && tile < total_tiles; tile += workers) {
+      const int ks = tile % p.splits, ot = tile / p.splits;
+      const int mt = ot / n_tiles * CG + crank, nt = ot % n_tiles;
+      for (int kb0 = 0; kb0 < nkb; ++kb0) {
+        const int kb = ks * nkb + kb0;
+        if (!ako::tc::mbar_wait_warp(ako::smem_u32(&s_empty[stage]), ph ^ 1u, &s_err, kErrGLoad)) { ok = false; break; }
+        const uint32_t bar = ako::smem_u32(&s_full[stage]);
+        const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
+        const int brow = nt * BN + crank * Cfg::B_ROWS;
+        if (ako::tc::elect_one()) {
+          // the even CTA announces the bytes of both; the odd CTA's copies count down on its barrier.
+          // The empty half of an odd last pair reads zero fill.
+          if (crank == 0) ako::tc::mbar_arrive_expect_tx(bar, stage_tx);
+          if (CG == 2) {
+            const uint32_t bar0 = ako::tc::t2_mapa(bar, 0);
+            ako::tc::t2_tma_load_2d(sa, &tm_a, kb * G_BK_BYTES, mt * G_BM, bar0);
+            ako::tc::t2_tma_load_2d(sa + G_A_BYTES, &tm_b, kb * G_BK_BYTES, brow, bar0);
+          } else {
+            ako::tc::tma_load_2d(sa, &tm_a, kb * G_BK_BYTES, mt * G_BM, bar);
+            ako::tc::tma_load_2d(sa + G_A_BYTES, &tm_b, kb * G_BK_BYTES, brow, bar);
+          }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; ph ^= 1u; }
       }
     }
   } else if (warp == 5) {
-    // ================================ MMA issuer ===============================================
-    if (lane == 0) {
+    // ================================ MMA issuer (of a pair: in the even CTA) ===================
+    if (crank == 0) {
       const uint32_t a_lo0 = ako::tc::smem_desc_lo(smem_base);
       const uint32_t b_lo0 = ako::tc::smem_desc_lo(smem_base + G_A_BYTES);
-      int g = 0, lt = 0;
+      int stage = 0, lt = 0;
+      uint32_t ph = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++lt) {
+      for (int tile = worker; ok && tile < total_tiles; tile += workers, ++lt) {
         const int buf = lt & 1;
-        if (!ako::tc::mbar_wait(ako::smem_u32(&s_acc_empty[buf]), (uint32_t)(((lt >> 1) & 1) ^ 1), &s_err, kErrGAcc)) break;
+        if (!ako::tc::mbar_wait_warp(ako::smem_u32(&s_acc_empty[buf]), (uint32_t)(((lt >> 1) & 1) ^ 1), &s_err, kErrGAcc)) break;
         const uint32_t d = tmem_base + buf * BN;
-        for (int kb = 0; kb < nkb; ++kb, ++g) {
-          const int stage = g % STAGES;
-          if (!ako::tc::mbar_wait(ako::smem_u32(&s_full[stage]), (uint32_t)((g / STAGES) & 1), &s_err, kErrGMma)) { ok = false; break; }
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!ako::tc::mbar_wait_warp(ako::smem_u32(&s_full[stage]), ph, &s_err, kErrGMma)) { ok = false; break; }
           ako::tc::fence_after_thread_sync();
           const uint32_t a_lo = a_lo0 + stage * (Cfg::STAGE_BYTES >> 4);
           const uint32_t b_lo = b_lo0 + stage * (Cfg::STAGE_BYTES >> 4);
-          ako::tc::mma_bf16_lohi(d, a_lo, b_lo, IDESC, kb > 0 ? 1u : 0u);
-          ako::tc::mma_bf16_lohi(d, a_lo + 2, b_lo + 2, IDESC, 1u);
-          ako::tc::mma_bf16_lohi(d, a_lo + 4, b_lo + 4, IDESC, 1u);
-          ako::tc::mma_bf16_lohi(d, a_lo + 6, b_lo + 6, IDESC, 1u);
-          ako::tc::mma_commit(ako::smem_u32(&s_empty[stage]));
+          if (ako::tc::elect_one()) {
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) {
+              const uint32_t acc = (kb > 0 || ks > 0) ? 1u : 0u;
+              if (CG == 2) ako::tc::t2_mma_bf16(d, a_lo + 2 * ks, b_lo + 2 * ks, IDESC, acc);
+              else ako::tc::mma_bf16_lohi(d, a_lo + 2 * ks, b_lo + 2 * ks, IDESC, acc);
+            }
+            if (CG == 2) ako::tc::t2_commit_both(ako::smem_u32(&s_empty[stage]));
+            else ako::tc::mma_commit(ako::smem_u32(&s_empty[stage]));
+            if (kb == nkb - 1) {
+              if (CG == 2) ako::tc::t2_commit_both(ako::smem_u32(&s_acc_full[buf]));
+              else ako::tc::mma_commit(ako::smem_u32(&s_acc_full[buf]));
+            }
+          }
+          __syncwarp();
+          if (++stage == STAGES) { stage = 0; ph ^= 1u; }
         }
-        if (ok) ako::tc::mma_commit(ako::smem_u32(&s_acc_full[buf]));
       }
     }
   } else {
     // ================================ epilogue warps ===========================================
     const int row_in_tile = 32 * warp + lane;   // TMEM lane = accumulator row
     int lt = 0;
-    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++lt) {
+    for (int tile = worker; tile < total_tiles; tile += workers, ++lt) {
       const int ks = tile % p.splits, ot = tile / p.splits;
-      const int mt = ot / n_tiles, nt = ot % n_tiles;
+      const int mt = ot / n_tiles * CG + crank, nt = ot % n_tiles;
       const int buf = lt & 1;
       if (!ako::tc::mbar_wait_warp(ako::smem_u32(&s_acc_full[buf]), (uint32_t)((lt >> 1) & 1), &s_err, kErrGEpi)) break;
       ako::tc::fence_after_thread_sync();
@@ -183,17 +217,22 @@ gemm_f16_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tm_a, const _
       }
       ako::tc::fence_before_thread_sync();
       __syncwarp();
-      if (lane == 0) ako::tc::mbar_arrive(ako::smem_u32(&s_acc_empty[buf]));
+      if (lane == 0) {
+        if (CG == 2) ako::tc::t2_arrive_cluster(ako::tc::t2_mapa(ako::smem_u32(&s_acc_empty[buf]), 0));
+        else ako::tc::mbar_arrive(ako::smem_u32(&s_acc_empty[buf]));
+      }
     }
   }
 
   // ================================ common exit ================================================
   ako::tc::fence_before_thread_sync();
   __syncthreads();
+  if (CG == 2) ako::tc::t2_cluster_sync();  // the peer may still be reading this CTA's shared memory or writing its TMEM
   if (tid == 0 && s_err != 0) atomicCAS(&g_gemm_status, 0, s_err);
   if (warp == 4) {
     ako::tc::fence_after_thread_sync();
-    ako::tc::tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+    if (CG == 2) ako::tc::t2_tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+    else ako::tc::tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
   }
 }
 
@@ -230,16 +269,33 @@ __global__ void __launch_bounds__(256) gemm_splitk_reduce_kernel(const float* __
   *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(c) + i) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// CTAs of a pair kernel that can be resident at once (2 x the co-resident clusters), per device.
 template <int BN, bool BF16>
+int pair_ctas(cudaLaunchConfig_t cfg) {
+  static std::atomic<int> cached[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cfg.gridDim = dim3((unsigned)(ako::sm_count() & ~1));
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, gemm_f16_tc_kernel<BN, BF16, 2>, &cfg) != cudaSuccess) return 0;
+    n = 2 * clusters;
+    cached[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+template <int BN, bool BF16, int CG>
 int launch_gemm(const void* a, const void* b, void* c, int64_t m, int64_t n, int64_t k, int splits, float* partial,
                 cudaStream_t st) {
-  using Cfg = GemmCfg<BN>;
+  using Cfg = GemmCfg<BN, CG>;
   const int a_box_rows = (m >= G_BM) ? G_BM : (int)((m + 7) / 8 * 8);
   CUtensorMap tm_a, tm_b;
   if (!ako::tma::byte_matrix_map(&tm_a, a, (uint64_t)m, (uint64_t)k * 2, (uint32_t)a_box_rows) ||
-      !ako::tma::byte_matrix_map(&tm_b, b, (uint64_t)n, (uint64_t)k * 2, (uint32_t)BN))
+      !ako::tma::byte_matrix_map(&tm_b, b, (uint64_t)n, (uint64_t)k * 2, (uint32_t)Cfg::B_ROWS))
     return AKO4X_ELAUNCH;
-  if (!ako::ensure_dynamic_smem<gemm_f16_tc_kernel<BN, BF16>>((int)Cfg::SMEM)) return AKO4X_ELAUNCH;
+  if (!ako::ensure_dynamic_smem<gemm_f16_tc_kernel<BN, BF16, CG>>((int)Cfg::SMEM)) return AKO4X_ELAUNCH;
   GemmArgs p;
   p.c = c;
   p.m = (int)m;
@@ -248,10 +304,23 @@ int launch_gemm(const void* a, const void* b, void* c, int64_t m, int64_t n, int
   p.a_box_rows = a_box_rows;
   p.splits = splits;
   p.partial = partial;
-  const int64_t tiles = ((m + G_BM - 1) / G_BM) * (n / BN) * splits;
-  const int grid = (int)std::min<int64_t>(tiles, ako::sm_count());
-  gemm_f16_tc_kernel<BN, BF16><<<grid, G_THREADS, Cfg::SMEM, st>>>(p, tm_a, tm_b);
-  AKO_CHECK_LAUNCH();
+  const int64_t tiles = ((m + CG * G_BM - 1) / (CG * G_BM)) * (n / BN) * splits;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(G_THREADS);
+  cfg.dynamicSmemBytes = Cfg::SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CG;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = (CG == 2) ? 1 : 0;
+  int ctas = ako::sm_count();
+  if constexpr (CG == 2) ctas = pair_ctas<BN, BF16>(cfg);
+  if (ctas < CG) return AKO4X_ELAUNCH;
+  cfg.gridDim = dim3((unsigned)std::min<int64_t>(CG * tiles, ctas));
+  if (cudaLaunchKernelEx(&cfg, gemm_f16_tc_kernel<BN, BF16, CG>, p, tm_a, tm_b) != cudaSuccess) return AKO4X_ELAUNCH;
   if (splits > 1) {
     const int64_t mn = m * n;
     const unsigned blocks = (unsigned)((mn / 8 + 255) / 256);
@@ -262,23 +331,50 @@ int launch_gemm(const void* a, const void* b, void* c, int64_t m, int64_t n, int
   return AKO4X_OK;
 }
 
-// Tile width and K split by how many work items the GPU gets. Full-width tiles (256 columns)
-// without a split once they fill three quarters of the SMs. Below that a tile's K loop (256 MMAs
-// whatever the tile width) is what a call waits for: tiles of 128 columns, and K cut into 2, 4 or 8
-// pieces handled by different CTAs (summed by a second kernel) until there are 128 work items.
-// Measured, whole call, cold L2: M = 16: 15.4 us (unsplit 26.6), M = 128: 17.4, M = 256: 19.5,
-// M = 512: 23.5, M = 969: 30.7 (no split; 256 columns x 2 splits: 29.7).
+// Tile width, CTAs per tile and K split by how many work items the GPU gets. A K block of 64 costs a
+// CTA about the same time whatever its tile is (it waits for operands, not for the tensor pipe), so
+// the plan looks for the widest tiles that still give every SM work: pairs (256 rows) from the second
+// row tile on, 256 columns once 128 would need a second wave, K cut into 2, 4 or 8 pieces (summed by
+// a second kernel) while less than half of the GPU has work. One-CTA tiles stay for up to 128 rows
+// (a pair would be half empty) and where they fit one wave and pairs of the same width do not.
+// Measured, whole call, N = 2048, K = 4096, against one-CTA tiles everywhere (us): M = 256: 15.6
+// (20.0), 512: 18.5 (20.0), 640: 23.5 (29.2), 969: 22.6 (26.0), 1536: 28.8 (44.5), 4000: 52.3 (57.7),
+// 16294: 182 (204); M = 640 as 256 x 128 pairs with K in two, 96 of them for 74 places: 26.7.
 struct GemmPlan {
-  int bn, splits;
+  int bn, splits, cg;
 };
 inline GemmPlan gemm_plan(int64_t m, int64_t n, int64_t k, bool have_workspace) {
-  const int64_t mt = (m + G_BM - 1) / G_BM;
+  const int64_t mt = (m + G_BM - 1) / G_BM, mp = (mt + 1) / 2;
   const int sms = ako::sm_count();
-  if (mt * (n / 256) * 4 >= 3 * sms) return {256, 1};
-  if (!have_workspace) return {(mt * (n / 128) * 4 >= 3 * sms) ? 128 : 32, 1};
+  if (mt > 1) {
+    // more 256 x 128 tiles than one wave of pairs
+    if (2 * mp * (n / 128) > sms) {
+      if (mt * (n / 128) <= sms) return {128, 1, 1};
+      return {256, 1, 2};
+    }
+    int s = 1;
+    while (have_workspace && s < 8 && 4 * mp * (n / 128) * s <= sms && (k / 64) % (2 * s) == 0) s *= 2;
+    if (s > 1) return {128, s, 2};
+    // between a quarter and a half of the GPU with full-width tiles: those, K in two
+    if (have_workspace && 4 * mp * (n / 256) * 3 <= 2 * sms && (k / 64) % 2 == 0) return {256, 2, 2};
+    if (4 * mp * (n / 128) >= sms) return {128, 1, 2};
+  }
+  if (mt * (n / 256) * 4 >= 3 * sms) return {256, 1, 1};
+  if (!have_workspace) return {(mt * (n / 128) * 4 >= 3 * sms) ? 128 : 32, 1, 1};
   int s = 1;
   while (s < 8 && mt * (n / 128) * s < 128 && (k / 64) % (2 * s) == 0) s *= 2;
-  return {128, s};
+  return {128, s, 1};
+}
+
+template <bool BF16>
+int launch_plan(const GemmPlan& pl, const void* a, const void* b, void* c, int64_t m, int64_t n, int64_t k,
+                float* part, cudaStream_t st) {
+  if (pl.cg == 2)
+    return (pl.bn == 256) ? launch_gemm<256, BF16, 2>(a, b, c, m, n, k, pl.splits, part, st)
+                          : launch_gemm<128, BF16, 2>(a, b, c, m, n, k, pl.splits, part, st);
+  if (pl.bn == 256) return launch_gemm<256, BF16, 1>(a, b, c, m, n, k, 1, part, st);
+  if (pl.bn == 128) return launch_gemm<128, BF16, 1>(a, b, c, m, n, k, pl.splits, part, st);
+  return launch_gemm<32, BF16, 1>(a, b, c, m, n, k, 1, part, st);
 }
 
 }  // namespace
@@ -300,14 +396,7 @@ static int gemm_entry(const void* a, const void* b, void* c, int64_t m, int64_t 
   const GemmPlan pl = gemm_plan(m, n, k, workspace != nullptr);
   if (pl.splits > 1 && workspace_bytes < (size_t)pl.splits * (size_t)m * (size_t)n * sizeof(float)) return AKO4X_EWORKSPACE;
   float* part = (float*)workspace;
-  if (is_bf16) {
-    if (pl.bn == 256) return launch_gemm<256, true>(a, b, c, m, n, k, pl.splits, part, st);
-    if (pl.bn == 128) return launch_gemm<128, true>(a, b, c, m, n, k, pl.splits, part, st);
-    return launch_gemm<32, true>(a, b, c, m, n, k, 1, part, st);
-  }
-  if (pl.bn == 256) return launch_gemm<256, false>(a, b, c, m, n, k, pl.splits, part, st);
-  if (pl.bn == 128) return launch_gemm<128, false>(a, b, c, m, n, k, pl.splits, part, st);
-  return launch_gemm<32, false>(a, b, c, m, n, k, 1, part, st);
+  return is_bf16 ? launch_plan<true>(pl, a, b, c, m, n, k, part, st) : launch_plan<false>(pl, a, b, c, m, n, k, part, st);
 }
 
 extern "C" int ako4x_gemm_f16_nt(const void* a, const void* b, void* c, int64_t m, int64_t n, int64_t k,

@@ -37,6 +37,26 @@ def test_against_oracle(m):
     assert _cabi.lib().ako4x_gemm_device_status() == 0
 
 
+# both sides of every line of the plan: one-CTA tiles and pairs (odd and even numbers of row tiles), their
+# widths and K splits; reductions of one block and of a number of blocks that does not split
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k", [(m, 2048, 4096) for m in (255, 257, 385, 512, 513, 769, 1024, 1025, 1153, 2561)] +
+                         [(130, 256, 64), (700, 2048, 192), (300, 512, 4096), (129, 8192, 128), (100, 32768, 64)])
+def test_plan_edges(dtype, m, n, k):
+    g = torch.Generator().manual_seed(m + n + k)
+    a = torch.randn(m, k, generator=g).to(dtype)
+    b = (torch.randn(n, k, generator=g) * 0.05).to(dtype)
+    ws = _cabi.lib().ako4x_gemm_workspace_bytes(m, n, k)
+    for use_ws in ((False, True) if ws else (False,)):
+        ad, bd, c = a.cuda(), b.cuda(), torch.full((m, n), float("nan"), dtype=dtype, device="cuda")
+        w = torch.empty(max(ws, 16), dtype=torch.uint8, device="cuda")
+        st = _cabi.lib().ako4x_gemm_f16_nt_ws(_cabi.ptr(ad), _cabi.ptr(bd), _cabi.ptr(c), m, n, k, int(dtype == torch.bfloat16),
+                                              _cabi.ptr(w) if use_ws else None, ws if use_ws else 0, _cabi.stream())
+        assert st == 0
+        _check(c.cpu(), oracle.gemm_nt(a, b), 2e-3 if dtype == torch.float16 else 8e-3)
+    assert _cabi.lib().ako4x_gemm_device_status() == 0
+
+
 def test_unsplit_entry_point_agrees():
     """The entry point without a workspace (no K split) against the oracle, and the split form
     against it: same products, fp32 sums in another grouping."""
