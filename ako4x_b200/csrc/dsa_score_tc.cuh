@@ -304,9 +304,9 @@ dsa_score_tc_kernel(ScoreParams p, const __grid_constant__ CUtensorMap tm_q, con
     }
   } else if (warp >= TS_MMA_WARP && warp < TS_MMA_WARP + TS_ACCS) {
     // ================================ MMA issuers ==============================================
-    // The barrier waits and the descriptor read for the issuer's NEXT key tile are done between
-    // the second and third MMA of the current one.
-    if (lane == 0) {
+    // The barrier waits and the descriptor read for the issuer's NEXT key tile are done while the MMAs
+    // of the current one run.
+    {  // the whole warp waits, one lane issues
       constexpr uint32_t IDESC_SHARED = ako::tc::idesc_e4m3_f32(128, TS_ACC_COLS);
       constexpr uint32_t IDESC_ROW = ako::tc::idesc_e4m3_f32(128, NH);
       // a_lo, b_lo: descriptor low words; mma: this issuer's rows take part in the tile;
@@ -324,14 +324,16 @@ dsa_score_tc_kernel(ScoreParams p, const __grid_constant__ CUtensorMap tm_q, con
       auto prepare = [&](Tile& t) -> int {
         if (sub == subs) {  // next unit
           const int slot = n % TS_SLOTS;
-          if (!ako::tc::mbar_wait(ako::smem_u32(&s_slot_full[slot]), (uint32_t)((n / TS_SLOTS) & 1), &s_err, 4)) return -1;
+          if (!ako::tc::mbar_wait_warp(ako::smem_u32(&s_slot_full[slot]), (uint32_t)((n / TS_SLOTS) & 1), &s_err, 4)) return -1;
           const volatile ScoreDesc* dp = reinterpret_cast<const volatile ScoreDesc*>(slot_ptr + slot * TS_SLOT_BYTES + TS_ROWS * TS_SCALE_BYTES);
           const int flags = dp->flags, qc = dp->qc;
           ac = dp->ac0;
-          ako::tc::mbar_arrive(ako::smem_u32(&s_slot_empty[slot]));
+          __syncwarp();
+          if (ako::tc::elect_one()) ako::tc::mbar_arrive(ako::smem_u32(&s_slot_empty[slot]));
+          __syncwarp();
           if (flags & TS_F_END) return 0;
           if ((flags & TS_F_NEWGROUP) &&
-              !ako::tc::mbar_wait(ako::smem_u32(&s_q_full), (uint32_t)(qc & 1), &s_err, 5)) return -1;
+              !ako::tc::mbar_wait_warp(ako::smem_u32(&s_q_full), (uint32_t)(qc & 1), &s_err, 5)) return -1;
           shared = flags & TS_F_SHARED;
           last_unit = flags & TS_F_LASTGROUP;
           subs = shared ? 1 : TS_ROWS;
@@ -342,7 +344,7 @@ dsa_score_tc_kernel(ScoreParams p, const __grid_constant__ CUtensorMap tm_q, con
         // Tiles of the other row pairs are waited for as well: the stage's release counts all
         // issuers, and this keeps an issuer from arriving for the stage's next use too early.
         const int stage = ac % TS_A_STAGES;
-        if (!ako::tc::mbar_wait(ako::smem_u32(&s_a_full[stage]), (uint32_t)((ac / TS_A_STAGES) & 1), &s_err, 7)) return -1;
+        if (!ako::tc::mbar_wait_warp(ako::smem_u32(&s_a_full[stage]), (uint32_t)((ac / TS_A_STAGES) & 1), &s_err, 7)) return -1;
         ako::tc::fence_after_thread_sync();
         t.mma = shared || (sub >> 1) == me;
         t.a_lo = a_lo0 + stage * (TS_A_BYTES >> 4);
@@ -363,22 +365,25 @@ dsa_score_tc_kernel(ScoreParams p, const __grid_constant__ CUtensorMap tm_q, con
         if (cur.mma) {
           // This issuer's units share one accumulator: the team must have read the previous result.
           if (cur.acc_wait >= 0 &&
-              !ako::tc::mbar_wait(ako::smem_u32(&s_acc_empty[me]), (uint32_t)cur.acc_wait, &s_err, 6)) break;
-          ako::tc::mma_f8_lohi<false>(cur.d, cur.a_lo, cur.b_lo, cur.idesc);  // K = 32 slices: +32 B = +2
-          ako::tc::mma_f8_lohi<true>(cur.d, cur.a_lo + 2, cur.b_lo + 2, cur.idesc);
-          if (!cur.q_done) r = prepare(nxt);
-          ako::tc::mma_f8_lohi<true>(cur.d, cur.a_lo + 4, cur.b_lo + 4, cur.idesc);
-          ako::tc::mma_f8_lohi<true>(cur.d, cur.a_lo + 6, cur.b_lo + 6, cur.idesc);
-          ako::tc::mma_commit(ako::smem_u32(&s_a_empty[cur.stage]));
-          if (cur.last) ako::tc::mma_commit(ako::smem_u32(&s_acc_full[me]));
+              !ako::tc::mbar_wait_warp(ako::smem_u32(&s_acc_empty[me]), (uint32_t)cur.acc_wait, &s_err, 6)) break;
+          if (ako::tc::elect_one()) {
+            ako::tc::mma_f8_lohi<false>(cur.d, cur.a_lo, cur.b_lo, cur.idesc);  // K = 32 slices: +32 B = +2
+            ako::tc::mma_f8_lohi<true>(cur.d, cur.a_lo + 2, cur.b_lo + 2, cur.idesc);
+            ako::tc::mma_f8_lohi<true>(cur.d, cur.a_lo + 4, cur.b_lo + 4, cur.idesc);
+            ako::tc::mma_f8_lohi<true>(cur.d, cur.a_lo + 6, cur.b_lo + 6, cur.idesc);
+            ako::tc::mma_commit(ako::smem_u32(&s_a_empty[cur.stage]));
+            if (cur.last) ako::tc::mma_commit(ako::smem_u32(&s_acc_full[me]));
+          }
         } else {
-          ako::tc::mbar_arrive(ako::smem_u32(&s_a_empty[cur.stage]));
-          if (!cur.q_done) r = prepare(nxt);
+          if (ako::tc::elect_one()) ako::tc::mbar_arrive(ako::smem_u32(&s_a_empty[cur.stage]));
         }
+        __syncwarp();
+        if (!cur.q_done) r = prepare(nxt);
         if (cur.q_done) {
           // The group's last tile: hand the query buffer back once this issuer's MMAs are done,
           // and only then look at the next unit (its group cannot be loaded before).
-          ako::tc::mma_commit(ako::smem_u32(&s_q_empty));
+          if (ako::tc::elect_one()) ako::tc::mma_commit(ako::smem_u32(&s_q_empty));
+          __syncwarp();
           r = prepare(nxt);
         }
         cur = nxt;

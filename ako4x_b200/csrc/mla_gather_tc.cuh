@@ -465,58 +465,70 @@ __global__ void __launch_bounds__(THREADS, 1) mla_gather_tc_kernel(Params p, int
     ako::cp_async_wait<0>();  // nothing of this thread is in flight when the CTA leaves
   } else {
     ako::tc::reg_dec<REGS_ISSUER>();
-    if (warp == 12 && lane == 0) {
-      // =================================== MMA issuer ============================================
+    if (warp == 12) {
+      // ============================== MMA issuer (whole warp, one lane issues) ====================
       const uint32_t p_lo = ako::tc::smem_desc_lo(base + OFF_P);
       const uint32_t k_lo = ako::tc::smem_desc_lo(base + OFF_KPE);
       const uint32_t d_s = tmem, d_pv = tmem + 32;
       bool ok = true;
       int gt = 0, seg = 0;
       do {
-        if (!ako::tc::mbar_wait(ako::smem_u32(&b_q_full[seg & 1]), (uint32_t)((seg >> 1) & 1), err, kErrMmaQ)) { ok = false; break; }
+        if (!ako::tc::mbar_wait_warp(ako::smem_u32(&b_q_full[seg & 1]), (uint32_t)((seg >> 1) & 1), err, kErrMmaQ)) { ok = false; break; }
         ako::tc::fence_proxy_async_smem();
         const uint32_t q_lo = ako::tc::smem_desc_lo(base + OFF_Q + (seg & 1) * Q_BYTES);
         for (int it = 0; it < w.nt && ok; ++it, ++gt) {
           // ---- S^T = K Q^T: the kpe chunk first (it was fetched ahead), then the four pairs ----
-          if (gt > 0 && !ako::tc::mbar_wait(ako::smem_u32(&b_s_empty), (uint32_t)((gt - 1) & 1), err, kErrMmaS)) { ok = false; break; }
-          if (!ako::tc::mbar_wait(ako::smem_u32(&b_kpe_full), (uint32_t)(gt & 1), err, kErrMmaKpe)) { ok = false; break; }
+          if (gt > 0 && !ako::tc::mbar_wait_warp(ako::smem_u32(&b_s_empty), (uint32_t)((gt - 1) & 1), err, kErrMmaS)) { ok = false; break; }
+          if (!ako::tc::mbar_wait_warp(ako::smem_u32(&b_kpe_full), (uint32_t)(gt & 1), err, kErrMmaKpe)) { ok = false; break; }
           ako::tc::fence_proxy_async_smem();  // cp.async wrote the block through the generic proxy
           ako::tc::fence_after_thread_sync();
+          if (ako::tc::elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            ako::tc::mma_bf16_lohi(d_s, k_lo + 2 * k, q_lo + (uint32_t)(8 * (QCH >> 4)) + 2 * k, IDESC_S, k ? 1u : 0u);
-          ako::tc::mma_commit(ako::smem_u32(&b_kpe_empty));
+            for (int k = 0; k < 4; ++k)
+              ako::tc::mma_bf16_lohi(d_s, k_lo + 2 * k, q_lo + (uint32_t)(8 * (QCH >> 4)) + 2 * k, IDESC_S, k ? 1u : 0u);
+            ako::tc::mma_commit(ako::smem_u32(&b_kpe_empty));
+          }
+          __syncwarp();
           for (int pr = 0; pr < 4 && ok; ++pr) {
             const int g = gt * 4 + pr, slot = g % NPAIR;
-            if (!ako::tc::mbar_wait(ako::smem_u32(&b_pair_full[slot]), (uint32_t)((g / NPAIR) & 1), err, kErrMmaPair)) { ok = false; break; }
+            if (!ako::tc::mbar_wait_warp(ako::smem_u32(&b_pair_full[slot]), (uint32_t)((g / NPAIR) & 1), err, kErrMmaPair)) { ok = false; break; }
             ako::tc::fence_proxy_async_smem();
             ako::tc::fence_after_thread_sync();
+            if (ako::tc::elect_one()) {
 #pragma unroll
-            for (int fbk = 0; fbk < 8; ++fbk) {
-              const int f2 = fbk >> 2, k = fbk & 3;
-              const uint32_t a_lo = ako::tc::smem_desc_lo(base + slot * PAIR + f2 * BLK) + 2 * k;
-              const uint32_t b_lo = q_lo + (uint32_t)((2 * pr + f2) * (QCH >> 4)) + 2 * k;
-              ako::tc::mma_bf16_lohi(d_s, a_lo, b_lo, IDESC_S, 1u);
+              for (int fbk = 0; fbk < 8; ++fbk) {
+                const int f2 = fbk >> 2, k = fbk & 3;
+                const uint32_t a_lo = ako::tc::smem_desc_lo(base + slot * PAIR + f2 * BLK) + 2 * k;
+                const uint32_t b_lo = q_lo + (uint32_t)((2 * pr + f2) * (QCH >> 4)) + 2 * k;
+                ako::tc::mma_bf16_lohi(d_s, a_lo, b_lo, IDESC_S, 1u);
+              }
+              if (pr == 3) {
+                ako::tc::mma_commit(ako::smem_u32(&b_s_full));
+                if (it + 1 == w.nt) ako::tc::mma_commit(ako::smem_u32(&b_q_empty[seg & 1]));  // last S of this row
+              }
             }
+            __syncwarp();
           }
           if (!ok) break;
-          ako::tc::mma_commit(ako::smem_u32(&b_s_full));
-          if (it + 1 == w.nt) ako::tc::mma_commit(ako::smem_u32(&b_q_empty[seg & 1]));  // last S of this row
           // ---- O^T partial = V^T P^T ----
-          if (!ako::tc::mbar_wait(ako::smem_u32(&b_p_full), (uint32_t)(gt & 1), err, kErrMmaP)) { ok = false; break; }
-          if (gt > 0 && !ako::tc::mbar_wait(ako::smem_u32(&b_pv_empty), (uint32_t)((gt - 1) & 1), err, kErrMmaPv)) { ok = false; break; }
+          if (!ako::tc::mbar_wait_warp(ako::smem_u32(&b_p_full), (uint32_t)(gt & 1), err, kErrMmaP)) { ok = false; break; }
+          if (gt > 0 && !ako::tc::mbar_wait_warp(ako::smem_u32(&b_pv_empty), (uint32_t)((gt - 1) & 1), err, kErrMmaPv)) { ok = false; break; }
           ako::tc::fence_after_thread_sync();
-          for (int mb = 0; mb < 4; ++mb) {
-            const int g = gt * 4 + mb, slot = g % NPAIR;
-            const uint32_t a0 = ako::tc::smem_desc_lo_mn(base + slot * PAIR, BLK);
+          if (ako::tc::elect_one()) {
+#pragma unroll 1
+            for (int mb = 0; mb < 4; ++mb) {
+              const int g = gt * 4 + mb, slot = g % NPAIR;
+              const uint32_t a0 = ako::tc::smem_desc_lo_mn(base + slot * PAIR, BLK);
 #pragma unroll
-            for (int kt = 0; kt < 8; ++kt)  // 16 tokens per MMA: two 8-token groups of 1024 bytes
-              ako::tc::mma_bf16_lohi(d_pv + 16 * mb, a0 + (uint32_t)(kt * (2048 >> 4)),
-                                     p_lo + (uint32_t)((kt >> 2) * (QCH >> 4)) + 2 * (kt & 3), IDESC_PV, kt ? 1u : 0u);
-            ako::tc::mma_commit(ako::smem_u32(&b_pair_empty[slot]));
+              for (int kt = 0; kt < 8; ++kt)  // 16 tokens per MMA: two 8-token groups of 1024 bytes
+                ako::tc::mma_bf16_lohi(d_pv + 16 * mb, a0 + (uint32_t)(kt * (2048 >> 4)),
+                                       p_lo + (uint32_t)((kt >> 2) * (QCH >> 4)) + 2 * (kt & 3), IDESC_PV, kt ? 1u : 0u);
+              ako::tc::mma_commit(ako::smem_u32(&b_pair_empty[slot]));
+            }
+            ako::tc::mma_commit(ako::smem_u32(&b_pv_full));
+            ako::tc::mma_commit(ako::smem_u32(&b_p_empty));
           }
-          ako::tc::mma_commit(ako::smem_u32(&b_pv_full));
-          ako::tc::mma_commit(ako::smem_u32(&b_p_empty));
+          __syncwarp();
         }
         ++seg;
       } while (ok && w.next());

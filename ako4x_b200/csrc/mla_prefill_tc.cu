@@ -23,8 +23,8 @@
 // Why a pair: one CTA per tile was bound by the bytes that cross shared memory (128 B/clk per SM):
 // 644 KB per 128-key tile, of which 294 KB were TMA writes of Q and K chunks and 288 KB S operands.
 // A pair reads half of every K chunk and half of V per CTA and leaves room for a resident Q tile:
-// 352 KB. Eight ragged prompts (9 101 queries, 39 794 keys): 2 274 -> 1 785 us with the gather, 745
-// TFLOP/s of algorithmic flops, 1 140 counting S of both halves.
+// 352 KB. Eight ragged prompts (9 101 queries, 39 794 keys): 2 239 -> 1 730 us with the gather, 769
+// TFLOP/s of algorithmic flops, 1 180 counting S of both halves.
 // Warps: 0-7 softmax, rescale and output, 8 Q/K producer, 9 S issuer (even CTA), 10 V producer,
 // 11 PV issuer (even CTA). Rows of a partial last tile and keys past the causal limit are masked;
 // every mbarrier wait is bounded and a timeout sets the status word.
@@ -331,41 +331,50 @@ mla_prefill_tc_kernel(PfParams p, const __grid_constant__ CUtensorMap tm_qn, con
         }
       }
     }
-  } else if (warp == 8 && lane == 0 && ntk > 0) {
+  } else if (warp == 8 && ntk > 0) {
     // ================================ Q / K producer (each CTA its rows and keys) ================
-    ako::tc::tma_prefetch_desc(&tm_qn);
-    ako::tc::tma_prefetch_desc(&tm_qp);
-    ako::tc::tma_prefetch_desc(&tm_k);
+    // this role and the next three: the whole warp waits, one lane issues
+    if (ako::tc::elect_one()) {
+      ako::tc::tma_prefetch_desc(&tm_qn);
+      ako::tc::tma_prefetch_desc(&tm_qp);
+      ako::tc::tma_prefetch_desc(&tm_k);
+    }
     int g = 0;
     bool ok = true;
     for (int j = 0; ok && j < ntk; ++j) {
       for (int c = 0; c < NCH; ++c, ++g) {
         const int stage = g % NST;
-        if (!ako::tc::mbar_wait(ako::smem_u32(&st_empty[stage]), (uint32_t)(((g / NST) & 1) ^ 1), &g_pf_status, 5)) { ok = false; break; }
+        if (!ako::tc::mbar_wait_warp(ako::smem_u32(&st_empty[stage]), (uint32_t)(((g / NST) & 1) ^ 1), &g_pf_status, 5)) { ok = false; break; }
         const uint32_t bar = ako::tc::t2_mapa(ako::smem_u32(&st_full[stage]), 0);
-        // the even CTA announces the bytes of both; the first tile's stages bring the Q chunk along
-        if (crank == 0)
-          ako::tc::mbar_arrive_expect_tx(ako::smem_u32(&st_full[stage]), 2 * (K_CH_BYTES + (j == 0 ? Q_CH_BYTES : 0)));
-        if (j == 0) {
-          if (c < DC / 64) ako::tc::t2_tma_load_2d(q_base + c * Q_CH_BYTES, &tm_qn, c * 64, q0 * H, bar);
-          else ako::tc::t2_tma_load_2d(q_base + c * Q_CH_BYTES, &tm_qp, 0, q0 * H, bar);
+        if (ako::tc::elect_one()) {
+          // the even CTA announces the bytes of both; the first tile's stages bring the Q chunk along
+          if (crank == 0)
+            ako::tc::mbar_arrive_expect_tx(ako::smem_u32(&st_full[stage]), 2 * (K_CH_BYTES + (j == 0 ? Q_CH_BYTES : 0)));
+          if (j == 0) {
+            if (c < DC / 64) ako::tc::t2_tma_load_2d(q_base + c * Q_CH_BYTES, &tm_qn, c * 64, q0 * H, bar);
+            else ako::tc::t2_tma_load_2d(q_base + c * Q_CH_BYTES, &tm_qp, 0, q0 * H, bar);
+          }
+          ako::tc::t2_tma_load_2d(k_base + stage * K_CH_BYTES, &tm_k, c * 64, (int)(kbase + (int64_t)j * BK + crank * (BK / 2)), bar);
         }
-        ako::tc::t2_tma_load_2d(k_base + stage * K_CH_BYTES, &tm_k, c * 64, (int)(kbase + (int64_t)j * BK + crank * (BK / 2)), bar);
+        __syncwarp();
       }
     }
-  } else if (warp == 10 && lane == 0 && ntk > 0) {
+  } else if (warp == 10 && ntk > 0) {
     // ================================ V producer (each CTA its 128 columns) ======================
-    ako::tc::tma_prefetch_desc(&tm_v);
+    if (ako::tc::elect_one()) ako::tc::tma_prefetch_desc(&tm_v);
     const uint32_t bar = ako::tc::t2_mapa(ako::smem_u32(&v_full), 0);
     const int x = half * 256 + crank * 128;
     for (int j = 0; j < ntk; ++j) {
-      if (j > 0 && !ako::tc::mbar_wait(ako::smem_u32(&pv_done[(j - 1) & 1]), (uint32_t)(((j - 1) >> 1) & 1), &g_pf_status, 6)) break;
-      if (crank == 0) ako::tc::mbar_arrive_expect_tx(ako::smem_u32(&v_full), 2 * V_BYTES);
-      const int y = (int)(kbase + (int64_t)j * BK);
-      ako::tc::t2_tma_load_2d(v_base, &tm_v, x, y, bar);
-      ako::tc::t2_tma_load_2d(v_base + V_BOX_BYTES, &tm_v, x + 64, y, bar);
+      if (j > 0 && !ako::tc::mbar_wait_warp(ako::smem_u32(&pv_done[(j - 1) & 1]), (uint32_t)(((j - 1) >> 1) & 1), &g_pf_status, 6)) break;
+      if (ako::tc::elect_one()) {
+        if (crank == 0) ako::tc::mbar_arrive_expect_tx(ako::smem_u32(&v_full), 2 * V_BYTES);
+        const int y = (int)(kbase + (int64_t)j * BK);
+        ako::tc::t2_tma_load_2d(v_base, &tm_v, x, y, bar);
+        ako::tc::t2_tma_load_2d(v_base + V_BOX_BYTES, &tm_v, x + 64, y, bar);
+      }
+      __syncwarp();
     }
-  } else if (warp == 9 && lane == 0 && crank == 0 && ntk > 0) {
+  } else if (warp == 9 && crank == 0 && ntk > 0) {
     // ================================ S issuer (for the pair) ====================================
     constexpr uint32_t IDESC_S = ako::tc::idesc_bf16_f32(2 * BM, BK);
     const uint32_t q_lo = ako::tc::smem_desc_lo(q_base), k_lo = ako::tc::smem_desc_lo(k_base);
@@ -375,22 +384,25 @@ mla_prefill_tc_kernel(PfParams p, const __grid_constant__ CUtensorMap tm_qn, con
     for (int j = 0; ok && j < ntk; ++j) {
       const int buf = j & 1;
       // the PV MMAs of tile j-2 have read P out of this buffer
-      if (!ako::tc::mbar_wait(ako::smem_u32(&pv_done[buf]), (uint32_t)(((j >> 1) & 1) ^ 1), &g_pf_status, 7)) break;
+      if (!ako::tc::mbar_wait_warp(ako::smem_u32(&pv_done[buf]), (uint32_t)(((j >> 1) & 1) ^ 1), &g_pf_status, 7)) break;
       const uint32_t d = tmem + buf * BK;
       for (int c = 0; c < NCH; ++c) {
-        if (!ako::tc::mbar_wait(ako::smem_u32(&st_full[stage]), ph, &g_pf_status, 8)) { ok = false; break; }
+        if (!ako::tc::mbar_wait_warp(ako::smem_u32(&st_full[stage]), ph, &g_pf_status, 8)) { ok = false; break; }
         ako::tc::fence_after_thread_sync();
         const uint32_t a_lo = q_lo + c * (Q_CH_BYTES >> 4);
         const uint32_t b_lo = k_lo + stage * (K_CH_BYTES >> 4);
+        if (ako::tc::elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          ako::tc::t2_mma_bf16(d, a_lo + 2 * ks, b_lo + 2 * ks, IDESC_S, (c > 0 || ks > 0) ? 1u : 0u);
-        ako::tc::t2_commit_both(ako::smem_u32(&st_empty[stage]));
+          for (int ks = 0; ks < 4; ++ks)
+            ako::tc::t2_mma_bf16(d, a_lo + 2 * ks, b_lo + 2 * ks, IDESC_S, (c > 0 || ks > 0) ? 1u : 0u);
+          ako::tc::t2_commit_both(ako::smem_u32(&st_empty[stage]));
+          if (c == NCH - 1) ako::tc::t2_commit_both(ako::smem_u32(&s_full[buf]));
+        }
+        __syncwarp();
         if (++stage == NST) { stage = 0; ph ^= 1u; }
       }
-      if (ok) ako::tc::t2_commit_both(ako::smem_u32(&s_full[buf]));
     }
-  } else if (warp == 11 && lane == 0 && crank == 0 && ntk > 0) {
+  } else if (warp == 11 && crank == 0 && ntk > 0) {
     // ================================ PV issuer (for the pair) ===================================
     // a thread of its own: PV of tile j goes to the tensor pipe the moment P is written, while
     // the S issuer is still waiting on the operand stream of a later tile
@@ -399,15 +411,18 @@ mla_prefill_tc_kernel(PfParams p, const __grid_constant__ CUtensorMap tm_qn, con
     const uint32_t d = tmem + 256;
     for (int j = 0; j < ntk; ++j) {
       const int buf = j & 1;
-      if (!ako::tc::mbar_wait(ako::smem_u32(&p_full[buf]), (uint32_t)((j >> 1) & 1), &g_pf_status, 9)) break;
-      if (!ako::tc::mbar_wait(ako::smem_u32(&v_full), (uint32_t)(j & 1), &g_pf_status, 10)) break;
+      if (!ako::tc::mbar_wait_warp(ako::smem_u32(&p_full[buf]), (uint32_t)((j >> 1) & 1), &g_pf_status, 9)) break;
+      if (!ako::tc::mbar_wait_warp(ako::smem_u32(&v_full), (uint32_t)(j & 1), &g_pf_status, 10)) break;
       ako::tc::fence_after_thread_sync();
+      if (ako::tc::elect_one()) {
 #pragma unroll
-      for (int ks = 0; ks < BK / 16; ++ks)  // 16 keys = two 8-row groups of 1024 bytes
-        ako::tc::t2_mma_bf16_tmem_a(d, tmem + buf * BK + 8 * ks, v_lo + ks * (2048 >> 4), IDESC_PV, (j > 0 || ks > 0) ? 1u : 0u);
-      // P (inside the S buffer) and V have been read, O is up to date. Both CTAs wait for the last of
-      // these, so no signal is on its way to a CTA that leaves.
-      ako::tc::t2_commit_both(ako::smem_u32(&pv_done[buf]));
+        for (int ks = 0; ks < BK / 16; ++ks)  // 16 keys = two 8-row groups of 1024 bytes
+          ako::tc::t2_mma_bf16_tmem_a(d, tmem + buf * BK + 8 * ks, v_lo + ks * (2048 >> 4), IDESC_PV, (j > 0 || ks > 0) ? 1u : 0u);
+        // P (inside the S buffer) and V have been read, O is up to date. Both CTAs wait for the last of
+        // these, so no signal is on its way to a CTA that leaves.
+        ako::tc::t2_commit_both(ako::smem_u32(&pv_done[buf]));
+      }
+      __syncwarp();
     }
   }
 

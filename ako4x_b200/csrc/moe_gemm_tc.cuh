@@ -131,9 +131,11 @@ moe_gemm_tc_kernel(GemmParams p, const __grid_constant__ CUtensorMap tm_a, const
   } else if (warp == 9) {
     // ================================ TMA producer =============================================
     ako::tc::reg_dec<TC_REGS_OTHER>();
-    if (lane == 0) {
-      ako::tc::tma_prefetch_desc(&tm_a);
-      ako::tc::tma_prefetch_desc(&tm_b);
+    {  // the whole warp waits, one lane issues
+      if (ako::tc::elect_one()) {
+        ako::tc::tma_prefetch_desc(&tm_a);
+        ako::tc::tma_prefetch_desc(&tm_b);
+      }
       int g = 0;
       bool ok = true;
       for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
@@ -142,28 +144,31 @@ moe_gemm_tc_kernel(GemmParams p, const __grid_constant__ CUtensorMap tm_a, const
           const int stage = g % STAGES;
           const uint32_t ph = (g / STAGES) & 1;
           const uint32_t bar = ako::smem_u32(&s_full[stage]);
-          if (!ako::tc::mbar_wait(ako::smem_u32(&s_empty[stage]), ph ^ 1u, p.error, kErrLoad)) { ok = false; break; }
+          if (!ako::tc::mbar_wait_warp(ako::smem_u32(&s_empty[stage]), ph ^ 1u, p.error, kErrLoad)) { ok = false; break; }
           const uint32_t sa = smem_base + stage * STAGE_BYTES;
           const uint32_t sb = sa + A_BYTES;
-          ako::tc::mbar_arrive_expect_tx(bar, STAGE_BYTES);
-          ako::tc::tma_load_2d(sa, &tm_a, kb * 128, ti.row0, bar);
-          if (WHICH == 2) ako::tc::tma_load_2d(sa + TC_A_BYTES, &tm_a, INTER + kb * 128, ti.row0, bar);   // the lo piece
-          if (WHICH == 1) {
-            const int wr = ti.e * (2 * INTER) + ti.nt * 128;
-            ako::tc::tma_load_2d(sb, &tm_b, kb * 128, wr, bar);                         // g1, h cols 0-63
-            ako::tc::tma_load_2d(sb + 64 * 128, &tm_b, kb * 128, wr + INTER, bar);       // g2, h cols 0-63
-            ako::tc::tma_load_2d(sb + 128 * 128, &tm_b, kb * 128, wr + 64, bar);         // g1, 64-127
-            ako::tc::tma_load_2d(sb + 192 * 128, &tm_b, kb * 128, wr + INTER + 64, bar); // g2, 64-127
-          } else {
-            ako::tc::tma_load_2d(sb, &tm_b, kb * 128, ti.e * HID + ti.nt * TC_BN, bar);
+          if (ako::tc::elect_one()) {
+            ako::tc::mbar_arrive_expect_tx(bar, STAGE_BYTES);
+            ako::tc::tma_load_2d(sa, &tm_a, kb * 128, ti.row0, bar);
+            if (WHICH == 2) ako::tc::tma_load_2d(sa + TC_A_BYTES, &tm_a, INTER + kb * 128, ti.row0, bar);   // the lo piece
+            if (WHICH == 1) {
+              const int wr = ti.e * (2 * INTER) + ti.nt * 128;
+              ako::tc::tma_load_2d(sb, &tm_b, kb * 128, wr, bar);                         // g1, h cols 0-63
+              ako::tc::tma_load_2d(sb + 64 * 128, &tm_b, kb * 128, wr + INTER, bar);       // g2, h cols 0-63
+              ako::tc::tma_load_2d(sb + 128 * 128, &tm_b, kb * 128, wr + 64, bar);         // g1, 64-127
+              ako::tc::tma_load_2d(sb + 192 * 128, &tm_b, kb * 128, wr + INTER + 64, bar); // g2, 64-127
+            } else {
+              ako::tc::tma_load_2d(sb, &tm_b, kb * 128, ti.e * HID + ti.nt * TC_BN, bar);
+            }
           }
+          __syncwarp();
         }
       }
     }
   } else if (warp == 8) {
     // ================================ MMA issuer ===============================================
     ako::tc::reg_dec<TC_REGS_OTHER>();
-    if (lane == 0) {
+    {  // the whole warp waits, one lane issues
       // descriptor low words: +2 per K = 32 slice, bytes >> 4 per stage
       const uint32_t a_lo0 = ako::tc::smem_desc_lo(smem_base);
       const uint32_t b_lo0 = ako::tc::smem_desc_lo(smem_base + A_BYTES);
@@ -174,25 +179,28 @@ moe_gemm_tc_kernel(GemmParams p, const __grid_constant__ CUtensorMap tm_a, const
         for (int kb = 0; kb < NKB; ++kb, ++g) {
           const int buf = g & 1;
           const uint32_t aph = (g >> 1) & 1;
-          if (!ako::tc::mbar_wait(ako::smem_u32(&s_acc_empty[buf]), aph ^ 1u, p.error, kErrMmaAcc)) { ok = false; break; }
-          if (!ako::tc::mbar_wait(ako::smem_u32(&s_full[stage]), ph, p.error, kErrMmaFull)) { ok = false; break; }
+          if (!ako::tc::mbar_wait_warp(ako::smem_u32(&s_acc_empty[buf]), aph ^ 1u, p.error, kErrMmaAcc)) { ok = false; break; }
+          if (!ako::tc::mbar_wait_warp(ako::smem_u32(&s_full[stage]), ph, p.error, kErrMmaFull)) { ok = false; break; }
           ako::tc::fence_after_thread_sync();
           const uint32_t a_lo = a_lo0 + stage * (STAGE_BYTES >> 4);
           const uint32_t b_lo = b_lo0 + stage * (STAGE_BYTES >> 4);
           const uint32_t d = tmem_base + buf * TC_BN;
-          ako::tc::mma_f8_lohi<false>(d, a_lo, b_lo, IDESC);
-          ako::tc::mma_f8_lohi<true>(d, a_lo + 2, b_lo + 2, IDESC);
-          ako::tc::mma_f8_lohi<true>(d, a_lo + 4, b_lo + 4, IDESC);
-          ako::tc::mma_f8_lohi<true>(d, a_lo + 6, b_lo + 6, IDESC);
-          if (WHICH == 2) {   // the lo piece of h against the same weight block
-            const uint32_t a2 = a_lo + (TC_A_BYTES >> 4);
-            ako::tc::mma_f8_lohi<true>(d, a2, b_lo, IDESC);
-            ako::tc::mma_f8_lohi<true>(d, a2 + 2, b_lo + 2, IDESC);
-            ako::tc::mma_f8_lohi<true>(d, a2 + 4, b_lo + 4, IDESC);
-            ako::tc::mma_f8_lohi<true>(d, a2 + 6, b_lo + 6, IDESC);
+          if (ako::tc::elect_one()) {
+            ako::tc::mma_f8_lohi<false>(d, a_lo, b_lo, IDESC);
+            ako::tc::mma_f8_lohi<true>(d, a_lo + 2, b_lo + 2, IDESC);
+            ako::tc::mma_f8_lohi<true>(d, a_lo + 4, b_lo + 4, IDESC);
+            ako::tc::mma_f8_lohi<true>(d, a_lo + 6, b_lo + 6, IDESC);
+            if (WHICH == 2) {   // the lo piece of h against the same weight block
+              const uint32_t a2 = a_lo + (TC_A_BYTES >> 4);
+              ako::tc::mma_f8_lohi<true>(d, a2, b_lo, IDESC);
+              ako::tc::mma_f8_lohi<true>(d, a2 + 2, b_lo + 2, IDESC);
+              ako::tc::mma_f8_lohi<true>(d, a2 + 4, b_lo + 4, IDESC);
+              ako::tc::mma_f8_lohi<true>(d, a2 + 6, b_lo + 6, IDESC);
+            }
+            ako::tc::mma_commit(ako::smem_u32(&s_empty[stage]));
+            ako::tc::mma_commit(ako::smem_u32(&s_acc_full[buf]));
           }
-          ako::tc::mma_commit(ako::smem_u32(&s_empty[stage]));
-          ako::tc::mma_commit(ako::smem_u32(&s_acc_full[buf]));
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; ph ^= 1u; }
         }
       }
