@@ -444,7 +444,10 @@ mla_prefill_tc_kernel(PfParams p, const __grid_constant__ CUtensorMap tm_qn, con
 size_t ako_mla_prefill_tc_workspace_bytes(int64_t batch, int64_t num_kv_indices, int64_t page_size) {
   const int64_t ntok = num_kv_indices * page_size;
   if (ntok <= 0 || batch <= 0) return 0;
-  return ((size_t)ntok * DQK * 2 + 255) / 256 * 256;
+  const size_t kc = ((size_t)ntok * DQK * 2 + 255) / 256 * 256;
+  // The C ABI promises callers a size of 2 176 bytes per key and refuses less (the values were once
+  // copied a second time, transposed). The promise stands; only the first part is used.
+  return kc + (size_t)DC * 2 * (((size_t)ntok + 8 * (size_t)batch + 8 + 7) / 8 * 8);
 }
 
 int ako_mla_prefill_tc_launch(const void* q_nope, const void* q_pe, const void* ckv_cache, const void* kpe_cache,

@@ -4,7 +4,7 @@
 #include <stddef.h>
 #include <stdint.h>
 
-// Scratch the tensor-core prefill needs: a contiguous copy of the keys.
+// Scratch the tensor-core prefill asks for; it holds a contiguous copy of the keys.
 size_t ako_mla_prefill_tc_workspace_bytes(int64_t batch, int64_t num_kv_indices, int64_t page_size);
 
 // Returns an AKO4X_* status. All pointers are device pointers; nothing is read on the host.
