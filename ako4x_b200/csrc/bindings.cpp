@@ -420,9 +420,11 @@ PyObject* moe(PyObject*, PyObject* const* a, Py_ssize_t n) {
   need(shape_is(x0, {tokens, H}) && x0.element_size() == 1, "moe: hidden_states must be e4m3 [tokens, 7168]");
   need(shape_is(xs0, {H / 128, tokens}) && xs0.scalar_type() == at::kFloat, "moe: hidden_states_scale must be fp32 [56, tokens]");
   need(shape_is(w13, {n_local, 2 * I, H}) && w13.element_size() == 1, "moe: gemm1_weights must be e4m3 [E, 4096, 7168]");
-  need(shape_is(s13_0, {n_local, 2 * I / 128, H / 128}), "moe: gemm1_weights_scale must be fp32 [E, 32, 56]");
+  need(shape_is(s13_0, {n_local, 2 * I / 128, H / 128}) && s13_0.scalar_type() == at::kFloat,
+       "moe: gemm1_weights_scale must be fp32 [E, 32, 56]");
   need(shape_is(w2, {n_local, H, I}) && w2.element_size() == 1, "moe: gemm2_weights must be e4m3 [E, 7168, 2048]");
-  need(shape_is(s2_0, {n_local, H / 128, I / 128}), "moe: gemm2_weights_scale must be fp32 [E, 56, 16]");
+  need(shape_is(s2_0, {n_local, H / 128, I / 128}) && s2_0.scalar_type() == at::kFloat,
+       "moe: gemm2_weights_scale must be fp32 [E, 56, 16]");
   const Tensor lg = dense(lg0), rb = dense(rb0), x = dense(x0), xs = dense(xs0), s13 = dense(s13_0), s2 = dense(s2_0);
   Tensor out = empty({tokens, H}, at::kBFloat16, x);
   Workspace ws(ako4x_moe_fp8_block_scale_workspace_bytes(tokens, n_local), x);

@@ -166,6 +166,8 @@ class ExpertParallelMoE:
         dev = hidden_states.device
         if gemm1_weights.shape[0] != EXPERTS_PER_RANK:
             raise _cabi.Ako4xError("moe_ep: every rank holds 32 experts")
+        if gemm1_weights_scale.dtype != torch.float32 or gemm2_weights_scale.dtype != torch.float32:
+            raise _cabi.Ako4xError("moe_ep: gemm1_weights_scale and gemm2_weights_scale must be fp32")
         if T > self._cap:
             raise _cabi.Ako4xError("moe_ep: call prepare(tokens) on every rank before a larger step")
         out = torch.empty((T, H), dtype=torch.bfloat16, device=dev)

@@ -3,8 +3,9 @@ without a GPU (every call below is rejected, or is a zero-size no-op, before any
 import ctypes
 
 import pytest
+import torch
 
-from ako4x_b200 import _cabi
+from ako4x_b200 import _cabi, moe, moe_ep
 
 OK, EINVAL, EWORKSPACE = 0, -1, -4
 P = ctypes.c_void_p
@@ -84,3 +85,24 @@ def test_sparse_attention_and_moe_validation(L):
     need = L.ako4x_moe_fp8_block_scale_workspace_bytes(8, 32)
     assert need > 0
     assert moe(x, x, 0, x, x, x, x, x, x, 0, 2.5, x, 8, 32, None, 0, None) == EWORKSPACE
+
+
+@pytest.mark.parametrize("name", ["gemm1_weights_scale", "gemm2_weights_scale"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float64])
+def test_moe_weight_scales_of_another_type_are_refused(built_lib, name, dtype):
+    """The kernels read the weight scales as fp32: a narrower tensor of the right shape would be read
+    past its end. Refused before any device is touched, by the operator and by its expert-parallel form."""
+    e4m3 = torch.float8_e4m3fn
+    a = {"routing_logits": torch.zeros(4, 256), "routing_bias": torch.zeros(256),
+         "hidden_states": torch.empty((4, 7168), dtype=e4m3), "hidden_states_scale": torch.zeros(56, 4),
+         "gemm1_weights": torch.empty((32, 4096, 7168), dtype=e4m3, device="meta"),
+         "gemm1_weights_scale": torch.zeros(32, 32, 56),
+         "gemm2_weights": torch.empty((32, 7168, 2048), dtype=e4m3, device="meta"),
+         "gemm2_weights_scale": torch.zeros(32, 56, 16)}
+    a[name] = a[name].to(dtype)
+    with pytest.raises(_cabi.Ako4xError, match=f"{name} must be fp32"):
+        moe.run(*a.values(), 0, 2.5)
+    ep = moe_ep.ExpertParallelMoE(0, 2, backend="p2p")
+    ep._cap = 4
+    with pytest.raises(_cabi.Ako4xError, match="must be fp32"):
+        ep._run_p2p(*a.values(), 2.5)
