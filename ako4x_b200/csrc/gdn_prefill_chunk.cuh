@@ -19,6 +19,11 @@
 // own logarithms, never as a difference of two prefix sums, so strong decay elsewhere in a chunk
 // costs it nothing.
 //
+// Values that are not finite: a product takes in every token of its 8- or 16-token step, later ones with
+// coefficient zero, and 0 x NaN is NaN. A token whose right-hand side or delta is not finite is therefore
+// kept out of the tiles of earlier tokens, so that it spoils its row of the state from that token on and
+// nothing before it, as in the recurrence. Tiles with finite values only pay the check (1 to 3 %).
+//
 // Split: the state rows never interact, so a CTA owns 16 rows (v) of one (sequence, head). Two groups
 // of four warps share it. The chain group holds S: its warps split k (32 columns each), which makes
 // S0 k a sum over the warps but keeps every part of S in registers for the whole sequence, as mma
@@ -181,10 +186,11 @@ __global__ void __launch_bounds__(128, 7) gdn_chunk_prep_kernel(
     coef[lane] = exp2f(lc);
     coef[C_TOK + lane] = exp2f(run);
     __syncwarp();
+    const float bj = s_beta[e][j];          // may be NaN: enters at the diagonal, so that zeros above it stay zeros
     float t[C_TOK];
 #pragma unroll
     for (int i = 0; i < C_TOK; ++i) {
-      float x[4] = {(i == j) ? 1.f : 0.f, 0.f, 0.f, 0.f};
+      float x[4] = {(i == j) ? bj : 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int l = 0; l < i; l += 4) {
         const float4 w = *reinterpret_cast<const float4*>(out + i * A_PITCH + l);
@@ -195,10 +201,9 @@ __global__ void __launch_bounds__(128, 7) gdn_chunk_prep_kernel(
       }
       t[i] = (x[0] + x[1]) + (x[2] + x[3]);
     }
-    const float bj = s_beta[e][j];
     __syncwarp();
 #pragma unroll
-    for (int i = 0; i < C_TOK; ++i) out[i * C_TOK + ((j + i) & 31)] = t[i] * bj;
+    for (int i = 0; i < C_TOK; ++i) out[i * C_TOK + ((j + i) & 31)] = t[i];
   } else {
     float run = 0.f;
 #pragma unroll
@@ -278,6 +283,22 @@ __device__ __forceinline__ void mma_6(float (&d0)[4], float (&d1)[4], const uint
   ako::mma_bf16_16816(d0, A[1], B[1].x, B[1].y);
   ako::mma_bf16_16816(d1, A[0], B[2].x, B[2].y);
 }
+// The same over the first 8 of the 16 tokens: the last step of an even tile, where the other 8 come after
+// every token of the tile.
+__device__ __forceinline__ void mma_k8(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(b));
+}
+__device__ __forceinline__ void mma_6_half(float (&d0)[4], float (&d1)[4], const uint32_t (&A)[3][4], const uint2 (&B)[3]) {
+  mma_k8(d0, A[0][0], A[0][1], B[0].x);
+  mma_k8(d1, A[1][0], A[1][1], B[0].x);
+  mma_k8(d0, A[0][0], A[0][1], B[1].x);
+  mma_k8(d1, A[2][0], A[2][1], B[0].x);
+  mma_k8(d0, A[1][0], A[1][1], B[1].x);
+  mma_k8(d1, A[0][0], A[0][1], B[2].x);
+}
 // The A fragments (16 rows x 16 tokens, three pieces) of two neighbouring token tiles.
 __device__ __forceinline__ void frag_pieces(uint32_t (&A)[3][4], const uint2* src) {
 #pragma unroll
@@ -285,6 +306,34 @@ __device__ __forceinline__ void frag_pieces(uint32_t (&A)[3][4], const uint2* sr
     const uint2 x = src[p * 128], y = src[p * 128 + 32];
     A[p][0] = x.x; A[p][1] = x.y; A[p][2] = y.x; A[p][3] = y.y;
   }
+}
+// ---- values that are not finite ----
+__device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
+__device__ __forceinline__ float not_finite_sum(const float (&x)[4]) {   // 0, or NaN where one of them is not finite
+  return fmaf(x[0], 0.f, fmaf(x[1], 0.f, fmaf(x[2], 0.f, x[3] * 0.f)));
+}
+// Sign bits of the halves of a bf16 pair that are not finite.
+__device__ __forceinline__ uint32_t not_finite_pair(uint32_t u) { return ((u & 0x7f807f80u) + 0x00800080u) & 0x80008000u; }
+// Of a 16 x 8 tile (lane (g, t): tokens 2t, 2t + 1 of row g and of row g + 8), given as leading pieces: the
+// tokens in front of a row's first one that is not finite, as masks of the lane's two pairs.
+__device__ __forceinline__ void keep_before(uint32_t lead0, uint32_t lead1, int t, uint32_t& keep0, uint32_t& keep1) {
+  const uint32_t b0 = not_finite_pair(lead0), b1 = not_finite_pair(lead1);
+  int f0 = (b0 & 0x8000u) ? 2 * t : b0 ? 2 * t + 1 : 8, f1 = (b1 & 0x8000u) ? 2 * t : b1 ? 2 * t + 1 : 8;
+#pragma unroll
+  for (int o = 1; o <= 2; o <<= 1) {
+    f0 = min(f0, __shfl_xor_sync(0xffffffffu, f0, o));
+    f1 = min(f1, __shfl_xor_sync(0xffffffffu, f1, o));
+  }
+  keep0 = (2 * t < f0 ? 0xffffu : 0u) | (2 * t + 1 < f0 ? 0xffff0000u : 0u);
+  keep1 = (2 * t < f1 ? 0xffffu : 0u) | (2 * t + 1 < f1 ? 0xffff0000u : 0u);
+}
+// The other tokens become NaN.
+__device__ __forceinline__ void spoil(float (&x)[4], uint32_t keep0, uint32_t keep1) {
+  const float nan = __uint_as_float(0x7fffffffu);
+  if (!(keep0 & 0xffffu)) x[0] = nan;
+  if (!(keep0 >> 16)) x[1] = nan;
+  if (!(keep1 & 0xffffu)) x[2] = nan;
+  if (!(keep1 >> 16)) x[3] = nan;
 }
 // 8 x 8 transpose of bf16 pairs across the warp.
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
@@ -354,18 +403,38 @@ __device__ __forceinline__ void store_pieces(uint2* dst, const float (&x)[4]) {
 #pragma unroll
   for (int p = 0; p < 3; ++p) dst[p * 128] = make_uint2(f[p][0], f[p][1]);
 }
-// d0 + d1 (+)= (pieces of token tiles 0 .. w) x (tile w of T or P): one or two 16-token steps.
+// d0 + d1 (+)= (pieces of token tiles 0 .. w) x (tile w of T or P): one or two 16-token steps. Of tile w itself
+// only the tokens that keep0 and keep1 hold are taken in (`spoilt`, warp-uniform: not all of them). The
+// caller makes the masks ahead, off its serial chain: a vote between these loads and products cost 5 %.
 template <bool FIRST>
-__device__ __forceinline__ void triangular_tile(float (&d0)[4], float (&d1)[4], const uint2* pieces, const uint2* frag, bool two) {
+__device__ __forceinline__ void triangular_tile(float (&d0)[4], float (&d1)[4], const uint2* pieces, const uint2* frag, int w,
+                                                bool spoilt, uint32_t keep0, uint32_t keep1) {
   uint32_t A[3][4];
   uint2 B[3];
+  if (w >= 2) {
+    frag_pieces(A, pieces);
+    B[0] = frag[0]; B[1] = frag[32]; B[2] = frag[64];
+    mma_6<FIRST>(d0, d1, A, B);
+    pieces += 64;
+    frag += 96;
+  } else if (FIRST) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d0[i] = d1[i] = 0.f;
+  }
   frag_pieces(A, pieces);
   B[0] = frag[0]; B[1] = frag[32]; B[2] = frag[64];
-  mma_6<FIRST>(d0, d1, A, B);
-  if (two) {
-    frag_pieces(A, pieces + 64);
-    B[0] = frag[96]; B[1] = frag[128]; B[2] = frag[160];
+  if (w & 1) {
+    if (spoilt) {
+#pragma unroll
+      for (int p = 0; p < 3; ++p) { A[p][2] &= keep0; A[p][3] &= keep1; }
+    }
     mma_6<false>(d0, d1, A, B);
+  } else {
+    if (spoilt) {
+#pragma unroll
+      for (int p = 0; p < 3; ++p) { A[p][0] &= keep0; A[p][1] &= keep1; }
+    }
+    mma_6_half(d0, d1, A, B);
   }
 }
 
@@ -384,7 +453,6 @@ __global__ void __launch_bounds__(2 * C_WARPS * 32, 2) gdn_chunk_kernel(
   const int len = (int)(t1 - t0);
   const int chunks = (len > 0) ? (len + C_TOK - 1) / C_TOK : 0;
   const uint32_t sm = ako::smem_u32(smem);
-  const bool two = w >= 2;                          // tile w needs two 16-token steps of T and P
   const int ft = gdn_frag_tile(w, 0) * 96 + lane;   // its first fragment
   const unsigned char* slot = ws + (gdn_chunk_slot(t0, seq, 0) * P_HV + h) * C_SLOT_BYTES;
   const int64_t kq_off = ((t0 + g) * P_HQ + hq) * P_D + 32 * w + 8 * t;
@@ -462,12 +530,18 @@ __global__ void __launch_bounds__(2 * C_WARPS * 32, 2) gdn_chunk_kernel(
 
       // 2. right-hand side of tile w: v - gam (S0 k), as pieces for the group
       add_partials(x, sX, w, lane);
+      bool spoilt;
+      uint32_t keep0 = ~0u, keep1 = ~0u;
       {
         const float2 gam = *reinterpret_cast<const float2*>(coef + 8 * w + 2 * t);
         const __nv_bfloat16* vv = reinterpret_cast<const __nv_bfloat16*>(stage + C_CH_V) + (8 * w + 2 * t) * C_ROWS + g;
         const float r[4] = {__bfloat162float(vv[0]) - gam.x * x[0], __bfloat162float(vv[C_ROWS]) - gam.y * x[1],
                             __bfloat162float(vv[8]) - gam.x * x[2], __bfloat162float(vv[C_ROWS + 8]) - gam.y * x[3]};
         store_pieces(sR + w * 32, r);
+        spoilt = __any_sync(0xffffffffu, !(not_finite_sum(r) == 0.f));
+        if (spoilt)
+          keep_before(__byte_perm(__float_as_uint(r[0]), __float_as_uint(r[1]), 0x7632),
+                      __byte_perm(__float_as_uint(r[2]), __float_as_uint(r[3]), 0x7632), t, keep0, keep1);
       }
       const float gC = coef[C_TOK - 1];
       const float2 dec = *reinterpret_cast<const float2*>(coef + C_TOK + 8 * w + 2 * t);
@@ -479,9 +553,10 @@ __global__ void __launch_bounds__(2 * C_WARPS * 32, 2) gdn_chunk_kernel(
 
       // 3. delta of tile w = T (right-hand side)
       float d0[4], d1[4];
-      triangular_tile<true>(d0, d1, sR, reinterpret_cast<const uint2*>(stage + C_CH_SLOT) + ft, two);
+      triangular_tile<true>(d0, d1, sR, reinterpret_cast<const uint2*>(stage + C_CH_SLOT) + ft, w, spoilt, keep0, keep1);
 #pragma unroll
       for (int i = 0; i < 4; ++i) d0[i] += d1[i];
+      if (spoilt) spoil(d0, keep0, keep1);
       {
         const float e[4] = {d0[0] * dec.x, d0[1] * dec.y, d0[2] * dec.x, d0[3] * dec.y};
         store_pieces(sE + w * 32, e);
@@ -553,15 +628,20 @@ __global__ void __launch_bounds__(2 * C_WARPS * 32, 2) gdn_chunk_kernel(
       ako::cp_async_wait<1>();
       __syncwarp();
       const unsigned char* stage = smem + C_OFF_OUT + b * C_OUT_STAGE;
+      const uint2 own = (reinterpret_cast<const uint2*>(smem + C_OFF_D + b * C_D_BYTES) + lane)[w * 32];   // leading pieces of tile w
       float y[4];
       partial_products(y, As, sm + C_OFF_OUT + b * C_OUT_STAGE + w * C_KQ_WARP, sY, w, lane);
+      const bool spoilt = __any_sync(0xffffffffu, (not_finite_pair(own.x) | not_finite_pair(own.y)) != 0u);
+      uint32_t keep0 = ~0u, keep1 = ~0u;
+      if (spoilt) keep_before(own.x, own.y, t, keep0, keep1);
       bar_sync(C_BAR_OUT, GROUP);
       add_partials(y, sY, w, lane);
       const float2 gam = *reinterpret_cast<const float2*>(reinterpret_cast<const float*>(stage + C_OUT_COEF) + 8 * w + 2 * t);
       float o0[4] = {scale * gam.x * y[0], scale * gam.y * y[1], scale * gam.x * y[2], scale * gam.y * y[3]};
       float o1[4] = {0.f, 0.f, 0.f, 0.f};
       triangular_tile<false>(o0, o1, reinterpret_cast<const uint2*>(smem + C_OFF_D + b * C_D_BYTES) + lane,
-                             reinterpret_cast<const uint2*>(stage + C_OUT_SLOT) + ft, two);
+                             reinterpret_cast<const uint2*>(stage + C_OUT_SLOT) + ft, w, spoilt, keep0, keep1);
+      if (spoilt) spoil(o0, keep0, keep1);
       if (c + 2 < chunks) bar_arrive(C_BAR_EMPTY + b, 2 * GROUP);
       // transposed across the warp: lane (g, t) gets token g, rows 2t, 2t+1 (and + 8)
       const uint32_t y0 = movmatrix_trans(ako::pack_bf16x2(o0[0] + o1[0], o0[1] + o1[1]));
@@ -594,6 +674,36 @@ static_assert(CW_STAGE % 128 == 0 && 3 * (CW_SMEM + 1024) <= 228 * 1024, "three 
 __device__ __forceinline__ void tile_pieces(uint32_t (&A)[3][4], int half, const float (&x)[4]) {
   split3_exact(x[0], x[1], A[0][2 * half], A[1][2 * half], A[2][2 * half]);
   split3_exact(x[2], x[3], A[0][2 * half + 1], A[1][2 * half + 1], A[2][2 * half + 1]);
+}
+
+__device__ __forceinline__ bool wide_not_finite(const float (&x)[4][4]) {
+  const float z = (not_finite_sum(x[0]) + not_finite_sum(x[1])) + (not_finite_sum(x[2]) + not_finite_sum(x[3]));
+  return __any_sync(0xffffffffu, !(z == 0.f));
+}
+// Moves f0 and f1 (rows g, g + 8) up to the row's first token that is not finite.
+__device__ __forceinline__ void wide_first_not_finite(const float (&x)[4][4], int& f0, int& f1, int t) {
+#pragma unroll
+  for (int n = 0; n < 4; ++n)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if (not_finite(x[n][i])) f0 = min(f0, 8 * n + 2 * t + i);
+      if (not_finite(x[n][2 + i])) f1 = min(f1, 8 * n + 2 * t + i);
+    }
+#pragma unroll
+  for (int o = 1; o <= 2; o <<= 1) {
+    f0 = min(f0, __shfl_xor_sync(0xffffffffu, f0, o));
+    f1 = min(f1, __shfl_xor_sync(0xffffffffu, f1, o));
+  }
+}
+// Sets the tokens from f0 (f1) on to `value`.
+__device__ __forceinline__ void wide_set(float (&x)[4][4], float value, int f0, int f1, int t) {
+#pragma unroll
+  for (int n = 0; n < 4; ++n)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if (8 * n + 2 * t + i >= f0) x[n][i] = value;
+      if (8 * n + 2 * t + i >= f1) x[n][2 + i] = value;
+    }
 }
 
 __global__ void __launch_bounds__(128, 3) gdn_chunk_wide_kernel(
@@ -726,6 +836,13 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_wide_kernel(
         yr[0] *= scale * gam.x; yr[1] *= scale * gam.y; yr[2] *= scale * gam.x; yr[3] *= scale * gam.y;
       }
     }
+    // the first token of rows g and g + 8 that is not finite; it and later ones are left out of the products
+    int f0 = C_TOK, f1 = C_TOK;
+    bool spoilt = wide_not_finite(x);
+    if (spoilt) {
+      wide_first_not_finite(x, f0, f1, t);
+      wide_set(x, 0.f, f0, f1, t);
+    }
     // 3. delta = T (right-hand side), tile by tile
     float d[4][4];
     {
@@ -735,18 +852,30 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_wide_kernel(
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
         float d1[4];
+        if (n == 0) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) d[n][i] = d1[i] = 0.f;
+        }
 #pragma unroll
         for (int s = 0; s <= n / 2; ++s) {
           const uint2* f = sT + gdn_frag_tile(n, s) * 96;
           const uint2 B[3] = {f[0], f[32], f[64]};
-          if (s == 0) mma_6<true>(d[n], d1, A[s], B);
+          if (s == n / 2 && n % 2 == 0) mma_6_half(d[n], d1, A[s], B);
+          else if (s == 0) mma_6<true>(d[n], d1, A[s], B);
           else mma_6<false>(d[n], d1, A[s], B);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) d[n][i] += d1[i];
       }
     }
+    if (wide_not_finite(d)) spoilt = true;   // also an overflow
     // 4. outputs
+    const float nan = __uint_as_float(0x7fffffffu);
+    if (spoilt) {
+      wide_first_not_finite(d, f0, f1, t);
+      wide_set(d, 0.f, f0, f1, t);
+      wide_set(y, nan, f0, f1, t);
+    }
     {
       uint32_t A[2][3][4];
 #pragma unroll
@@ -754,11 +883,17 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_wide_kernel(
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
         float o1[4];
+        if (n == 0) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) o1[i] = 0.f;
+        }
 #pragma unroll
         for (int s = 0; s <= n / 2; ++s) {
           const uint2* f = sP + gdn_frag_tile(n, s) * 96;
           const uint2 B[3] = {f[0], f[32], f[64]};
-          if (s == 0) {
+          if (s == n / 2 && n % 2 == 0) {
+            mma_6_half(y[n], o1, A[s], B);
+          } else if (s == 0) {
             ako::mma_bf16_16816(y[n], A[0][0], B[0].x, B[0].y);
             mma_zero(o1, A[0][1], B[0].x, B[0].y);
             ako::mma_bf16_16816(y[n], A[0][0], B[1].x, B[1].y);
@@ -788,13 +923,13 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_wide_kernel(
         const float e[4] = {d[n][0] * dec.x, d[n][1] * dec.y, d[n][2] * dec.x, d[n][3] * dec.y};
         tile_pieces(A[n >> 1], n & 1, e);
       }
-      const float gC = coef[C_TOK - 1];
+      const float gC = coef[C_TOK - 1], g0 = (spoilt && f0 < C_TOK) ? nan : gC, g1 = (spoilt && f1 < C_TOK) ? nan : gC;
 #pragma unroll
       for (int n = 0; n < 16; n += 2) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          S[n][i] *= gC;
-          S[n + 1][i] *= gC;
+          S[n][i] *= (i < 2) ? g0 : g1;
+          S[n + 1][i] *= (i < 2) ? g0 : g1;
         }
 #pragma unroll
         for (int s = 0; s < 2; ++s) {

@@ -115,3 +115,34 @@ def test_chunk_edges_and_tokens_outside(lens, lead, tail):
     assert (s1 - s2).abs().max().item() <= 2e-6 * max(lens) ** 0.5 * s1.abs().max().item()
     assert_close_bf16(o2.cpu(), o1.cpu(), atol=2e-3, rtol=2e-2)
     assert (o1 == o2).float().mean().item() > 0.99
+
+
+@pytest.mark.parametrize("kind,value", [("v", "inf"), ("v", "nan"), ("k", "nan"), ("k", "-inf"), ("q", "nan"), ("a", "nan"),
+                                        ("b", "nan"), ("a", "inf"), ("b", "-inf"), ("state", "nan"), ("state", "inf")])
+@pytest.mark.parametrize("lens", [[75], [40, 7, 75], [75, 1, 40] + [5] * 21])
+def test_values_that_are_not_finite_reach_no_earlier_token(kind, value, lens):
+    """A value that is not finite spoils what the recurrence makes of it (its own output, or its row of the
+    state from its token on) and nothing else: every other output and state element is as in the
+    token-by-token form. Tokens at the edges and inside of the 8-, 16- and 32-token steps of the chunked
+    form, and where there are several sequences the first one of another (the gate values +inf of `a` and
+    -inf of `b` are zero decay and zero update: nothing is spoilt)."""
+    a = W.make_gdn_prefill(lens, shape_id=77 + len(lens))
+    start = 0 if lens[0] == 75 else lens[0] + lens[1]
+    x = float(value)
+    if kind == "state":
+        a["state"][lens.index(75), 3, 17, 5] = x
+        a["state"][lens.index(75), 6, 90, 127] = x
+    else:
+        t = {("v", "inf"): 20, ("v", "nan"): 63, ("k", "nan"): 9, ("k", "-inf"): 47, ("q", "nan"): 16, ("a", "nan"): 5,
+             ("b", "nan"): 30, ("a", "inf"): 12, ("b", "-inf"): 55}[kind, value]
+        a[kind][start + t].view(-1)[::3] = x
+        if len(lens) > 1:
+            a[kind][(start + 75) % sum(lens)].view(-1)[1] = x
+    args = [a[k].cuda() for k in KEYS]
+    o1, s1 = gdn_prefill.run(*args, a["scale"], _chunked=False)
+    o2, s2 = gdn_prefill.run(*args, a["scale"])
+    fo, fs = torch.isfinite(o1.float()), torch.isfinite(s1)
+    assert torch.equal(torch.isfinite(o2.float()), fo) and torch.equal(torch.isfinite(s2), fs)
+    if fs.any():
+        assert (s1[fs] - s2[fs]).abs().max().item() <= 2e-6 * 75 ** 0.5 * s1[fs].abs().max().item()
+    assert_close_bf16(o2[fo], o1[fo], atol=2e-3, rtol=2e-2)
