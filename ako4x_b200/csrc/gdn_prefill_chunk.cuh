@@ -628,17 +628,17 @@ __global__ void __launch_bounds__(2 * C_WARPS * 32, 2) gdn_chunk_kernel(
       ako::cp_async_wait<1>();
       __syncwarp();
       const unsigned char* stage = smem + C_OFF_OUT + b * C_OUT_STAGE;
-      const uint2 own = (reinterpret_cast<const uint2*>(smem + C_OFF_D + b * C_D_BYTES) + lane)[w * 32];   // leading pieces of tile w
       float y[4];
       partial_products(y, As, sm + C_OFF_OUT + b * C_OUT_STAGE + w * C_KQ_WARP, sY, w, lane);
-      const bool spoilt = __any_sync(0xffffffffu, (not_finite_pair(own.x) | not_finite_pair(own.y)) != 0u);
-      uint32_t keep0 = ~0u, keep1 = ~0u;
-      if (spoilt) keep_before(own.x, own.y, t, keep0, keep1);
       bar_sync(C_BAR_OUT, GROUP);
       add_partials(y, sY, w, lane);
       const float2 gam = *reinterpret_cast<const float2*>(reinterpret_cast<const float*>(stage + C_OUT_COEF) + 8 * w + 2 * t);
       float o0[4] = {scale * gam.x * y[0], scale * gam.y * y[1], scale * gam.x * y[2], scale * gam.y * y[3]};
       float o1[4] = {0.f, 0.f, 0.f, 0.f};
+      const uint2 own = (reinterpret_cast<const uint2*>(smem + C_OFF_D + b * C_D_BYTES) + lane)[w * 32];   // leading pieces of tile w
+      const bool spoilt = __any_sync(0xffffffffu, (not_finite_pair(own.x) | not_finite_pair(own.y)) != 0u);
+      uint32_t keep0 = ~0u, keep1 = ~0u;
+      if (spoilt) keep_before(own.x, own.y, t, keep0, keep1);
       triangular_tile<false>(o0, o1, reinterpret_cast<const uint2*>(smem + C_OFF_D + b * C_D_BYTES) + lane,
                              reinterpret_cast<const uint2*>(stage + C_OUT_SLOT) + ft, w, spoilt, keep0, keep1);
       if (spoilt) spoil(o0, keep0, keep1);
