@@ -6,7 +6,8 @@
 //   out_t[v] = scale S[v,:].q_t = scale (g S_old[v,:].q_t + (q_t.k_t) delta[v])
 // (the recurrence reference/gdn-prefill/variants/cuda_graph_v5/kernel.py evaluates in chunked form,
 // :1333-1400 for its entry point). Calls with a workspace run it in chunks on the tensor cores
-// (gdn_prefill_chunk.cuh). The kernel in this file needs no workspace: the rows S[v,:] of a state never
+// (gdn_prefill_chunk.cuh) unless their sequences are a few tokens long. The kernel in this file needs no
+// workspace: the rows S[v,:] of a state never
 // interact, so it runs the recurrence as it is written, token by token: a row is held by 8 or 16 lanes
 // (16 or 8 state values each, in registers for the whole sequence), four compute warps own 16 or 8
 // rows of one (sequence, head) -- 64 or 128 CTAs per sequence --, q_t / k_t pass through shared memory
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(P_THREADS) gdn_prefill_kernel(
     const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
     const float* __restrict__ state, const float* __restrict__ A_log, const __nv_bfloat16* __restrict__ a,
     const float* __restrict__ dt_bias, const __nv_bfloat16* __restrict__ b, const int64_t* __restrict__ cu_seqlens,
-    float scale, __nv_bfloat16* __restrict__ out, float* __restrict__ new_state) {
+    float scale, __nv_bfloat16* __restrict__ out, float* __restrict__ new_state, int64_t zero_total) {
   constexpr int EPL = P_D / LPR;            // state values per lane (16 or 8)
   constexpr int NI = EPL / 4;               // float4 pieces per lane
   constexpr int ISTR = 4 * LPR;             // elements between a lane's pieces
@@ -122,6 +123,14 @@ __global__ void __launch_bounds__(P_THREADS) gdn_prefill_kernel(
   const int seg = lane % LPR;
   float* ns = new_state + (((int64_t)seq * P_HV + h) * P_D + row) * P_D + seg * 4;
 
+  if (zero_total > 0) {   // tokens outside every sequence: zero, by the CTAs of the first and of the last sequence
+    for (int side = 0; side < 2; ++side) {
+      if (seq != (side ? (int)gridDim.z - 1 : 0)) continue;
+      const int64_t z0 = side ? max(t1, (int64_t)0) : 0, z1 = side ? zero_total : min(t0, zero_total);
+      for (int64_t i = z0 * (P_ROWS / 8) + tid; i < z1 * (P_ROWS / 8); i += P_THREADS)
+        *reinterpret_cast<uint4*>(out + (i / (P_ROWS / 8) * P_HV + h) * P_D + rg * P_ROWS + i % (P_ROWS / 8) * 8) = make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
   float S[EPL];
   if (len <= 0) {   // the definition leaves the new state of an empty sequence at zero
     if (!producer) {
@@ -226,6 +235,16 @@ __global__ void __launch_bounds__(P_THREADS) gdn_prefill_kernel(
 
 #include "gdn_prefill_chunk.cuh"
 
+// Sequences so short on average that the second launch and the fixed cost of a 32-token chunk are more than
+// the serial steps: token by token then, although there is a workspace. Measured, token by token against
+// chunked (us): 1 x 8 tokens 5.1 against 9.4, 3 x 8 6.8 (9.8), 3 x 16 9.6 (9.8); 16 x 8 18.6 (19.9);
+// 20 x 4 14.5 (17.2), 20 x 8 19.3 (17.2); 32 x 2 18.2 (20.5), 32 x 4 22.4 (20.5); 48 x 2 25.6 (27.4), 64 x 1
+// 30.3 (30.1). A longer sequence among them stays below 152 tokens, 30 us.
+bool few_tokens(int64_t total_tokens, int64_t num_seqs) {
+  const int64_t most = num_seqs < 20 ? 8 : num_seqs < 32 ? 4 : num_seqs < 64 ? 2 : 0;
+  return total_tokens <= most * num_seqs;
+}
+
 }  // namespace
 
 extern "C" size_t ako4x_gdn_prefill_workspace_bytes(int64_t total_tokens, int64_t num_seqs) {
@@ -246,10 +265,13 @@ extern "C" int ako4x_gdn_prefill(const void* q, const void* k, const void* v, co
   cudaStream_t st = (cudaStream_t)stream;
   const __nv_bfloat16 *qb = (const __nv_bfloat16*)q, *kb = (const __nv_bfloat16*)k, *vb = (const __nv_bfloat16*)v;
   const __nv_bfloat16 *ab = (const __nv_bfloat16*)a, *bb = (const __nv_bfloat16*)b;
-  if (workspace != nullptr && total_tokens > 0) {
-    // chunked form: the token-only matrices of every chunk first, then 64 CTAs per sequence
+  const bool with_workspace = workspace != nullptr && total_tokens > 0;
+  if (with_workspace) {
     if (((uintptr_t)workspace & 15) || workspace_bytes < ako4x_gdn_prefill_workspace_bytes(total_tokens, num_seqs))
       return AKO4X_EWORKSPACE;
+  }
+  if (with_workspace && !few_tokens(total_tokens, num_seqs)) {
+    // chunked form: the token-only matrices of every chunk first, then 64 CTAs per sequence
     const int64_t slots = total_tokens / C_TOK + num_seqs;
     if (slots > 0x7fffffffLL) return AKO4X_EINVAL;
     if (!ako::ensure_dynamic_smem<gdn_chunk_kernel>(C_SMEM_ALONE)) return AKO4X_ELAUNCH;
@@ -278,15 +300,16 @@ extern "C" int ako4x_gdn_prefill(const void* q, const void* k, const void* v, co
       return AKO4X_ELAUNCH;
     return AKO4X_OK;
   }
-  // No workspace: token by token. One or two sequences: 16 lanes per row (128 CTAs per sequence, the
+  // Token by token. One or two sequences: 16 lanes per row (128 CTAs per sequence, the
   // shorter serial chain per token); more: 8 lanes per row (half the instructions per row and token;
   // measured better from three sequences on, 4 x 2 048: 675 against 734 us).
+  const int64_t zero_total = with_workspace ? total_tokens : 0;
   if (num_seqs <= 2) {
     gdn_prefill_kernel<16><<<dim3(P_D / 8, P_HV, (unsigned)num_seqs), P_THREADS, 0, st>>>(
-        qb, kb, vb, state, A_log, ab, dt_bias, bb, cu_seqlens, scale, (__nv_bfloat16*)out, new_state);
+        qb, kb, vb, state, A_log, ab, dt_bias, bb, cu_seqlens, scale, (__nv_bfloat16*)out, new_state, zero_total);
   } else {
     gdn_prefill_kernel<8><<<dim3(P_D / 16, P_HV, (unsigned)num_seqs), P_THREADS, 0, st>>>(
-        qb, kb, vb, state, A_log, ab, dt_bias, bb, cu_seqlens, scale, (__nv_bfloat16*)out, new_state);
+        qb, kb, vb, state, A_log, ab, dt_bias, bb, cu_seqlens, scale, (__nv_bfloat16*)out, new_state, zero_total);
   }
   AKO_CHECK_LAUNCH();
   return AKO4X_OK;

@@ -312,10 +312,11 @@ int ako4x_gemm_device_status(void);
  * output taken after each update. An empty sequence gets a zero new_state (as the definition
  * does).
  * With a workspace of ako4x_gdn_prefill_workspace_bytes(total_tokens, num_seqs) bytes (16-byte
- * aligned) the recurrence runs in chunks of 32 tokens on the tensor cores (a kernel that makes the
- * token-only triangular matrices of all chunks, then the state kernel), and tokens that belong to no
- * sequence are set to zero; with a NULL workspace it runs token by token in one launch and leaves such
- * tokens as they are. Same results up to fp32 rounding order. */
+ * aligned) tokens that belong to no sequence are set to zero, and the recurrence runs in chunks of 32
+ * tokens on the tensor cores (a kernel that makes the token-only triangular matrices of all chunks, then
+ * the state kernel), or token by token in one launch where the sequences have a few tokens on average;
+ * with a NULL workspace it always runs token by token and leaves such tokens as they are. Same results up
+ * to fp32 rounding order. */
 size_t ako4x_gdn_prefill_workspace_bytes(int64_t total_tokens, int64_t num_seqs);
 int ako4x_gdn_prefill(const void* q, const void* k, const void* v, const float* state,
                       const float* A_log, const void* a, const float* dt_bias, const void* b,

@@ -146,3 +146,27 @@ def test_values_that_are_not_finite_reach_no_earlier_token(kind, value, lens):
     if fs.any():
         assert (s1[fs] - s2[fs]).abs().max().item() <= 2e-6 * 75 ** 0.5 * s1[fs].abs().max().item()
     assert_close_bf16(o2[fo], o1[fo], atol=2e-3, rtol=2e-2)
+
+
+@pytest.mark.parametrize("lens", [[1], [8], [1, 1, 1], [24, 0, 0], [0, 9, 15], [8] * 19, [1] * 18 + [134], [4] * 20, [2] * 63, [9], [25, 0, 0],
+                                  [8] * 18 + [9], [4] * 19 + [5], [2] * 62 + [3], [1] * 64])
+@pytest.mark.parametrize("state", [True, False])
+def test_few_tokens_per_sequence(lens, state):
+    """Sequences of a few tokens on average run token by token (up to 8 tokens for fewer than 20 sequences,
+    4 for fewer than 32, 2 for fewer than 64), which is then the very same kernel; just above the line the
+    two forms differ in the order of fp32 sums. Tokens in front of and behind the sequences are zero."""
+    n = len(lens)
+    most = n * (8 if n < 20 else 4 if n < 32 else 2 if n < 64 else 0)
+    for lead, tail in ((0, 0), (2, 1)):
+        a = W.make_gdn_prefill([lead] + lens + [tail], shape_id=13 + n, with_state=state)
+        a["cu_seqlens"] = a["cu_seqlens"][1:n + 2].contiguous()
+        if state:
+            a["state"] = a["state"][1:n + 1].contiguous()
+        args = [a[k].cuda() if a[k] is not None else None for k in KEYS]
+        o1, s1 = gdn_prefill.run(*args, a["scale"], _chunked=False)
+        o2, s2 = gdn_prefill.run(*args, a["scale"])
+        assert torch.all(o2[:lead] == 0) and torch.all(o2[lead + sum(lens):] == 0)
+        if lead + sum(lens) + tail <= most:
+            assert torch.equal(o1, o2) and torch.equal(s1, s2)
+        assert (s1 - s2).abs().max().item() <= 2e-6 * max(lens) ** 0.5 * max(s1.abs().max().item(), 1e-3)
+        assert_close_bf16(o2.cpu(), o1.cpu(), atol=2e-3, rtol=2e-2)
