@@ -265,11 +265,12 @@ extern "C" int ako4x_gdn_prefill(const void* q, const void* k, const void* v, co
   cudaStream_t st = (cudaStream_t)stream;
   const __nv_bfloat16 *qb = (const __nv_bfloat16*)q, *kb = (const __nv_bfloat16*)k, *vb = (const __nv_bfloat16*)v;
   const __nv_bfloat16 *ab = (const __nv_bfloat16*)a, *bb = (const __nv_bfloat16*)b;
-  const bool with_workspace = workspace != nullptr && total_tokens > 0;
-  if (with_workspace) {
-    if (((uintptr_t)workspace & 15) || workspace_bytes < ako4x_gdn_prefill_workspace_bytes(total_tokens, num_seqs))
-      return AKO4X_EWORKSPACE;
-  }
+  // From three sequences on, a workspace that cannot be used counts as none, as it did when only calls with
+  // one or two sequences used one at all; those refuse it.
+  const bool usable = ((uintptr_t)workspace & 15) == 0 &&
+                      workspace_bytes >= ako4x_gdn_prefill_workspace_bytes(total_tokens, num_seqs);
+  if (workspace != nullptr && !usable && num_seqs <= 2) return AKO4X_EWORKSPACE;
+  const bool with_workspace = workspace != nullptr && usable && total_tokens > 0;
   if (with_workspace && !few_tokens(total_tokens, num_seqs)) {
     // chunked form: the token-only matrices of every chunk first, then 64 CTAs per sequence
     const int64_t slots = total_tokens / C_TOK + num_seqs;

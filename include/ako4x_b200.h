@@ -316,7 +316,8 @@ int ako4x_gemm_device_status(void);
  * tokens on the tensor cores (a kernel that makes the token-only triangular matrices of all chunks, then
  * the state kernel), or token by token in one launch where the sequences have a few tokens on average;
  * with a NULL workspace it always runs token by token and leaves such tokens as they are. Same results up
- * to fp32 rounding order. */
+ * to fp32 rounding order. A workspace that is too small or not aligned is refused (AKO4X_EWORKSPACE) for
+ * one or two sequences and counts as NULL for more. */
 size_t ako4x_gdn_prefill_workspace_bytes(int64_t total_tokens, int64_t num_seqs);
 int ako4x_gdn_prefill(const void* q, const void* k, const void* v, const float* state,
                       const float* A_log, const void* a, const float* dt_bias, const void* b,

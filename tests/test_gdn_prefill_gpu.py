@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import oracle
-from ako4x_b200 import gdn_decode, gdn_prefill, workloads as W
+from ako4x_b200 import _cabi, gdn_decode, gdn_prefill, workloads as W
 from conftest import assert_close_bf16, load_golden
 
 pytestmark = pytest.mark.gpu
@@ -170,3 +170,25 @@ def test_few_tokens_per_sequence(lens, state):
             assert torch.equal(o1, o2) and torch.equal(s1, s2)
         assert (s1 - s2).abs().max().item() <= 2e-6 * max(lens) ** 0.5 * max(s1.abs().max().item(), 1e-3)
         assert_close_bf16(o2.cpu(), o1.cpu(), atol=2e-3, rtol=2e-2)
+
+
+@pytest.mark.parametrize("lens,offset,short,expected", [([40, 9, 50], 0, 16, 0), ([40, 9, 50], 8, 0, 0), ([40, 9, 50], 0, 0, 0),
+                                                        ([40, 9], 0, 16, -4), ([40, 9], 8, 0, -4), ([40, 9], 0, 0, 0)])
+def test_workspace_that_cannot_be_used(lens, offset, short, expected):
+    """Too small (by `short` bytes) or misaligned: refused for one or two sequences, as good as none for more
+    (the token-by-token form, whose outputs leave tokens outside the sequences as they are)."""
+    L = _cabi.lib()
+    a = W.make_gdn_prefill([3] + lens, shape_id=3, device="cuda")
+    n, T = len(lens), 3 + sum(lens)
+    a["state"], a["cu_seqlens"] = a["state"][1:].contiguous(), a["cu_seqlens"][1:].contiguous()
+    need = L.ako4x_gdn_prefill_workspace_bytes(T, n)
+    ws = torch.empty(need + 16, dtype=torch.uint8, device="cuda")
+    o = torch.full((T, 8, 128), 7.0, dtype=torch.bfloat16, device="cuda")
+    s = torch.empty((n, 8, 128, 128), device="cuda")
+    st = L.ako4x_gdn_prefill(*[_cabi.ptr(a[k]) for k in KEYS], a["scale"], _cabi.ptr(o), _cabi.ptr(s), T, n,
+                             ws.data_ptr() + offset, need - short, _cabi.stream())
+    assert st == expected
+    if expected == 0:
+        ro, rs = gdn_prefill.run(*[a[k] for k in KEYS], a["scale"], _chunked=bool(not offset and not short))
+        assert torch.equal(s, rs) and torch.equal(o[3:], ro[3:])
+        assert torch.all(o[:3] == (7.0 if offset or short else 0.0))
