@@ -193,6 +193,13 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gqa_decode_kernel(Params
       s[3] = ako::fast_exp2(s[3] - m1);
       l0 += s[0] + s[2];
       l1 += s[1] + s[3];
+      if (tile * TILE + TILE > len) {   // past the end: weight 0, but the row read in their place may hold infinities
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (!v0) vc[0][j] = make_uint4(0u, 0u, 0u, 0u);
+          if (!v1) vc[1][j] = make_uint4(0u, 0u, 0u, 0u);
+        }
+      }
       const uint32_t b0 = movmatrix_trans(ako::pack_bf16x2(s[0], s[1])), b1 = movmatrix_trans(ako::pack_bf16x2(s[2], s[3]));
 #pragma unroll
       for (int j = 0; j < 4; ++j) {

@@ -126,3 +126,18 @@ def test_shares_and_whole_sequences(built_lib, lens):
     """Many short sequences (one share each, no partials, no merge), a batch just inside that rule, and
     few sequences whose partials come from one or from hundreds of shares; empty ones in between."""
     _check(W.make_gqa_decode(len(lens), shape_id=60 + len(lens) % 7, lens=lens, extra_pages=11))
+
+
+@pytest.mark.parametrize("lens", [[1], [5], [8, 9], [21, 16, 47], [700, 30], [7] * 230])
+def test_infinity_in_the_last_value_row(built_lib, lens):
+    """The lanes of a last tile that have no token of their own read the last one again, with weight 0: an
+    infinity there stays one (0 x inf would make it NaN)."""
+    a = W.make_gqa_decode(len(lens), shape_id=5, lens=lens, extra_pages=3)
+    for b in range(len(lens)):
+        a["v_cache"][int(a["kv_indices"][int(a["kv_indptr"][b + 1]) - 1]), 0, b % 8, 40 + b % 64] = float("inf") if b % 2 else float("-inf")
+    o, lse = _run(a)
+    ro, rlse = oracle.gqa_paged_decode(*[a[k] for k in KEYS])
+    assert torch.equal(o.cpu()[~torch.isfinite(ro)], ro[~torch.isfinite(ro)]) and torch.isfinite(o.cpu()[torch.isfinite(ro)]).all()
+    assert torch.isinf(ro).any() and not torch.isnan(ro).any()
+    assert_close_bf16(o.cpu()[torch.isfinite(ro)], ro[torch.isfinite(ro)])
+    assert_lse_close(lse, rlse)
