@@ -19,6 +19,8 @@
 // bulk copies through shared memory and a planning kernel before -> now): 64 sequences of up to 8 192 tokens
 // 245 -> 188 us (6.3 TB/s = 0.96 of the measured copy bandwidth), 256 of them 841 -> 680 (0.99), 16 of up to
 // 1 200 25 -> 17, one of 547 12.6 -> 10.2 us.
+#include <cfloat>
+
 #include "flat_share.cuh"
 
 namespace {
@@ -144,7 +146,9 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gqa_decode_kernel(Params
       for (int u = 0; u < 2; ++u)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[j][u][i] = 0.f;
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;   // heads 2t, 2t+1; l over this lane's tokens
+    // heads 2t, 2t+1; l over this lane's tokens. The maxima start at the lowest finite value, so that a score
+    // of -inf weighs 0 whatever else a tile or a share holds.
+    float m0 = -FLT_MAX, m1 = -FLT_MAX, l0 = 0.f, l1 = 0.f;
 
     for (int tile = ts; tile < te; ++tile) {
       float s[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};
@@ -172,7 +176,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gqa_decode_kernel(Params
         n0 = fmaxf(n0, __shfl_xor_sync(0xffffffffu, n0, o));
         n1 = fmaxf(n1, __shfl_xor_sync(0xffffffffu, n1, o));
       }
-      if (__any_sync(0xffffffffu, n0 > m0 || n1 > m1)) {   // every tile holds at least one valid token: finite
+      if (__any_sync(0xffffffffu, n0 > m0 || n1 > m1)) {
         n0 = fmaxf(n0, m0);
         n1 = fmaxf(n1, m1);
         const float f0 = ako::fast_exp2(m0 - n0), f1 = ako::fast_exp2(m1 - n1);

@@ -141,3 +141,19 @@ def test_infinity_in_the_last_value_row(built_lib, lens):
     assert torch.isinf(ro).any() and not torch.isnan(ro).any()
     assert_close_bf16(o.cpu()[torch.isfinite(ro)], ro[torch.isfinite(ro)])
     assert_lse_close(lse, rlse)
+
+
+@pytest.mark.parametrize("length,masked", [(64, range(0, 32)), (64, range(32, 64)), (2100, range(0, 700)), (2100, range(900, 2100)), (40, range(0, 39)),
+                                           (3000, range(16, 32))])
+def test_keys_that_score_minus_infinity(built_lib, length, masked):
+    """Keys whose dot product overflows to -inf weigh nothing, also where they fill whole tiles and shares."""
+    a = W.make_gqa_decode(2, shape_id=9, lens=[length, 50], extra_pages=3)
+    a["q"] = a["q"].abs() + 1e3
+    rows = a["kv_indices"][:length][torch.tensor(list(masked))].long()
+    a["k_cache"] *= 1e-3
+    a["k_cache"][rows] = -3e38
+    o, lse = _run(a)
+    ro, rlse = oracle.gqa_paged_decode(*[a[k] for k in KEYS])
+    assert torch.isfinite(ro.float()).all() and torch.isfinite(o.float()).all()
+    assert_close_bf16(o, ro)
+    assert_lse_close(lse, rlse)
