@@ -1,8 +1,7 @@
 // Work split of the decode attention kernels: the key tiles of all rows (sequences, query tokens) form
 // one flat sequence and every CTA takes an equal contiguous share of it (+-1 tile whatever the mix of
 // row lengths), which it cuts at row boundaries into segments. A row inside one share is finished by
-// its CTA; a segment of a longer row leaves one partial in slot row + share index: both only grow
-// along the sequence, so the sum is unique and below rows + shares.
+// its CTA; the segments of a longer row leave one partial each for a merge kernel.
 #pragma once
 #include "common.cuh"
 
@@ -12,21 +11,22 @@ struct Share {
   int row;    // row of the first tile
   int skip;   // tiles of that row in front of the share
   int left;   // tiles of the share
+  int per;    // tiles of a full share
 };
 
-// Finds share `index` of `shares` with 128 threads; `tiles(r)` is the tile count of row r < nrows. When
-// `table` is set the exclusive prefix of the tile counts (and the total) also goes to prefix[0 .. nrows],
-// for the merge kernel. s_scan: six ints of shared memory.
-template <class Tiles>
-__device__ __forceinline__ Share find_share(int nrows, int index, int shares, bool table, int* __restrict__ prefix, int* s_scan,
-                                            Tiles tiles) {
+// Finds share `index` of `shares` with 128 threads; `tiles(r)` is the tile count of row r < nrows and
+// `empty(r)` is called (by one thread) for the share's part of the rows that have none. s_scan: six ints of
+// shared memory.
+template <class Tiles, class Empty>
+__device__ __forceinline__ Share find_share(int nrows, int index, int shares, int* s_scan, Tiles tiles, Empty empty) {
   constexpr int NT = 128;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  Share sh = {0, 0, 0};
+  Share sh = {0, 0, 0, 1};
   int first = 0, mine = 0;                          // `first`: the thread's row of the first 128
   for (int r = tid; r < nrows; r += NT) {
     const int n = tiles(r);
     if (r == tid) first = n;
+    if (n == 0 && r % shares == index) empty(r);
     mine += n;
   }
 #pragma unroll
@@ -37,8 +37,7 @@ __device__ __forceinline__ Share find_share(int nrows, int index, int shares, bo
   const int total = s_scan[0] + s_scan[1] + s_scan[2] + s_scan[3];
   const int per = (total + shares - 1) / shares;
   const int begin = index * per;
-  if (table && tid == 0) prefix[nrows] = total;
-  if (begin >= total && !table) return sh;
+  if (begin >= total) return sh;
   int base = 0;
   for (int r0 = 0; r0 < nrows; r0 += NT) {
     const int r = r0 + tid;
@@ -54,20 +53,18 @@ __device__ __forceinline__ Share find_share(int nrows, int index, int shares, bo
     __syncthreads();
     x += base;
     for (int i = 0; i < w; ++i) x += s_scan[i];     // inclusive prefix
-    if (table && r < nrows) prefix[r] = x - n;
     if (x - n <= begin && begin < x) {
       s_scan[4] = r;
       s_scan[5] = begin - (x - n);
     }
     base += s_scan[0] + s_scan[1] + s_scan[2] + s_scan[3];
     __syncthreads();
-    if (!table && s_scan[4] >= 0) break;
+    if (s_scan[4] >= 0) break;
   }
-  if (begin < total) {
-    sh.row = s_scan[4];
-    sh.skip = s_scan[5];
-    sh.left = min(per, total - begin);
-  }
+  sh.row = s_scan[4];
+  sh.skip = s_scan[5];
+  sh.left = min(per, total - begin);
+  sh.per = per;
   return sh;
 }
 

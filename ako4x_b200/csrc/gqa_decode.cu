@@ -18,7 +18,11 @@
 // heads); a second kernel merges the partials of rows that several shares touch. Measured (whole call,
 // bulk copies through shared memory and a planning kernel before -> now): 64 sequences of up to 8 192 tokens
 // 245 -> 188 us (6.3 TB/s = 0.96 of the measured copy bandwidth), 256 of them 841 -> 680 (0.99), 16 of up to
-// 1 200 25 -> 17, one of 547 12.6 -> 10.2 us.
+// 1 200 25 -> 17, one of 547 12.6 -> 10.2 us. Shares also for batches of short sequences, where one CTA pair
+// per sequence needs no merge: equal sequences lose a few us (222 x 64 tokens 13.5 -> 16.0, 888 x 100 67.4 ->
+// 69.6, 3 000 x 30 79 -> 90), but one long sequence among them no longer keeps a single pair busy (eight of
+// 8 192 tokens among 248 of 256: 580 -> 94; one of 60 000 among 229 of 100: 4 074 -> 78).
+#include <algorithm>
 #include <cfloat>
 
 #include "flat_share.cuh"
@@ -45,13 +49,25 @@ struct Params {
   float* lse;
   float* part_acc;  // [slot][32][128]
   float* part_ml;   // [slot][32][2]
-  int32_t* prefix;  // [batch + 1] tiles in front of a sequence
+  int2* cut;        // sequences that several shares touch: see below
   float scale_log2;
   int page_size;
   int batch;
   bool whole_rows;  // a share is one sequence
 };
 
+// For the merge the split kernel leaves entries {sequence, first share | shares << 16}; one share or none:
+// nothing to merge. With no more sequences than shares there is one entry per sequence (written by the CTA
+// that starts it), otherwise one per share, for the sequence that starts in it and goes on: the merge has at
+// most `shares` of them to look at, however many sequences there are. The partial of share c lies in slot
+// sequence + c, or, with one entry per share, in slot 2 c, the first one of a sequence in 2 c + 1.
+__device__ __forceinline__ int2 cut_entry(int b, int first, int n) { return make_int2(b, first | n << 16); }
+
+__device__ __forceinline__ void empty_head(const Params& p, int64_t row_head) {   // one thread
+  uint4* op = reinterpret_cast<uint4*>(p.o + row_head * D);
+  for (int i = 0; i < D / 8; ++i) op[i] = make_uint4(0u, 0u, 0u, 0u);
+  p.lse[row_head] = -INFINITY;
+}
 __device__ __forceinline__ int seq_tokens(const Params& p, int b) {
   return max(0, p.indptr[b + 1] - p.indptr[b]) * p.page_size;
 }
@@ -74,18 +90,20 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gqa_decode_kernel(Params
   const int kvh = half * HPC + warp;
   ako::pdl_trigger();  // the merge kernel may be scheduled early; it waits for this grid to finish
   auto seq_tiles = [&](int b) { return (seq_tokens(p, b) + TILE - 1) / TILE; };
+  const int shares = gridDim.x / HALVES;
+  const bool by_share = p.batch > shares;
+  const bool keeper = half == 0 && threadIdx.x == 0;   // writes the entries
   ako::Share sh;
   if (p.whole_rows) {
-    sh = {share, 0, seq_tiles(share)};
-    if (sh.left == 0) {                              // an empty sequence
-      const int64_t h0 = (int64_t)share * HQ + kvh * GROUP;
-      uint4* op = reinterpret_cast<uint4*>(p.o + h0 * D);
-      for (int i = lane; i < GROUP * D / 8; i += 32) op[i] = make_uint4(0u, 0u, 0u, 0u);
-      if (lane < GROUP) p.lse[h0 + lane] = -INFINITY;
-    }
+    sh = {share, 0, seq_tiles(share), 0};
+    if (sh.left == 0 && lane < GROUP) empty_head(p, (int64_t)share * HQ + kvh * GROUP + lane);
   } else {
-    sh = ako::find_share(p.batch, share, gridDim.x / HALVES, blockIdx.x == 0, p.prefix, s_scan, seq_tiles);
+    sh = ako::find_share(p.batch, share, shares, s_scan, seq_tiles, [&](int r) {
+      for (int h = 0; h < HQ / HALVES; ++h) empty_head(p, (int64_t)r * HQ + half * (HQ / HALVES) + h);
+      if (!by_share && half == 0) p.cut[r] = cut_entry(r, 0, 0);
+    });
   }
+  int2 cut = cut_entry(0, 0, 0);
 
   int b = sh.row, ts = sh.skip;
   while (sh.left > 0) {
@@ -228,7 +246,11 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gqa_decode_kernel(Params
     const bool whole = te - ts == tiles;
     const float i0 = (whole && l0 > 0.f) ? 1.f / l0 : 1.f, i1 = (whole && l1 > 0.f) ? 1.f / l1 : 1.f;
     const bool odd = g & 1;
-    const int64_t slot = (int64_t)b + share;
+    const int64_t slot = by_share ? 2 * (int64_t)share + (ts == 0) : (int64_t)b + share;
+    if (ts == 0 && !p.whole_rows) {
+      cut = cut_entry(b, share, whole ? 1 : 1 + (tiles - te + sh.per - 1) / sh.per);
+      if (!by_share && keeper) p.cut[b] = cut;
+    }
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh) {
       const int head = kvh * GROUP + 2 * t + hh;
@@ -258,13 +280,13 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gqa_decode_kernel(Params
     ++b;
     ts = 0;
   }
+  if (by_share && !p.whole_rows && keeper) p.cut[share] = cut;
 }
 
 // Merge: WARPS warps per (sequence, head), every warp 32 threads x 4 columns of every WARPS-th partial;
 // a block holds four heads (WARPS = 1) or one (WARPS = 8: few sequences with many partials each, where
-// one warp would walk up to 222 partials in a row). The partials of sequence b are the slots b + c of
-// the shares c that touch it; a sequence inside one share is already written, an empty one gets its
-// zeros here.
+// one warp would walk up to 222 partials in a row). Sequences inside one share, and empty ones, are already
+// written.
 constexpr int MERGE_MAX = 512;                       // shares of a call never exceed this (three CTAs per SM)
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS == 1 ? 128 : WARPS * 32) gqa_merge_kernel(Params p, int shares) {
@@ -272,31 +294,25 @@ __global__ void __launch_bounds__(WARPS == 1 ? 128 : WARPS * 32) gqa_merge_kerne
   __shared__ float s_w[HEADS][MERGE_MAX];
   __shared__ float4 s_acc[WARPS][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int b = blockIdx.x / (HQ / HEADS), hl = (WARPS == 1) ? w : 0, part = (WARPS == 1) ? 0 : w;
+  const int hl = (WARPS == 1) ? w : 0, part = (WARPS == 1) ? 0 : w;
   const int head = (blockIdx.x % (HQ / HEADS)) * HEADS + hl;
   ako::pdl_wait();
-  const int t0 = p.prefix[b], t1 = p.prefix[b + 1], total = p.prefix[p.batch];
-  const int64_t oi = (int64_t)b * HQ + head;
+  const int2 cut = p.cut[blockIdx.x / (HQ / HEADS)];
+  const int c0 = cut.y & 0xffff, n = cut.y >> 16;
+  if (n <= 1) return;
+  const bool by_share = p.batch > shares;
+  const int64_t oi = (int64_t)cut.x * HQ + head, slot0 = by_share ? 2 * (int64_t)c0 : (int64_t)cut.x + c0;
+  auto slot = [&](int i) { return by_share ? 2 * i + (i == 0) : i; };
   uint2* op = reinterpret_cast<uint2*>(p.o + oi * D) + lane;
-  if (t1 <= t0) {
-    if (part == 0) {
-      *op = make_uint2(0u, 0u);
-      if (lane == 0) p.lse[oi] = -INFINITY;
-    }
-    return;
-  }
-  const int per = (total + shares - 1) / shares;
-  const int c0 = t0 / per, n = (t1 - 1) / per - c0 + 1;
-  if (n == 1) return;
-  const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + ((int64_t)(b + c0) * HQ + head);
-  const float4* pa = reinterpret_cast<const float4*>(p.part_acc + ((int64_t)(b + c0) * HQ + head) * D) + lane;
+  const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + (slot0 * HQ + head);
+  const float4* pa = reinterpret_cast<const float4*>(p.part_acc + (slot0 * HQ + head) * D) + lane;
   // every warp of the head finds the maximum over all partials for itself
   float2 mine[MERGE_MAX / 32];
   float M = -INFINITY, L = 0.f;
 #pragma unroll
   for (int i = 0; i < MERGE_MAX / 32; ++i) {
     mine[i] = make_float2(-INFINITY, 0.f);
-    if (i * 32 < n && i * 32 + lane < n) mine[i] = ml[(int64_t)(i * 32 + lane) * HQ];
+    if (i * 32 < n && i * 32 + lane < n) mine[i] = ml[(int64_t)slot(i * 32 + lane) * HQ];
     M = fmaxf(M, mine[i].x);
   }
 #pragma unroll
@@ -314,7 +330,7 @@ __global__ void __launch_bounds__(WARPS == 1 ? 128 : WARPS * 32) gqa_merge_kerne
 #pragma unroll 8
   for (int i = part; i < n; i += WARPS) {
     const float wgt = s_w[hl][i];
-    const float4 x = pa[(int64_t)i * (HQ * D / 4)];
+    const float4 x = pa[(int64_t)slot(i) * (HQ * D / 4)];
     acc.x = fmaf(x.x, wgt, acc.x);
     acc.y = fmaf(x.y, wgt, acc.y);
     acc.z = fmaf(x.z, wgt, acc.z);
@@ -337,15 +353,14 @@ __global__ void __launch_bounds__(WARPS == 1 ? 128 : WARPS * 32) gqa_merge_kerne
   if (lane == 0) p.lse[oi] = (L > 0.f) ? M + log2f(L) : -INFINITY;
 }
 
-// Whole sequences as shares, without partials and without the merge: batches that fill the GPU and are
-// short (at most 32 tiles) or many (four times as many sequences as shares fit at once).
+// Calls that can do without a workspace, with whole sequences as shares: batches that fill the GPU and are
+// short on average or many. A long sequence among them is then walked by one pair of CTAs.
 bool whole_rows(int64_t batch, int64_t num_kv_indices, int64_t page_size) {
   const int64_t most = (int64_t)CTAS_PER_SM * ako::sm_count() / HALVES;
   return batch >= 4 * most || (batch >= most && num_kv_indices * page_size <= batch * 512);
 }
 // Shares of a call: all CTAs resident at once, and at least one tile (16 tokens, 64 KB of K and V) each.
-int pick_shares(int64_t batch, int64_t num_kv_indices, int64_t page_size) {
-  if (whole_rows(batch, num_kv_indices, page_size)) return (int)batch;
+int pick_shares(int64_t num_kv_indices, int64_t page_size) {
   const int64_t most = (int64_t)CTAS_PER_SM * ako::sm_count() / HALVES;
   const int64_t tiles = ako::cdiv(num_kv_indices * page_size, (int64_t)TILE);   // at least; rows round up
   int64_t s = tiles < most ? tiles : most;
@@ -353,14 +368,18 @@ int pick_shares(int64_t batch, int64_t num_kv_indices, int64_t page_size) {
   return (int)(s < 1 ? 1 : s);
 }
 struct Carve {
-  size_t acc, ml, total;   // offsets; the prefix table is first
+  size_t acc, ml, total;   // offsets; the entries are first
 };
-Carve carve(int64_t batch, int shares) {
-  const size_t slots = (size_t)batch + (size_t)shares;
+Carve carve(int64_t batch, int64_t num_kv_indices, int64_t page_size) {
+  const int shares = pick_shares(num_kv_indices, page_size);
+  const size_t entries = (size_t)(batch < shares ? batch : shares), slots = entries + (size_t)shares;
   Carve c;
-  c.acc = (((size_t)batch + 1) * sizeof(int32_t) + 255) / 256 * 256;
+  c.acc = (entries * sizeof(int2) + 255) / 256 * 256;
   c.ml = c.acc + slots * HQ * D * sizeof(float);
-  c.total = c.ml + slots * HQ * 2 * sizeof(float);
+  // Callers that cannot do without were promised (and are refused below) a size of a slot for every sequence
+  // and share, as if each sequence could be cut; at most `shares` can.
+  const size_t promised = whole_rows(batch, num_kv_indices, page_size) ? slots : (size_t)batch + (size_t)shares;
+  c.total = c.acc + promised * HQ * (D + 2) * sizeof(float);
   return c;
 }
 
@@ -368,8 +387,8 @@ Carve carve(int64_t batch, int shares) {
 
 extern "C" size_t ako4x_gqa_paged_decode_workspace_bytes(int64_t batch, int64_t num_kv_indices,
                                                          int64_t page_size) {
-  if (batch <= 0 || whole_rows(batch, num_kv_indices, page_size)) return 0;
-  return carve(batch, pick_shares(batch, num_kv_indices, page_size)).total;
+  if (batch <= 0) return 0;
+  return carve(batch, num_kv_indices, page_size).total;
 }
 
 extern "C" int ako4x_gqa_paged_decode(const void* q, const void* k_cache, const void* v_cache,
@@ -383,12 +402,13 @@ extern "C" int ako4x_gqa_paged_decode(const void* q, const void* k_cache, const 
   if (num_kv_indices > 0 && !kv_indices) return AKO4X_EINVAL;
   if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)o) & 15) return AKO4X_EINVAL;
   if (batch > 0x7fffffffLL / HQ || page_size > 0x7fffffffLL) return AKO4X_EINVAL;
-  const bool whole = whole_rows(batch, num_kv_indices, page_size);
-  const int shares = pick_shares(batch, num_kv_indices, page_size);
-  const Carve c = carve(batch, shares);
-  if (!whole) {
-    if (!workspace || workspace_bytes < c.total) return AKO4X_EWORKSPACE;
-    if ((uintptr_t)workspace & 15) return AKO4X_EINVAL;
+  int shares = pick_shares(num_kv_indices, page_size);
+  const Carve c = carve(batch, num_kv_indices, page_size);
+  bool whole = false;
+  if (!workspace || workspace_bytes < c.total || ((uintptr_t)workspace & 15)) {
+    whole = whole_rows(batch, num_kv_indices, page_size);
+    if (!whole) return (!workspace || workspace_bytes < c.total) ? AKO4X_EWORKSPACE : AKO4X_EINVAL;
+    shares = (int)batch;
   }
   cudaStream_t st = (cudaStream_t)stream;
 
@@ -400,7 +420,7 @@ extern "C" int ako4x_gqa_paged_decode(const void* q, const void* k_cache, const 
   p.indices = kv_indices;
   p.o = (__nv_bfloat16*)o;
   p.lse = lse;
-  p.prefix = (int32_t*)workspace;
+  p.cut = (int2*)workspace;
   p.part_acc = (float*)((unsigned char*)workspace + c.acc);
   p.part_ml = (float*)((unsigned char*)workspace + c.ml);
   p.scale_log2 = sm_scale * AKO_LOG2E;
@@ -409,10 +429,11 @@ extern "C" int ako4x_gqa_paged_decode(const void* q, const void* k_cache, const 
   p.whole_rows = whole;
   gqa_decode_kernel<<<(unsigned)(shares * HALVES), THREADS, 0, st>>>(p);
   AKO_CHECK_LAUNCH();
-  if (whole) return AKO4X_OK;
+  if (whole || shares == 1) return AKO4X_OK;          // nothing is cut
   const bool many = shares >= 8 * batch;              // partials per sequence
-  const cudaError_t e = many ? ako::launch_pdl(true, gqa_merge_kernel<8>, dim3((unsigned)(batch * HQ)), dim3(256), 0, st, p, shares)
-                             : ako::launch_pdl(true, gqa_merge_kernel<1>, dim3((unsigned)(batch * (HQ / 4))), dim3(128), 0, st, p, shares);
+  const unsigned entries = (unsigned)std::min<int64_t>(batch, shares);
+  const cudaError_t e = many ? ako::launch_pdl(true, gqa_merge_kernel<8>, dim3(entries * HQ), dim3(256), 0, st, p, shares)
+                             : ako::launch_pdl(true, gqa_merge_kernel<1>, dim3(entries * (HQ / 4)), dim3(128), 0, st, p, shares);
   if (e != cudaSuccess)
     return AKO4X_ELAUNCH;
   return AKO4X_OK;

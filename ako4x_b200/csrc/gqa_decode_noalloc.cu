@@ -23,8 +23,8 @@
 
 namespace {
 
-// Enough for every batch of up to 282 sequences, and for the larger ones whose sequences are short
-// (those need no partials at all).
+// Enough for every batch of up to 282 sequences, and for the larger ones that are also accepted without a
+// workspace (at most 444 partials on 148 SMs).
 constexpr size_t kScratchBytes = 8u << 20;
 
 // In host code this name is only a handle for the runtime, not a device address: it must go

@@ -50,8 +50,8 @@ int ako4x_rmsnorm_h128(const void* x, const void* weight, void* y, int64_t rows,
  * [batch+1]; kv_indices int32 [kv_indptr[batch]] (page ids); o bf16 [batch,32,128];
  * lse fp32 [batch,32] = log2(sum exp(logit)); empty sequence gives o = 0, lse = -inf.
  * `num_kv_indices` (the length of kv_indices) sizes the work split and the workspace; it is a shape,
- * not device data, and kv_indptr[batch] <= num_kv_indices must hold. The workspace is 0 bytes for large
- * batches of short sequences.
+ * not device data, and kv_indptr[batch] <= num_kv_indices must hold. Large batches of short sequences
+ * are also accepted without a workspace; a long sequence among them then takes as long as one alone.
  */
 size_t ako4x_gqa_paged_decode_workspace_bytes(int64_t batch, int64_t num_kv_indices,
                                               int64_t page_size);

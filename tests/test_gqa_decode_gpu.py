@@ -3,7 +3,7 @@ import pytest
 import torch
 
 import oracle
-from ako4x_b200 import gqa_decode, workloads as W
+from ako4x_b200 import _cabi, gqa_decode, workloads as W
 from conftest import assert_close_bf16, assert_lse_close, load_golden
 
 pytestmark = pytest.mark.gpu
@@ -157,3 +157,42 @@ def test_keys_that_score_minus_infinity(built_lib, length, masked):
     assert torch.isfinite(ro.float()).all() and torch.isfinite(o.float()).all()
     assert_close_bf16(o, ro)
     assert_lse_close(lse, rlse)
+
+
+@pytest.mark.parametrize("lens", [[512] * 222, [513] * 222, [512] * 221, [100] * 221 + [4000, 3], [3000] + [0, 17] * 130, [0, 31, 5] * 300 + [2500],
+                                  [16] * 889, [6000, 0, 0] + [1] * 250 + [0] * 40 + [700, 650]])
+def test_large_batches_with_and_without_a_workspace(built_lib, lens):
+    """Batches on both sides of what is accepted without a workspace (mean length 512 from 222 sequences on,
+    any from 888 on, on 148 SMs), some with one sequence far longer than the rest: cut at share boundaries with
+    one merge entry per share, and whole sequences per CTA pair, against the oracle and each other."""
+    a = W.make_gqa_decode(len(lens), shape_id=3, lens=lens, extra_pages=5)
+    _check(a)
+    d = W.to_device(a, "cuda")
+    L, n, idx = _cabi.lib(), len(lens), a["kv_indices"].numel()
+    o, lse = torch.full_like(d["q"], float("nan")), torch.full((n, 32), float("nan"), device="cuda")
+    st = L.ako4x_gqa_paged_decode(*[_cabi.ptr(d[k]) for k in KEYS[:5]], d["sm_scale"], _cabi.ptr(o), _cabi.ptr(lse), n, idx, 1, None, 0,
+                                  _cabi.stream())
+    without = n >= 888 or (n >= 222 and idx <= 512 * n)
+    assert st == (0 if without else -4)
+    if without:
+        ro, rlse = gqa_decode.run(*[d[k] for k in KEYS])
+        assert_close_bf16(o, ro)
+        assert_lse_close(lse, rlse)
+
+
+def test_a_long_sequence_in_a_large_batch_is_shared(built_lib):
+    """256 sequences with a mean below 512 tokens, one of which holds half of the tokens: it must not be left to
+    one pair of CTAs, which takes more than ten times as long as a batch of equal sequences of the same size."""
+    def us(lens):
+        a = W.make_gqa_decode(len(lens), shape_id=1, lens=lens, device="cuda", extra_pages=3)
+        args = [a[k] for k in KEYS]
+        best = 1e9
+        for _ in range(5):
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record()
+            gqa_decode.run(*args)
+            ev[1].record()
+            torch.cuda.synchronize()
+            best = min(best, ev[0].elapsed_time(ev[1]) * 1e3)
+        return best
+    assert us([32768] + [128] * 255) < 3 * us([256] * 256)
