@@ -136,17 +136,35 @@ mla_prefill_tc_kernel(PfParams p, const __grid_constant__ CUtensorMap tm_qn, con
   int* s_work = reinterpret_cast<int*>(xch_full + 6);  // sequence, pair tile inside the sequence (or -1)
   static_assert(4 * BM * 4 + (2 * NST + 6 + 6) * 8 + 8 <= AUX_BYTES, "aux region");
 
-  if (tid == 0) {
+  if (warp == 0) {
     // reversed: within a sequence the later query tiles see more keys, so the long pairs start
-    // first and the short ones fill the end of the grid
-    int t = (int)((gridDim.x - 1 - blockIdx.x) >> 1), b = 0;
-    for (; b < p.batch; ++b) {
-      const int nt = (p.qo_indptr[b + 1] - p.qo_indptr[b] + PT - 1) / PT;
-      if (t < nt) break;
-      t -= nt;
+    // first and the short ones fill the end of the grid. 32 sequences per step: one thread alone
+    // walked 256 of them in 5 us, with every pair.
+    int t = (int)((gridDim.x - 1 - blockIdx.x) >> 1), seq = p.batch;
+    for (int b0 = 0; b0 < p.batch; b0 += 32) {
+      const int b = b0 + lane;
+      const int nt = (b < p.batch) ? (p.qo_indptr[b + 1] - p.qo_indptr[b] + PT - 1) / PT : 0;
+      int x = nt;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += up;
+      }
+      const unsigned hit = __ballot_sync(0xffffffffu, t < x);
+      if (hit) {
+        const int f = __ffs(hit) - 1;
+        t -= __shfl_sync(0xffffffffu, x - nt, f);
+        seq = b0 + f;
+        break;
+      }
+      t -= __shfl_sync(0xffffffffu, x, 31);
     }
-    s_work[0] = b;
-    s_work[1] = (b < p.batch) ? t : -1;
+    if (lane == 0) {
+      s_work[0] = seq;
+      s_work[1] = (seq < p.batch) ? t : -1;
+    }
+  }
+  if (tid == 0) {
     for (int s = 0; s < NST; ++s) {
       ako::tc::mbar_init(ako::smem_u32(&st_full[s]), 1);
       ako::tc::mbar_init(ako::smem_u32(&st_empty[s]), 1);

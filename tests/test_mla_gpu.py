@@ -246,3 +246,12 @@ def test_sparse_order_invariance_full_size(built_lib):
     o2, l2 = dsa_attention.run(*[a[k] for k in SKEYS])
     assert_close_bf16(o2, o1)
     assert_lse_close(l2, l1)
+
+
+@pytest.mark.parametrize("count", [31, 32, 33, 64, 100])
+def test_prefill_many_sequences(built_lib, count):
+    """Query tiles of more sequences than one step of the tile search looks at, empty ones among them."""
+    q_lens = [(0, 1, 16, 17, 8, 40, 0)[i % 7] for i in range(count)]
+    kv_lens = [q + (0, 5, 130, 60)[i % 4] for i, q in enumerate(q_lens)]
+    _check(mla_prefill, oracle.mla_paged_prefill, PKEYS,
+           W.make_mla_prefill(count, shape_id=count, q_lens=q_lens, kv_lens=kv_lens, extra_pages=3))
