@@ -3,7 +3,7 @@
 // to 16 294; the reference's campaign ended with cuBLAS as its best implementation, README.md of
 // that folder). Hand-written for sm_100a:
 //   * persistent CTAs, one per SM, over output tiles of 128 rows x BN columns, or pairs of CTAs
-//     (cta_group::2) over tiles of 256 rows x BN columns (BN = 256, 128 or 32, gemm_plan below), n
+//     (cta_group::2) over tiles of 256 rows x BN columns (BN = 256, 128 or 32, gemm_plan.h), n
 //     fastest so that the CTAs sharing an A tile run side by side and A crosses HBM once (B, 16 MB,
 //     stays in L2). Each CTA of a pair brings its own rows of A and half of B;
 //   * a TMA producer warp fills a ring of K = 64 slices (128-byte-swizzled boxes of A and B);
@@ -14,13 +14,14 @@
 // Small M: a tile's K loop is 256 MMAs whatever its width and an M128 x N32 x K16 MMA takes about
 // 80 cycles, so one CTA per tile needs 11 us (22-24 us per call, and keeping 64 KB instead of 32 KB
 // of B in flight per CTA changed nothing). With a workspace the K dimension is split over up to 8
-// CTAs per tile and a second kernel sums the fp32 partial products (gemm_plan below).
+// CTAs per tile and a second kernel sums the fp32 partial products (gemm_plan.h).
 // Every wait is bounded; a wait that gives up records its code in the status word below and the
 // CTA unwinds through the common exit that frees TMEM.
 #include <algorithm>
 #include <atomic>
 
 #include "common.cuh"
+#include "gemm_plan.h"
 #include "tcgen05.cuh"
 #include "tma_host.cuh"
 
@@ -269,17 +270,40 @@ __global__ void __launch_bounds__(256) gemm_splitk_reduce_kernel(const float* __
   *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(c) + i) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// CTAs of a pair kernel that can be resident at once (2 x the co-resident clusters), per device.
+template <int CG>
+cudaLaunchConfig_t launch_config(size_t smem, cudaStream_t st, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(G_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = CG;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = (CG == 2) ? 1 : 0;
+  return cfg;
+}
+
+// CTAs of a pair kernel that can be resident at once (2 x the co-resident clusters), per device; 0 when
+// none can, or the query fails (its error does not stay behind).
 template <int BN, bool BF16>
-int pair_ctas(cudaLaunchConfig_t cfg) {
+int pair_ctas() {
   static std::atomic<int> cached[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   int n = cached[dev].load(std::memory_order_relaxed);
   if (n == 0) {
+    using Cfg = GemmCfg<BN, 2>;
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg = launch_config<2>(Cfg::SMEM, nullptr, attr);
     cfg.gridDim = dim3((unsigned)(ako::sm_count() & ~1));
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, gemm_f16_tc_kernel<BN, BF16, 2>, &cfg) != cudaSuccess) return 0;
+    if (!ako::ensure_dynamic_smem<gemm_f16_tc_kernel<BN, BF16, 2>>((int)Cfg::SMEM) ||
+        cudaOccupancyMaxActiveClusters(&clusters, gemm_f16_tc_kernel<BN, BF16, 2>, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return 0;
+    }
     n = 2 * clusters;
     cached[dev].store(n, std::memory_order_relaxed);
   }
@@ -305,20 +329,10 @@ int launch_gemm(const void* a, const void* b, void* c, int64_t m, int64_t n, int
   p.splits = splits;
   p.partial = partial;
   const int64_t tiles = ((m + CG * G_BM - 1) / (CG * G_BM)) * (n / BN) * splits;
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(G_THREADS);
-  cfg.dynamicSmemBytes = Cfg::SMEM;
-  cfg.stream = st;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CG;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = (CG == 2) ? 1 : 0;
+  cudaLaunchConfig_t cfg = launch_config<CG>(Cfg::SMEM, st, attr);
   int ctas = ako::sm_count();
-  if constexpr (CG == 2) ctas = pair_ctas<BN, BF16>(cfg);
-  if (ctas < CG) return AKO4X_ELAUNCH;
+  if constexpr (CG == 2) ctas = pair_ctas<BN, BF16>();
   cfg.gridDim = dim3((unsigned)std::min<int64_t>(CG * tiles, ctas));
   if (cudaLaunchKernelEx(&cfg, gemm_f16_tc_kernel<BN, BF16, CG>, p, tm_a, tm_b) != cudaSuccess) return AKO4X_ELAUNCH;
   if (splits > 1) {
@@ -331,43 +345,8 @@ int launch_gemm(const void* a, const void* b, void* c, int64_t m, int64_t n, int
   return AKO4X_OK;
 }
 
-// Tile width, CTAs per tile and K split by how many work items the GPU gets. A K block of 64 costs a
-// CTA about the same time whatever its tile is (it waits for operands, not for the tensor pipe), so
-// the plan looks for the widest tiles that still give every SM work: pairs (256 rows) from the second
-// row tile on, 256 columns once 128 would need a second wave, K cut into 2, 4 or 8 pieces (summed by
-// a second kernel) while less than half of the GPU has work. One-CTA tiles stay for up to 128 rows
-// (a pair would be half empty) and where they fit one wave and pairs of the same width do not.
-// Measured, whole call, N = 2048, K = 4096, against one-CTA tiles everywhere (us): M = 256: 15.6
-// (20.0), 512: 18.5 (20.0), 640: 23.5 (29.2), 969: 22.6 (26.0), 1536: 28.8 (44.5), 4000: 52.3 (57.7),
-// 16294: 182 (204); M = 640 as 256 x 128 pairs with K in two, 96 of them for 74 places: 26.7.
-struct GemmPlan {
-  int bn, splits, cg;
-};
-inline GemmPlan gemm_plan(int64_t m, int64_t n, int64_t k, bool have_workspace) {
-  const int64_t mt = (m + G_BM - 1) / G_BM, mp = (mt + 1) / 2;
-  const int sms = ako::sm_count();
-  if (mt > 1) {
-    // more 256 x 128 tiles than one wave of pairs
-    if (2 * mp * (n / 128) > sms) {
-      if (mt * (n / 128) <= sms) return {128, 1, 1};
-      return {256, 1, 2};
-    }
-    int s = 1;
-    while (have_workspace && s < 8 && 4 * mp * (n / 128) * s <= sms && (k / 64) % (2 * s) == 0) s *= 2;
-    if (s > 1) return {128, s, 2};
-    // between a quarter and a half of the GPU with full-width tiles: those, K in two
-    if (have_workspace && 4 * mp * (n / 256) * 3 <= 2 * sms && (k / 64) % 2 == 0) return {256, 2, 2};
-    if (4 * mp * (n / 128) >= sms) return {128, 1, 2};
-  }
-  if (mt * (n / 256) * 4 >= 3 * sms) return {256, 1, 1};
-  if (!have_workspace) return {(mt * (n / 128) * 4 >= 3 * sms) ? 128 : 32, 1, 1};
-  int s = 1;
-  while (s < 8 && mt * (n / 128) * s < 128 && (k / 64) % (2 * s) == 0) s *= 2;
-  return {128, s, 1};
-}
-
 template <bool BF16>
-int launch_plan(const GemmPlan& pl, const void* a, const void* b, void* c, int64_t m, int64_t n, int64_t k,
+int launch_plan(const ako_gemm::Plan& pl, const void* a, const void* b, void* c, int64_t m, int64_t n, int64_t k,
                 float* part, cudaStream_t st) {
   if (pl.cg == 2)
     return (pl.bn == 256) ? launch_gemm<256, BF16, 2>(a, b, c, m, n, k, pl.splits, part, st)
@@ -381,8 +360,7 @@ int launch_plan(const GemmPlan& pl, const void* a, const void* b, void* c, int64
 
 extern "C" size_t ako4x_gemm_workspace_bytes(int64_t m, int64_t n, int64_t k) {
   if (m <= 0 || n <= 0 || k <= 0 || n % 256 != 0 || k % 64 != 0) return 0;
-  const GemmPlan pl = gemm_plan(m, n, k, true);
-  return pl.splits > 1 ? (size_t)pl.splits * (size_t)m * (size_t)n * sizeof(float) : 0;
+  return ako_gemm::workspace_bytes(ako_gemm::plan(m, n, k, true, ako::sm_count(), true), m, n);
 }
 
 static int gemm_entry(const void* a, const void* b, void* c, int64_t m, int64_t n, int64_t k, int is_bf16,
@@ -393,8 +371,12 @@ static int gemm_entry(const void* a, const void* b, void* c, int64_t m, int64_t 
   if (!a || !b || !c) return AKO4X_EINVAL;
   if (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)workspace) & 15) return AKO4X_EINVAL;
   cudaStream_t st = (cudaStream_t)stream;
-  const GemmPlan pl = gemm_plan(m, n, k, workspace != nullptr);
-  if (pl.splits > 1 && workspace_bytes < (size_t)pl.splits * (size_t)m * (size_t)n * sizeof(float)) return AKO4X_EWORKSPACE;
+  ako_gemm::Plan pl;
+  auto resident = [&](int bn) {
+    if (bn == 256) return is_bf16 ? pair_ctas<256, true>() : pair_ctas<256, false>();
+    return is_bf16 ? pair_ctas<128, true>() : pair_ctas<128, false>();
+  };
+  if (!ako_gemm::choose(m, n, k, workspace != nullptr, workspace_bytes, ako::sm_count(), resident, pl)) return AKO4X_EWORKSPACE;
   float* part = (float*)workspace;
   return is_bf16 ? launch_plan<true>(pl, a, b, c, m, n, k, part, st) : launch_plan<false>(pl, a, b, c, m, n, k, part, st);
 }
