@@ -8,6 +8,7 @@ import torch
 import oracle
 from ako4x_b200 import _cabi, gemm, workloads as W
 from conftest import load_golden
+from test_gemm_plan import FORMS
 
 pytestmark = pytest.mark.gpu
 
@@ -116,3 +117,15 @@ def test_empty_and_errors():
     with pytest.raises(_cabi.Ako4xError):
         gemm.run(torch.zeros((4, 4096), dtype=torch.float16, device="cuda"),
                  torch.zeros((200, 4096), dtype=torch.float16, device="cuda"))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k", FORMS.values())
+def test_every_form_of_the_kernel(dtype, m, n, k):
+    """One shape per tile width, number of pieces of K and CTAs per tile that a plan can name. Same
+    tolerance as above: fp32 sums in another order and one rounding."""
+    g = torch.Generator().manual_seed(m + n + k)
+    a = torch.randn(m, k, generator=g).to(dtype)
+    b = (torch.randn(n, k, generator=g) * 0.05).to(dtype)
+    _check(gemm.run(a.cuda(), b.cuda()).cpu(), oracle.gemm_nt(a, b), 2e-3 if dtype == torch.float16 else 8e-3)
+    assert _cabi.lib().ako4x_gemm_device_status() == 0

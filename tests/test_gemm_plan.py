@@ -53,3 +53,22 @@ def test_without_resident_pairs_a_call_runs_on_single_ctas(choose, m, n, k):
         bn, splits, cg = plan
         assert n % bn == 0 and (k // 64) % splits == 0
         assert splits == 1 or splits * m * n * 4 <= need
+
+
+# one shape for every form of the kernel that a plan can name: tile width, pieces of K, CTAs per tile
+FORMS = {(128, 1, 1): (1100, 2048, 512), (128, 2, 1): (1100, 1024, 4096), (128, 4, 1): (200, 2048, 2048), (128, 8, 1): (300, 512, 4096),
+         (128, 1, 2): (640, 2048, 4096), (128, 2, 2): (512, 2048, 4096), (128, 4, 2): (256, 2048, 4096), (128, 8, 2): (260, 512, 8192),
+         (256, 1, 1): (1000, 4096, 256), (256, 1, 2): (1153, 2048, 4096), (256, 2, 2): (1481, 1024, 8192), (256, 4, 2): (1444, 512, 8192)}
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_form_of_a_shape(choose, form):
+    assert choose(*FORMS[form], 1 << 60, 148) == form
+
+
+def test_a_missed_wave_and_short_k_loops(choose):
+    """144 single CTAs in one wave instead of 80 pairs for 74 places; no pairs and no pieces for short K loops."""
+    assert choose(1100, 4096, 4096, 1 << 60, 148)[2] == 1
+    assert choose(130, 32768, 64, 1 << 60, 148)[2] == 1
+    assert choose(300, 2048, 512, 1 << 60, 148) == (128, 1, 1)
+    assert choose(300, 2048, 4096, 1 << 60, 148)[2] == 2
