@@ -360,7 +360,7 @@ int launch_plan(const ako_gemm::Plan& pl, const void* a, const void* b, void* c,
 
 extern "C" size_t ako4x_gemm_workspace_bytes(int64_t m, int64_t n, int64_t k) {
   if (m <= 0 || n <= 0 || k <= 0 || n % 256 != 0 || k % 64 != 0) return 0;
-  return ako_gemm::workspace_bytes(ako_gemm::plan(m, n, k, true, ako::sm_count(), true), m, n);
+  return ako_gemm::workspace_bytes(m, n, k, ako::sm_count());
 }
 
 static int gemm_entry(const void* a, const void* b, void* c, int64_t m, int64_t n, int64_t k, int is_bf16,

@@ -71,14 +71,25 @@ inline Plan plan(int64_t m, int64_t n, int64_t k, bool have_workspace, int sms, 
 inline size_t workspace_bytes(const Plan& pl, int64_t m, int64_t n) {
   return pl.splits > 1 ? (size_t)pl.splits * (size_t)m * (size_t)n * sizeof(float) : 0;
 }
+// The workspace a caller is told to bring, and refused below: enough for the plan, and not less than what
+// callers were told while K was always split until there were 128 items of 128 columns.
+inline size_t workspace_bytes(int64_t m, int64_t n, int64_t k, int sms) {
+  const size_t need = workspace_bytes(plan(m, n, k, true, sms, true), m, n);
+  const int64_t mt = (m + kTileRows - 1) / kTileRows;
+  if (mt * (n / 256) * 4 >= 3 * sms) return need;
+  int s = 1;
+  while (s < 8 && mt * (n / 128) * s < 128 && (k / 64) % (2 * s) == 0) s *= 2;
+  const size_t told = workspace_bytes(Plan{128, s, 1}, m, n);
+  return need > told ? need : told;
+}
 
 // The plan of a call: false if its workspace is too small. `pair_ctas(bn)` tells how many CTAs of the pair
 // kernel can be resident; where none can (a partition of the GPU without a free pair of SMs), one-CTA
 // tiles, with whatever K split the workspace holds.
 template <class PairCtas>
 inline bool choose(int64_t m, int64_t n, int64_t k, bool have_workspace, size_t bytes, int sms, PairCtas pair_ctas, Plan& pl) {
+  if (have_workspace && bytes < workspace_bytes(m, n, k, sms)) return false;
   pl = plan(m, n, k, have_workspace, sms, true);
-  if (workspace_bytes(pl, m, n) > bytes) return false;
   if (pl.cg == 2 && pair_ctas(pl.bn) < 2) {
     pl = plan(m, n, k, have_workspace, sms, false);
     if (workspace_bytes(pl, m, n) > bytes) pl = plan(m, n, k, false, sms, false);

@@ -9,6 +9,9 @@ import pytest
 CSRC = Path(__file__).resolve().parents[1] / "ako4x_b200" / "csrc"
 SRC = """
 #include "gemm_plan.h"
+extern "C" unsigned long long workspace(long long m, long long n, long long k, int sms) {
+  return ako_gemm::workspace_bytes(m, n, k, sms);
+}
 extern "C" int choose(long long m, long long n, long long k, int have_ws, unsigned long long bytes, int sms, int resident,
                       int* plan) {
   ako_gemm::Plan pl;
@@ -28,13 +31,15 @@ def choose(tmp_path_factory):
     so = d / "plan.so"
     subprocess.run([os.environ.get("CXX") or "g++", "-std=c++17", "-shared", "-fPIC", "-I", str(CSRC), str(d / "plan.cpp"), "-o", str(so)],
                    check=True)
-    f = ctypes.CDLL(str(so)).choose
+    lib = ctypes.CDLL(str(so))
+    f, lib.workspace.restype = lib.choose, ctypes.c_ulonglong
     f.argtypes = [ctypes.c_longlong] * 3 + [ctypes.c_int, ctypes.c_ulonglong, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]
 
     def call(m, n, k, bytes_, resident):
         plan = (ctypes.c_int * 3)()
         ok = f(m, n, k, bytes_ is not None, bytes_ or 0, 148, resident, plan)
         return tuple(plan) if ok else None
+    call.workspace = lambda m, n, k: lib.workspace(*[ctypes.c_longlong(x) for x in (m, n, k)], 148)
     return call
 
 
@@ -45,7 +50,8 @@ def test_without_resident_pairs_a_call_runs_on_single_ctas(choose, m, n, k):
         need = 0
         if workspace:
             bn, splits, cg = choose(m, n, k, 1 << 60, 148)
-            need = splits * m * n * 4 if splits > 1 else 0
+            need = choose.workspace(m, n, k)
+            assert need >= (splits * m * n * 4 if splits > 1 else 0)
             if need:
                 assert choose(m, n, k, need - 1, 148) is None
         plan = choose(m, n, k, need if workspace else None, 0)
