@@ -159,10 +159,3 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 def stream() -> int:
     return torch.cuda.current_stream().cuda_stream
-
-
-def workspace(nbytes: int, device) -> torch.Tensor | None:
-    """Scratch from PyTorch's caching allocator; contents are undefined."""
-    if nbytes <= 0:
-        return None
-    return torch.empty(int(nbytes), dtype=torch.uint8, device=device)

@@ -335,12 +335,6 @@ __device__ __forceinline__ void spoil(float (&x)[4], uint32_t keep0, uint32_t ke
   if (!(keep1 & 0xffffu)) x[2] = nan;
   if (!(keep1 >> 16)) x[3] = nan;
 }
-// 8 x 8 transpose of bf16 pairs across the warp.
-__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
-  uint32_t y;
-  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(y) : "r"(x));
-  return y;
-}
 
 // A group's 128 threads copy `bytes` (a multiple of 16, at most 3 x 2 KB) to shared memory.
 template <int BYTES>
@@ -644,8 +638,8 @@ __global__ void __launch_bounds__(2 * C_WARPS * 32, 2) gdn_chunk_kernel(
       if (spoilt) spoil(o0, keep0, keep1);
       if (c + 2 < chunks) bar_arrive(C_BAR_EMPTY + b, 2 * GROUP);
       // transposed across the warp: lane (g, t) gets token g, rows 2t, 2t+1 (and + 8)
-      const uint32_t y0 = movmatrix_trans(ako::pack_bf16x2(o0[0] + o1[0], o0[1] + o1[1]));
-      const uint32_t y1 = movmatrix_trans(ako::pack_bf16x2(o0[2] + o1[2], o0[3] + o1[3]));
+      const uint32_t y0 = ako::movmatrix_trans(ako::pack_bf16x2(o0[0] + o1[0], o0[1] + o1[1]));
+      const uint32_t y1 = ako::movmatrix_trans(ako::pack_bf16x2(o0[2] + o1[2], o0[3] + o1[3]));
       if (c * C_TOK + 8 * w + g < len) {
         uint32_t* op = reinterpret_cast<uint32_t*>(out_h + (int64_t)(c * C_TOK + 8 * w + g) * (P_HV * P_D)) + t;
         op[0] = y0;
@@ -905,8 +899,8 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_wide_kernel(
           }
         }
         // transposed across the warp: lane (g, t) gets token g, rows 2t, 2t+1 (and + 8)
-        const uint32_t y0 = movmatrix_trans(ako::pack_bf16x2(y[n][0] + o1[0], y[n][1] + o1[1]));
-        const uint32_t y1 = movmatrix_trans(ako::pack_bf16x2(y[n][2] + o1[2], y[n][3] + o1[3]));
+        const uint32_t y0 = ako::movmatrix_trans(ako::pack_bf16x2(y[n][0] + o1[0], y[n][1] + o1[1]));
+        const uint32_t y1 = ako::movmatrix_trans(ako::pack_bf16x2(y[n][2] + o1[2], y[n][3] + o1[3]));
         if (c * C_TOK + 8 * n + g < len) {
           uint32_t* op = reinterpret_cast<uint32_t*>(out_h + (int64_t)(c * C_TOK + 8 * n + g) * (P_HV * P_D)) + t;
           op[0] = y0;

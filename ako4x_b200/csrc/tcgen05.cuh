@@ -288,10 +288,13 @@ __device__ __forceinline__ uint32_t t2_mapa(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
-// Arrival on a barrier of the pair's even CTA. Relaxed: what the barrier orders here is TMEM traffic
-// (the tcgen05.ld of this thread's warp against the next MMA into the buffer), which the
-// tcgen05 fences around the arrival and the wait take care of; a release at cluster scope measured
-// 1 500 - 2 400 cycles per arrival, once per warp and K block.
+// Arrival on a barrier of the pair's even CTA. Relaxed: what the barrier orders here is TMEM traffic, never
+// shared or global memory, and every use must keep to that. Either the tcgen05.ld of this thread's warp
+// against the next MMA into the buffer, or its tcgen05.st (attention weights, a rescaled accumulator) against
+// the MMA that reads them: the ld or st is complete (tcgen05.wait::ld, wait::st) before the arrival, and
+// tcgen05.fence::before_thread_sync in front of it and fence::after_thread_sync behind the issuer's wait order
+// it against the MMA. A release at cluster scope measured 1 500 - 2 400 cycles per arrival, once per warp and
+// K block.
 __device__ __forceinline__ void t2_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
 }

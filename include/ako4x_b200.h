@@ -61,8 +61,7 @@ int ako4x_gqa_paged_decode(const void* q, const void* k_cache, const void* v_cac
                            int64_t page_size, void* workspace, size_t workspace_bytes,
                            void* stream);
 
-/* Status word of the kernel (0: it has no wait that could give up). It synchronises the device: for
- * tests and post-mortems only. */
+/* Always 0: the kernels have no wait that could give up. */
 int ako4x_gqa_paged_decode_device_status(void);
 
 /* The same operator for callers that have no scratch memory to pass and cannot allocate any (a
@@ -95,8 +94,11 @@ int ako4x_mla_paged_decode(const void* q_nope, const void* q_pe, const void* ckv
                            int64_t batch, int64_t num_kv_indices, int64_t page_size,
                            void* workspace, size_t workspace_bytes, void* stream);
 
-/* Device status word shared by the MLA decode / prefill / DSA sparse attention kernels (same
- * meaning as ako4x_gqa_paged_decode_device_status; synchronises the device). */
+/* Device status word shared by the MLA decode / prefill / DSA sparse attention kernels. They wait on
+ * mbarriers with a cycle limit; a wait that gives up makes its CTA stop consuming and stores a non-zero
+ * code here (0 = no wait has given up since the library was loaded). A non-zero word means that the
+ * outputs of the call that set it are invalid; later calls are not affected by it (every launch starts its
+ * waits afresh). It synchronises the device: for tests and post-mortems only. */
 int ako4x_mla_attention_device_status(void);
 
 /* ---- a4. Paged causal MLA prefill ----------------------------------------------------------
@@ -142,7 +144,7 @@ int ako4x_dsa_topk_select(const float* scores, const int32_t* seq_lens, const in
                           int32_t* topk_indices, int64_t rows, int64_t max_pages, void* stream);
 
 /* Device status word of the tensor-core score kernel (same meaning as
- * ako4x_gqa_paged_decode_device_status; synchronises the device). */
+ * ako4x_mla_attention_device_status; synchronises the device). */
 int ako4x_dsa_indexer_device_status(void);
 
 /* ---- a6. DSA sparse MLA attention ----------------------------------------------------------
