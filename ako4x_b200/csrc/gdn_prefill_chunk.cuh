@@ -15,9 +15,10 @@
 // three bf16 pieces each (8 + 8 + 8 mantissa bits: by truncation the three pieces of an fp32 value
 // ADD UP TO IT EXACTLY; T and P are rounded piece by piece, which leaves 2^-26). A product with one
 // bf16 factor takes three mma, a product of two fp32 factors takes the six pairs of pieces down to
-// 2^-24: the sums are those of an fp32 recurrence in another order. R is formed from the sum of its
-// own logarithms, never as a difference of two prefix sums, so strong decay elsewhere in a chunk
-// costs it nothing.
+// 2^-24: the sums are those of an fp32 recurrence in another order. R is the product of its own gates, as in
+// the recurrence: never a ratio of two prefix products, so that strong decay elsewhere in a chunk costs it
+// nothing, and not an exponential of summed logarithms, whose rounding made the state's error 1.8e-7 of an
+// fp64 recurrence instead of the token-by-token form's 6.5e-8.
 //
 // Values that are not finite: a product takes in every token of its 8- or 16-token step, later ones with
 // coefficient zero, and 0 x NaN is NaN. A token whose right-hand side or delta is not finite is therefore
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(128, 7) gdn_chunk_prep_kernel(
   constexpr int A_PITCH = C_TOK + 4, WARP_FLOATS = C_TOK * A_PITCH;
   __shared__ __align__(128) unsigned char s_x[4 * WARP_FLOATS * 4];
   __shared__ float s_g[2][C_TOK][C_TOK + 1];                         // k.k, q.k
-  __shared__ float s_lg[2][C_TOK], s_beta[2][C_TOK];
+  __shared__ float s_gate[2][C_TOK], s_beta[2][C_TOK];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t slot = blockIdx.x;
   const int hq = blockIdx.y;
@@ -119,14 +120,14 @@ __global__ void __launch_bounds__(128, 7) gdn_chunk_prep_kernel(
   if (tid < 64) {
     const int e = tid >> 5, h = 2 * hq + e;
     const int64_t t = tb + lane;
-    float lg = 0.f, beta = 0.f;             // tokens past the end: no decay, no update
+    float gate = 1.f, beta = 0.f;           // tokens past the end: no decay, no update
     if (t < t1) {
       const float y = __bfloat162float(a[t * P_HV + h]) + dt_bias[h];
       const float sp = (y > 20.f) ? y : log1pf(expf(y));
-      lg = -expf(A_log[h]) * 1.4426950408889634f * sp;
+      gate = expf(-expf(A_log[h]) * sp);
       beta = 1.f / (1.f + expf(-__bfloat162float(b[t * P_HV + h])));
     }
-    s_lg[e][lane] = lg;
+    s_gate[e][lane] = gate;
     s_beta[e][lane] = beta;
   }
   ako::cp_async_wait<0>();
@@ -170,21 +171,21 @@ __global__ void __launch_bounds__(128, 7) gdn_chunk_prep_kernel(
   unsigned char* dst = ws + (slot * P_HV + 2 * hq + e) * C_SLOT_BYTES + (warp >> 1) * C_FRAG_BYTES;
   float* out = reinterpret_cast<float*>(s_x) + warp * WARP_FLOATS;       // [i][j], columns rotated by i
   if (warp < 2) {
-    float run = 0.f;
+    float run = 1.f;
 #pragma unroll
     for (int i = 0; i < C_TOK; ++i) {
-      if (i > j) run += s_lg[e][i];
-      out[i * A_PITCH + j] = (i > j) ? s_beta[e][i] * exp2f(run) * s_g[0][i][j] : 0.f;
+      if (i > j) run *= s_gate[e][i];
+      out[i * A_PITCH + j] = (i > j) ? s_beta[e][i] * run * s_g[0][i][j] : 0.f;
     }
     float* coef = reinterpret_cast<float*>(ws + (slot * P_HV + 2 * hq + e) * C_SLOT_BYTES + 2 * C_FRAG_BYTES);
-    float lc = s_lg[e][lane];
+    float gam = s_gate[e][lane];
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-      const float up = __shfl_up_sync(0xffffffffu, lc, off);
-      if (lane >= off) lc += up;
+      const float up = __shfl_up_sync(0xffffffffu, gam, off);
+      if (lane >= off) gam *= up;
     }
-    coef[lane] = exp2f(lc);
-    coef[C_TOK + lane] = exp2f(run);
+    coef[lane] = gam;
+    coef[C_TOK + lane] = run;
     __syncwarp();
     const float bj = s_beta[e][j];          // may be NaN: enters at the diagonal, so that zeros above it stay zeros
     float t[C_TOK];
@@ -205,11 +206,11 @@ __global__ void __launch_bounds__(128, 7) gdn_chunk_prep_kernel(
 #pragma unroll
     for (int i = 0; i < C_TOK; ++i) out[i * C_TOK + ((j + i) & 31)] = t[i];
   } else {
-    float run = 0.f;
+    float run = 1.f;
 #pragma unroll
     for (int i = 0; i < C_TOK; ++i) {
-      if (i > j) run += s_lg[e][i];
-      out[i * C_TOK + ((j + i) & 31)] = (i >= j) ? scale * exp2f(run) * s_g[1][i][j] : 0.f;
+      if (i > j) run *= s_gate[e][i];
+      out[i * C_TOK + ((j + i) & 31)] = (i >= j) ? scale * run * s_g[1][i][j] : 0.f;
     }
   }
   __syncwarp();
