@@ -5,7 +5,8 @@
 // R_ij = prod_{j<l<=i} g_l (the decay between tokens j and i), unrolling
 //   delta_i = beta_i (v_i - g_i S_{i-1} k_i),   S_i = g_i S_{i-1} + delta_i k_i^T
 // gives, for every state row on its own,
-//   delta = T (v - gam (S0 k)),  T = (I + A)^-1 diag(beta),  A_ij = beta_i R_ij (k_i.k_j) for j < i
+//   delta = T (v - gam (S0 k)),  T = (I + A)^-1 diag(beta) (its diagonal is beta),
+//   A_ij = beta_i R_ij (k_i.k_j) for j < i
 //   out_i = gam_i scale (S0 q_i) + sum_{j<=i} P_ij delta_j,  P_ij = scale R_ij (q_i.k_j)
 //   S_C   = gam_C S0 + sum_j (R_Cj delta_j) k_j^T
 // T and P depend on the tokens only: gdn_chunk_prep_kernel makes them for all chunks at once.
@@ -15,10 +16,15 @@
 // three bf16 pieces each (8 + 8 + 8 mantissa bits: by truncation the three pieces of an fp32 value
 // ADD UP TO IT EXACTLY; T and P are rounded piece by piece, which leaves 2^-26). A product with one
 // bf16 factor takes three mma, a product of two fp32 factors takes the six pairs of pieces down to
-// 2^-24: the sums are those of an fp32 recurrence in another order. R is the product of its own gates, as in
-// the recurrence: never a ratio of two prefix products, so that strong decay elsewhere in a chunk costs it
-// nothing, and not an exponential of summed logarithms, whose rounding made the state's error 1.8e-7 of an
-// fp64 recurrence instead of the token-by-token form's 6.5e-8.
+// 2^-24: the sums are those of an fp32 recurrence in another order. The tensor core truncates where it
+// accumulates, which costs an fp32 result twice the error of a rounding and a bias: so what carries most of a
+// value is kept out of it or goes in last. The diagonal of T, which is beta, multiplies its right-hand side in
+// fp32 outside (the tiles of T hold what is below it); a product's small pieces are summed before the leading
+// ones; and a chunk's update is summed from zero and added to the state in fp32. R is the product of its own
+// gates, as in the recurrence: never a ratio of two prefix products, so that strong decay elsewhere in a chunk
+// costs it nothing, and not an exponential of summed logarithms. Error of the state from an fp64 recurrence,
+// rms (8 x 300, 1 x 2 000, 24 x 100 tokens): 6.7e-8, 6.9e-8, 8.3e-8; token by token in fp32 6.4e-8, 6.6e-8,
+// 6.7e-8; 1.8e-7, 1.7e-7, 2.0e-7 before that care was taken, for 4 to 7 % less time.
 //
 // Values that are not finite: a product takes in every token of its 8- or 16-token step, later ones with
 // coefficient zero, and 0 x NaN is NaN. A token whose right-hand side or delta is not finite is therefore
@@ -45,9 +51,9 @@ constexpr int C_TOK = 32;                                // tokens per chunk
 constexpr int C_ROWS = 16;                               // state rows per CTA (one m16 tile)
 constexpr int C_WARPS = 4;                               // k split
 constexpr int C_FRAG_BYTES = 6 * 3 * 32 * 8;             // six 8 x 16 tiles (i, j) on or below the diagonal, three pieces
-constexpr int C_COEF_FLOATS = 2 * C_TOK;                 // gam_i, then R_Cj
+constexpr int C_COEF_FLOATS = 3 * C_TOK;                 // gam_i, R_Cj, beta_i
 constexpr int C_SLOT_BYTES = 2 * C_FRAG_BYTES + C_COEF_FLOATS * 4;   // T, P, coefficients of one (chunk, head)
-static_assert(C_SLOT_BYTES % 256 == 0, "slots keep the alignment of the workspace");
+static_assert(C_SLOT_BYTES % 16 == 0, "slots are copied in 16-byte pieces");
 
 // Workspace slot of chunk c of sequence `seq` that starts at token t0: unique over all sequences
 // without a scan of cu_seqlens (every sequence start costs at most one extra partial chunk).
@@ -186,6 +192,7 @@ __global__ void __launch_bounds__(128, 7) gdn_chunk_prep_kernel(
     }
     coef[lane] = gam;
     coef[C_TOK + lane] = run;
+    coef[2 * C_TOK + lane] = s_beta[e][lane];
     __syncwarp();
     const float bj = s_beta[e][j];          // may be NaN: enters at the diagonal, so that zeros above it stay zeros
     float t[C_TOK];
@@ -204,7 +211,7 @@ __global__ void __launch_bounds__(128, 7) gdn_chunk_prep_kernel(
     }
     __syncwarp();
 #pragma unroll
-    for (int i = 0; i < C_TOK; ++i) out[i * C_TOK + ((j + i) & 31)] = t[i];
+    for (int i = 0; i < C_TOK; ++i) out[i * C_TOK + ((j + i) & 31)] = (i == j) ? 0.f : t[i];
   } else {
     float run = 1.f;
 #pragma unroll
@@ -359,7 +366,7 @@ __device__ __forceinline__ void load_token_tile(uint32_t (&bf)[4], uint32_t base
   const int row = 8 * tile + (lane & 7);
   ako::ldmatrix_x4(bf[0], bf[1], bf[2], bf[3], base + row * 64 + (((lane >> 3) ^ ((row >> 1) & 3)) << 4));
 }
-// acc[n] = (S0 pieces of this warp's 32 columns) x (token tile (w + n) mod 4); the three tiles that other
+// acc[n] = (S0 pieces of this warp's 32 columns) x (token tile (w + n) mod 4), small pieces first; the three tiles that other
 // warps finish go to shared memory, tile w itself is accumulator 0.
 __device__ __forceinline__ void partial_products(float (&own)[4], const uint32_t (&As)[2][3][4], uint32_t base, float4* part,
                                                  int w, int lane) {
@@ -368,11 +375,11 @@ __device__ __forceinline__ void partial_products(float (&own)[4], const uint32_t
 #pragma unroll
   for (int n = 0; n < 4; ++n) load_token_tile(bf[n], base, (w + n) & 3, lane);
 #pragma unroll
-  for (int n = 0; n < 4; ++n) mma_zero(acc[n], As[0][0], bf[n][0], bf[n][1]);
+  for (int n = 0; n < 4; ++n) mma_zero(acc[n], As[0][2], bf[n][0], bf[n][1]);
 #pragma unroll
-  for (int n = 0; n < 4; ++n) ako::mma_bf16_16816(acc[n], As[1][0], bf[n][2], bf[n][3]);
+  for (int n = 0; n < 4; ++n) ako::mma_bf16_16816(acc[n], As[1][2], bf[n][2], bf[n][3]);
 #pragma unroll
-  for (int p = 1; p < 3; ++p)
+  for (int p = 1; p >= 0; --p)
 #pragma unroll
     for (int s = 0; s < 2; ++s)
 #pragma unroll
@@ -527,11 +534,14 @@ __global__ void __launch_bounds__(2 * C_WARPS * 32, 2) gdn_chunk_kernel(
       add_partials(x, sX, w, lane);
       bool spoilt;
       uint32_t keep0 = ~0u, keep1 = ~0u;
+      float r[4];
       {
         const float2 gam = *reinterpret_cast<const float2*>(coef + 8 * w + 2 * t);
         const __nv_bfloat16* vv = reinterpret_cast<const __nv_bfloat16*>(stage + C_CH_V) + (8 * w + 2 * t) * C_ROWS + g;
-        const float r[4] = {__bfloat162float(vv[0]) - gam.x * x[0], __bfloat162float(vv[C_ROWS]) - gam.y * x[1],
-                            __bfloat162float(vv[8]) - gam.x * x[2], __bfloat162float(vv[C_ROWS + 8]) - gam.y * x[3]};
+        r[0] = __bfloat162float(vv[0]) - gam.x * x[0];
+        r[1] = __bfloat162float(vv[C_ROWS]) - gam.y * x[1];
+        r[2] = __bfloat162float(vv[8]) - gam.x * x[2];
+        r[3] = __bfloat162float(vv[C_ROWS + 8]) - gam.y * x[3];
         store_pieces(sR + w * 32, r);
         spoilt = __any_sync(0xffffffffu, !(not_finite_sum(r) == 0.f));
         if (spoilt)
@@ -540,17 +550,14 @@ __global__ void __launch_bounds__(2 * C_WARPS * 32, 2) gdn_chunk_kernel(
       }
       const float gC = coef[C_TOK - 1];
       const float2 dec = *reinterpret_cast<const float2*>(coef + C_TOK + 8 * w + 2 * t);
-#pragma unroll
-      for (int n = 0; n < 4; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) S[n][i] *= gC;
+      const float2 beta = *reinterpret_cast<const float2*>(coef + 2 * C_TOK + 8 * w + 2 * t);
       bar_sync(C_BAR_CHAIN, GROUP);
 
       // 3. delta of tile w = T (right-hand side)
       float d0[4], d1[4];
       triangular_tile<true>(d0, d1, sR, reinterpret_cast<const uint2*>(stage + C_CH_SLOT) + ft, w, spoilt, keep0, keep1);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) d0[i] += d1[i];
+      for (int i = 0; i < 4; ++i) d0[i] = fmaf((i & 1) ? beta.y : beta.x, r[i], d0[i] + d1[i]);
       if (spoilt) spoil(d0, keep0, keep1);
       {
         const float e[4] = {d0[0] * dec.x, d0[1] * dec.y, d0[2] * dec.x, d0[3] * dec.y};
@@ -560,20 +567,34 @@ __global__ void __launch_bounds__(2 * C_WARPS * 32, 2) gdn_chunk_kernel(
       store_pieces(reinterpret_cast<uint2*>(smem + C_OFF_D + b * C_D_BYTES) + lane + w * 32, d0);
       bar_arrive(C_BAR_FULL + b, 2 * GROUP);
 
-      // 4. the state at the end of the chunk
+      // 4. the state at the end of the chunk, 16 columns at a time; the leading pieces last
+      uint32_t A[2][3][4];
+      frag_pieces(A[0], sE);
+      frag_pieces(A[1], sE + 64);
 #pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        uint32_t A[3][4], bf[8];
-        frag_pieces(A, sE + 64 * s);
-        const int row = 16 * s + (lane & 15);
+      for (int n0 = 0; n0 < 4; n0 += 2) {
+        uint32_t bf[2][4];
 #pragma unroll
-        for (int n = 0; n < 4; n += 2)
-          ako::ldmatrix_x4_trans(bf[2 * n], bf[2 * n + 1], bf[2 * n + 2], bf[2 * n + 3],
-                                 kbase + row * 64 + (((n + (lane >> 4)) ^ ((row >> 1) & 3)) << 4));
+        for (int s = 0; s < 2; ++s) {
+          const int row = 16 * s + (lane & 15);
+          ako::ldmatrix_x4_trans(bf[s][0], bf[s][1], bf[s][2], bf[s][3],
+                                 kbase + row * 64 + (((n0 + (lane >> 4)) ^ ((row >> 1) & 3)) << 4));
+        }
+        float U[2][4];
 #pragma unroll
-        for (int p = 0; p < 3; ++p)
+        for (int n = 0; n < 2; ++n) mma_zero(U[n], A[0][2], bf[0][2 * n], bf[0][2 * n + 1]);
 #pragma unroll
-          for (int n = 0; n < 4; ++n) ako::mma_bf16_16816(S[n], A[p], bf[2 * n], bf[2 * n + 1]);
+        for (int n = 0; n < 2; ++n) ako::mma_bf16_16816(U[n], A[1][2], bf[1][2 * n], bf[1][2 * n + 1]);
+#pragma unroll
+        for (int p = 1; p >= 0; --p)
+#pragma unroll
+          for (int s = 0; s < 2; ++s)
+#pragma unroll
+            for (int n = 0; n < 2; ++n) ako::mma_bf16_16816(U[n], A[s][p], bf[s][2 * n], bf[s][2 * n + 1]);
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) S[n0 + n][i] = fmaf(gC, S[n0 + n][i], U[n][i]);
       }
       __syncwarp();   // the warp's k of this chunk is read: the next load may overwrite it
     }
@@ -859,8 +880,9 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_wide_kernel(
           else if (s == 0) mma_6<true>(d[n], d1, A[s], B);
           else mma_6<false>(d[n], d1, A[s], B);
         }
+        const float2 beta = *reinterpret_cast<const float2*>(coef + 2 * C_TOK + 8 * n + 2 * t);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) d[n][i] += d1[i];
+        for (int i = 0; i < 4; ++i) d[n][i] = fmaf((i & 1) ? beta.y : beta.x, x[n][i], d[n][i] + d1[i]);
       }
     }
     if (wide_not_finite(d)) spoilt = true;   // also an overflow
@@ -921,21 +943,28 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_wide_kernel(
       const float gC = coef[C_TOK - 1], g0 = (spoilt && f0 < C_TOK) ? nan : gC, g1 = (spoilt && f1 < C_TOK) ? nan : gC;
 #pragma unroll
       for (int n = 0; n < 16; n += 2) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          S[n][i] *= (i < 2) ? g0 : g1;
-          S[n + 1][i] *= (i < 2) ? g0 : g1;
-        }
+        uint32_t bf[2][4];
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
-          uint32_t bf[4];
           const int row = 16 * s + (lane & 15);
-          ako::ldmatrix_x4_trans(bf[0], bf[1], bf[2], bf[3], st + row * 256 + (((n + (lane >> 4)) ^ (row & 7)) << 4));
+          ako::ldmatrix_x4_trans(bf[s][0], bf[s][1], bf[s][2], bf[s][3], st + row * 256 + (((n + (lane >> 4)) ^ (row & 7)) << 4));
+        }
+        float U[2][4];
+        mma_zero(U[0], A[0][2], bf[0][0], bf[0][1]);
+        mma_zero(U[1], A[0][2], bf[0][2], bf[0][3]);
+        ako::mma_bf16_16816(U[0], A[1][2], bf[1][0], bf[1][1]);
+        ako::mma_bf16_16816(U[1], A[1][2], bf[1][2], bf[1][3]);
 #pragma unroll
-          for (int p = 0; p < 3; ++p) {
-            ako::mma_bf16_16816(S[n], A[s][p], bf[0], bf[1]);
-            ako::mma_bf16_16816(S[n + 1], A[s][p], bf[2], bf[3]);
+        for (int p = 1; p >= 0; --p)
+#pragma unroll
+          for (int s = 0; s < 2; ++s) {
+            ako::mma_bf16_16816(U[0], A[s][p], bf[s][0], bf[s][1]);
+            ako::mma_bf16_16816(U[1], A[s][p], bf[s][2], bf[s][3]);
           }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          S[n][i] = fmaf((i < 2) ? g0 : g1, S[n][i], U[0][i]);
+          S[n + 1][i] = fmaf((i < 2) ? g0 : g1, S[n + 1][i], U[1][i]);
         }
       }
     }
