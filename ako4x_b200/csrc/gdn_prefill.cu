@@ -279,9 +279,10 @@ extern "C" int ako4x_gdn_prefill(const void* q, const void* k, const void* v, co
     gdn_chunk_prep_kernel<<<dim3((unsigned)slots, P_HQ), 128, 0, st>>>(qb, kb, A_log, ab, dt_bias, bb, cu_seqlens,
                                                                       (int)num_seqs, scale, (unsigned char*)workspace);
     AKO_CHECK_LAUNCH();
-    // One warp per 16 rows and no exchanges from 20 sequences on, where it fills the GPU: equal at 16
-    // sequences (16 x 200 tokens: 60 against 58 us), ahead from 20 (20 x 200: 60 against 70, 64 x 128: 84
-    // against 128, 64 x 4: 31 against 53) and far behind for few long ones (1 x 8 192: 800 against 275).
+    // One warp per 16 rows and no exchanges from 20 sequences on, where it fills the GPU. Measured (us, uniform
+    // lengths): behind or ahead by length at 16 sequences (16 x 64 tokens 24.4 against 25.0, x 200 59 against 55,
+    // x 500 124 against 113), ahead from 20 (20 x 32 17.6 against 22.7, x 400 106 against 120, 64 x 4 31 against 52,
+    // 64 x 128 86 against 128) and far behind for few long ones (8 000 tokens in one of 20: 642 against 290).
     if (num_seqs >= 20) {
       if (!ako::ensure_dynamic_smem<gdn_chunk_wide_kernel>(CW_SMEM) ||
           ako::launch_pdl(true, gdn_chunk_wide_kernel, dim3(P_D / CW_ROWS, P_HV, (unsigned)num_seqs), dim3(128), CW_SMEM, st, qb, kb, vb,

@@ -11,7 +11,10 @@
 //     m16n8k16 with tokens as M, over a permuted order of the reduction in which Q's B fragments are
 //     loaded too. S^T = K Q^T is [16 tokens x 8 heads], four of them real.
 //   * V is loaded the same way; movmatrix turns an 8 x 8 block of pairs into the A fragment of
-//     O^T = V^T P^T ([128 x 8 heads], features as M), and P's own pairs into the B fragment.
+//     O^T = V^T P^T ([128 x 8 heads], features as M), and P's own pairs into the B fragment. P goes in as two
+//     bf16 pieces (16 bits): in one, its rounding showed in the output (2.2e-3 of an fp64 result at 64 sequences
+//     of up to 8 192 tokens, and more the longer a share is; now 1.67e-3, which is the bf16 output's own
+//     rounding) for 8 of 24 mma a tile, hidden behind the loads (0 to 0.3 us a call).
 //   * K of the next tile is requested when S has been computed, V of it when O has.
 //
 // Work split: flat_share.cuh, tiles of 16 tokens, one share per pair of CTAs (the two halves of the KV
@@ -136,12 +139,6 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gqa_decode_kernel(Params
 #pragma unroll
         for (int i = 0; i < 2; ++i) x[i][j] = ld_row16(base + off[i] + 64 * j);
     };
-    fetch_ids(ts);
-    locate(ts);
-    load(kc, p.k);
-    load(vc, p.v);
-    fetch_ids(ts + 1);
-
     // Q of the four heads as B fragments (n = head g, heads 4-7 are zero), in the order of the K pieces
     uint4 qb[4];
 #pragma unroll
@@ -150,83 +147,112 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gqa_decode_kernel(Params
       if (g < GROUP)
         qb[j] = __ldg(reinterpret_cast<const uint4*>(p.q + ((int64_t)b * HQ + kvh * GROUP + g) * D + 32 * j + 8 * t));
     }
+    // P goes in as two pieces, and once more as one where an output came out NaN or infinite: an infinite value
+    // must not meet a piece of zero or of the other sign.
+    bool two = true;
     float acc[4][2][4];   // [block j][u]: features 32 j + 8 (g / 2) + (g & 1) + 4 u (regs 0, 1) and + 2 (2, 3), heads 2t, 2t+1
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[j][u][i] = 0.f;
     // heads 2t, 2t+1; l over this lane's tokens. The maxima start at the lowest finite value, so that a score
     // of -inf weighs 0 whatever else a tile or a share holds.
-    float m0 = -FLT_MAX, m1 = -FLT_MAX, l0 = 0.f, l1 = 0.f;
+    float m0, m1, l0, l1;
+    while (true) {
+      fetch_ids(ts);
+      locate(ts);
+      load(kc, p.k);
+      load(vc, p.v);
+      fetch_ids(ts + 1);
+      m0 = m1 = -FLT_MAX;
+      l0 = l1 = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[j][u][i] = 0.f;
 
-    for (int tile = ts; tile < te; ++tile) {
-      float s[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t a0[4] = {kc[0][j].x, kc[1][j].x, kc[0][j].y, kc[1][j].y};
-        const uint32_t a1[4] = {kc[0][j].z, kc[1][j].z, kc[0][j].w, kc[1][j].w};
-        ako::mma_bf16_16816(s, a0, qb[j].x, qb[j].y);
-        ako::mma_bf16_16816(s2, a1, qb[j].z, qb[j].w);
-      }
-      const bool more = tile + 1 < te;
-      if (more) {
-        locate(tile + 1);
-        load(kc, p.k);
-      }
-      // softmax over the tokens: rows g and g + 8 of this lane, 8 lanes apart by 4
-      const bool v0 = tile * TILE + g < len, v1 = tile * TILE + 8 + g < len;
-      s[0] = v0 ? (s[0] + s2[0]) * p.scale_log2 : -INFINITY;
-      s[1] = v0 ? (s[1] + s2[1]) * p.scale_log2 : -INFINITY;
-      s[2] = v1 ? (s[2] + s2[2]) * p.scale_log2 : -INFINITY;
-      s[3] = v1 ? (s[3] + s2[3]) * p.scale_log2 : -INFINITY;
-      float n0 = fmaxf(s[0], s[2]), n1 = fmaxf(s[1], s[3]);
-#pragma unroll
-      for (int o = 4; o <= 16; o <<= 1) {
-        n0 = fmaxf(n0, __shfl_xor_sync(0xffffffffu, n0, o));
-        n1 = fmaxf(n1, __shfl_xor_sync(0xffffffffu, n1, o));
-      }
-      if (__any_sync(0xffffffffu, n0 > m0 || n1 > m1)) {
-        n0 = fmaxf(n0, m0);
-        n1 = fmaxf(n1, m1);
-        const float f0 = ako::fast_exp2(m0 - n0), f1 = ako::fast_exp2(m1 - n1);
-        m0 = n0;
-        m1 = n1;
-        l0 *= f0;
-        l1 *= f1;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            acc[j][u][0] *= f0; acc[j][u][1] *= f1; acc[j][u][2] *= f0; acc[j][u][3] *= f1;
-          }
-      }
-      s[0] = ako::fast_exp2(s[0] - m0);
-      s[1] = ako::fast_exp2(s[1] - m1);
-      s[2] = ako::fast_exp2(s[2] - m0);
-      s[3] = ako::fast_exp2(s[3] - m1);
-      l0 += s[0] + s[2];
-      l1 += s[1] + s[3];
-      if (tile * TILE + TILE > len) {   // past the end: weight 0, but the row read in their place may hold infinities
+      for (int tile = ts; tile < te; ++tile) {
+        float s[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          if (!v0) vc[0][j] = make_uint4(0u, 0u, 0u, 0u);
-          if (!v1) vc[1][j] = make_uint4(0u, 0u, 0u, 0u);
+          const uint32_t a0[4] = {kc[0][j].x, kc[1][j].x, kc[0][j].y, kc[1][j].y};
+          const uint32_t a1[4] = {kc[0][j].z, kc[1][j].z, kc[0][j].w, kc[1][j].w};
+          ako::mma_bf16_16816(s, a0, qb[j].x, qb[j].y);
+          ako::mma_bf16_16816(s2, a1, qb[j].z, qb[j].w);
+        }
+        const bool more = tile + 1 < te;
+        if (more) {
+          locate(tile + 1);
+          load(kc, p.k);
+        }
+        // softmax over the tokens: rows g and g + 8 of this lane, 8 lanes apart by 4
+        const bool v0 = tile * TILE + g < len, v1 = tile * TILE + 8 + g < len;
+        s[0] = v0 ? (s[0] + s2[0]) * p.scale_log2 : -INFINITY;
+        s[1] = v0 ? (s[1] + s2[1]) * p.scale_log2 : -INFINITY;
+        s[2] = v1 ? (s[2] + s2[2]) * p.scale_log2 : -INFINITY;
+        s[3] = v1 ? (s[3] + s2[3]) * p.scale_log2 : -INFINITY;
+        float n0 = fmaxf(s[0], s[2]), n1 = fmaxf(s[1], s[3]);
+#pragma unroll
+        for (int o = 4; o <= 16; o <<= 1) {
+          n0 = fmaxf(n0, __shfl_xor_sync(0xffffffffu, n0, o));
+          n1 = fmaxf(n1, __shfl_xor_sync(0xffffffffu, n1, o));
+        }
+        if (__any_sync(0xffffffffu, n0 > m0 || n1 > m1)) {
+          n0 = fmaxf(n0, m0);
+          n1 = fmaxf(n1, m1);
+          const float f0 = ako::fast_exp2(m0 - n0), f1 = ako::fast_exp2(m1 - n1);
+          m0 = n0;
+          m1 = n1;
+          l0 *= f0;
+          l1 *= f1;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              acc[j][u][0] *= f0; acc[j][u][1] *= f1; acc[j][u][2] *= f0; acc[j][u][3] *= f1;
+            }
+        }
+        s[0] = ako::fast_exp2(s[0] - m0);
+        s[1] = ako::fast_exp2(s[1] - m1);
+        s[2] = ako::fast_exp2(s[2] - m0);
+        s[3] = ako::fast_exp2(s[3] - m1);
+        l0 += s[0] + s[2];
+        l1 += s[1] + s[3];
+        if (tile * TILE + TILE > len) {   // past the end: weight 0, but the row read in their place may hold infinities
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (!v0) vc[0][j] = make_uint4(0u, 0u, 0u, 0u);
+            if (!v1) vc[1][j] = make_uint4(0u, 0u, 0u, 0u);
+          }
+        }
+        const uint32_t h0 = ako::pack_bf16x2(s[0], s[1]), h1 = ako::pack_bf16x2(s[2], s[3]);
+        const uint32_t b0 = ako::movmatrix_trans(h0), b1 = ako::movmatrix_trans(h1);
+        // what the rounding of the weights left
+        const uint32_t c0 = ako::movmatrix_trans(ako::pack_bf16x2(s[0] - ako::bf16_lo(h0), s[1] - ako::bf16_hi(h0)));
+        const uint32_t c1 = ako::movmatrix_trans(ako::pack_bf16x2(s[2] - ako::bf16_lo(h1), s[3] - ako::bf16_hi(h1)));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t a0[4] = {ako::movmatrix_trans(vc[0][j].x), ako::movmatrix_trans(vc[0][j].y), ako::movmatrix_trans(vc[1][j].x), ako::movmatrix_trans(vc[1][j].y)};
+          const uint32_t a1[4] = {ako::movmatrix_trans(vc[0][j].z), ako::movmatrix_trans(vc[0][j].w), ako::movmatrix_trans(vc[1][j].z), ako::movmatrix_trans(vc[1][j].w)};
+          if (two) {
+            ako::mma_bf16_16816(acc[j][0], a0, c0, c1);
+            ako::mma_bf16_16816(acc[j][1], a1, c0, c1);
+          }
+          ako::mma_bf16_16816(acc[j][0], a0, b0, b1);
+          ako::mma_bf16_16816(acc[j][1], a1, b0, b1);
+        }
+        if (more) {
+          load(vc, p.v);
+          fetch_ids(tile + 2);
         }
       }
-      const uint32_t b0 = ako::movmatrix_trans(ako::pack_bf16x2(s[0], s[1])), b1 = ako::movmatrix_trans(ako::pack_bf16x2(s[2], s[3]));
+      float z = 0.f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t a0[4] = {ako::movmatrix_trans(vc[0][j].x), ako::movmatrix_trans(vc[0][j].y), ako::movmatrix_trans(vc[1][j].x), ako::movmatrix_trans(vc[1][j].y)};
-        const uint32_t a1[4] = {ako::movmatrix_trans(vc[0][j].z), ako::movmatrix_trans(vc[0][j].w), ako::movmatrix_trans(vc[1][j].z), ako::movmatrix_trans(vc[1][j].w)};
-        ako::mma_bf16_16816(acc[j][0], a0, b0, b1);
-        ako::mma_bf16_16816(acc[j][1], a1, b0, b1);
-      }
-      if (more) {
-        load(vc, p.v);
-        fetch_ids(tile + 2);
-      }
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) z = fmaf(acc[j][u][i], 0.f, z);
+      if (!two || !__any_sync(0xffffffffu, !(z == 0.f))) break;
+      two = false;
     }
 
 #pragma unroll
