@@ -39,12 +39,12 @@
 // Per chunk and pair of warps: 96 mma (24 S0 k, 24 S0 q, <= 12 T, <= 12 P, 24 S update) of 8.2 cycles of
 // an SM sub-partition (mma.sync m16n8k16 measured at 2.0 cycles per SM).
 //
-// What bounds it: one CTA per SM, the chain (2 100 cycles per chunk, of which three exchanges through
-// shared memory); two CTAs per SM, the LSU data pipe (ncu: 77 %, 1 130 wavefronts per chunk; tensor pipe
-// 43 %). Measured, whole call against the fp32 CUDA-core form this replaces: 8 ragged sequences of
-// 7 244 tokens 605 -> 121 us, 1 x 8 192 1 000 -> 275, 64 x 128 510 -> 120. One group of four warps that
-// also makes the outputs: 128 us for the 8 (three CTAs per SM) and 1.2 instead of 1.08 us per chunk for
-// one sequence. Loads by TMA instead of cp.async: no difference for 8, 1.22 us per chunk for one.
+// What bounds it: one CTA per SM, the chain (2 150 cycles per chunk, of which three exchanges through
+// shared memory); two CTAs per SM, the LSU data pipe (ncu: 67 %, 1 130 wavefronts per chunk; tensor pipe
+// 39 %). Measured, whole call against the fp32 CUDA-core form this replaces: 8 ragged sequences of
+// 7 244 tokens 605 -> 121 us, 1 x 8 192 1 000 -> 288. One group of four warps that also makes the outputs:
+// 128 us for the 8 (three CTAs per SM) and 1.2 instead of 1.08 us per chunk for one sequence. Loads by TMA
+// instead of cp.async: no difference for 8, 1.22 us per chunk for one.
 #pragma once
 
 constexpr int C_TOK = 32;                                // tokens per chunk
@@ -676,7 +676,8 @@ __global__ void __launch_bounds__(2 * C_WARPS * 32, 2) gdn_chunk_kernel(
 // all 128 columns of its 16 rows, so that a chunk needs no exchange at all (everything from S0 k to the
 // new S stays in its registers) and the CTA's four warps (64 rows) only share the loads: 264 LSU
 // wavefronts per 16 rows and chunk instead of 1 130, 360 mma in a row instead of 96. Bound by the tensor
-// pipe (2 950 cycles of a sub-partition per chunk and warp) where at least two warps share one.
+// pipe (2 950 cycles of a sub-partition per chunk and warp; ncu: 58 %) where at least two warps share one.
+// 64 x 128 tokens: 86 us against 128 with the kernel above and 499 token by token.
 constexpr int CW_ROWS = 64;
 constexpr int CW_V_PITCH = CW_ROWS * 2 + 16;                          // ldmatrix of eight rows: no bank conflict
 constexpr int CW_OFF_Q = C_TOK * 256;                                 // stage: k | q | T, P, coefficients | v

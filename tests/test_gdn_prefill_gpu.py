@@ -46,8 +46,8 @@ def test_against_oracle(lens):
 
 @pytest.mark.parametrize("lens", [[370], [33], [129], [16], [5], [70, 300], [0, 33], [17, 0]])
 def test_both_forms_agree(lens):
-    """One or two sequences run in the chunked form (16 tokens per step of the state), more run
-    token by token; `_chunked=False` forces the latter. Both against the oracle and each other."""
+    """Calls with a workspace run in the chunked form (32 tokens per step of the state) unless their sequences
+    are a few tokens long; `_chunked=False` forces token by token. Both against the oracle and each other."""
     a = W.make_gdn_prefill(lens, shape_id=21 + len(lens))
     args = [a[k].cuda() if a[k] is not None else None for k in KEYS]
     o1, s1 = gdn_prefill.run(*args, a["scale"], _chunked=False)

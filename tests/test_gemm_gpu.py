@@ -38,7 +38,7 @@ def test_against_oracle(m):
     assert _cabi.lib().ako4x_gemm_device_status() == 0
 
 
-# both sides of every line of the plan: one-CTA tiles and pairs (odd and even numbers of row tiles), their
+# row counts around the tile and wave edges: one-CTA tiles and pairs (odd and even numbers of row tiles), their
 # widths and K splits; reductions of one block and of a number of blocks that does not split
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("m,n,k", [(m, 2048, 4096) for m in (255, 257, 385, 512, 513, 769, 1024, 1025, 1153, 2561)] +

@@ -42,8 +42,8 @@ def test_config_shapes(built_lib, batch):
 
 
 def test_work_list_mode_ragged(built_lib):
-    """A batch large and long enough for the work-list mode (equal chunks per CTA): very long next to
-    very short and empty sequences, checked against the oracle for every row."""
+    """Very long next to very short and empty sequences, cut into equal shares, checked against the oracle for
+    every row."""
     lens = [8192] * 20 + [1, 17, 300, 0, 2049, 255, 256, 257] + [5000, 16, 0, 777] * 5
     assert sum(lens) >= 160 * 1024
     _check(W.make_gqa_decode(len(lens), shape_id=41, lens=lens, extra_pages=29))
@@ -81,8 +81,8 @@ def test_full_size_split_invariance(built_lib):
 
 
 def test_full_length_sampled_sequences(built_lib):
-    """B = 256 with the configured lengths (128..8192), i.e. the work-list mode at full size: eight
-    sampled sequences against the CPU oracle (their cache rows compacted into a small cache)."""
+    """B = 256 with the configured lengths (128..8192): eight sampled sequences against the CPU oracle
+    (their cache rows compacted into a small cache)."""
     a = W.make_gqa_decode(256, shape_id=256, device="cuda")
     o, lse = gqa_decode.run(*[a[k] for k in KEYS])
     sel = [0, 1, 50, 99, 128, 200, 254, 255]
@@ -123,8 +123,8 @@ def test_same_buffers_new_contents(built_lib):
 
 @pytest.mark.parametrize("lens", [[15, 16, 17, 0, 33, 1] * 40, [600] * 3 + [0] + [3] * 230, [5, 0, 8192, 2, 0], [7000, 16, 1]])
 def test_shares_and_whole_sequences(built_lib, lens):
-    """Many short sequences (one share each, no partials, no merge), a batch just inside that rule, and
-    few sequences whose partials come from one or from hundreds of shares; empty ones in between."""
+    """Many short sequences, most of them inside one share, some longer ones among them, and few sequences whose
+    partials come from one or from hundreds of shares; empty ones in between."""
     _check(W.make_gqa_decode(len(lens), shape_id=60 + len(lens) % 7, lens=lens, extra_pages=11))
 
 

@@ -65,7 +65,7 @@ def test_oversized_request_is_refused_cleanly(built_lib):
     """A shape whose partials exceed the built-in scratch returns AKO4X_ETOOLARGE before any
     pointer is touched (the pointers below are never dereferenced)."""
     limit = built_lib.ako4x_gqa_paged_decode_noalloc_max_scratch_bytes()
-    batch, n_idx = 512, 512 * 8192   # two splits of 512 x 32 heads: about 17 MB of partials
+    batch, n_idx = 512, 512 * 8192   # a size of 512 + 222 partials of 32 heads: about 12 MB
     assert built_lib.ako4x_gqa_paged_decode_workspace_bytes(batch, n_idx, 1) > limit
     a = W.make_gqa_decode(1, shape_id=33, device="cuda", lens=[64])
     st = built_lib.ako4x_gqa_paged_decode_noalloc(
