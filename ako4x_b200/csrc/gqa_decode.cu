@@ -22,8 +22,8 @@
 // bulk copies through shared memory and a planning kernel before -> now): 64 sequences of up to 8 192 tokens
 // 245 -> 188 us (6.3 TB/s = 0.96 of the measured copy bandwidth), 256 of them 841 -> 680 (0.99), 16 of up to
 // 1 200 25 -> 17, one of 547 12.6 -> 10.2 us. Shares also for batches of short sequences, where one CTA pair
-// per sequence needs no merge: equal sequences lose a few us (222 x 64 tokens 13.5 -> 16.0, 888 x 100 67.4 ->
-// 69.6, 3 000 x 30 79 -> 90), but one long sequence among them no longer keeps a single pair busy (eight of
+// per sequence needs no merge: equal sequences lose a few us (222 x 64 tokens 13.5 -> 16.4, 888 x 100 67.4 ->
+// 71.3, 3 000 x 30 79 -> 94), but one long sequence among them no longer keeps a single pair busy (eight of
 // 8 192 tokens among 248 of 256: 580 -> 94; one of 60 000 among 229 of 100: 4 074 -> 78).
 #include <algorithm>
 #include <cfloat>
